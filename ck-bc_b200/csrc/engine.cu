@@ -30,6 +30,7 @@
 #include "bcg_common.hpp"
 #include "engine.cuh"
 #include "engine_internal.hpp"
+#include "wide.cuh"
 
 namespace bcg {
 
@@ -168,6 +169,7 @@ static void graph_free(bcg_graph *g) {
     dev_free(g->d_level_out);
     dev_free(g->d_slot_level);
     dev_free(g->d_ext);
+    wide_free(g);
     dev_free(g->d_rows); dev_free(g->d_ctrl);
     dev_free(g->d_roots); dev_free(g->d_pend); dev_free(g->d_mult); dev_free(g->d_rstat);
     if (g->ev0) cudaEventDestroy(g->ev0);
@@ -331,6 +333,7 @@ struct RunPlan {
     // pruned: sources in components that are trees (no search needed)
     uint64_t tree_only = 0, tree_edges = 0, tree_verts = 0;
     uint64_t launches = 0;  // kernels the planning launched (the source gather)
+    bool plain = false;  // every root has an edge and no pendant sources (plan_run's roots)
 };
 
 // A pruned graph: the closed-form bc of the tree vertices (and the anchors' tree
@@ -394,6 +397,7 @@ static int plan_run(bcg_graph *g, const uint32_t *src, uint64_t nsrc, RunPlan &p
         p.mult[k] += 1.0;
         p.count[k] += 1;
     }
+    p.plain = true;
     return BCG_OK;
 }
 
@@ -433,6 +437,38 @@ struct DebugOut {
     double *delta = nullptr;
 };
 
+// Whether a run of nroots plain sources goes to the wide-batch kernel: a
+// width not forced, counts not extended from the start, and a graph that is
+// not of low degree (grids, meshes, chains: deep, with small frontiers).
+static bool takes_wide(const bcg_graph *g, uint64_t nroots) {
+    const double n = g->tile_n ? g->tile_n : g->n;
+    return !g->forced_width && g->sigma_mode != BCG_SIGMA_EXTENDED && nroots >= 4 && (double)g->nnz_pruned >= 6.0 * n &&
+           n < (double)(1u << 28);
+}
+
+// Totals of the plan's roots (rs in plan order) and the kernels' time.
+static void finish_stats(bcg_graph *g, const RunPlan &p, const std::vector<RootStat> &rs, bcg_stats *stats) {
+    uint64_t teps = 0, vis = 0, cv = 0, se = 0;
+    uint32_t md = 0;
+    for (size_t i = 0; i < p.roots.size(); ++i) {
+        teps += p.count[i] * (rs[i].mc2 / 2);
+        cv += p.count[i] * rs[i].wsum;
+        vis += rs[i].visited;
+        // mc2 = sum of (deg + 2 reach) and wsum = sum of (1 + reach) over
+        // the visited vertices: the searched degrees sum to mc2 - 2 (wsum - visited)
+        se += (rs[i].mc2 - 2 * (rs[i].wsum - rs[i].visited)) / 2;
+        md = std::max(md, rs[i].depth);
+    }
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, g->ev0, g->ev1);
+    stats->teps_edges = teps;
+    stats->visited = vis;
+    stats->comp_vertices = cv;
+    stats->max_depth = md;
+    stats->kernel_ms = ms;
+    stats->search_edges = se;
+}
+
 // rs_out (with stats): every root's own totals, in plan order.
 static int run_plan(bcg_graph *g, const RunPlan &p, cudaStream_t st, bcg_stats *stats, const DebugOut &dbg,
                     std::vector<RootStat> *rs_out = nullptr) {
@@ -444,8 +480,23 @@ static int run_plan(bcg_graph *g, const RunPlan &p, cudaStream_t st, bcg_stats *
         stats->launches = p.launches;
     }
     if (nroots == 0) return BCG_OK;
+    int rc;
+    if (!debug && takes_wide(g, nroots) && (stats || g->sigma_mode == 0) && p.plain) {
+        WideResult res;
+        rc = wide_run(g, p.roots.data(), p.mult.data(), nroots, st, &res);
+        if (rc) return rc;
+        if (res.done) {
+            if (stats) {
+                stats->launches += res.launches;
+                stats->batches = res.batches;
+                stats->batch_width = kWideSlots;
+                finish_stats(g, p, res.rstat, stats);
+            }
+            return BCG_OK;
+        }
+    }
     const uint32_t S = debug ? dbg.width : choose_width(g, nroots);
-    int rc = ensure_state(g, S);
+    rc = ensure_state(g, S);
     if (rc) return rc;
     const uint64_t nbatch = (nroots + S - 1) / S;
     const size_t slots = nbatch * S;
@@ -564,28 +615,10 @@ static int run_plan(bcg_graph *g, const RunPlan &p, cudaStream_t st, bcg_stats *
         std::vector<RootStat> rs(slots);
         CK(cudaMemcpy(rs.data(), g->d_rstat, slots * sizeof(RootStat), cudaMemcpyDeviceToHost));
         if (rs_out) rs_out->assign(rs.begin(), rs.begin() + nroots);
-        uint64_t teps = 0, vis = 0, cv = 0, se = 0;
-        uint32_t md = 0;
-        for (uint64_t i = 0; i < nroots; ++i) {
-            teps += p.count[i] * (rs[i].mc2 / 2);
-            cv += p.count[i] * rs[i].wsum;
-            vis += rs[i].visited;
-            // mc2 = sum of (deg + 2 reach) and wsum = sum of (1 + reach) over
-            // the visited vertices: the searched degrees sum to mc2 - 2 (wsum - visited)
-            se += (rs[i].mc2 - 2 * (rs[i].wsum - rs[i].visited)) / 2;
-            md = std::max(md, rs[i].depth);
-        }
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, g->ev0, g->ev1);
         stats->batches = nbatch;
-        stats->teps_edges = teps;
-        stats->visited = vis;
-        stats->comp_vertices = cv;
-        stats->max_depth = md;
         stats->batch_width = S;
-        stats->kernel_ms = ms;
+        finish_stats(g, p, rs, stats);
         stats->extended_sigma = ext ? 1u : 0u;
-        stats->search_edges = se;
     }
     return BCG_OK;
 }

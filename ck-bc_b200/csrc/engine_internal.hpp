@@ -16,6 +16,8 @@ using bcg::kTileEdges;
 using bcg::kTileVerts;
 
 namespace bcg {
+struct WideGraph;  // wide.cu
+
 // Pendant trees of a graph on the device (BCG_PRUNE_TREES, and one peeling
 // round for BCG_PRUNE_DEGREE1; trees_gpu.cu), caller's numbering.
 struct TreeDev {
@@ -85,6 +87,7 @@ struct bcg_graph {
     double *d_bc_save = nullptr;      // accumulators before an automatic-mode run
     unsigned long long wait_ns = kDefaultWaitNs;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    bcg::WideGraph *wide = nullptr;  // the graph's form for wide-batch runs (wide.cu), built by the first one
 };
 
 namespace bcg {
@@ -110,6 +113,22 @@ inline cudaError_t dev_free(void *p) { return tmp_free(p, 0); }
 
 // ext: sigma and X as extended-range numbers (ext64.cuh) instead of uint64 / double
 int launch_sweep(int S, const BatchArgs &a, cudaStream_t st, int *grid_out, bool ext = false);
+
+// out[i] = in[0] + ... + in[i-1] on stream st (in and out may be the same
+// array; every partial sum fits 32 bits).
+int scan_exclusive(const uint32_t *d_in, uint32_t *d_out, uint64_t len, cudaStream_t st);
+
+// Wide-batch runs (wide.cu).  Adds the dependencies of the given roots
+// (engine ids with an edge, weights mult) into g's bc on stream st and waits.
+// done = false: the graph is too deep for it, a count overflowed or memory ran
+// out; bc is as before and nothing else was changed.
+struct WideResult {
+    bool done = false;
+    uint64_t batches = 0, launches = 0;
+    std::vector<RootStat> rstat;  // per root, in order (padded to whole jobs)
+};
+int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, cudaStream_t st, WideResult *res);
+void wide_free(bcg_graph *g);
 
 // Component-packed batches already on the device (see BatchArgs::xbeg).
 struct PackedRun {

@@ -64,7 +64,7 @@ constexpr uint32_t kKept = 0xFFFFFFFFu;  // rem[v] of a vertex that is not peele
 
 inline unsigned nblocks(uint64_t work, unsigned per) { return (unsigned)std::max<uint64_t>(1, (work + per - 1) / per); }
 
-// ---- exclusive scan of uint32 counts (every partial sum fits 32 bits)
+// ---- exclusive scan of uint32 counts
 constexpr int kScanBlock = 1024;
 
 __global__ void __launch_bounds__(kScanBlock) k_scan_block(const uint32_t *__restrict__ in, uint32_t *__restrict__ out,
@@ -101,7 +101,8 @@ __global__ void k_scan_add(uint32_t *__restrict__ out, const uint32_t *__restric
     if (i < len) out[i] += boff[blockIdx.x];
 }
 
-// out[i] = in[0] + ... + in[i-1] (in and out may be the same array).
+}  // namespace
+
 int scan_exclusive(const uint32_t *d_in, uint32_t *d_out, uint64_t len, cudaStream_t st) {
     if (len == 0) return BCG_OK;
     const uint64_t nb = (len + kScanBlock - 1) / kScanBlock;
@@ -120,6 +121,8 @@ int scan_exclusive(const uint32_t *d_in, uint32_t *d_out, uint64_t len, cudaStre
     tmp_free(bsum, st);
     return rc;
 }
+
+namespace {
 
 // ---- peeling
 __global__ void k_tp_init(uint32_t n, const uint32_t *__restrict__ offs, uint32_t *__restrict__ deg,

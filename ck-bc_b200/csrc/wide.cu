@@ -1,0 +1,1351 @@
+// Wide-batch Brandes searches (sm_100a): 16 sources a job, for graphs whose
+// searches are a few levels deep.
+//
+// What bounds it.  On a small-diameter graph nearly every vertex is in the
+// frontier of some source of a batch at the two or three middle levels, so a
+// level is a sparse-matrix times dense-matrix product: every vertex adds the
+// 16 values of each neighbour.  The rows are gathered from L2, and an SM
+// takes in 64 bytes a clock from there.  So the design is about bytes per
+// (edge, source) and about whole rows per request:
+//   - 16 sources share a row: 64 bytes of 32-bit path counts forward, 128
+//     bytes of doubles backward, no level words in between.  A row holds the
+//     value of the slots that sit exactly at the level being read and 0 in
+//     the others, so a gather needs no test per slot: 4 lanes take a row with
+//     one 16- or 32-byte load each and add.  (Measured on an R-MAT graph of
+//     31 M entries: 141 us and 201 us a pass, 14 and 20 TB/s out of L2, the
+//     whole port; the 64-byte rows of levels and values of sweep.cu carry 6
+//     sources and take about 500 us.)
+//   - a bit per vertex and level says whether any slot sits there, so a
+//     gather skips the rows of other vertices, rows are never cleared, and
+//     backward sweeps visit a level's vertices only.
+//   - path counts are 64-bit; the 32-bit rows are used while every count of
+//     the level is below 2^28 (the sweep that finds them says so), and otherwise the
+//     sweep reads levels and 64-bit counts (kFwdFull), with overflow checked.
+// All forward sweeps pull: no atomics on values, sums in a fixed order.
+//
+// Work split.  Vertices are numbered by descending degree class.  A vertex
+// of up to 32 entries is taken by four lanes (eight vertices of like degree a
+// warp), one of up to 256 by a warp (its edges dealt to the eight groups of
+// four lanes), a heavier one in chunks of 256 entries by one warp each, whose
+// sums meet in a buffer and are added in a fixed order by the chunk that
+// arrives last.  Warps draw items from a counter in shared memory, heaviest
+// first.
+//
+// Teams.  The CTAs of the launch are cut into teams; a team runs one job at
+// a time on state of its own, with a barrier over its own CTAs only, and
+// draws its next job from a counter.  On a small graph a team is one CTA and
+// the barrier is __syncthreads; on a large one the team is the whole grid.
+// Every job writes its dependencies to its own vector, and k_wide_reduce
+// adds the vectors in job order, so the result does not depend on which team
+// ran a job, nor on what else ran.
+//
+// Coherence.  Rows, levels and counts are read with .cg loads.  The bitmaps
+// are read through L1: they are written in one sweep and read in later ones,
+// and the barrier's acquire and fences order the two.
+#include <algorithm>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+
+#include "bcg_common.hpp"
+#include "engine_internal.hpp"
+#include "wide.cuh"
+
+namespace bcg {
+
+namespace {
+
+constexpr uint32_t kFull = 0xffffffffu;
+constexpr uint32_t kNone = 0xffffffffu;
+constexpr uint32_t kUnseen = 0xFFu;  // level byte of a vertex not reached yet
+constexpr uint32_t kEmpty = 0xFEu;   // level byte of a slot without a source
+
+// What a sweep does: forward over 32-bit rows, forward over levels and
+// 64-bit counts, backward, backward at the deepest level (no child exists).
+enum : int { kFwd32 = 0, kFwdFull = 1, kBack = 2, kBackLast = 3 };
+
+struct WideCtx {
+    uint32_t T, rank;  // CTAs of the team, this one's place
+    unsigned char *lvl;
+    uint32_t *done, *act;  // bitmaps: all slots reached; by level: some slot at it
+    size_t words;
+    unsigned long long *sig;
+    unsigned char *g0;  // rows of even levels,
+    ptrdiff_t g01;      // and how far behind them the odd levels' are
+    unsigned long long *part;
+    uint32_t *hcnt;
+    double *bc;
+};
+
+// The rows of level d.
+__device__ __forceinline__ unsigned char *rows_of(const WideCtx &x, uint32_t d) { return x.g0 + ((d & 1u) ? x.g01 : 0); }
+
+struct WideSmem {
+    WideSub sub;
+    WideCtx x;
+    uint32_t roots[kWideSlots];
+    double mult[kWideSlots];
+    uint32_t nmed;      // end of the vertices a warp takes alone (WideSub::nmed by degree bound)
+    uint32_t next;      // items drawn in the current sweep
+    uint32_t found;     // this CTA's part of WideTeam::any
+    uint32_t any;       // the team's, after the barrier
+    unsigned long long count;   // this CTA's part of WideTeam::count
+    uint32_t met[kWideLevels];  // vertices that some slot holds at a level, at most
+    uint32_t left;              // vertices that some slot has not reached
+    int ok;
+    uint32_t edges[kWideSlots + 1];             // entries of the sources before each
+    unsigned long long reach[3 * kWideSlots];   // this CTA's part of the sources' totals
+    unsigned char list[kWideWarps][32];
+};
+
+__device__ __forceinline__ unsigned long long wide_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+__device__ __forceinline__ void ld32(const void *p, uint32_t (&w)[8]) {
+    asm volatile("ld.global.cg.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                 : "l"(p));
+}
+__device__ __forceinline__ void st32(void *p, const uint32_t (&w)[8]) {
+    asm volatile("st.global.v8.u32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};" ::"r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+                 "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "l"(p)
+                 : "memory");
+}
+// A lane's part of row u of doubles (0 where u is kNone).  Not volatile: rows
+// do not change during the sweep that reads them, so the loads may move.
+__device__ __forceinline__ void ld_row(uint32_t u, const unsigned char *rows, double (&r)[4]) {
+    r[0] = r[1] = r[2] = r[3] = 0.0;
+    if (u != kNone)
+        asm("ld.global.cg.v4.f64 {%0,%1,%2,%3}, [%4];"
+            : "=d"(r[0]), "=d"(r[1]), "=d"(r[2]), "=d"(r[3])
+            : "l"(rows + (size_t)u * 128));
+}
+// An adjacency entry: streamed, so evicted before the rows.
+__device__ __forceinline__ uint32_t ld_adj(const uint32_t *p, unsigned long long pol) {
+    uint32_t v;
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
+    return v;
+}
+
+__device__ __forceinline__ bool wide_stopped(const WideCtrl *c) {
+    const volatile int *p = &c->error;
+    return p[0] | p[1] | p[2];
+}
+
+// Barrier of a team: one arrival per CTA on the team's counter.  Returns
+// false when any CTA of the launch recorded an error; a waiting CTA sees that
+// too, so nobody waits for one that has left.
+__device__ bool team_sync(const WideArgs &a, const WideCtx &x, WideTeam *t, WideSmem &sm, unsigned long long wait_ns,
+                          uint32_t slot, uint32_t level = 0) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        bool ok = true;
+        uint32_t any = sm.found;
+        unsigned long long met = sm.count;
+        if (x.T > 1) {
+            if (slot < 4) {
+                if (any) atomicOr(&t->any[slot], any);
+                if (met) atomicAdd(&t->count[slot], met);
+            }
+            __threadfence();
+            const unsigned long long arrived = atomicAdd(&t->arrived, 1ull) + 1ull;
+            const unsigned long long target = (arrived + x.T - 1) / x.T * x.T;
+            if (arrived != target) {
+                const unsigned long long t0 = wide_ns();
+                uint32_t spins = 0;
+                for (;;) {
+                    unsigned long long v;
+                    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(&t->arrived) : "memory");
+                    if (v >= target) break;
+                    if ((++spins & 63u) == 0) {
+                        if (wide_stopped(a.ctrl)) break;
+                        if (wide_ns() - t0 > wait_ns) {
+                            atomicCAS(&a.ctrl->error, 0, BCG_ERR_TIMEOUT);
+                            break;
+                        }
+                    }
+                }
+            }
+            __threadfence();
+            if (slot < 4) {
+                any = *reinterpret_cast<volatile uint32_t *>(&t->any[slot]);
+                met = *reinterpret_cast<volatile unsigned long long *>(&t->count[slot]);
+            }
+            ok = !wide_stopped(a.ctrl);
+        } else {
+            __threadfence();
+            if (slot == 5) ok = !wide_stopped(a.ctrl);  // a team of one looks once a job
+        }
+        sm.next = 0;
+        sm.found = 0;
+        sm.count = 0;
+        sm.any = any;
+        if (slot < 4) {
+            sm.met[level] = (uint32_t)met;
+            sm.left -= (uint32_t)(met >> 32);
+        }
+        sm.ok = ok;
+    }
+    __syncthreads();
+    return sm.ok != 0;
+}
+
+template <int KIND>
+struct AccOf { using T = unsigned long long; };
+template <>
+struct AccOf<kBack> { using T = double; };
+template <>
+struct AccOf<kBackLast> { using T = double; };
+
+template <int KIND, class T>
+__device__ __forceinline__ T wide_add(T x, T y, bool &ovf) {
+    const T s = x + y;
+    if (KIND == kFwdFull) ovf |= s < y;
+    return s;
+}
+
+// The ids of a lane's edges base + step * j, j < 4, below end.
+__device__ __forceinline__ void load_ids(uint32_t (&id)[4], const uint32_t *__restrict__ adj, uint32_t base,
+                                         uint32_t end, uint32_t step, unsigned long long pol) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t e = base + step * j;
+        id[j] = e < end ? ld_adj(adj + e, pol) : kNone;
+    }
+}
+
+// The first J of a lane's four edges: a group of four lanes takes its lanes'
+// edges one after the other, each lane 4 slots of a row, the next rows in
+// flight while the last are added.
+template <int KIND, int J, class T>
+__device__ __forceinline__ void add_rows(const unsigned char *rows, const uint32_t (&id)[4], T (&acc)[4]) {
+    const unsigned sh = threadIdx.x & 28u;
+    if constexpr (KIND == kFwd32) {
+        uint32_t part[4] = {0u, 0u, 0u, 0u};  // at most 16 counts below 2^28
+        uint4 r[2][4];
+        auto fetch = [&](int j, uint4 (&o)[4]) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t u = __shfl_sync(kFull, id[j], sh + q);
+                o[q] = make_uint4(0u, 0u, 0u, 0u);
+                if (u != kNone) o[q] = __ldcg(reinterpret_cast<const uint4 *>(rows + (size_t)u * 64));
+            }
+        };
+        fetch(0, r[0]);
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            if (j + 1 < J) fetch(j + 1, r[(j + 1) & 1]);
+            const uint4 *o = r[j & 1];
+            part[0] += (o[0].x + o[1].x) + (o[2].x + o[3].x);
+            part[1] += (o[0].y + o[1].y) + (o[2].y + o[3].y);
+            part[2] += (o[0].z + o[1].z) + (o[2].z + o[3].z);
+            part[3] += (o[0].w + o[1].w) + (o[2].w + o[3].w);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[k] += (T)part[k];
+    } else if constexpr (KIND == kBack) {
+        double r[2][2][4];
+        auto fetch = [&](int s, double (&o)[2][4]) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) ld_row(__shfl_sync(kFull, id[s >> 1], sh + 2 * (s & 1) + q), rows, o[q]);
+        };
+        fetch(0, r[0]);
+#pragma unroll
+        for (int s = 0; s < 2 * J; ++s) {
+            if (s + 1 < 2 * J) fetch(s + 1, r[(s + 1) & 1]);
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) acc[k] += r[s & 1][q][k];
+        }
+    }
+}
+
+// Adds the rows of a block's neighbours: every lane holds the ids of its own
+// four edges.  Ids that no slot holds at the level are dropped first.
+template <int KIND, class T>
+__device__ __forceinline__ void add_block(const WideCtx &x, uint32_t d, uint32_t (&id)[4], T (&acc)[4], bool &ovf) {
+    const unsigned l = threadIdx.x & 3u, sh = threadIdx.x & 28u;
+    const uint32_t *act = x.act + (size_t)(KIND == kBack ? d + 1 : d) * x.words;
+    uint32_t wd[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) wd[j] = id[j] != kNone ? act[id[j] >> 5] : 0u;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (!((wd[j] >> (id[j] & 31u)) & 1u)) id[j] = kNone;
+    if constexpr (KIND == kFwdFull) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll 1
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t u = __shfl_sync(kFull, id[j], sh + q);
+                if (u == kNone) continue;
+                uint32_t r[8];
+                ld32(x.sig + (size_t)u * kWideSlots + l * 4, r);
+                const uint32_t lv = __ldcg(reinterpret_cast<const uint32_t *>(x.lvl) + (size_t)u * 4 + l);
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (((lv >> (8 * k)) & 0xFFu) == d)
+                        acc[k] = wide_add<KIND>(acc[k], (T)((unsigned long long)r[2 * k + 1] << 32 | r[2 * k]), ovf);
+            }
+    } else {
+        const unsigned char *rows = rows_of(x, KIND == kBack ? d + 1 : d) + l * (KIND == kFwd32 ? 16 : 32);
+        const bool low = id[0] != kNone || id[1] != kNone, high = id[2] != kNone || id[3] != kNone;
+        if (__any_sync(kFull, high)) add_rows<KIND, 4>(rows, id, acc);
+        else if (__any_sync(kFull, low)) add_rows<KIND, 2>(rows, id, acc);
+    }
+}
+
+// The eight groups' sums of a warp's vertex, added in a fixed order and dealt
+// out one slot a lane: lane 4g + l gets slot 4l + k, k = own_slot's low bits
+// (the lanes of groups g and g ^ 1 the same).
+__device__ __forceinline__ uint32_t own_slot() {
+    const unsigned lane = threadIdx.x & 31;
+    return 4u * (lane & 3u) + ((lane >> 3) & 3u);
+}
+template <int KIND, class T>
+__device__ __forceinline__ T wide_fold(const T (&acc)[4], bool &ovf) {
+    const unsigned lane = threadIdx.x & 31;
+    T a0 = (lane & 16u) ? acc[2] : acc[0], a1 = (lane & 16u) ? acc[3] : acc[1];
+    const T b0 = (lane & 16u) ? acc[0] : acc[2], b1 = (lane & 16u) ? acc[1] : acc[3];
+    a0 = wide_add<KIND>(a0, (T)__shfl_xor_sync(kFull, b0, 16), ovf);
+    a1 = wide_add<KIND>(a1, (T)__shfl_xor_sync(kFull, b1, 16), ovf);
+    T c = (lane & 8u) ? a1 : a0;
+    const T e = (lane & 8u) ? a0 : a1;
+    c = wide_add<KIND>(c, (T)__shfl_xor_sync(kFull, e, 8), ovf);
+    return wide_add<KIND>(c, (T)__shfl_xor_sync(kFull, c, 4), ovf);
+}
+
+// Finishing a vertex whose sums lie one slot a lane (wide_fold's order): the
+// whole warp calls, the lanes of even groups store.
+__device__ __forceinline__ uint32_t finish_fwd_warp(const WideCtx &x, uint32_t v, unsigned long long sum, uint32_t d,
+                                                    uint32_t &found) {
+    const unsigned lane = threadIdx.x & 31;
+    const uint32_t k = own_slot();
+    const bool mine = !(lane & 4u);
+    unsigned char *lp = x.lvl + (size_t)v * kWideSlots + k;
+    const uint32_t lv = __ldcg(lp);
+    const bool fresh = lv == kUnseen && sum != 0ull;
+    const bool got = __any_sync(kFull, fresh), left = __any_sync(kFull, lv == kUnseen && !fresh);
+    if (got) {
+        found |= 1u;
+        if (mine) reinterpret_cast<uint32_t *>(rows_of(x, d + 1) + (size_t)v * 64)[k] = fresh ? (uint32_t)sum : 0u;
+        if (mine && fresh) {
+            *lp = (unsigned char)(d + 1);
+            x.sig[(size_t)v * kWideSlots + k] = sum;
+            if (sum >> 28) found |= 2u;
+        }
+    }
+    return (got ? 1u : 0u) | (left ? 0u : 2u);
+}
+
+__device__ __forceinline__ void finish_back_warp(const WideCtx &x, const double *mult, uint32_t v, uint32_t reach,
+                                                 double sum, uint32_t d) {
+    const unsigned lane = threadIdx.x & 31;
+    const uint32_t k = own_slot();
+    const uint32_t lv = __ldcg(x.lvl + (size_t)v * kWideSlots + k);
+    double s = 0.0, xo = 0.0;
+    if (lv == d) {
+        const double sg = (double)__ldcg(x.sig + (size_t)v * kWideSlots + k);
+        const double delta = (double)reach + sg * sum;
+        xo = (1.0 + delta) / sg;
+        s = mult[k] * delta;
+    }
+    if (!(lane & 4u)) reinterpret_cast<double *>(rows_of(x, d) + (size_t)v * 128)[k] = xo;
+#pragma unroll
+    for (int o = 1; o <= 16; o = o == 2 ? 8 : 2 * o) s += __shfl_xor_sync(kFull, s, o);
+    // one add per vertex and sweep, sweeps ordered by the barrier
+    if (lane == 0) atomicAdd(x.bc + v, s);
+}
+
+// Finishes vertex v from its sums (lane l of its group holds slots 4l ..
+// 4l + 3); every lane of the warp calls it, the ones without a vertex with
+// valid = false.  Forward: the slots not reached yet whose sum is not 0 are
+// at level d + 1.  Returns the bits of v's group: 1 some slot was reached, 2 none is left.
+__device__ __forceinline__ uint32_t finish_fwd(const WideCtx &x, uint32_t v, const unsigned long long (&acc)[4],
+                                               bool valid, uint32_t d, uint32_t &found) {
+    const unsigned lane = threadIdx.x & 31, l = lane & 3u;
+    uint32_t *lp = reinterpret_cast<uint32_t *>(x.lvl) + (size_t)v * 4 + l;
+    const uint32_t lv = valid ? __ldcg(lp) : 0u;
+    uint32_t nl = lv, f[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const bool fresh = ((lv >> (8 * k)) & 0xFFu) == kUnseen && acc[k] != 0ull;
+        f[k] = fresh ? (uint32_t)acc[k] : 0u;
+        if (fresh) {
+            nl = (nl & ~(0xFFu << (8 * k))) | ((d + 1) << (8 * k));
+            x.sig[(size_t)v * kWideSlots + 4 * l + k] = acc[k];
+            if (acc[k] >> 28) found |= 2u;
+        }
+    }
+    const unsigned got = __ballot_sync(kFull, nl != lv);
+    const unsigned left = __ballot_sync(kFull, valid && __vcmpeq4(nl, kFull) != 0u);
+    const unsigned sh = lane & ~3u;
+    if ((got >> sh) & 15u) {
+        found |= 1u;
+        *reinterpret_cast<uint4 *>(rows_of(x, d + 1) + (size_t)v * 64 + l * 16) = make_uint4(f[0], f[1], f[2], f[3]);
+        if (nl != lv) *lp = nl;
+    }
+    return (((got >> sh) & 15u) ? 1u : 0u) | (((left >> sh) & 15u) ? 0u : 2u);
+}
+
+// Backward: delta = reach + sigma * sum of X over the children, X = (1 +
+// delta) / sigma for the slots at level d, and the weighted delta into the
+// job's vector.
+__device__ __forceinline__ void finish_back(const WideCtx &x, const WideSmem &sm, uint32_t v, const double (&acc)[4],
+                                            bool valid, uint32_t d) {
+    const unsigned l = threadIdx.x & 3u;
+    double s = 0.0;
+    if (valid) {
+        const uint32_t lv = __ldcg(reinterpret_cast<const uint32_t *>(x.lvl) + (size_t)v * 4 + l);
+        uint32_t w[8];
+        uint32_t r[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) w[k] = 0u;
+        if (__vcmpeq4(lv, d * 0x01010101u)) {
+            const double reach = (double)sm.sub.vinfo[v].y;
+            ld32(x.sig + (size_t)v * kWideSlots + 4 * l, r);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (((lv >> (8 * k)) & 0xFFu) != d) continue;
+                const double sg = (double)((unsigned long long)r[2 * k + 1] << 32 | r[2 * k]);
+                const double delta = reach + sg * acc[k];
+                const double xo = (1.0 + delta) / sg;
+                w[2 * k] = (uint32_t)__double2loint(xo);
+                w[2 * k + 1] = (uint32_t)__double2hiint(xo);
+                s += sm.mult[4 * l + k] * delta;
+            }
+        }
+        st32(rows_of(x, d) + (size_t)v * 128 + l * 32, w);
+    }
+    s += __shfl_xor_sync(kFull, s, 1);
+    s += __shfl_xor_sync(kFull, s, 2);
+    // one add per vertex and sweep, sweeps ordered by the barrier
+    if (valid && l == 0) atomicAdd(x.bc + v, s);
+}
+
+// One sweep over the team's share of the job's vertices.
+// (Not inlined: each kind then has the registers to itself.)
+template <int KIND>
+__device__ __noinline__ void wide_sweep(WideSmem &sm, uint32_t d) {
+    const WideCtx &x = sm.x;
+    using T = typename AccOf<KIND>::T;
+    constexpr bool kForward = KIND == kFwd32 || KIND == kFwdFull;
+    constexpr int side = kForward ? 0 : 1;
+    const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const WideSub &g = sm.sub;
+    const uint32_t *offs = g.offs[side], *adj = g.adj[side];
+    const uint32_t W = x.T * kWideWarps;
+    unsigned long long pol;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+    // items: chunks of the heavy vertices, runs of medium ones, (parts of)
+    // words of light ones; as many a draw as leave every warp about four draws
+    constexpr bool kGather = KIND != kBackLast;  // nothing to gather: every vertex is a light one
+    const uint32_t nchunk = kGather ? g.nchunk[side] : 0u;
+    const uint32_t light0 = kGather ? sm.nmed : 0u;
+    const uint32_t nmedv = kGather ? sm.nmed - g.nheavy : 0u;
+    const uint32_t left = kForward ? sm.left : sm.met[d];  // vertices the sweep does something for, at most
+    const uint32_t thin = left >= g.n ? 1u : min(32u, g.n / max(1u, left));  // 1 in so many
+    // (the few are the heavy ones first, so chunks are not drawn in larger lots)
+    const uint32_t cb = min(4u, max(1u, nchunk / (4u * W)));
+    const uint32_t mb = min(8u, max(1u, nmedv / (4u * W)));
+    const uint32_t nl = g.n - light0;
+    const uint32_t lp = thin > 1u ? 1u : (nl >= 128u * W ? 1u : (nl >= 64u * W ? 2u : 4u));  // parts of a word
+    const uint32_t lw = min(thin, max(1u, nl / (64u * W)));  // or words of a draw
+    const uint32_t nci = (nchunk + cb - 1) / cb, nmi = (nmedv + mb - 1) / mb;
+    const uint32_t w0 = light0 >> 5, nli = nl ? ((((g.n + 31u) >> 5) - w0) * lp + lw - 1u) / lw : 0u;
+    const uint32_t total = nci + nmi + nli;
+    const uint32_t *need_map = kForward ? x.done : x.act + (size_t)d * x.words;
+    uint32_t found = 0, fresh = 0, gone = 0;  // of the lane
+    bool ovf = false;
+    for (;;) {
+        uint32_t c = 0;
+        if (lane == 0) c = atomicAdd(&sm.next, 1u);
+        c = __shfl_sync(kFull, c, 0);
+        if (c >= total) break;  // so that c * T below cannot wrap
+        const uint32_t it = x.rank + c * x.T;
+        if (it >= total) break;
+        if (it < nci + nmi) {
+            // up to 32 segments of a warp each, lane i holding the i-th: chunks
+            // of heavy vertices, or whole medium vertices
+            const bool heavy = it < nci;
+            uint32_t v = 0, e0 = 0, e1 = 0;
+            bool need = false;
+            if (heavy) {
+                const uint32_t i = it * cb + lane;
+                if (lane < cb && i < nchunk) {
+                    const uint2 ch = g.chunk[side][i];
+                    v = ch.x;
+                    e0 = offs[v] + ch.y * g.chunk_len;
+                    e1 = min(offs[v + 1], e0 + g.chunk_len);
+                    need = true;
+                }
+            } else {
+                v = g.nheavy + (it - nci) * mb + lane;
+                if (lane < mb && v < sm.nmed) {
+                    e0 = offs[v];
+                    e1 = offs[v + 1];
+                    need = true;
+                }
+            }
+            if (need) {
+                const uint32_t w = need_map[v >> 5] >> (v & 31u);
+                need = kForward ? !(w & 1u) : (w & 1u) != 0u;
+            }
+            unsigned todo = __ballot_sync(kFull, need);
+            uint32_t nxt[4];
+            uint32_t sb = 0, se = 0;
+            if (todo) {
+                sb = __shfl_sync(kFull, e0, __ffs(todo) - 1);
+                se = __shfl_sync(kFull, e1, __ffs(todo) - 1);
+                load_ids(nxt, adj, sb + lane, se, 32u, pol);
+            }
+#pragma unroll 1
+            while (todo) {
+                const int i = __ffs(todo) - 1;
+                todo &= todo - 1;
+                const uint32_t vi = __shfl_sync(kFull, v, i), end = se;
+                T acc[4] = {0, 0, 0, 0};
+                uint32_t at = sb;
+                bool more;
+#pragma unroll 1
+                do {
+                    // the next block of this segment, or the next segment's
+                    // first, is on its way while this one is added
+                    uint32_t id[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) id[j] = nxt[j];
+                    at += 128u;
+                    more = at < end;
+                    if (more) {
+                        load_ids(nxt, adj, at + lane, end, 32u, pol);
+                    } else if (todo) {
+                        sb = __shfl_sync(kFull, e0, __ffs(todo) - 1);
+                        se = __shfl_sync(kFull, e1, __ffs(todo) - 1);
+                        load_ids(nxt, adj, sb + lane, se, 32u, pol);
+                    }
+                    if constexpr (kGather) add_block<KIND>(x, d, id, acc, ovf);
+                } while (more);
+                T sum = wide_fold<KIND>(acc, ovf);
+                if (heavy) {
+                    const uint32_t ci = it * cb + i;
+                    const uint32_t c0 = g.cbeg[side][vi], nc = g.cbeg[side][vi + 1] - c0;
+                    if (nc > 1) {
+                        // the chunks meet: the one that arrives last adds them,
+                        // half warps the even and the odd ones, in order
+                        const uint32_t k = own_slot();
+                        T *part = reinterpret_cast<T *>(x.part);
+                        if (!(lane & 4u)) __stcg(part + (size_t)ci * kWideSlots + k, sum);
+                        __syncwarp();
+                        uint32_t last = 0;
+                        if (lane == 0) {
+                            __threadfence();
+                            last = atomicAdd(x.hcnt + vi, 1u) == nc - 1u;
+                            if (last) __threadfence();
+                        }
+                        last = __shfl_sync(kFull, last, 0);
+                        if (!last) continue;
+                        if (lane == 0) x.hcnt[vi] = 0u;
+                        sum = 0;
+#pragma unroll 4
+                        for (uint32_t q = (lane >> 2) & 1u; q < nc; q += 2)
+                            sum = wide_add<KIND>(sum, __ldcg(part + (size_t)(c0 + q) * kWideSlots + k), ovf);
+                        sum = wide_add<KIND>(sum, (T)__shfl_xor_sync(kFull, sum, 4), ovf);
+                    }
+                }
+                if constexpr (kForward) {
+                    const uint32_t b = finish_fwd_warp(x, vi, sum, d, found);
+                    if (lane == 0) {
+                        if (b & 1u) {
+                            atomicOr(x.act + (size_t)(d + 1) * x.words + (vi >> 5), 1u << (vi & 31u));
+                            ++fresh;
+                        }
+                        if (b & 2u) {
+                            atomicOr(x.done + (vi >> 5), 1u << (vi & 31u));
+                            ++gone;
+                        }
+                    }
+                } else {
+                    finish_back_warp(x, sm.mult, vi, g.vinfo[vi].y, sum, d);
+                }
+            }
+        } else {
+            // lw words, one a lane, or part of one
+            const uint32_t li = (it - nci - nmi) * lw, wl = w0 + li / lp + lane;
+            uint32_t ml = 0;
+            if (lane < lw && wl << 5 < g.n) {
+                const uint32_t vl = wl << 5;
+                ml = need_map[wl];
+                if (kForward) ml = ~ml;
+                if (lp > 1) ml &= ((1u << (32u / lp)) - 1u) << ((li % lp) * (32u / lp));
+                if (kGather && vl < light0) ml &= kFull << (light0 - vl);
+                if (vl + 32u > g.n) ml &= (1u << (g.n - vl)) - 1u;
+            }
+#pragma unroll 1
+            for (unsigned full = __ballot_sync(kFull, ml != 0u); full; full &= full - 1) {
+            const int wi = __ffs(full) - 1;
+            const uint32_t w = w0 + li / lp + wi, vb = w << 5, m = __shfl_sync(kFull, ml, wi);
+            uint32_t e0 = 0, e1 = 0;
+            if (kGather && vb + lane < g.n) {
+                e0 = offs[vb + lane];
+                e1 = offs[vb + lane + 1];
+            }
+            if ((m >> lane) & 1u) sm.list[wid][__popc(m & ((1u << lane) - 1u))] = (unsigned char)lane;
+            __syncwarp();
+            const uint32_t cnt = __popc(m);
+            // eight vertices at a time, four lanes each
+            auto pick = [&](uint32_t i0, bool &ok, uint32_t &p, uint32_t &b, uint32_t &e) {
+                const uint32_t i = i0 + (lane >> 2);
+                ok = i < cnt;
+                p = ok ? sm.list[wid][i] : 0u;
+                b = __shfl_sync(kFull, e0, p);
+                e = __shfl_sync(kFull, e1, p);
+                if (!ok) e = b;
+            };
+            bool ok;
+            uint32_t p, sb, se, nxt[4];
+            pick(0, ok, p, sb, se);
+            if constexpr (kGather) load_ids(nxt, adj, sb + (lane & 3u), se, 4u, pol);
+#pragma unroll 1
+            for (uint32_t i0 = 0; i0 < cnt; i0 += 8) {
+                const bool valid = ok;
+                const uint32_t v = vb + p;
+                T acc[4] = {0, 0, 0, 0};
+                if constexpr (kGather) {
+                    const uint32_t b = sb, e = se;
+                    const uint32_t nblk = max(1u, __reduce_max_sync(kFull, (e - b + 15u) / 16u));
+#pragma unroll 1
+                    for (uint32_t k = 1; k <= nblk; ++k) {
+                        uint32_t id[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) id[j] = nxt[j];
+                        if (k < nblk) {
+                            load_ids(nxt, adj, b + 16u * k + (lane & 3u), e, 4u, pol);
+                        } else if (i0 + 8 < cnt) {
+                            pick(i0 + 8, ok, p, sb, se);
+                            load_ids(nxt, adj, sb + (lane & 3u), se, 4u, pol);
+                        }
+                        add_block<KIND>(x, d, id, acc, ovf);
+                    }
+                } else {
+                    pick(i0 + 8, ok, p, sb, se);
+                }
+                if constexpr (kForward) {
+                    const uint32_t b = finish_fwd(x, v, acc, valid, d, found);
+                    const uint32_t bit = valid ? 1u << (v & 31u) : 0u;
+                    const uint32_t am = __reduce_or_sync(kFull, (b & 1u) ? bit : 0u);
+                    const uint32_t dm = __reduce_or_sync(kFull, (b & 2u) ? bit : 0u);
+                    if (lane == 0) {
+                        if (am) {
+                            atomicOr(x.act + (size_t)(d + 1) * x.words + w, am);
+                            fresh += __popc(am);
+                        }
+                        if (dm) {
+                            atomicOr(x.done + w, dm);
+                            gone += __popc(dm);
+                        }
+                    }
+                } else {
+                    finish_back(x, sm, v, acc, valid, d);
+                }
+            }
+            __syncwarp();
+            }
+        }
+    }
+    if (KIND == kFwdFull && ovf) found |= 4u;
+    if (kForward) {
+        found = __reduce_or_sync(kFull, found);
+        if (lane == 0 && found) atomicOr(&sm.found, found);
+        if (lane == 0 && (fresh | gone)) atomicAdd(&sm.count, (unsigned long long)gone << 32 | fresh);
+    }
+}
+
+__device__ __forceinline__ void wide_trace(const WideArgs &a, uint32_t job, uint32_t kind, uint32_t level,
+                                           uint32_t info) {
+    if (!a.trace || blockIdx.x != 0 || threadIdx.x != 0) return;
+    const unsigned int i = *a.trace_cnt;
+    if (i >= a.trace_cap) return;
+    a.trace[i] = TraceRec{wide_ns(), job, kind, level, info, 0ull};
+    *a.trace_cnt = i + 1;
+}
+
+__global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
+    __shared__ WideSmem sm;
+    WideCtx &x = sm.x;
+    const uint32_t team = blockIdx.x / a.team_ctas;
+    if (team >= a.teams) return;
+    WideTeam *t = a.team + team;
+    const unsigned long long wait_ns = a.ctrl->wait_ns ? a.ctrl->wait_ns : kDefaultWaitNs;
+    if (threadIdx.x == 0) {
+        unsigned char *st = a.state + (size_t)team * a.stride;
+        x.T = a.team_ctas;
+        x.rank = blockIdx.x % a.team_ctas;
+        x.lvl = st;
+        x.done = reinterpret_cast<uint32_t *>(st + a.o_done);
+        x.act = reinterpret_cast<uint32_t *>(st + a.o_act);
+        x.words = a.words;
+        x.sig = reinterpret_cast<unsigned long long *>(st + a.o_sig);
+        x.g0 = st + a.o_g0;
+        x.g01 = (ptrdiff_t)(a.o_g1 - a.o_g0);
+        x.part = reinterpret_cast<unsigned long long *>(st + a.o_part);
+        x.hcnt = reinterpret_cast<uint32_t *>(st + a.o_hcnt);
+    }
+    __syncthreads();
+    const unsigned lane = threadIdx.x & 31;
+    const uint32_t tid = x.rank * kWideThreads + threadIdx.x, nt = x.T * kWideThreads;
+    if (threadIdx.x == 0) {
+        sm.next = 0;
+        sm.found = 0;
+        sm.count = 0;
+    }
+    uint32_t job = team;
+    for (uint32_t par = 0; job < a.njobs; par ^= 1u) {
+        const WideJob J = a.jobs[job];
+        if (threadIdx.x < sizeof(WideSub) / 4)
+            reinterpret_cast<uint32_t *>(&sm.sub)[threadIdx.x] =
+                reinterpret_cast<const uint32_t *>(a.subs + J.sub)[threadIdx.x];
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            // four lanes take a vertex while its blocks are no more than
+            // about half of a warp's share of a sweep
+            const uint32_t blocks = sm.sub.offs[1][sm.sub.n] / (128u * x.T * kWideWarps);
+            sm.nmed = sm.sub.nmed[blocks >= 32 ? 3 : (blocks >= 16 ? 2 : (blocks >= 8 ? 1 : 0))];
+        }
+        if (threadIdx.x < kWideSlots) {
+            const bool has = threadIdx.x < J.nroots;
+            uint32_t r = kNone;
+            if (has) r = sm.sub.inv[a.roots[J.root0 + threadIdx.x]];
+            sm.roots[threadIdx.x] = r;
+            sm.mult[threadIdx.x] = has ? a.mult[J.root0 + threadIdx.x] : 0.0;
+        }
+        if (threadIdx.x == 0) x.bc = a.jobbc + J.out;
+        __syncthreads();
+        const uint32_t n = sm.sub.n;
+        const uint32_t *offs1 = sm.sub.offs[1], *adj1 = sm.sub.adj[1];
+        if (threadIdx.x == 0) sm.left = n;
+        if (threadIdx.x < 32) {
+            // (16 lists of one graph: the sum may pass 2^32 only on graphs refused on the host)
+            const uint32_t r = lane < kWideSlots ? sm.roots[lane] : kNone;
+            uint32_t s = r != kNone ? offs1[r + 1] - offs1[r] : 0u;
+#pragma unroll
+            for (int o = 1; o < kWideSlots; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFull, s, o);
+                if (lane >= (unsigned)o) s += y;
+            }
+            if (lane < kWideSlots) sm.edges[lane + 1] = s;
+            if (lane == 0) sm.edges[0] = 0;
+        }
+        __syncthreads();
+        // f(k, w) for every neighbour w of the source in slot k
+        auto each_first = [&](auto f) {
+            for (uint32_t i = tid; i < sm.edges[kWideSlots]; i += nt) {
+                int k = 0;
+                while (sm.edges[k + 1] <= i) ++k;
+                f(k, adj1[offs1[sm.roots[k]] + (i - sm.edges[k])]);
+            }
+        };
+        // reset: levels, the bitmaps of levels 0 and 1, the job's vector; the
+        // sources at level 0 with one path
+        if (x.rank == 0 && threadIdx.x == 0) {
+            t->job[par] = a.teams + atomicAdd(&a.ctrl->next_job, 1u);
+            for (int i = 0; i < 4; ++i) {
+                t->any[i] = 0;
+                t->count[i] = 0ull;
+            }
+        }
+        for (uint32_t v = tid; v < n; v += nt) {
+            uint32_t w[4] = {kFull, kFull, kFull, kFull};
+            bool root = false;
+#pragma unroll
+            for (int k = 0; k < kWideSlots; ++k) {
+                const uint32_t r = sm.roots[k];
+                if (r == kNone) w[k >> 2] = (w[k >> 2] & ~(0xFFu << (8 * (k & 3)))) | (kEmpty << (8 * (k & 3)));
+                if (r == v) {
+                    w[k >> 2] &= ~(0xFFu << (8 * (k & 3)));
+                    root = true;
+                }
+            }
+            reinterpret_cast<uint4 *>(x.lvl)[v] = make_uint4(w[0], w[1], w[2], w[3]);
+            x.bc[v] = 0.0;
+            if (root) {
+                uint32_t *row = reinterpret_cast<uint32_t *>(x.g0) + (size_t)v * kWideSlots;
+                for (int k = 0; k < kWideSlots; ++k) {
+                    row[k] = sm.roots[k] == v;
+                    if (sm.roots[k] == v) x.sig[(size_t)v * kWideSlots + k] = 1ull;
+                }
+            }
+        }
+        for (uint32_t w = tid; w < (n + 31u) >> 5; w += nt) {
+            uint32_t m = 0;
+            for (int k = 0; k < kWideSlots; ++k)
+                if (sm.roots[k] >> 5 == w && sm.roots[k] != kNone) m |= 1u << (sm.roots[k] & 31u);
+            x.done[w] = 0;
+            x.act[w] = m;
+            x.act[x.words + w] = 0;
+        }
+        for (uint32_t i = tid; i < sm.sub.nheavy; i += nt) x.hcnt[i] = 0;
+        // the rows of level 1 start from 0
+        each_first([&](int k, uint32_t w) {
+            if (w != sm.roots[k]) x.sig[(size_t)w * kWideSlots + k] = 0ull;
+            uint4 *row = reinterpret_cast<uint4 *>(rows_of(x, 1) + (size_t)w * 64);
+#pragma unroll
+            for (int h = 0; h < 4; ++h) row[h] = make_uint4(0u, 0u, 0u, 0u);
+        });
+        if (!team_sync(a, x, t, sm, wait_ns, 5)) return;
+        wide_trace(a, job, 0, 0, n);
+
+        // ---- forward
+        uint32_t d = 0;
+        bool big = false;  // some count of level d is 2^28 or more
+        for (;; ++d) {
+            if (d + 2 >= kWideLevels) {
+                if (threadIdx.x == 0) a.ctrl->deep = 1;
+                return;
+            }
+            for (uint32_t w = tid; w < (n + 31u) >> 5; w += nt) x.act[(size_t)(d + 2) * x.words + w] = 0;
+            if (x.rank == 0 && threadIdx.x == 0) {
+                t->any[(d + 2) & 3] = 0;
+                t->count[(d + 2) & 3] = 0ull;
+            }
+            if (d == 0) {
+                // level 1: the sources' neighbours, one path for each time
+                // they are listed
+                each_first([&](int k, uint32_t w) {
+                    if (w == sm.roots[k]) return;
+                    x.lvl[(size_t)w * kWideSlots + k] = 1;
+                    atomicAdd(x.sig + (size_t)w * kWideSlots + k, 1ull);
+                    atomicAdd(reinterpret_cast<uint32_t *>(rows_of(x, 1)) + (size_t)w * kWideSlots + k, 1u);
+                    atomicOr(x.act + x.words + (w >> 5), 1u << (w & 31u));
+                });
+                if (threadIdx.x == 0 && sm.edges[kWideSlots]) {
+                    sm.found = 1;
+                    if (x.rank == 0) sm.count = sm.edges[kWideSlots];  // at most
+                }
+            } else if (big) wide_sweep<kFwdFull>(sm, d);
+            else wide_sweep<kFwd32>(sm, d);
+            if (!team_sync(a, x, t, sm, wait_ns, d & 3, d + 1)) return;
+            const uint32_t any = sm.any;
+            wide_trace(a, job, 2, d, any);
+            if (any & 4u) {
+                if (threadIdx.x == 0) a.ctrl->overflow = 1;
+                return;
+            }
+            if (!(any & 1u)) break;
+            big = (any & 2u) != 0;
+        }
+        const uint32_t D = d;
+
+        // ---- what each source reached: a thread's vertices, four slots each
+        if (threadIdx.x < 3 * kWideSlots) sm.reach[threadIdx.x] = 0ull;
+        __syncthreads();
+        {
+            uint32_t vis[4] = {0, 0, 0, 0};
+            unsigned long long ws[4] = {0, 0, 0, 0}, mc[4] = {0, 0, 0, 0};
+            for (uint32_t i = tid; i < n * 4u; i += nt) {  // n * 4 < 2^32 (checked on the host)
+                const uint32_t lv = __ldcg(reinterpret_cast<const uint32_t *>(x.lvl) + i);
+                const uint2 vi = sm.sub.vinfo[i >> 2];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (((lv >> (8 * k)) & 0xFFu) >= kWideLevels) continue;
+                    ++vis[k];
+                    ws[k] += 1ull + vi.y;
+                    mc[k] += (unsigned long long)vi.x + 2ull * vi.y;
+                }
+            }
+            // nt is a multiple of 4, so a thread's words all belong to slots 4 (lane & 3) ..
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                unsigned long long s0 = vis[k], s1 = ws[k], s2 = mc[k];
+#pragma unroll
+                for (int o = 4; o <= 16; o <<= 1) {
+                    s0 += __shfl_xor_sync(kFull, s0, o);
+                    s1 += __shfl_xor_sync(kFull, s1, o);
+                    s2 += __shfl_xor_sync(kFull, s2, o);
+                }
+                if (lane < 4 && s0) {
+                    atomicAdd(&sm.reach[4 * lane + k], s0);
+                    atomicAdd(&sm.reach[kWideSlots + 4 * lane + k], s1);
+                    atomicAdd(&sm.reach[2 * kWideSlots + 4 * lane + k], s2);
+                }
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < kWideSlots && sm.reach[threadIdx.x]) {
+            RootStat *rs = a.rstat + (size_t)job * kWideSlots + threadIdx.x;
+            atomicAdd(&rs->visited, sm.reach[threadIdx.x]);
+            atomicAdd(&rs->wsum, sm.reach[kWideSlots + threadIdx.x]);
+            atomicAdd(&rs->mc2, sm.reach[2 * kWideSlots + threadIdx.x]);
+            rs->depth = D;
+        }
+
+        // ---- backward
+        for (uint32_t e = D; e >= 1; --e) {
+            if (e == D) wide_sweep<kBackLast>(sm, e);
+            else wide_sweep<kBack>(sm, e);
+            if (!team_sync(a, x, t, sm, wait_ns, 4)) return;
+            wide_trace(a, job, 3, e, 0);
+        }
+        if (D == 0 && !team_sync(a, x, t, sm, wait_ns, 4)) return;
+        job = *reinterpret_cast<volatile uint32_t *>(&t->job[par]);
+        __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Adding up the jobs: vertex v of a graph gets its jobs' dependencies, eight
+// interleaved partial sums in job order, then those in order.
+// ---------------------------------------------------------------------------
+
+struct WideOut {
+    unsigned long long out0;  // jobs j < njobs: jobbc[out0 + j * n + v]
+    uint32_t njobs, n;
+    const uint32_t *map;      // v -> index into bc
+    double *bc;
+};
+
+__global__ void __launch_bounds__(256) k_wide_reduce(const WideCtrl *__restrict__ ctrl,
+                                                     const WideOut *__restrict__ outs, WideOut one,
+                                                     const double *__restrict__ jobbc) {
+    __shared__ double part[8][32];
+    if (ctrl->error | ctrl->overflow | ctrl->deep) return;  // nothing of a stopped launch is kept
+    const WideOut o = outs ? outs[blockIdx.y] : one;
+    const unsigned lane = threadIdx.x & 31, p = threadIdx.x >> 5;
+    for (uint32_t v0 = blockIdx.x * 32; v0 < o.n; v0 += gridDim.x * 32) {
+        const uint32_t v = v0 + lane;
+        double s = 0.0;
+        if (v < o.n) {
+            const double *q = jobbc + o.out0 + v;
+#pragma unroll 4
+            for (uint32_t j = p; j < o.njobs; j += 8) s += __ldcs(q + (size_t)j * o.n);
+        }
+        part[p][lane] = s;
+        __syncthreads();
+        if (p == 0 && v < o.n) {
+#pragma unroll
+            for (int k = 1; k < 8; ++k) s += part[k][lane];
+            o.bc[o.map[v]] += s;
+        }
+        __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The numbering by descending degree class, built on the device.
+// ---------------------------------------------------------------------------
+
+constexpr uint32_t kClasses = 112;  // key of degree class c: kClasses - 1 - c
+constexpr uint32_t kSortVerts = 2048;  // vertices of a sorting block
+
+// Degrees up to 32 are classes of their own (a warp takes eight vertices of
+// one class), then eights up to 256, then two classes an octave; 0 is last.
+__device__ __forceinline__ uint32_t degree_key(uint32_t d) {
+    uint32_t c;
+    if (d <= 32u) c = d;
+    else if (d <= 256u) c = 33u + (d - 33u) / 8u;
+    else {
+        const uint32_t lg = 31u - __clz(d);
+        c = 61u + 2u * (lg - 8u) + ((d >> (lg - 1u)) & 1u);
+    }
+    return kClasses - 1u - c;
+}
+constexpr uint32_t kKeyZero = kClasses - 1u;
+
+__device__ __forceinline__ uint32_t sort_degree(const uint32_t *offs, const uint32_t *toffs, uint32_t v) {
+    const uint32_t d = offs[v + 1] - offs[v];
+    return toffs ? max(d, toffs[v + 1] - toffs[v]) : d;
+}
+
+__global__ void __launch_bounds__(256) k_wide_hist(uint32_t n, const uint32_t *__restrict__ offs,
+                                                   const uint32_t *__restrict__ toffs, uint32_t *__restrict__ hist) {
+    __shared__ uint32_t cnt[kClasses];
+    for (uint32_t i = threadIdx.x; i < kClasses; i += 256) cnt[i] = 0;
+    __syncthreads();
+    const uint32_t v0 = blockIdx.x * kSortVerts;
+    for (uint32_t i = threadIdx.x; i < kSortVerts && v0 + i < n; i += 256)
+        atomicAdd(&cnt[degree_key(sort_degree(offs, toffs, v0 + i))], 1u);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < kClasses; i += 256) hist[i * gridDim.x + blockIdx.x] = cnt[i];
+}
+
+// hist: exclusive prefix sums.  Stable: vertices of a class keep their order.
+// meta: {vertices with an entry, nheavy, the four nmed}.
+__global__ void __launch_bounds__(256) k_wide_number(uint32_t n, const uint32_t *__restrict__ offs,
+                                                     const uint32_t *__restrict__ toffs,
+                                                     const uint32_t *__restrict__ hist, uint32_t *__restrict__ perm,
+                                                     uint32_t *__restrict__ inv, uint32_t chunk,
+                                                     uint32_t *__restrict__ meta) {
+    __shared__ uint32_t base[kClasses], cnt[8][kClasses];
+    const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (uint32_t i = threadIdx.x; i < kClasses; i += 256) base[i] = hist[i * gridDim.x + blockIdx.x];
+    for (uint32_t i = threadIdx.x; i < 8 * kClasses; i += 256) (&cnt[0][0])[i] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        meta[0] = hist[kKeyZero * gridDim.x];
+        meta[1] = hist[(degree_key(chunk + 1u) + 1u) * gridDim.x];  // the classes from chunk's octave on
+        for (uint32_t b = 0; b < 4; ++b)  // more than 32, 64, 128, 256 entries
+            meta[2 + b] = max(meta[1], hist[(degree_key(kWideLight << b)) * gridDim.x]);
+    }
+    __syncthreads();
+    const uint32_t b0 = blockIdx.x * kSortVerts;
+    for (uint32_t i0 = 0; i0 < kSortVerts; i0 += 256) {
+        const uint32_t v = b0 + i0 + threadIdx.x;
+        const bool ok = v < n && i0 + threadIdx.x < kSortVerts;
+        const uint32_t key = ok ? degree_key(sort_degree(offs, toffs, v)) : kClasses;
+        const unsigned peers = __match_any_sync(kFull, key);
+        const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
+        if (ok && rank == 0) cnt[wid][key] = __popc(peers);
+        __syncthreads();
+        if (ok) {
+            uint32_t pos = base[key] + rank;
+            for (unsigned w = 0; w < wid; ++w) pos += cnt[w][key];
+            perm[pos] = v;
+            inv[v] = pos;
+        }
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < kClasses; i += 256) {
+            uint32_t s = 0;
+            for (unsigned w = 0; w < 8; ++w) {
+                s += cnt[w][i];
+                cnt[w][i] = 0;
+            }
+            base[i] += s;
+        }
+        __syncthreads();
+    }
+}
+
+// Row lengths in the new numbering (len[n] = 0 for the scan), the degree and
+// reach words, and where a vertex's bc goes.
+__global__ void k_wide_len(uint32_t n, const uint32_t *__restrict__ perm, const uint32_t *__restrict__ offs,
+                           const uint32_t *__restrict__ toffs, const uint2 *__restrict__ vinfo,
+                           const uint32_t *__restrict__ ext, uint32_t *__restrict__ len, uint32_t *__restrict__ tlen,
+                           uint2 *__restrict__ vi2, uint32_t *__restrict__ map) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > n) return;
+    if (i == n) {
+        len[n] = 0;
+        if (toffs) tlen[n] = 0;
+        return;
+    }
+    const uint32_t v = perm[i];
+    len[i] = offs[v + 1] - offs[v];
+    if (toffs) tlen[i] = toffs[v + 1] - toffs[v];
+    vi2[i] = vinfo[v];
+    map[i] = ext ? ext[v] : v;
+}
+
+// The lists in the new numbering, one warp a vertex, order kept.
+__global__ void k_wide_fill(uint32_t n, const uint32_t *__restrict__ perm, const uint32_t *__restrict__ inv,
+                            const uint32_t *__restrict__ offs, const uint32_t *__restrict__ adj,
+                            const uint32_t *__restrict__ offs2, uint32_t *__restrict__ adj2) {
+    const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const unsigned lane = threadIdx.x & 31;
+    if (w >= n) return;
+    const uint32_t v = perm[w], e0 = offs[v], len = offs[v + 1] - e0, o = offs2[w];
+    for (uint32_t i = lane; i < len; i += 32) adj2[o + i] = inv[adj[e0 + i]];
+}
+
+// Chunks of the heavy vertices (at least one each): counts, then the table.
+// cap: entries of cnt (an upper bound of nheavy); cnt[cap] closes the scan.
+__global__ void k_wide_chunks(uint32_t cap, const uint32_t *__restrict__ meta, const uint32_t *__restrict__ offs2,
+                              uint32_t chunk, uint32_t *__restrict__ cnt) {
+    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v > cap) return;
+    cnt[v] = v < meta[1] ? max(1u, (offs2[v + 1] - offs2[v] + chunk - 1u) / chunk) : 0u;
+}
+
+__global__ void k_wide_table(uint32_t cap, uint32_t *__restrict__ meta, int side, const uint32_t *__restrict__ cbeg,
+                             uint2 *__restrict__ chunk) {
+    const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const unsigned lane = threadIdx.x & 31;
+    if (w == 0 && lane == 0) meta[6 + side] = cbeg[cap];
+    if (w >= meta[1]) return;
+    const uint32_t c0 = cbeg[w], c1 = cbeg[w + 1];
+    for (uint32_t c = c0 + lane; c < c1; c += 32) chunk[c] = make_uint2((uint32_t)w, c - c0);
+}
+
+// Transposed lists of a directed graph (the order within a list is free: path
+// counts are integers).
+__global__ void k_wide_indeg(uint64_t nnz, const uint32_t *__restrict__ adj, uint32_t *__restrict__ deg) {
+    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += (uint64_t)gridDim.x * blockDim.x)
+        atomicAdd(deg + adj[e], 1u);
+}
+__global__ void k_wide_transpose(uint32_t n, const uint32_t *__restrict__ offs, const uint32_t *__restrict__ adj,
+                                 uint32_t *__restrict__ cursor, uint32_t *__restrict__ tadj) {
+    const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const unsigned lane = threadIdx.x & 31;
+    if (w >= n) return;
+    for (uint32_t e = offs[w] + lane; e < offs[w + 1]; e += 32) tadj[atomicAdd(cursor + adj[e], 1u)] = (uint32_t)w;
+}
+
+#define CKW(call)                                                                                      do {                                                                                                   cudaError_t e_ = (call);                                                                           if (e_ != cudaSuccess)                                                                                 return set_error(e_ == cudaErrorMemoryAllocation ? BCG_ERR_OOM : BCG_ERR_CUDA, "%s failed: %s",                              #call, cudaGetErrorString(e_));                                           } while (0)
+
+inline unsigned wblocks(uint64_t work, unsigned per) { return (unsigned)std::max<uint64_t>(1, (work + per - 1) / per); }
+
+size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
+
+}  // namespace
+
+// A graph's wide form (bcg_graph::wide): its lists in the wide numbering and
+// the buffers of its runs.
+struct WideGraph {
+    WideSub sub{};
+    uint32_t *perm = nullptr, *inv = nullptr, *map = nullptr, *offs[2] = {nullptr, nullptr},
+             *adj[2] = {nullptr, nullptr}, *cbeg[2] = {nullptr, nullptr};
+    uint2 *vinfo = nullptr, *chunk[2] = {nullptr, nullptr};
+    // run buffers
+    unsigned char *state = nullptr, *blob = nullptr, *stat = nullptr;
+    double *jobbc = nullptr;
+    size_t state_cap = 0, blob_cap = 0, stat_cap = 0, jobbc_cap = 0;
+};
+
+void wide_free(bcg_graph *g) {
+    WideGraph *w = g->wide;
+    if (!w) return;
+    dev_free(w->perm); dev_free(w->inv); dev_free(w->map); dev_free(w->vinfo);
+    for (int s = 0; s < 2; ++s) {
+        if (s && w->offs[1] == w->offs[0]) break;
+        dev_free(w->offs[s]); dev_free(w->adj[s]); dev_free(w->cbeg[s]); dev_free(w->chunk[s]);
+    }
+    dev_free(w->state); dev_free(w->blob); dev_free(w->stat); dev_free(w->jobbc);
+    delete w;
+    g->wide = nullptr;
+}
+
+// Builds g's wide form on stream 0 (the caller's later work on any stream
+// follows: the call ends with a device synchronisation).
+static int wide_build(bcg_graph *g) {
+    WideGraph *w = g->wide = new WideGraph();
+    const uint32_t n = g->tile_n ? g->tile_n : g->n;
+    const uint64_t nnz = g->nnz_pruned;
+    const bool dir = (g->flags & BCG_DIRECTED) != 0;
+    cudaStream_t st = 0;
+    uint32_t *toffs = nullptr, *tadj = nullptr, *tmp = nullptr, *hist = nullptr, *meta = nullptr;
+    auto cleanup = [&]() {
+        tmp_free(toffs, st); tmp_free(tadj, st); tmp_free(tmp, st); tmp_free(hist, st); tmp_free(meta, st);
+    };
+    struct Guard { decltype(cleanup) &f; ~Guard() { f(); } } guard{cleanup};
+    int rc;
+    CKW(tmp_alloc(&meta, 8 * sizeof(uint32_t), st));
+    CKW(tmp_alloc(&tmp, 2 * ((size_t)n + 1) * sizeof(uint32_t), st));
+    if (dir) {
+        CKW(tmp_alloc(&toffs, ((size_t)n + 1) * sizeof(uint32_t), st));
+        CKW(tmp_alloc(&tadj, std::max<uint64_t>(1, nnz) * sizeof(uint32_t), st));
+        CKW(cudaMemsetAsync(tmp, 0, ((size_t)n + 1) * sizeof(uint32_t), st));
+        k_wide_indeg<<<148 * 8, 256, 0, st>>>(nnz, g->d_adj, tmp);
+        if ((rc = scan_exclusive(tmp, toffs, (uint64_t)n + 1, st))) return rc;
+        CKW(cudaMemcpyAsync(tmp, toffs, (size_t)n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
+        k_wide_transpose<<<wblocks((uint64_t)n * 32, 256), 256, 0, st>>>(n, g->d_offs, g->d_adj, tmp, tadj);
+        CKW(cudaGetLastError());
+    }
+    // entries of a warp's share of a heavy vertex: longer ones meet less
+    // often, shorter ones leave more warps something to do
+    uint32_t chunk = kWideChunk;
+    while (chunk < 8 * kWideChunk && nnz / (148ull * kWideWarps * 8) >= chunk) chunk *= 2;
+    const uint32_t nb = wblocks(n, kSortVerts);
+    CKW(tmp_alloc(&hist, (size_t)kClasses * nb * sizeof(uint32_t), st));
+    CKW(dev_alloc(&w->perm, (size_t)n * sizeof(uint32_t)));
+    CKW(dev_alloc(&w->inv, (size_t)n * sizeof(uint32_t)));
+    CKW(dev_alloc(&w->map, (size_t)n * sizeof(uint32_t)));
+    CKW(dev_alloc(&w->vinfo, (size_t)n * sizeof(uint2)));
+    k_wide_hist<<<nb, 256, 0, st>>>(n, g->d_offs, toffs, hist);
+    if ((rc = scan_exclusive(hist, hist, (uint64_t)kClasses * nb, st))) return rc;
+    k_wide_number<<<nb, 256, 0, st>>>(n, g->d_offs, toffs, hist, w->perm, w->inv, chunk, meta);
+    k_wide_len<<<wblocks((uint64_t)n + 1, 256), 256, 0, st>>>(n, w->perm, g->d_offs, toffs, g->d_vinfo, g->d_ext, tmp,
+                                                              tmp + n + 1, w->vinfo, w->map);
+    CKW(cudaGetLastError());
+    // a heavy vertex has at least chunk entries in one direction
+    const uint32_t cap = (uint32_t)std::min<uint64_t>(n, (dir ? 2 : 1) * (nnz / chunk) + 1);
+    const size_t maxchunk = nnz / chunk + cap + 1;
+    for (int s = 0; s < (dir ? 2 : 1); ++s) {
+        // side 0: who leads to v (the transposed lists of a directed graph), side 1: where v leads
+        const uint32_t *o = (dir && s == 0) ? toffs : g->d_offs, *a = (dir && s == 0) ? tadj : g->d_adj;
+        const uint32_t *len = (dir && s == 0) ? tmp + n + 1 : tmp;
+        CKW(dev_alloc(&w->offs[s], ((size_t)n + 1) * sizeof(uint32_t)));
+        CKW(dev_alloc(&w->adj[s], std::max<uint64_t>(1, nnz) * sizeof(uint32_t)));
+        CKW(dev_alloc(&w->cbeg[s], ((size_t)cap + 1) * sizeof(uint32_t)));
+        CKW(dev_alloc(&w->chunk[s], maxchunk * sizeof(uint2)));
+        if ((rc = scan_exclusive(len, w->offs[s], (uint64_t)n + 1, st))) return rc;
+        k_wide_fill<<<wblocks((uint64_t)n * 32, 256), 256, 0, st>>>(n, w->perm, w->inv, o, a, w->offs[s], w->adj[s]);
+        k_wide_chunks<<<wblocks((uint64_t)cap + 1, 256), 256, 0, st>>>(cap, meta, w->offs[s], chunk, w->cbeg[s]);
+        if ((rc = scan_exclusive(w->cbeg[s], w->cbeg[s], (uint64_t)cap + 1, st))) return rc;
+        k_wide_table<<<wblocks((uint64_t)cap * 32, 256), 256, 0, st>>>(cap, meta, s, w->cbeg[s], w->chunk[s]);
+        CKW(cudaGetLastError());
+    }
+    uint32_t h[8] = {};
+    CKW(cudaMemcpy(h, meta, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost));
+    CKW(cudaDeviceSynchronize());
+    if (!dir) {
+        h[7] = h[6];
+        w->offs[1] = w->offs[0]; w->adj[1] = w->adj[0]; w->cbeg[1] = w->cbeg[0]; w->chunk[1] = w->chunk[0];
+    }
+    WideSub &b = w->sub;
+    b.n = h[0];
+    b.nheavy = h[1];
+    for (int i = 0; i < 4; ++i) b.nmed[i] = h[2 + i];
+    b.chunk_len = chunk;
+    for (int s = 0; s < 2; ++s) {
+        b.nchunk[s] = h[6 + s];
+        b.offs[s] = w->offs[s];
+        b.adj[s] = w->adj[s];
+        b.chunk[s] = w->chunk[s];
+        b.cbeg[s] = w->cbeg[s];
+    }
+    b.vinfo = w->vinfo;
+    b.inv = w->inv;
+    return BCG_OK;
+}
+
+// Grows *p to bytes (the old buffer may be in use on any stream).
+static int grow(unsigned char **p, size_t *cap, size_t bytes) {
+    if (*cap >= bytes) return BCG_OK;
+    CKW(cudaDeviceSynchronize());
+    dev_free(*p);
+    *p = nullptr;
+    *cap = 0;
+    CKW(dev_alloc(p, bytes));
+    CKW(cudaDeviceSynchronize());
+    *cap = bytes;
+    return BCG_OK;
+}
+
+int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, cudaStream_t st, WideResult *res) {
+    res->done = false;
+    int rc;
+    if (!g->wide && (rc = wide_build(g))) {
+        wide_free(g);
+        return rc == BCG_ERR_OOM ? BCG_OK : rc;
+    }
+    WideGraph *w = g->wide;
+    const WideSub &b = w->sub;
+    const uint64_t njobs = (nroots + kWideSlots - 1) / kWideSlots;
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    // state of a team
+    const size_t n = b.n, words = (n + 31) / 32, nch = std::max(b.nchunk[0], b.nchunk[1]);
+    WideArgs a{};
+    size_t o = up256(n * 16);
+    a.o_done = o; o += up256(words * 4);
+    a.o_act = o; o += up256(words * 4 * kWideLevels);
+    a.o_sig = o; o += up256(n * 128);
+    a.o_g0 = o; o += up256(n * 128);
+    a.o_g1 = o; o += up256(n * 128);
+    a.o_part = o; o += up256(std::max<size_t>(1, nch) * 128);
+    a.o_hcnt = o; o += up256(std::max<size_t>(1, b.nheavy) * 4);
+    a.stride = o;
+    a.words = words;
+    // teams
+    uint64_t teams = std::min<uint64_t>(njobs, (uint64_t)nsm);
+    double budget = 128.0 * 1024 * 1024;
+    if (const char *e = getenv("BCG_WIDE_TEAM_MB")) budget = atof(e) * 1024 * 1024;
+    teams = std::max<uint64_t>(1, std::min<uint64_t>(teams, (uint64_t)(budget / (double)a.stride)));
+    a.teams = (uint32_t)teams;
+    a.team_ctas = (uint32_t)(nsm / teams);
+    // jobs of one launch: their vectors stay under 512 MB
+    const uint64_t per = std::max<uint64_t>(teams, (512ull << 20) / (n * 8 + 1));
+    const uint64_t jl = std::min(per, njobs);
+    if ((rc = grow(&w->state, &w->state_cap, a.stride * teams)) ||
+        (rc = grow(reinterpret_cast<unsigned char **>(&w->jobbc), &w->jobbc_cap, jl * n * 8)))
+        return rc == BCG_ERR_OOM ? BCG_OK : rc;
+    // one upload: the sub, the jobs, the sources
+    const size_t o_jobs = up256(sizeof(WideSub)), o_mult = o_jobs + up256(njobs * sizeof(WideJob)),
+                 o_roots = o_mult + up256(nroots * 8), blob = o_roots + up256(nroots * 4);
+    std::vector<unsigned char> h(blob);
+    memcpy(h.data(), &b, sizeof(b));
+    WideJob *hj = reinterpret_cast<WideJob *>(h.data() + o_jobs);
+    for (uint64_t j = 0; j < njobs; ++j) {
+        hj[j] = WideJob{};
+        hj[j].root0 = (uint32_t)(j * kWideSlots);
+        hj[j].nroots = (uint32_t)std::min<uint64_t>(kWideSlots, nroots - j * kWideSlots);
+        hj[j].out = (j % jl) * n;
+    }
+    memcpy(h.data() + o_mult, mult, nroots * 8);
+    memcpy(h.data() + o_roots, roots, nroots * 4);
+    // control words, teams, per-source totals: one block, cleared together
+    const size_t o_team = sizeof(WideCtrl), o_rstat = o_team + teams * sizeof(WideTeam),
+                 stat = o_rstat + njobs * kWideSlots * sizeof(RootStat);
+    if ((rc = grow(&w->blob, &w->blob_cap, blob)) || (rc = grow(&w->stat, &w->stat_cap, stat)))
+        return rc == BCG_ERR_OOM ? BCG_OK : rc;
+    CKW(cudaMemcpyAsync(w->blob, h.data(), blob, cudaMemcpyHostToDevice, st));
+    a.subs = reinterpret_cast<const WideSub *>(w->blob);
+    a.mult = reinterpret_cast<const double *>(w->blob + o_mult);
+    a.roots = reinterpret_cast<const uint32_t *>(w->blob + o_roots);
+    a.jobbc = w->jobbc;
+    a.state = w->state;
+    a.ctrl = reinterpret_cast<WideCtrl *>(w->stat);
+    a.team = reinterpret_cast<WideTeam *>(w->stat + o_team);
+    TraceRec *d_trace = nullptr;
+    unsigned int *d_tcnt = nullptr;
+    const char *trace_path = getenv("BCG_TRACE_FILE");
+    if (trace_path && *trace_path) {
+        a.trace_cap = 1u << 20;
+        CKW(dev_alloc(&d_trace, a.trace_cap * sizeof(TraceRec)));
+        CKW(dev_alloc(&d_tcnt, sizeof(unsigned int)));
+        CKW(cudaMemsetAsync(d_tcnt, 0, sizeof(unsigned int), st));
+        a.trace = d_trace;
+        a.trace_cnt = d_tcnt;
+    }
+    std::vector<unsigned char> hs(stat);
+    CKW(cudaMemsetAsync(w->stat, 0, stat, st));
+    CKW(cudaEventRecord(g->ev0, st));
+    // The jobs are added into bc on the device only if none of them stopped.
+    // Several launches add one after the other, so bc is saved before them.
+    const bool several = jl < njobs;
+    if (several) {
+        if (!g->d_bc_save) CKW(dev_alloc(&g->d_bc_save, (size_t)g->n * sizeof(double)));
+        CKW(cudaMemcpyAsync(g->d_bc_save, g->d_bc, (size_t)g->n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    }
+    const WideCtrl *c = reinterpret_cast<const WideCtrl *>(hs.data());
+    for (uint64_t j0 = 0; j0 < njobs; j0 += jl) {
+        a.njobs = (uint32_t)std::min(jl, njobs - j0);
+        a.jobs = reinterpret_cast<const WideJob *>(w->blob + o_jobs) + j0;
+        a.rstat = reinterpret_cast<RootStat *>(w->stat + o_rstat) + j0 * kWideSlots;
+        if (j0) CKW(cudaMemsetAsync(w->stat, 0, o_rstat, st));
+        void *params[] = {&a};
+        CKW(cudaLaunchCooperativeKernel((const void *)bc_wide_kernel, dim3(a.teams * a.team_ctas), dim3(kWideThreads),
+                                        params, 0, st));
+        WideOut out{0, a.njobs, (uint32_t)n, w->map, g->d_bc};
+        k_wide_reduce<<<wblocks(n, 32), 256, 0, st>>>(a.ctrl, nullptr, out, w->jobbc);
+        CKW(cudaGetLastError());
+        res->launches += 2;
+        const bool last = j0 + a.njobs >= njobs;
+        if (last) CKW(cudaEventRecord(g->ev1, st));
+        CKW(cudaMemcpyAsync(hs.data(), w->stat, last ? stat : sizeof(WideCtrl), cudaMemcpyDeviceToHost, st));
+        CKW(cudaStreamSynchronize(st));
+        if (c->error || c->overflow || c->deep) break;
+    }
+    if (d_trace) {
+        unsigned int cnt = 0;
+        CKW(cudaStreamSynchronize(st));
+        CKW(cudaMemcpy(&cnt, d_tcnt, sizeof(cnt), cudaMemcpyDeviceToHost));
+        std::vector<TraceRec> recs(cnt);
+        if (cnt) CKW(cudaMemcpy(recs.data(), d_trace, cnt * sizeof(TraceRec), cudaMemcpyDeviceToHost));
+        if (FILE *f = fopen(trace_path, "a")) {
+            fprintf(f, "# wide roots %zu vertices %zu teams %u x %u\n", (size_t)nroots, n, a.teams, a.team_ctas);
+            for (const TraceRec &r : recs)
+                fprintf(f, "%u,%u,%u,%u,%llu,%llu\n", r.batch, r.kind, r.level, r.nwork, r.disc, r.t_ns);
+            fclose(f);
+        }
+        dev_free(d_trace);
+        dev_free(d_tcnt);
+    }
+    if (c->error) return set_error(c->error, "device reported error %d (a bounded wait gave up)", c->error);
+    if (c->overflow || c->deep) {
+        // an overflowing count or a deep search: the caller runs the sweep kernel
+        if (several)
+            CKW(cudaMemcpyAsync(g->d_bc, g->d_bc_save, (size_t)g->n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+        res->launches = 0;
+        return BCG_OK;
+    }
+    res->rstat.resize(njobs * kWideSlots);
+    memcpy(res->rstat.data(), hs.data() + o_rstat, res->rstat.size() * sizeof(RootStat));
+    res->batches = njobs;
+    res->done = true;
+    return BCG_OK;
+}
+
+}  // namespace bcg

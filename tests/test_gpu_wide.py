@@ -1,0 +1,123 @@
+"""The wide-batch searches (16 sources a job, teams of CTAs) against the oracle.
+
+Plain runs of four roots or more go there on graphs of mean degree 6 and up.
+The cases sit at the edges of its work split: vertices of 31 to 33, 64, 256
+and several thousand entries (four lanes, a warp, chunks), vertex counts
+around 32-vertex words, one to 17 and 33 roots, several components, every
+pruning mode, directed lists, counts of 2^28 and more (the 32-bit rows do not
+hold them), counts past 2^64 and searches of more than 62 levels (both leave
+the kernel: the run is redone).  The bar is the suite's 1e-9; path counts are
+exact, so only the order of FP64 sums differs."""
+import numpy as np
+import pytest
+
+import bcg
+import oracle
+from test_gpu_parity import assert_bc_close
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows(n, degrees, seed):
+    """Vertices 0, 1, ... with the given numbers of random neighbours, among n."""
+    rng = np.random.default_rng(seed)
+    pairs = [np.stack([np.full(d, v), rng.choice(n, size=d, replace=False)], 1) for v, d in enumerate(degrees)]
+    fill = rng.integers(0, n, (4 * n, 2))
+    return bcg.from_pairs(np.concatenate(pairs + [fill]), n)
+
+
+GRAPHS = {
+    "degrees": lambda: _rows(5000, [4000, 3000, 1025, 1024, 513, 512, 300, 257, 256, 255, 129, 128, 65, 64, 63, 33, 32, 31, 1], 3),
+    "word31": lambda: bcg.generate("er:scale=5,ef=6,seed=8"),
+    "word33": lambda: _rows(33, [30, 20], 4),
+    "rmat13": lambda: bcg.generate("rmat:scale=13,ef=16,a=0.57,b=0.19,c=0.19,seed=3"),
+    "pendants": lambda: bcg.generate("rmat:scale=11,ef=16,seed=9,pendant_frac=0.1,pendant_mean=4"),
+    "er15": lambda: bcg.generate("er:scale=15,ef=12,seed=6"),
+}
+
+
+@pytest.fixture(scope="module")
+def graphs():
+    return {k: f() for k, f in GRAPHS.items()}
+
+
+@pytest.mark.parametrize("flags", [0, bcg.PRUNE_DEGREE1, bcg.PRUNE_TREES])
+@pytest.mark.parametrize("gname", list(GRAPHS))
+def test_matches_oracle(graphs, gname, flags):
+    offs, adj = graphs[gname]
+    n = len(offs) - 1
+    live = np.nonzero(np.diff(offs))[0].astype(np.uint32)
+    for k in (4, 16, 17, 33):
+        src = live[np.linspace(0, len(live) - 1, min(k, len(live))).astype(int)]
+        ref, ost = oracle.bc(offs, adj, src, nthreads=oracle.max_threads())
+        with bcg.Graph(offs, adj, flags) as G:
+            st = G.run(src)
+            got = G.bc()
+            G.run(src)
+            twice = G.bc()
+        assert flags or st.batch_width == 16
+        assert_bc_close(got, ref, f"{gname} k={k} flags={flags}")
+        assert_bc_close(twice, 2 * ref, f"{gname} k={k} flags={flags} accumulated")
+        assert st.teps_edges == ost["teps_edges"] and st.skipped == ost["skipped"]
+        assert flags or (st.max_depth == ost["max_depth"] and st.visited == ost["visited"])
+
+
+def test_all_sources_many_teams(graphs):
+    """More jobs than CTAs: a team is one CTA and draws job after job."""
+    offs, adj = graphs["rmat13"]
+    src = np.arange(len(offs) - 1, dtype=np.uint32)
+    ref, _ = oracle.bc(offs, adj, src, nthreads=oracle.max_threads())
+    with bcg.Graph(offs, adj) as G:
+        G.run(src)
+        first = G.bc()
+        G.reset()
+        G.run(src)
+        assert np.array_equal(first.view(np.uint64), G.bc().view(np.uint64))
+    assert_bc_close(first, ref, "rmat13 all sources")
+
+
+def test_directed():
+    rng = np.random.default_rng(12)
+    n = 3000
+    hub = np.stack([np.zeros(2000, int), rng.choice(np.arange(1, n), 2000, replace=False)], 1)
+    into = np.stack([rng.choice(np.arange(2, n), 700, replace=False), np.ones(700, int)], 1)
+    offs, adj = bcg.from_pairs(np.concatenate([rng.integers(0, n, (40000, 2)), hub, into]), n, undirected=False)
+    src = bcg.sample_sources(n, 100, 1)
+    ref, ost = oracle.bc(offs, adj, src)
+    with bcg.Graph(offs, adj, bcg.DIRECTED) as G:
+        st = G.run(src)
+        assert st.batch_width == 16
+        assert_bc_close(G.bc(), ref, "directed")
+
+
+def _layers(width, depth):
+    """Complete bipartite layers: width^i paths to layer i + 1."""
+    ids = np.arange(width * depth).reshape(depth, width)
+    pairs = [np.stack(np.meshgrid(ids[i], ids[i + 1]), -1).reshape(-1, 2) for i in range(depth - 1)]
+    return bcg.from_pairs(np.concatenate(pairs), width * depth)
+
+
+@pytest.mark.parametrize("depth,ext", [(9, 0), (12, 0), (15, 0), (30, 1)])
+def test_large_counts(depth, ext):
+    """16 paths more a layer: 2^28 is passed from depth 9 on, 2^64 at 18."""
+    offs, adj = _layers(16, depth)
+    src = np.arange(0, 16 * depth, 3, dtype=np.uint32)
+    ref, _ = oracle.bc_q(offs, adj, src)
+    with bcg.Graph(offs, adj) as G:
+        st = G.run(src)
+        assert st.extended_sigma == ext and (ext or st.batch_width == 16)
+        assert_bc_close(G.bc(), ref, f"layers {depth}")
+
+
+def test_deep_search_leaves():
+    """Mean degree above 6, 120 levels: the run is redone by the sweep kernel,
+    and what was in bc before stays."""
+    offs, adj = _layers(4, 120)
+    src = np.arange(0, 480, 30, dtype=np.uint32)
+    ref, _ = oracle.bc_q(offs, adj, src)
+    with bcg.Graph(offs, adj) as G:
+        st = G.run(src)
+        assert st.max_depth > 62 and st.batch_width != 16
+        assert_bc_close(G.bc(), ref, "deep")
+        G.run(src)
+        assert_bc_close(G.bc(), 2 * ref, "deep twice")

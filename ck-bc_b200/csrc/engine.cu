@@ -62,11 +62,12 @@ __global__ void k_vinfo_plain(uint32_t n, const uint32_t *__restrict__ offs, uin
 // staging limits).
 // Only vertices [0, tn) get tiles.  A tile never spans a vertex listed in
 // `breaks` (sorted) and the vertex before it.  tile_of[v] = index of v's tile (of its first chunk, with
-// kHubFlag, when v is split).
+// kHubFlag, when v is split).  max_deg: the largest degree met.
 static void build_tiles(const uint32_t *offs, uint32_t n, uint32_t tn, uint32_t vcap, uint32_t ecap,
                         const std::vector<uint32_t> &breaks, std::vector<Tile> &tiles, uint32_t &nhub,
-                        uint32_t &nhubchunks, std::vector<uint32_t> &tile_of) {
+                        uint32_t &nhubchunks, std::vector<uint32_t> &tile_of, uint32_t &max_deg) {
     tiles.clear();
+    max_deg = 0;
     tile_of.assign(n, 0);  // vertices past tn (no edges: never reached) keep tile 0
     n = tn;
     nhub = 0;
@@ -78,6 +79,7 @@ static void build_tiles(const uint32_t *offs, uint32_t n, uint32_t tn, uint32_t 
         const uint32_t stop = nb < breaks.size() ? breaks[nb] : n;
         const uint32_t dv = offs[v + 1] - offs[v];
         if (dv > ecap) {
+            max_deg = std::max(max_deg, dv);
             const uint32_t nch = (dv + ecap - 1) / ecap;
             tile_of[v] = (uint32_t)tiles.size() | kHubFlag;
             for (uint32_t c = 0; c < nch; ++c) {
@@ -101,6 +103,7 @@ static void build_tiles(const uint32_t *offs, uint32_t n, uint32_t tn, uint32_t 
             const uint32_t d = offs[v + 1] - offs[v];
             if (d > ecap || sum + d > ecap) break;
             sum += d;
+            max_deg = std::max(max_deg, d);
             tile_of[v] = (uint32_t)tiles.size();
             ++v;
         }
@@ -170,6 +173,7 @@ static void graph_free(bcg_graph *g) {
     dev_free(g->d_slot_level);
     dev_free(g->d_ext);
     wide_free(g);
+    deep_free(g);
     dev_free(g->d_rows); dev_free(g->d_ctrl);
     dev_free(g->d_roots); dev_free(g->d_pend); dev_free(g->d_mult); dev_free(g->d_rstat);
     if (g->ev0) cudaEventDestroy(g->ev0);
@@ -239,7 +243,7 @@ static int setup_tiles(bcg_graph *g, const uint32_t *h_offs) {
     std::vector<Tile> tiles;
     std::vector<uint32_t> tile_of;
     build_tiles(h_offs, n, g->tile_n ? g->tile_n : n, g->tile_vcap, g->tile_ecap, g->tile_breaks, tiles, g->nhub,
-                g->nhubchunks, tile_of);
+                g->nhubchunks, tile_of, g->max_deg);
     g->ntiles = (uint32_t)tiles.size();
     CK(dev_alloc(&g->d_tiles, std::max<size_t>(1, tiles.size()) * sizeof(Tile)));
     if (!tiles.empty())
@@ -481,7 +485,10 @@ static int run_plan(bcg_graph *g, const RunPlan &p, cudaStream_t st, bcg_stats *
     }
     if (nroots == 0) return BCG_OK;
     int rc;
-    if (!debug && takes_wide(g, nroots) && (stats || g->sigma_mode == 0) && p.plain) {
+    // plain runs of a width that is not forced: the wide-batch kernel, or one
+    // CTA a source on graphs of few neighbours (both wait for their results)
+    const bool free_run = !debug && p.plain && !g->forced_width && (stats || g->sigma_mode == BCG_SIGMA_AUTO);
+    if (free_run && takes_wide(g, nroots)) {
         WideResult res;
         rc = wide_run(g, p.roots.data(), p.mult.data(), nroots, st, &res);
         if (rc) return rc;
@@ -490,6 +497,27 @@ static int run_plan(bcg_graph *g, const RunPlan &p, cudaStream_t st, bcg_stats *
                 stats->launches += res.launches;
                 stats->batches = res.batches;
                 stats->batch_width = kWideSlots;
+                finish_stats(g, p, res.rstat, stats);
+            }
+            return BCG_OK;
+        }
+    }
+    if (free_run && deep_takes(g)) {
+        DeepResult res;
+        bool extended = g->sigma_mode == BCG_SIGMA_EXTENDED;
+        rc = deep_run(g, p.roots.data(), p.mult.data(), nroots, extended, st, &res);
+        if (!rc && res.overflow && g->sigma_mode == BCG_SIGMA_AUTO) {
+            extended = true;
+            rc = deep_run(g, p.roots.data(), p.mult.data(), nroots, true, st, &res);
+        }
+        if (rc) return rc;
+        if (res.overflow) return set_error(BCG_ERR_OVERFLOW, "a shortest-path count exceeded 2^64");
+        if (res.done) {
+            if (stats) {
+                stats->launches += res.launches;
+                stats->batches = nroots;
+                stats->batch_width = 1;
+                stats->extended_sigma = extended ? 1u : 0u;
                 finish_stats(g, p, res.rstat, stats);
             }
             return BCG_OK;

@@ -17,6 +17,7 @@ using bcg::kTileVerts;
 
 namespace bcg {
 struct WideGraph;  // wide.cu
+struct DeepGraph;  // deep.cu
 
 // Pendant trees of a graph on the device (BCG_PRUNE_TREES, and one peeling
 // round for BCG_PRUNE_DEGREE1; trees_gpu.cu), caller's numbering.
@@ -88,6 +89,8 @@ struct bcg_graph {
     unsigned long long wait_ns = kDefaultWaitNs;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     bcg::WideGraph *wide = nullptr;  // the graph's form for wide-batch runs (wide.cu), built by the first one
+    bcg::DeepGraph *deep = nullptr;  // the same for deep runs (deep.cu)
+    uint32_t max_deg = 0;            // largest degree in the searched graph
 };
 
 namespace bcg {
@@ -129,6 +132,19 @@ struct WideResult {
 };
 int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, cudaStream_t st, WideResult *res);
 void wide_free(bcg_graph *g);
+
+// Runs one CTA a source on a graph of at most 8 neighbours a vertex (deep.cu);
+// as wide_run otherwise.  overflow: a uint64 count wrapped (done = false, bc as
+// before).  done and overflow false: no memory, or more levels than kMaxLevel.
+struct DeepResult {
+    bool done = false, overflow = false;
+    uint64_t launches = 0;
+    std::vector<RootStat> rstat;
+};
+bool deep_takes(const bcg_graph *g);
+int deep_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, bool ext, cudaStream_t st,
+             DeepResult *res);
+void deep_free(bcg_graph *g);
 
 // Component-packed batches already on the device (see BatchArgs::xbeg).
 struct PackedRun {

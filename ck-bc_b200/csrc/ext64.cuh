@@ -91,6 +91,14 @@ __host__ __device__ __forceinline__ unsigned long long ext_mul(unsigned long lon
 __host__ __device__ __forceinline__ unsigned long long ext_from_double(double x, int k = 0) {
     if (!(x > 0.0)) return 0ull;
     int q;
+#ifdef __CUDA_ARCH__
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
+    const int be = (int)(bits >> 52);
+    if (be != 0) {  // a normal number: its fields are the significand and exponent
+        q = be - 1022;
+        return ext_round(((bits & ((1ull << 52) - 1)) | (1ull << 52)) << 8, false, q + k - 50 + kExtBias);
+    }
+#endif
     const double m = frexp(x, &q);  // x = m * 2^q, m in [0.5, 1)
     // 53-bit integer significand D = m * 2^53, x * 2^k = D * 2^(q - 53 + k);
     // s = D * 2^8 in [2^60, 2^61) stands for s * 2^(e - bias - 11), so
@@ -103,6 +111,12 @@ __host__ __device__ __forceinline__ unsigned long long ext_from_double(double x,
 __host__ __device__ __forceinline__ double ext_to_double(unsigned long long a) {
     if (!a) return 0.0;
     const unsigned long long m = (a & kExtFrac) | (1ull << 48);
+#ifdef __CUDA_ARCH__
+    // 49 bits fit a double's 53: inside its normal range the fields are moved over
+    const int be = (int)(a >> 48) - kExtBias + 48 + 1023;
+    if (be > 0 && be < 2047)
+        return __longlong_as_double((long long)((unsigned long long)be << 52 | (a & kExtFrac) << 4));
+#endif
     return ldexp((double)m, (int)(a >> 48) - kExtBias);
 }
 

@@ -14,6 +14,16 @@
 // batch resets and first pulls only the rows and tiles of that prefix.  The whole schedule runs in one cooperative launch,
 // captured once into a CUDA graph and replayed by every bcg_batch_run.
 //
+// Sets of shallow graphs (wide_shallow: every graph of mean degree 6 and up, or
+// of a few vertices) do not run that schedule: their sources go to the
+// wide-batch searches (wide.cu), 16 of one graph a job, a CTA or a few to a
+// job, largest graphs first, in as many launches as the job vectors' memory
+// asks for, captured the same way.  One with a search of more than 62 levels
+// goes back to the packed schedule.  (48 graphs of 250 to 2,500 vertices: the
+// packed schedule advances all by six sources a batch and pays about 13
+// barriers of the whole chip for it, 108 ms; a CTA that runs 16 sources of one
+// graph has no such barrier: 6.8 ms.)
+//
 // The autotuner times a prefix of the schedule for each candidate batch width
 // S in {1, 3, 6} and tile shape (vertices x adjacency entries per tile), keeps
 // the fastest per root, and rebuilds the schedule for it.
@@ -24,6 +34,7 @@
 
 #include "bcg_common.hpp"
 #include "engine_internal.hpp"
+#include "wide.cuh"
 
 using namespace bcg;
 
@@ -48,6 +59,19 @@ struct bcg_batch {
     cudaGraphExec_t exec = nullptr;
     int captured = 0;  // 1: runs replay a captured CUDA graph; 0: direct launches
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    // the wide searches of the set (wide = false: the packed schedule runs)
+    bool wide = false, packed = false;  // packed: its schedule is built
+    WideForm form;
+    struct Launch {
+        WideArgs a;
+        size_t outs;  // offset of its WideOut entries in d_wide
+        uint32_t nouts, nmax;
+    };
+    std::vector<Launch> launches;
+    uint64_t njobs = 0;
+    unsigned char *d_wide = nullptr, *d_stat = nullptr, *d_state = nullptr;
+    double *d_jobbc = nullptr, *d_save = nullptr;
+    size_t stat_bytes = 0, o_total = 0;
 };
 
 namespace {
@@ -73,6 +97,145 @@ void free_schedule(bcg_batch *b) {
     b->exec = nullptr;
     b->graph = nullptr;
     b->captured = 0;
+    b->packed = false;
+}
+
+void free_wide(bcg_batch *b) {
+    wide_form_free(b->form);
+    dev_free(b->d_wide); dev_free(b->d_stat); dev_free(b->d_state); dev_free(b->d_jobbc); dev_free(b->d_save);
+    b->d_wide = b->d_stat = b->d_state = nullptr;
+    b->d_jobbc = b->d_save = nullptr;
+    b->launches.clear();
+    b->wide = false;
+}
+
+// The set's jobs and launches (b->wide = true), if every graph is shallow.
+// Running out of memory leaves the packed schedule to do the work.
+int build_wide(bcg_batch *b) {
+    bcg_graph *g = b->g;
+    const uint32_t G = b->ngraphs;
+    std::vector<uint32_t> ubase(G + 1);
+    std::vector<uint32_t> act(G, 0);
+    std::vector<uint64_t> gnnz(G, 0);
+    WideInput in = wide_input(g);
+    in.graphs = G;
+    in.base = ubase.data();
+    in.big_nnz = 0;
+    uint64_t nroots = 0;
+    for (uint32_t p = 0; p < G; ++p) {
+        const uint32_t v0 = ubase[p] = b->base[b->order[p]], nv = b->gn[b->order[p]];
+        uint64_t &nnz = gnnz[p];
+        for (uint32_t v = v0; v < v0 + nv; ++v) {
+            nnz += b->hdeg[v];
+            act[p] += b->hdeg[v] != 0;
+        }
+        if (!wide_shallow(act[p], nnz)) return BCG_OK;
+        in.big_nnz = std::max(in.big_nnz, nnz);
+        nroots += act[p];
+    }
+    ubase[G] = g->n;
+    if (nroots == 0 || g->n >= (1u << 28)) return BCG_OK;
+    auto give_up = [&](int rc) {
+        free_wide(b);
+        return rc == BCG_ERR_OOM ? (cudaGetLastError(), BCG_OK) : rc;
+    };
+    int rc = wide_form_make(b->form, in);
+    if (rc) return give_up(rc);
+    // jobs in union order (largest graphs first); a launch ends when its jobs'
+    // vectors take 512 MB, or when the graphs have become a quarter of its
+    // first one's size and it has work for four rounds of the chip
+    constexpr uint64_t kCells = (512ull << 20) / 8;
+    std::vector<WideJob> jobs;
+    std::vector<uint32_t> roots;
+    std::vector<WideOut> outs;
+    struct Span { size_t job0, njobs, out0, nouts; uint64_t cells, entries; uint32_t nmax, nch, nheavy; };
+    std::vector<Span> spans;
+    uint64_t most_cells = 0;
+    roots.reserve(nroots);
+    for (uint32_t p = 0; p < G; ++p) {
+        const WideSub &s = b->form.subs[p];
+        if (!act[p]) continue;
+        const size_t r0 = roots.size();
+        for (uint32_t v = ubase[p]; v < ubase[p + 1]; ++v)
+            if (b->hdeg[v]) roots.push_back(v);
+        for (uint32_t r = 0; r < act[p]; r += kWideSlots) {
+            if (spans.empty() || spans.back().cells + s.n > kCells ||
+                (r == 0 && s.n < spans.back().nmax / 4 && spans.back().njobs >= 4 * 148))
+                spans.push_back(Span{jobs.size(), 0, outs.size(), 0, 0, 0, s.n, 1, 1});
+            Span &l = spans.back();
+            if (l.nouts == 0 || r == 0) {
+                outs.push_back(WideOut{l.cells, 0, s.n, b->form.map + s.base, g->d_bc});
+                ++l.nouts;
+            }
+            ++outs.back().njobs;
+            jobs.push_back(WideJob{p, (uint32_t)(r0 + r), std::min<uint32_t>(kWideSlots, act[p] - r), 0, l.cells});
+            ++l.njobs;
+            l.cells += s.n;
+            l.entries += gnnz[p];
+            l.nmax = std::max(l.nmax, s.n);
+            l.nch = std::max({l.nch, s.nchunk[0], s.nchunk[1]});
+            l.nheavy = std::max(l.nheavy, s.nheavy);
+            most_cells = std::max(most_cells, l.cells);
+        }
+    }
+    auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
+    const size_t o_roots = up(jobs.size() * sizeof(WideJob)), o_outs = o_roots + up(roots.size() * 4),
+                 blob = o_outs + outs.size() * sizeof(WideOut);
+    size_t stat = 0, state = 0;
+    for (const Span &l : spans) {
+        bcg_batch::Launch L{};
+        state = std::max(state, (wide_layout(L.a, l.nmax, l.nch, l.nheavy), wide_teams(L.a, l.njobs, l.entries / l.njobs),
+                                 L.a.stride * L.a.teams));
+        L.a.njobs = (uint32_t)l.njobs;
+        L.outs = o_outs + l.out0 * sizeof(WideOut);
+        L.nouts = (uint32_t)l.nouts;
+        L.nmax = l.nmax;
+        b->launches.push_back(L);
+        stat += sizeof(WideCtrl) + L.a.teams * sizeof(WideTeam);
+    }
+    b->o_total = stat;
+    b->stat_bytes = stat + sizeof(RootStat);
+    cudaError_t e;
+    if ((e = dev_alloc(&b->d_wide, blob)) != cudaSuccess || (e = dev_alloc(&b->d_stat, b->stat_bytes)) != cudaSuccess ||
+        (e = dev_alloc(&b->d_state, state)) != cudaSuccess ||
+        (e = dev_alloc(&b->d_jobbc, most_cells * sizeof(double))) != cudaSuccess ||
+        (spans.size() > 1 && (e = dev_alloc(&b->d_save, (size_t)g->n * sizeof(double))) != cudaSuccess))
+        return give_up(set_error(e == cudaErrorMemoryAllocation ? BCG_ERR_OOM : BCG_ERR_CUDA, "wide searches: %s",
+                                 cudaGetErrorString(e)));
+    CKB(cudaMemcpy(b->d_wide, jobs.data(), jobs.size() * sizeof(WideJob), cudaMemcpyHostToDevice));
+    CKB(cudaMemcpy(b->d_wide + o_roots, roots.data(), roots.size() * 4, cudaMemcpyHostToDevice));
+    CKB(cudaMemcpy(b->d_wide + o_outs, outs.data(), outs.size() * sizeof(WideOut), cudaMemcpyHostToDevice));
+    CKB(cudaDeviceSynchronize());  // everything is ready for the batch's stream
+    size_t at = 0;
+    for (size_t i = 0; i < spans.size(); ++i) {
+        WideArgs &a = b->launches[i].a;
+        a.subs = b->form.d_subs;
+        a.jobs = reinterpret_cast<const WideJob *>(b->d_wide) + spans[i].job0;
+        a.roots = reinterpret_cast<const uint32_t *>(b->d_wide + o_roots);
+        a.jobbc = b->d_jobbc;
+        a.state = b->d_state;
+        a.ctrl = reinterpret_cast<WideCtrl *>(b->d_stat + at);
+        a.team = reinterpret_cast<WideTeam *>(b->d_stat + at + sizeof(WideCtrl));
+        a.total = reinterpret_cast<RootStat *>(b->d_stat + b->o_total);
+        at += sizeof(WideCtrl) + a.teams * sizeof(WideTeam);
+    }
+    b->njobs = jobs.size();
+    b->nroots = nroots;
+    b->wide = true;
+    return BCG_OK;
+}
+
+// Enqueues the wide launches on b->stream.
+int enqueue_wide(bcg_batch *b) {
+    CKB(cudaMemsetAsync(b->d_stat, 0, b->stat_bytes, b->stream));
+    if (b->d_save)  // launches add to bc one after the other: what it was before them
+        CKB(cudaMemcpyAsync(b->d_save, b->g->d_bc, (size_t)b->g->n * sizeof(double), cudaMemcpyDeviceToDevice, b->stream));
+    for (const bcg_batch::Launch &l : b->launches) {
+        const int rc = wide_enqueue(l.a, reinterpret_cast<const WideOut *>(b->d_wide + l.outs), l.nouts, WideOut{}, l.nmax,
+                                    b->stream);
+        if (rc) return rc;
+    }
+    return BCG_OK;
 }
 
 // Builds and uploads the packed schedule for width b->width and the graph's
@@ -148,6 +311,7 @@ int build_schedule(bcg_batch *b) {
     CKB(cudaMalloc(&b->d_xrange, nb * sizeof(uint2)));
     CKB(cudaMemcpy(b->d_xrbeg, xrbeg.data(), (nb + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice));
     CKB(cudaMemcpy(b->d_xrange, xrange.data(), nb * sizeof(uint2), cudaMemcpyHostToDevice));
+    b->packed = true;
     return ensure_state(g, S);
 }
 
@@ -264,7 +428,8 @@ int bcg_batch_create(uint32_t ngraphs, const uint32_t *const *offsets, const uin
     if ((e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaEventCreate(&b->ev0)) != cudaSuccess || (e = cudaEventCreate(&b->ev1)) != cudaSuccess)
         return fail(set_error(BCG_ERR_CUDA, "stream/event: %s", cudaGetErrorString(e)));
-    rc = build_schedule(b);
+    rc = build_wide(b);
+    if (!rc && !b->wide) rc = build_schedule(b);
     if (rc) return fail(rc);
     *out = b;
     return BCG_OK;
@@ -273,7 +438,9 @@ int bcg_batch_create(uint32_t ngraphs, const uint32_t *const *offsets, const uin
 int bcg_batch_destroy(bcg_batch *b) {
     clear_error();
     if (!b) return set_error(BCG_ERR_ARG, "null handle");
+    if (b->stream) cudaStreamSynchronize(b->stream);
     free_schedule(b);
+    free_wide(b);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
     if (b->stream) cudaStreamDestroy(b->stream);
@@ -282,68 +449,118 @@ int bcg_batch_destroy(bcg_batch *b) {
     return BCG_OK;
 }
 
+// Runs the set's launches on b->stream, captured into a CUDA graph by the
+// first run and replayed; if the capture cannot be made, runs launch directly
+// (b->captured says which).
+static int replay(bcg_batch *b) {
+    auto enqueue = [&]() {
+        return b->wide ? enqueue_wide(b) : enqueue_packed(b->g, packed_prefix(b, b->nbatch), b->width, b->stream);
+    };
+    if (!b->exec) {
+        cudaGraph_t graph = nullptr;
+        int rc = BCG_ERR_CUDA;
+        if (cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeRelaxed) == cudaSuccess) {
+            rc = enqueue();
+            const cudaError_t ee = cudaStreamEndCapture(b->stream, &graph);
+            if (rc == BCG_OK && ee == cudaSuccess && graph && cudaGraphInstantiate(&b->exec, graph, 0) == cudaSuccess) {
+                b->graph = graph;
+                b->captured = 1;
+            } else {
+                if (graph) cudaGraphDestroy(graph);
+                b->exec = nullptr;
+            }
+        }
+        cudaGetLastError();  // a refused capture leaves no sticky error
+        clear_error();
+    }
+    CKB(cudaEventRecord(b->ev0, b->stream));
+    if (b->exec) {
+        CKB(cudaGraphLaunch(b->exec, b->stream));
+    } else {
+        const int rc = enqueue();
+        if (rc) return rc;
+    }
+    CKB(cudaEventRecord(b->ev1, b->stream));
+    return BCG_OK;
+}
+
 int bcg_batch_run(bcg_batch *b, bcg_stats *stats) {
     clear_error();
     if (!b) return set_error(BCG_ERR_ARG, "null handle");
     if (stats) *stats = bcg_stats{};
-    if (b->nbatch) {
-        if (!b->exec) {
-            // capture the whole packed launch once; if the capture cannot be
-            // made, runs launch directly (b->captured says which)
-            cudaGraph_t graph = nullptr;
-            int rc = BCG_ERR_CUDA;
-            if (cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeRelaxed) == cudaSuccess) {
-                rc = enqueue_packed(b->g, packed_prefix(b, b->nbatch), b->width, b->stream);
-                const cudaError_t ee = cudaStreamEndCapture(b->stream, &graph);
-                if (rc == BCG_OK && ee == cudaSuccess && graph &&
-                    cudaGraphInstantiate(&b->exec, graph, 0) == cudaSuccess) {
-                    b->graph = graph;
-                    b->captured = 1;
-                } else {
-                    if (graph) cudaGraphDestroy(graph);
-                    b->exec = nullptr;
-                }
-            }
-            cudaGetLastError();  // a refused capture leaves no sticky error
-            clear_error();
+    uint64_t teps = 0, vis = 0, cv = 0;
+    uint32_t md = 0, width = 0;
+    uint64_t batches = 0;
+    if (b->wide) {
+        int rc = replay(b);
+        if (rc) return rc;
+        std::vector<unsigned char> hs(b->stat_bytes);
+        CKB(cudaMemcpyAsync(hs.data(), b->d_stat, b->stat_bytes, cudaMemcpyDeviceToHost, b->stream));
+        CKB(cudaStreamSynchronize(b->stream));
+        bool deep = false, overflow = false;
+        int error = 0;
+        for (const bcg_batch::Launch &l : b->launches) {
+            const WideCtrl *c =
+                reinterpret_cast<const WideCtrl *>(hs.data() + (reinterpret_cast<unsigned char *>(l.a.ctrl) - b->d_stat));
+            deep |= c->deep != 0;
+            overflow |= c->overflow != 0;
+            if (c->error) error = c->error;
         }
-        CKB(cudaEventRecord(b->ev0, b->stream));
-        if (b->exec) {
-            CKB(cudaGraphLaunch(b->exec, b->stream));
+        if ((deep || overflow || error) && b->d_save) {
+            CKB(cudaMemcpyAsync(b->g->d_bc, b->d_save, (size_t)b->g->n * sizeof(double), cudaMemcpyDeviceToDevice, b->stream));
+            CKB(cudaStreamSynchronize(b->stream));
+        }
+        if (error) return set_error(error, "device reported error %d (a bounded wait gave up)", error);
+        if (overflow) return set_error(BCG_ERR_OVERFLOW, "a shortest-path count exceeded 2^64");
+        if (deep) {  // from here on the packed schedule runs
+            free_schedule(b);
+            free_wide(b);
+            rc = build_schedule(b);
+            if (rc) return rc;
         } else {
-            const int rc = enqueue_packed(b->g, packed_prefix(b, b->nbatch), b->width, b->stream);
+            const RootStat *t = reinterpret_cast<const RootStat *>(hs.data() + b->o_total);
+            teps = t->mc2 / 2;  // every source's share is even
+            vis = t->visited;
+            cv = t->wsum;
+            md = t->depth;
+            batches = b->njobs;
+            width = kWideSlots;
+        }
+    }
+    if (!b->wide) {
+        batches = b->nbatch;
+        width = b->width;
+        if (b->nbatch) {
+            int rc = replay(b);
+            if (!rc) rc = check_ctrl(b->g, b->stream);
             if (rc) return rc;
         }
-        CKB(cudaEventRecord(b->ev1, b->stream));
-        const int rc = check_ctrl(b->g, b->stream);
-        if (rc) return rc;
+        if (stats) {
+            std::vector<RootStat> rs((size_t)b->nbatch * b->width);
+            if (!rs.empty())
+                CKB(cudaMemcpy(rs.data(), b->d_rstat, rs.size() * sizeof(RootStat), cudaMemcpyDeviceToHost));
+            for (const RootStat &r : rs) {
+                teps += r.mc2 / 2;
+                vis += r.visited;
+                cv += r.wsum;
+                md = std::max(md, r.depth);
+            }
+        }
     }
     if (stats) {
-        const uint32_t S = b->width;
-        std::vector<RootStat> rs((size_t)b->nbatch * S);
-        if (!rs.empty())
-            CKB(cudaMemcpy(rs.data(), b->d_rstat, rs.size() * sizeof(RootStat), cudaMemcpyDeviceToHost));
-        uint64_t teps = 0, vis = 0, cv = 0;
-        uint32_t md = 0;
-        for (const RootStat &r : rs) {
-            teps += r.mc2 / 2;
-            vis += r.visited;
-            cv += r.wsum;
-            md = std::max(md, r.depth);
-        }
         uint64_t nsrc = 0;
         for (uint32_t i = 0; i < b->ngraphs; ++i) nsrc += b->gn[i];
         float ms = 0.f;
-        if (b->nbatch) cudaEventElapsedTime(&ms, b->ev0, b->ev1);
+        if (batches) cudaEventElapsedTime(&ms, b->ev0, b->ev1);
         stats->sources = nsrc;
         stats->roots = b->nroots;
         stats->skipped = nsrc - b->nroots;
-        stats->batches = b->nbatch;
+        stats->batches = batches;
         stats->teps_edges = teps;
         stats->visited = vis;
         stats->comp_vertices = cv;
         stats->max_depth = md;
-        stats->batch_width = S;
+        stats->batch_width = width;
         stats->kernel_ms = ms;
     }
     return BCG_OK;
@@ -372,6 +589,12 @@ int bcg_batch_autotune(bcg_batch *b, uint32_t sample_batches, uint32_t *width, u
     if (!b) return set_error(BCG_ERR_ARG, "null handle");
     static const uint32_t widths[] = {1, 3, 6};
     static const uint32_t shapes[][2] = {{32, 512}, {32, 256}, {32, 128}, {16, 128}, {16, 64}};
+    if (b->wide) {  // nothing to tune: the widths and tiles are the packed schedule's
+        if (width) *width = b->width;
+        if (tile_vertices) *tile_vertices = b->g->tile_vcap;
+        if (tile_entries) *tile_entries = b->g->tile_ecap;
+        return bcg_reset_bc(b->g);
+    }
     double best = 0.0;
     uint32_t bw = b->width, bv = b->g->tile_vcap, be = b->g->tile_ecap;
     for (const auto &sh : shapes) {
@@ -413,7 +636,7 @@ int bcg_batch_info(bcg_batch *b, uint32_t *nbatch, uint32_t *width, uint32_t *ti
                    uint32_t *tile_entries, int *captured) {
     clear_error();
     if (!b) return set_error(BCG_ERR_ARG, "null handle");
-    if (nbatch) *nbatch = b->nbatch;
+    if (nbatch) *nbatch = b->wide ? (uint32_t)std::min<uint64_t>(b->njobs, 0xFFFFFFFFull) : b->nbatch;
     if (width) *width = b->width;
     if (tile_vertices) *tile_vertices = b->g->tile_vcap;
     if (tile_entries) *tile_entries = b->g->tile_ecap;

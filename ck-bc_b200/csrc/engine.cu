@@ -441,13 +441,13 @@ struct DebugOut {
     double *delta = nullptr;
 };
 
-// Whether a run of nroots plain sources goes to the wide-batch kernel: a
-// width not forced, counts not extended from the start, and a graph that is
-// not of low degree (grids, meshes, chains: deep, with small frontiers).
+// Whether a run of nroots plain sources goes to the wide-batch kernel: counts
+// not extended from the start, and a graph that is not of low degree (grids,
+// meshes, chains: deep, with small frontiers).
 static bool takes_wide(const bcg_graph *g, uint64_t nroots) {
-    const double n = g->tile_n ? g->tile_n : g->n;
-    return !g->forced_width && g->sigma_mode != BCG_SIGMA_EXTENDED && nroots >= 4 && (double)g->nnz_pruned >= 6.0 * n &&
-           n < (double)(1u << 28);
+    const uint32_t n = g->tile_n ? g->tile_n : g->n;
+    if (g->sigma_mode == BCG_SIGMA_EXTENDED || nroots < 4 || n >= (1u << 28)) return false;
+    return wide_shallow(n, g->nnz_pruned) && (g->nnz_pruned >= 6ull * n || !deep_takes(g));
 }
 
 // Totals of the plan's roots (rs in plan order) and the kernels' time.

@@ -120,6 +120,9 @@ int launch_sweep(int S, const BatchArgs &a, cudaStream_t st, int *grid_out, bool
 // out[i] = in[0] + ... + in[i-1] on stream st (in and out may be the same
 // array; every partial sum fits 32 bits).
 int scan_exclusive(const uint32_t *d_in, uint32_t *d_out, uint64_t len, cudaStream_t st);
+// The same with the caller's scratch of scan_scratch(len) entries.
+uint64_t scan_scratch(uint64_t len);
+int scan_exclusive(const uint32_t *d_in, uint32_t *d_out, uint64_t len, uint32_t *scratch, cudaStream_t st);
 
 // Wide-batch runs (wide.cu).  Adds the dependencies of the given roots
 // (engine ids with an edge, weights mult) into g's bc on stream st and waits.

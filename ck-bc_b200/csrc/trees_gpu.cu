@@ -103,22 +103,29 @@ __global__ void k_scan_add(uint32_t *__restrict__ out, const uint32_t *__restric
 
 }  // namespace
 
-int scan_exclusive(const uint32_t *d_in, uint32_t *d_out, uint64_t len, cudaStream_t st) {
+uint64_t scan_scratch(uint64_t len) {
+    uint64_t s = 0;
+    for (uint64_t nb = (len + kScanBlock - 1) / kScanBlock; nb > 1; nb = (nb + kScanBlock - 1) / kScanBlock) s += nb;
+    return s + 1;
+}
+
+int scan_exclusive(const uint32_t *d_in, uint32_t *d_out, uint64_t len, uint32_t *scratch, cudaStream_t st) {
     if (len == 0) return BCG_OK;
     const uint64_t nb = (len + kScanBlock - 1) / kScanBlock;
-    uint32_t *bsum = nullptr;
-    CKT(tmp_alloc(&bsum, nb * sizeof(uint32_t), st));
-    k_scan_block<<<(unsigned)nb, kScanBlock, 0, st>>>(d_in, d_out, bsum, len);
-    int rc = BCG_OK;
-    if (cudaGetLastError() != cudaSuccess) rc = set_error(BCG_ERR_CUDA, "scan launch failed");
-    if (!rc && nb > 1) {
-        rc = scan_exclusive(bsum, bsum, nb, st);
-        if (!rc) {
-            k_scan_add<<<(unsigned)nb, kScanBlock, 0, st>>>(d_out, bsum, len);
-            if (cudaGetLastError() != cudaSuccess) rc = set_error(BCG_ERR_CUDA, "scan launch failed");
-        }
+    k_scan_block<<<(unsigned)nb, kScanBlock, 0, st>>>(d_in, d_out, scratch, len);
+    if (nb > 1) {
+        const int rc = scan_exclusive(scratch, scratch, nb, scratch + nb, st);
+        if (rc) return rc;
+        k_scan_add<<<(unsigned)nb, kScanBlock, 0, st>>>(d_out, scratch, len);
     }
-    tmp_free(bsum, st);
+    return cudaGetLastError() == cudaSuccess ? BCG_OK : set_error(BCG_ERR_CUDA, "scan launch failed");
+}
+
+int scan_exclusive(const uint32_t *d_in, uint32_t *d_out, uint64_t len, cudaStream_t st) {
+    uint32_t *scratch = nullptr;
+    CKT(tmp_alloc(&scratch, scan_scratch(len) * sizeof(uint32_t), st));
+    const int rc = scan_exclusive(d_in, d_out, len, scratch, st);
+    tmp_free(scratch, st);
     return rc;
 }
 

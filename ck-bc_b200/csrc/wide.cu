@@ -164,6 +164,7 @@ __device__ bool team_sync(const WideArgs &a, const WideCtx &x, WideTeam *t, Wide
                         if (wide_stopped(a.ctrl)) break;
                         if (wide_ns() - t0 > wait_ns) {
                             atomicCAS(&a.ctrl->error, 0, BCG_ERR_TIMEOUT);
+                            if (a.poison) *a.poison = 1;
                             break;
                         }
                     }
@@ -478,7 +479,7 @@ __device__ __noinline__ void wide_sweep(WideSmem &sm, uint32_t d) {
                 const uint32_t i = it * cb + lane;
                 if (lane < cb && i < nchunk) {
                     const uint2 ch = g.chunk[side][i];
-                    v = ch.x;
+                    v = ch.x - g.base;
                     e0 = offs[v] + ch.y * g.chunk_len;
                     e1 = min(offs[v + 1], e0 + g.chunk_len);
                     need = true;
@@ -532,7 +533,7 @@ __device__ __noinline__ void wide_sweep(WideSmem &sm, uint32_t d) {
                 T sum = wide_fold<KIND>(acc, ovf);
                 if (heavy) {
                     const uint32_t ci = it * cb + i;
-                    const uint32_t c0 = g.cbeg[side][vi], nc = g.cbeg[side][vi + 1] - c0;
+                    const uint32_t c0 = g.cbeg[side][vi] - g.chunk0[side], nc = g.cbeg[side][vi + 1] - g.chunk0[side] - c0;
                     if (nc > 1) {
                         // the chunks meet: the one that arrives last adds them,
                         // half warps the even and the odd ones, in order
@@ -678,6 +679,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
     WideCtx &x = sm.x;
     const uint32_t team = blockIdx.x / a.team_ctas;
     if (team >= a.teams) return;
+    if (a.poison && *reinterpret_cast<volatile int *>(a.poison)) return;
     WideTeam *t = a.team + team;
     const unsigned long long wait_ns = a.ctrl->wait_ns ? a.ctrl->wait_ns : kDefaultWaitNs;
     if (threadIdx.x == 0) {
@@ -704,7 +706,14 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
     }
     uint32_t job = team;
     for (uint32_t par = 0; job < a.njobs; par ^= 1u) {
-        const WideJob J = a.jobs[job];
+        WideJob J{0u, 0u, 0u, 0u, 0ull};
+        if (a.jobs) {
+            J = a.jobs[job];
+        } else {  // one graph's sources in order
+            J.root0 = (a.job0 + job) * kWideSlots;
+            J.nroots = min((uint32_t)kWideSlots, a.nroots - J.root0);
+            J.out = (unsigned long long)job * a.subs[0].n;
+        }
         if (threadIdx.x < sizeof(WideSub) / 4)
             reinterpret_cast<uint32_t *>(&sm.sub)[threadIdx.x] =
                 reinterpret_cast<const uint32_t *>(a.subs + J.sub)[threadIdx.x];
@@ -712,7 +721,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
         if (threadIdx.x == 0) {
             // four lanes take a vertex while its blocks are no more than
             // about half of a warp's share of a sweep
-            const uint32_t blocks = sm.sub.offs[1][sm.sub.n] / (128u * x.T * kWideWarps);
+            const uint32_t blocks = (sm.sub.offs[1][sm.sub.n] - sm.sub.offs[1][0]) / (128u * x.T * kWideWarps);
             sm.nmed = sm.sub.nmed[blocks >= 32 ? 3 : (blocks >= 16 ? 2 : (blocks >= 8 ? 1 : 0))];
         }
         if (threadIdx.x < kWideSlots) {
@@ -720,7 +729,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
             uint32_t r = kNone;
             if (has) r = sm.sub.inv[a.roots[J.root0 + threadIdx.x]];
             sm.roots[threadIdx.x] = r;
-            sm.mult[threadIdx.x] = has ? a.mult[J.root0 + threadIdx.x] : 0.0;
+            sm.mult[threadIdx.x] = !has ? 0.0 : (a.mult ? a.mult[J.root0 + threadIdx.x] : 1.0);
         }
         if (threadIdx.x == 0) x.bc = a.jobbc + J.out;
         __syncthreads();
@@ -803,7 +812,10 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
         bool big = false;  // some count of level d is 2^28 or more
         for (;; ++d) {
             if (d + 2 >= kWideLevels) {
-                if (threadIdx.x == 0) a.ctrl->deep = 1;
+                if (threadIdx.x == 0) {
+                    a.ctrl->deep = 1;
+                    if (a.poison) *a.poison = 1;
+                }
                 return;
             }
             for (uint32_t w = tid; w < (n + 31u) >> 5; w += nt) x.act[(size_t)(d + 2) * x.words + w] = 0;
@@ -831,7 +843,10 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
             const uint32_t any = sm.any;
             wide_trace(a, job, 2, d, any);
             if (any & 4u) {
-                if (threadIdx.x == 0) a.ctrl->overflow = 1;
+                if (threadIdx.x == 0) {
+                    a.ctrl->overflow = 1;
+                    if (a.poison) *a.poison = 1;
+                }
                 return;
             }
             if (!(any & 1u)) break;
@@ -874,7 +889,12 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
             }
         }
         __syncthreads();
-        if (threadIdx.x < kWideSlots && sm.reach[threadIdx.x]) {
+        if (threadIdx.x < kWideSlots && sm.reach[threadIdx.x] && a.total) {
+            atomicAdd(&a.total->visited, sm.reach[threadIdx.x]);
+            atomicAdd(&a.total->wsum, sm.reach[kWideSlots + threadIdx.x]);
+            atomicAdd(&a.total->mc2, sm.reach[2 * kWideSlots + threadIdx.x]);
+            atomicMax(&a.total->depth, D);
+        } else if (threadIdx.x < kWideSlots && sm.reach[threadIdx.x] && a.rstat) {
             RootStat *rs = a.rstat + (size_t)job * kWideSlots + threadIdx.x;
             atomicAdd(&rs->visited, sm.reach[threadIdx.x]);
             atomicAdd(&rs->wsum, sm.reach[kWideSlots + threadIdx.x]);
@@ -900,18 +920,13 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
 // interleaved partial sums in job order, then those in order.
 // ---------------------------------------------------------------------------
 
-struct WideOut {
-    unsigned long long out0;  // jobs j < njobs: jobbc[out0 + j * n + v]
-    uint32_t njobs, n;
-    const uint32_t *map;      // v -> index into bc
-    double *bc;
-};
-
 __global__ void __launch_bounds__(256) k_wide_reduce(const WideCtrl *__restrict__ ctrl,
+                                                     const int *__restrict__ poison,
                                                      const WideOut *__restrict__ outs, WideOut one,
                                                      const double *__restrict__ jobbc) {
     __shared__ double part[8][32];
     if (ctrl->error | ctrl->overflow | ctrl->deep) return;  // nothing of a stopped launch is kept
+    if (poison && *poison) return;
     const WideOut o = outs ? outs[blockIdx.y] : one;
     const unsigned lane = threadIdx.x & 31, p = threadIdx.x >> 5;
     for (uint32_t v0 = blockIdx.x * 32; v0 < o.n; v0 += gridDim.x * 32) {
@@ -933,170 +948,77 @@ __global__ void __launch_bounds__(256) k_wide_reduce(const WideCtrl *__restrict_
     }
 }
 
-// ---------------------------------------------------------------------------
-// The numbering by descending degree class, built on the device.
-// ---------------------------------------------------------------------------
-
-constexpr uint32_t kClasses = 112;  // key of degree class c: kClasses - 1 - c
-constexpr uint32_t kSortVerts = 2048;  // vertices of a sorting block
-
-// Degrees up to 32 are classes of their own (a warp takes eight vertices of
-// one class), then eights up to 256, then two classes an octave; 0 is last.
-__device__ __forceinline__ uint32_t degree_key(uint32_t d) {
-    uint32_t c;
-    if (d <= 32u) c = d;
-    else if (d <= 256u) c = 33u + (d - 33u) / 8u;
-    else {
-        const uint32_t lg = 31u - __clz(d);
-        c = 61u + 2u * (lg - 8u) + ((d >> (lg - 1u)) & 1u);
-    }
-    return kClasses - 1u - c;
-}
-constexpr uint32_t kKeyZero = kClasses - 1u;
-
-__device__ __forceinline__ uint32_t sort_degree(const uint32_t *offs, const uint32_t *toffs, uint32_t v) {
-    const uint32_t d = offs[v + 1] - offs[v];
-    return toffs ? max(d, toffs[v + 1] - toffs[v]) : d;
-}
-
-__global__ void __launch_bounds__(256) k_wide_hist(uint32_t n, const uint32_t *__restrict__ offs,
-                                                   const uint32_t *__restrict__ toffs, uint32_t *__restrict__ hist) {
-    __shared__ uint32_t cnt[kClasses];
-    for (uint32_t i = threadIdx.x; i < kClasses; i += 256) cnt[i] = 0;
-    __syncthreads();
-    const uint32_t v0 = blockIdx.x * kSortVerts;
-    for (uint32_t i = threadIdx.x; i < kSortVerts && v0 + i < n; i += 256)
-        atomicAdd(&cnt[degree_key(sort_degree(offs, toffs, v0 + i))], 1u);
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < kClasses; i += 256) hist[i * gridDim.x + blockIdx.x] = cnt[i];
-}
-
-// hist: exclusive prefix sums.  Stable: vertices of a class keep their order.
-// meta: {vertices with an entry, nheavy, the four nmed}.
-__global__ void __launch_bounds__(256) k_wide_number(uint32_t n, const uint32_t *__restrict__ offs,
-                                                     const uint32_t *__restrict__ toffs,
-                                                     const uint32_t *__restrict__ hist, uint32_t *__restrict__ perm,
-                                                     uint32_t *__restrict__ inv, uint32_t chunk,
-                                                     uint32_t *__restrict__ meta) {
-    __shared__ uint32_t base[kClasses], cnt[8][kClasses];
-    const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (uint32_t i = threadIdx.x; i < kClasses; i += 256) base[i] = hist[i * gridDim.x + blockIdx.x];
-    for (uint32_t i = threadIdx.x; i < 8 * kClasses; i += 256) (&cnt[0][0])[i] = 0;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        meta[0] = hist[kKeyZero * gridDim.x];
-        meta[1] = hist[(degree_key(chunk + 1u) + 1u) * gridDim.x];  // the classes from chunk's octave on
-        for (uint32_t b = 0; b < 4; ++b)  // more than 32, 64, 128, 256 entries
-            meta[2 + b] = max(meta[1], hist[(degree_key(kWideLight << b)) * gridDim.x]);
-    }
-    __syncthreads();
-    const uint32_t b0 = blockIdx.x * kSortVerts;
-    for (uint32_t i0 = 0; i0 < kSortVerts; i0 += 256) {
-        const uint32_t v = b0 + i0 + threadIdx.x;
-        const bool ok = v < n && i0 + threadIdx.x < kSortVerts;
-        const uint32_t key = ok ? degree_key(sort_degree(offs, toffs, v)) : kClasses;
-        const unsigned peers = __match_any_sync(kFull, key);
-        const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
-        if (ok && rank == 0) cnt[wid][key] = __popc(peers);
-        __syncthreads();
-        if (ok) {
-            uint32_t pos = base[key] + rank;
-            for (unsigned w = 0; w < wid; ++w) pos += cnt[w][key];
-            perm[pos] = v;
-            inv[v] = pos;
-        }
-        __syncthreads();
-        for (uint32_t i = threadIdx.x; i < kClasses; i += 256) {
-            uint32_t s = 0;
-            for (unsigned w = 0; w < 8; ++w) {
-                s += cnt[w][i];
-                cnt[w][i] = 0;
-            }
-            base[i] += s;
-        }
-        __syncthreads();
-    }
-}
-
-// Row lengths in the new numbering (len[n] = 0 for the scan), the degree and
-// reach words, and where a vertex's bc goes.
-__global__ void k_wide_len(uint32_t n, const uint32_t *__restrict__ perm, const uint32_t *__restrict__ offs,
-                           const uint32_t *__restrict__ toffs, const uint2 *__restrict__ vinfo,
-                           const uint32_t *__restrict__ ext, uint32_t *__restrict__ len, uint32_t *__restrict__ tlen,
-                           uint2 *__restrict__ vi2, uint32_t *__restrict__ map) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > n) return;
-    if (i == n) {
-        len[n] = 0;
-        if (toffs) tlen[n] = 0;
-        return;
-    }
-    const uint32_t v = perm[i];
-    len[i] = offs[v + 1] - offs[v];
-    if (toffs) tlen[i] = toffs[v + 1] - toffs[v];
-    vi2[i] = vinfo[v];
-    map[i] = ext ? ext[v] : v;
-}
-
-// The lists in the new numbering, one warp a vertex, order kept.
-__global__ void k_wide_fill(uint32_t n, const uint32_t *__restrict__ perm, const uint32_t *__restrict__ inv,
-                            const uint32_t *__restrict__ offs, const uint32_t *__restrict__ adj,
-                            const uint32_t *__restrict__ offs2, uint32_t *__restrict__ adj2) {
-    const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const unsigned lane = threadIdx.x & 31;
-    if (w >= n) return;
-    const uint32_t v = perm[w], e0 = offs[v], len = offs[v + 1] - e0, o = offs2[w];
-    for (uint32_t i = lane; i < len; i += 32) adj2[o + i] = inv[adj[e0 + i]];
-}
-
-// Chunks of the heavy vertices (at least one each): counts, then the table.
-// cap: entries of cnt (an upper bound of nheavy); cnt[cap] closes the scan.
-__global__ void k_wide_chunks(uint32_t cap, const uint32_t *__restrict__ meta, const uint32_t *__restrict__ offs2,
-                              uint32_t chunk, uint32_t *__restrict__ cnt) {
-    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v > cap) return;
-    cnt[v] = v < meta[1] ? max(1u, (offs2[v + 1] - offs2[v] + chunk - 1u) / chunk) : 0u;
-}
-
-__global__ void k_wide_table(uint32_t cap, uint32_t *__restrict__ meta, int side, const uint32_t *__restrict__ cbeg,
-                             uint2 *__restrict__ chunk) {
-    const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const unsigned lane = threadIdx.x & 31;
-    if (w == 0 && lane == 0) meta[6 + side] = cbeg[cap];
-    if (w >= meta[1]) return;
-    const uint32_t c0 = cbeg[w], c1 = cbeg[w + 1];
-    for (uint32_t c = c0 + lane; c < c1; c += 32) chunk[c] = make_uint2((uint32_t)w, c - c0);
-}
-
-// Transposed lists of a directed graph (the order within a list is free: path
-// counts are integers).
-__global__ void k_wide_indeg(uint64_t nnz, const uint32_t *__restrict__ adj, uint32_t *__restrict__ deg) {
-    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += (uint64_t)gridDim.x * blockDim.x)
-        atomicAdd(deg + adj[e], 1u);
-}
-__global__ void k_wide_transpose(uint32_t n, const uint32_t *__restrict__ offs, const uint32_t *__restrict__ adj,
-                                 uint32_t *__restrict__ cursor, uint32_t *__restrict__ tadj) {
-    const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const unsigned lane = threadIdx.x & 31;
-    if (w >= n) return;
-    for (uint32_t e = offs[w] + lane; e < offs[w + 1]; e += 32) tadj[atomicAdd(cursor + adj[e], 1u)] = (uint32_t)w;
-}
-
-#define CKW(call)                                                                                      do {                                                                                                   cudaError_t e_ = (call);                                                                           if (e_ != cudaSuccess)                                                                                 return set_error(e_ == cudaErrorMemoryAllocation ? BCG_ERR_OOM : BCG_ERR_CUDA, "%s failed: %s",                              #call, cudaGetErrorString(e_));                                           } while (0)
-
-inline unsigned wblocks(uint64_t work, unsigned per) { return (unsigned)std::max<uint64_t>(1, (work + per - 1) / per); }
+#define CKW(call)                                                                                  \
+    do {                                                                                           \
+        cudaError_t e_ = (call);                                                                   \
+        if (e_ != cudaSuccess)                                                                     \
+            return set_error(e_ == cudaErrorMemoryAllocation ? BCG_ERR_OOM : BCG_ERR_CUDA, "%s failed: %s", \
+                             #call, cudaGetErrorString(e_));                                       \
+    } while (0)
 
 size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
 
 }  // namespace
 
-// A graph's wide form (bcg_graph::wide): its lists in the wide numbering and
+size_t wide_layout(WideArgs &a, size_t n, size_t nchunk, size_t nheavy) {
+    const size_t words = (n + 31) / 32;
+    size_t o = up256(n * 16);
+    a.o_done = o; o += up256(words * 4);
+    a.o_act = o; o += up256(words * 4 * kWideLevels);
+    a.o_sig = o; o += up256(n * 128);
+    a.o_g0 = o; o += up256(n * 128);
+    a.o_g1 = o; o += up256(n * 128);
+    a.o_part = o; o += up256(std::max<size_t>(1, nchunk) * 128);
+    a.o_hcnt = o; o += up256(std::max<size_t>(1, nheavy) * 4);
+    a.stride = o;
+    a.words = words;
+    return o;
+}
+
+void wide_teams(WideArgs &a, uint64_t njobs, uint64_t entries) {
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    // A job on a team of T CTAs takes about 70 us of barriers and latency, and
+    // its entries at 9 ns an entry and CTA, 1.1 times that once the teams'
+    // rows are well beyond L2 (fitted on 16-source jobs of R-MAT graphs: 0.1 M
+    // entries 540 us on 1 CTA; 7.1 M entries 6,050 us on 13 and 590 us on 148;
+    // 30 M entries 8,800 us on 29 and 1,590 us on 148).  The number of teams
+    // that ends first, its states within 1 GiB.
+    constexpr double kFixed = 70.0, kEntry = 0.009, kBeyond = 1.1;
+    double best = 0.0;
+    for (uint64_t t = 1; t <= std::min<uint64_t>(njobs, (uint64_t)nsm); ++t) {
+        if (t > 1 && (double)a.stride * (double)t > 1024.0 * 1024 * 1024) break;
+        const double rows = (double)t * (double)a.words * 32.0 * 128.0;
+        const double job = kFixed + (double)entries * kEntry * (rows > 126e6 ? kBeyond : 1.0) / (double)(nsm / t);
+        const double all = (double)((njobs + t - 1) / t) * job;
+        if (t == 1 || all < best) {
+            best = all;
+            a.teams = (uint32_t)t;
+        }
+    }
+    a.team_ctas = (uint32_t)nsm / a.teams;
+}
+
+int wide_enqueue(const WideArgs &a, const WideOut *outs, uint32_t nouts, const WideOut &one, uint32_t nmax,
+                 cudaStream_t st) {
+    WideArgs args = a;
+    void *params[] = {&args};
+    CKW(cudaLaunchCooperativeKernel((const void *)bc_wide_kernel, dim3(a.teams * a.team_ctas), dim3(kWideThreads),
+                                    params, 0, st));
+    const unsigned bx = (unsigned)std::max<size_t>(1, ((size_t)nmax + 31) / 32);
+    // (65535 graphs at most in the second dimension)
+    for (uint32_t o = 0; o < nouts; o += 65535u)
+        k_wide_reduce<<<dim3(bx, std::min(65535u, nouts - o)), 256, 0, st>>>(a.ctrl, a.poison, outs ? outs + o : nullptr,
+                                                                           one, a.jobbc);
+    CKW(cudaGetLastError());
+    return BCG_OK;
+}
+
+// What a graph keeps for its wide runs (bcg_graph::wide): its wide form and
 // the buffers of its runs.
 struct WideGraph {
-    WideSub sub{};
-    uint32_t *perm = nullptr, *inv = nullptr, *map = nullptr, *offs[2] = {nullptr, nullptr},
-             *adj[2] = {nullptr, nullptr}, *cbeg[2] = {nullptr, nullptr};
-    uint2 *vinfo = nullptr, *chunk[2] = {nullptr, nullptr};
-    // run buffers
+    WideForm form;
     unsigned char *state = nullptr, *blob = nullptr, *stat = nullptr;
     double *jobbc = nullptr;
     size_t state_cap = 0, blob_cap = 0, stat_cap = 0, jobbc_cap = 0;
@@ -1105,174 +1027,75 @@ struct WideGraph {
 void wide_free(bcg_graph *g) {
     WideGraph *w = g->wide;
     if (!w) return;
-    dev_free(w->perm); dev_free(w->inv); dev_free(w->map); dev_free(w->vinfo);
-    for (int s = 0; s < 2; ++s) {
-        if (s && w->offs[1] == w->offs[0]) break;
-        dev_free(w->offs[s]); dev_free(w->adj[s]); dev_free(w->cbeg[s]); dev_free(w->chunk[s]);
-    }
+    wide_form_free(w->form);
     dev_free(w->state); dev_free(w->blob); dev_free(w->stat); dev_free(w->jobbc);
     delete w;
     g->wide = nullptr;
 }
 
-// Builds g's wide form on stream 0 (the caller's later work on any stream
-// follows: the call ends with a device synchronisation).
-static int wide_build(bcg_graph *g) {
-    WideGraph *w = g->wide = new WideGraph();
-    const uint32_t n = g->tile_n ? g->tile_n : g->n;
-    const uint64_t nnz = g->nnz_pruned;
-    const bool dir = (g->flags & BCG_DIRECTED) != 0;
-    cudaStream_t st = 0;
-    uint32_t *toffs = nullptr, *tadj = nullptr, *tmp = nullptr, *hist = nullptr, *meta = nullptr;
-    auto cleanup = [&]() {
-        tmp_free(toffs, st); tmp_free(tadj, st); tmp_free(tmp, st); tmp_free(hist, st); tmp_free(meta, st);
-    };
-    struct Guard { decltype(cleanup) &f; ~Guard() { f(); } } guard{cleanup};
-    int rc;
-    CKW(tmp_alloc(&meta, 8 * sizeof(uint32_t), st));
-    CKW(tmp_alloc(&tmp, 2 * ((size_t)n + 1) * sizeof(uint32_t), st));
-    if (dir) {
-        CKW(tmp_alloc(&toffs, ((size_t)n + 1) * sizeof(uint32_t), st));
-        CKW(tmp_alloc(&tadj, std::max<uint64_t>(1, nnz) * sizeof(uint32_t), st));
-        CKW(cudaMemsetAsync(tmp, 0, ((size_t)n + 1) * sizeof(uint32_t), st));
-        k_wide_indeg<<<148 * 8, 256, 0, st>>>(nnz, g->d_adj, tmp);
-        if ((rc = scan_exclusive(tmp, toffs, (uint64_t)n + 1, st))) return rc;
-        CKW(cudaMemcpyAsync(tmp, toffs, (size_t)n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
-        k_wide_transpose<<<wblocks((uint64_t)n * 32, 256), 256, 0, st>>>(n, g->d_offs, g->d_adj, tmp, tadj);
-        CKW(cudaGetLastError());
-    }
-    // entries of a warp's share of a heavy vertex: longer ones meet less
-    // often, shorter ones leave more warps something to do
-    uint32_t chunk = kWideChunk;
-    while (chunk < 8 * kWideChunk && nnz / (148ull * kWideWarps * 8) >= chunk) chunk *= 2;
-    const uint32_t nb = wblocks(n, kSortVerts);
-    CKW(tmp_alloc(&hist, (size_t)kClasses * nb * sizeof(uint32_t), st));
-    CKW(dev_alloc(&w->perm, (size_t)n * sizeof(uint32_t)));
-    CKW(dev_alloc(&w->inv, (size_t)n * sizeof(uint32_t)));
-    CKW(dev_alloc(&w->map, (size_t)n * sizeof(uint32_t)));
-    CKW(dev_alloc(&w->vinfo, (size_t)n * sizeof(uint2)));
-    k_wide_hist<<<nb, 256, 0, st>>>(n, g->d_offs, toffs, hist);
-    if ((rc = scan_exclusive(hist, hist, (uint64_t)kClasses * nb, st))) return rc;
-    k_wide_number<<<nb, 256, 0, st>>>(n, g->d_offs, toffs, hist, w->perm, w->inv, chunk, meta);
-    k_wide_len<<<wblocks((uint64_t)n + 1, 256), 256, 0, st>>>(n, w->perm, g->d_offs, toffs, g->d_vinfo, g->d_ext, tmp,
-                                                              tmp + n + 1, w->vinfo, w->map);
-    CKW(cudaGetLastError());
-    // a heavy vertex has at least chunk entries in one direction
-    const uint32_t cap = (uint32_t)std::min<uint64_t>(n, (dir ? 2 : 1) * (nnz / chunk) + 1);
-    const size_t maxchunk = nnz / chunk + cap + 1;
-    for (int s = 0; s < (dir ? 2 : 1); ++s) {
-        // side 0: who leads to v (the transposed lists of a directed graph), side 1: where v leads
-        const uint32_t *o = (dir && s == 0) ? toffs : g->d_offs, *a = (dir && s == 0) ? tadj : g->d_adj;
-        const uint32_t *len = (dir && s == 0) ? tmp + n + 1 : tmp;
-        CKW(dev_alloc(&w->offs[s], ((size_t)n + 1) * sizeof(uint32_t)));
-        CKW(dev_alloc(&w->adj[s], std::max<uint64_t>(1, nnz) * sizeof(uint32_t)));
-        CKW(dev_alloc(&w->cbeg[s], ((size_t)cap + 1) * sizeof(uint32_t)));
-        CKW(dev_alloc(&w->chunk[s], maxchunk * sizeof(uint2)));
-        if ((rc = scan_exclusive(len, w->offs[s], (uint64_t)n + 1, st))) return rc;
-        k_wide_fill<<<wblocks((uint64_t)n * 32, 256), 256, 0, st>>>(n, w->perm, w->inv, o, a, w->offs[s], w->adj[s]);
-        k_wide_chunks<<<wblocks((uint64_t)cap + 1, 256), 256, 0, st>>>(cap, meta, w->offs[s], chunk, w->cbeg[s]);
-        if ((rc = scan_exclusive(w->cbeg[s], w->cbeg[s], (uint64_t)cap + 1, st))) return rc;
-        k_wide_table<<<wblocks((uint64_t)cap * 32, 256), 256, 0, st>>>(cap, meta, s, w->cbeg[s], w->chunk[s]);
-        CKW(cudaGetLastError());
-    }
-    uint32_t h[8] = {};
-    CKW(cudaMemcpy(h, meta, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost));
-    CKW(cudaDeviceSynchronize());
-    if (!dir) {
-        h[7] = h[6];
-        w->offs[1] = w->offs[0]; w->adj[1] = w->adj[0]; w->cbeg[1] = w->cbeg[0]; w->chunk[1] = w->chunk[0];
-    }
-    WideSub &b = w->sub;
-    b.n = h[0];
-    b.nheavy = h[1];
-    for (int i = 0; i < 4; ++i) b.nmed[i] = h[2 + i];
-    b.chunk_len = chunk;
-    for (int s = 0; s < 2; ++s) {
-        b.nchunk[s] = h[6 + s];
-        b.offs[s] = w->offs[s];
-        b.adj[s] = w->adj[s];
-        b.chunk[s] = w->chunk[s];
-        b.cbeg[s] = w->cbeg[s];
-    }
-    b.vinfo = w->vinfo;
-    b.inv = w->inv;
-    return BCG_OK;
-}
-
 // Grows *p to bytes (the old buffer may be in use on any stream).
 static int grow(unsigned char **p, size_t *cap, size_t bytes) {
     if (*cap >= bytes) return BCG_OK;
-    CKW(cudaDeviceSynchronize());
+    if (*p) CKW(cudaDeviceSynchronize());
     dev_free(*p);
     *p = nullptr;
     *cap = 0;
     CKW(dev_alloc(p, bytes));
-    CKW(cudaDeviceSynchronize());
+    CKW(cudaStreamSynchronize(0));  // ready for any stream
     *cap = bytes;
     return BCG_OK;
 }
 
+WideInput wide_input(const bcg_graph *g) {
+    WideInput in{};
+    in.n = g->tile_n ? g->tile_n : g->n;
+    in.nnz = g->nnz_pruned;
+    in.offs = g->d_offs;
+    in.adj = g->d_adj;
+    in.vinfo = g->d_vinfo;
+    in.ext = g->d_ext;
+    in.directed = (g->flags & BCG_DIRECTED) != 0;
+    in.graphs = 1;
+    in.big_nnz = in.nnz;
+    return in;
+}
+
 int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, cudaStream_t st, WideResult *res) {
-    res->done = false;
+    *res = WideResult{};
     int rc;
-    if (!g->wide && (rc = wide_build(g))) {
-        wide_free(g);
-        return rc == BCG_ERR_OOM ? BCG_OK : rc;
+    // out of memory anywhere: the caller's other kernels need less
+    auto give_up = [](int code) { return code == BCG_ERR_OOM ? (cudaGetLastError(), BCG_OK) : code; };
+    if (!g->wide) {
+        g->wide = new WideGraph();
+        if ((rc = wide_form_make(g->wide->form, wide_input(g)))) {
+            wide_free(g);
+            return give_up(rc);
+        }
     }
     WideGraph *w = g->wide;
-    const WideSub &b = w->sub;
+    const WideSub &b = w->form.subs[0];
     const uint64_t njobs = (nroots + kWideSlots - 1) / kWideSlots;
-    int dev = 0, nsm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    // state of a team
-    const size_t n = b.n, words = (n + 31) / 32, nch = std::max(b.nchunk[0], b.nchunk[1]);
+    const size_t n = b.n;
     WideArgs a{};
-    size_t o = up256(n * 16);
-    a.o_done = o; o += up256(words * 4);
-    a.o_act = o; o += up256(words * 4 * kWideLevels);
-    a.o_sig = o; o += up256(n * 128);
-    a.o_g0 = o; o += up256(n * 128);
-    a.o_g1 = o; o += up256(n * 128);
-    a.o_part = o; o += up256(std::max<size_t>(1, nch) * 128);
-    a.o_hcnt = o; o += up256(std::max<size_t>(1, b.nheavy) * 4);
-    a.stride = o;
-    a.words = words;
-    // teams
-    uint64_t teams = std::min<uint64_t>(njobs, (uint64_t)nsm);
-    double budget = 128.0 * 1024 * 1024;
-    if (const char *e = getenv("BCG_WIDE_TEAM_MB")) budget = atof(e) * 1024 * 1024;
-    teams = std::max<uint64_t>(1, std::min<uint64_t>(teams, (uint64_t)(budget / (double)a.stride)));
-    a.teams = (uint32_t)teams;
-    a.team_ctas = (uint32_t)(nsm / teams);
+    wide_layout(a, n, std::max(b.nchunk[0], b.nchunk[1]), b.nheavy);
+    wide_teams(a, njobs, g->nnz_pruned);
     // jobs of one launch: their vectors stay under 512 MB
-    const uint64_t per = std::max<uint64_t>(teams, (512ull << 20) / (n * 8 + 1));
-    const uint64_t jl = std::min(per, njobs);
-    if ((rc = grow(&w->state, &w->state_cap, a.stride * teams)) ||
-        (rc = grow(reinterpret_cast<unsigned char **>(&w->jobbc), &w->jobbc_cap, jl * n * 8)))
-        return rc == BCG_ERR_OOM ? BCG_OK : rc;
-    // one upload: the sub, the jobs, the sources
-    const size_t o_jobs = up256(sizeof(WideSub)), o_mult = o_jobs + up256(njobs * sizeof(WideJob)),
-                 o_roots = o_mult + up256(nroots * 8), blob = o_roots + up256(nroots * 4);
-    std::vector<unsigned char> h(blob);
-    memcpy(h.data(), &b, sizeof(b));
-    WideJob *hj = reinterpret_cast<WideJob *>(h.data() + o_jobs);
-    for (uint64_t j = 0; j < njobs; ++j) {
-        hj[j] = WideJob{};
-        hj[j].root0 = (uint32_t)(j * kWideSlots);
-        hj[j].nroots = (uint32_t)std::min<uint64_t>(kWideSlots, nroots - j * kWideSlots);
-        hj[j].out = (j % jl) * n;
-    }
-    memcpy(h.data() + o_mult, mult, nroots * 8);
-    memcpy(h.data() + o_roots, roots, nroots * 4);
+    const uint64_t jl = std::min(njobs, std::max<uint64_t>(a.teams, (512ull << 20) / (n * 8 + 1)));
     // control words, teams, per-source totals: one block, cleared together
-    const size_t o_team = sizeof(WideCtrl), o_rstat = o_team + teams * sizeof(WideTeam),
+    const size_t o_team = sizeof(WideCtrl), o_rstat = o_team + a.teams * sizeof(WideTeam),
                  stat = o_rstat + njobs * kWideSlots * sizeof(RootStat);
-    if ((rc = grow(&w->blob, &w->blob_cap, blob)) || (rc = grow(&w->stat, &w->stat_cap, stat)))
-        return rc == BCG_ERR_OOM ? BCG_OK : rc;
+    const size_t o_roots = up256(nroots * 8), blob = o_roots + up256(nroots * 4);
+    if ((rc = grow(&w->state, &w->state_cap, a.stride * a.teams)) ||
+        (rc = grow(reinterpret_cast<unsigned char **>(&w->jobbc), &w->jobbc_cap, jl * n * 8)) ||
+        (rc = grow(&w->blob, &w->blob_cap, blob)) || (rc = grow(&w->stat, &w->stat_cap, stat)))
+        return give_up(rc);
+    std::vector<unsigned char> h(blob), hs(stat);
+    memcpy(h.data(), mult, nroots * 8);
+    memcpy(h.data() + o_roots, roots, nroots * 4);
     CKW(cudaMemcpyAsync(w->blob, h.data(), blob, cudaMemcpyHostToDevice, st));
-    a.subs = reinterpret_cast<const WideSub *>(w->blob);
-    a.mult = reinterpret_cast<const double *>(w->blob + o_mult);
+    a.subs = w->form.d_subs;
+    a.nroots = (uint32_t)nroots;
+    a.mult = reinterpret_cast<const double *>(w->blob);
     a.roots = reinterpret_cast<const uint32_t *>(w->blob + o_roots);
     a.jobbc = w->jobbc;
     a.state = w->state;
@@ -1285,11 +1108,11 @@ int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t n
         a.trace_cap = 1u << 20;
         CKW(dev_alloc(&d_trace, a.trace_cap * sizeof(TraceRec)));
         CKW(dev_alloc(&d_tcnt, sizeof(unsigned int)));
-        CKW(cudaMemsetAsync(d_tcnt, 0, sizeof(unsigned int), st));
+        CKW(cudaMemsetAsync(d_tcnt, 0, sizeof(unsigned int), 0));
+        CKW(cudaStreamSynchronize(0));
         a.trace = d_trace;
         a.trace_cnt = d_tcnt;
     }
-    std::vector<unsigned char> hs(stat);
     CKW(cudaMemsetAsync(w->stat, 0, stat, st));
     CKW(cudaEventRecord(g->ev0, st));
     // The jobs are added into bc on the device only if none of them stopped.
@@ -1302,15 +1125,11 @@ int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t n
     const WideCtrl *c = reinterpret_cast<const WideCtrl *>(hs.data());
     for (uint64_t j0 = 0; j0 < njobs; j0 += jl) {
         a.njobs = (uint32_t)std::min(jl, njobs - j0);
-        a.jobs = reinterpret_cast<const WideJob *>(w->blob + o_jobs) + j0;
+        a.job0 = (uint32_t)j0;
         a.rstat = reinterpret_cast<RootStat *>(w->stat + o_rstat) + j0 * kWideSlots;
         if (j0) CKW(cudaMemsetAsync(w->stat, 0, o_rstat, st));
-        void *params[] = {&a};
-        CKW(cudaLaunchCooperativeKernel((const void *)bc_wide_kernel, dim3(a.teams * a.team_ctas), dim3(kWideThreads),
-                                        params, 0, st));
-        WideOut out{0, a.njobs, (uint32_t)n, w->map, g->d_bc};
-        k_wide_reduce<<<wblocks(n, 32), 256, 0, st>>>(a.ctrl, nullptr, out, w->jobbc);
-        CKW(cudaGetLastError());
+        if ((rc = wide_enqueue(a, nullptr, 1, WideOut{0, a.njobs, (uint32_t)n, w->form.map, g->d_bc}, (uint32_t)n, st)))
+            return rc;
         res->launches += 2;
         const bool last = j0 + a.njobs >= njobs;
         if (last) CKW(cudaEventRecord(g->ev1, st));
@@ -1320,7 +1139,6 @@ int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t n
     }
     if (d_trace) {
         unsigned int cnt = 0;
-        CKW(cudaStreamSynchronize(st));
         CKW(cudaMemcpy(&cnt, d_tcnt, sizeof(cnt), cudaMemcpyDeviceToHost));
         std::vector<TraceRec> recs(cnt);
         if (cnt) CKW(cudaMemcpy(recs.data(), d_trace, cnt * sizeof(TraceRec), cudaMemcpyDeviceToHost));

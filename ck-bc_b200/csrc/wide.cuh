@@ -4,7 +4,11 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "engine.cuh"
+
+struct bcg_graph;
 
 namespace bcg {
 
@@ -25,9 +29,11 @@ struct WideSub {
     uint32_t n, nheavy, chunk_len, pad;
     uint32_t nmed[4];
     uint32_t nchunk[2];
-    const uint32_t *offs[2], *adj[2];
-    const uint2 *chunk[2];     // {vertex, index of the chunk within it}
-    const uint32_t *cbeg[2];   // nheavy + 1: first chunk of a heavy vertex
+    uint32_t base, pad2;       // the graph's first position in its union
+    uint32_t chunk0[2];        // its first chunk there
+    const uint32_t *offs[2], *adj[2];  // entries from offs[..][v] on in adj
+    const uint2 *chunk[2];     // {union position of the vertex, index of the chunk within it}
+    const uint32_t *cbeg[2];   // first chunk (of the union's) of a vertex
     const uint2 *vinfo;        // {out-degree, reach}
     const uint32_t *inv;       // the engine's vertex id -> this numbering
 };
@@ -58,13 +64,17 @@ static_assert(sizeof(WideCtrl) == 128, "one line");
 
 struct WideArgs {
     const WideSub *subs;
-    const WideJob *jobs;
-    uint32_t njobs;
+    const WideJob *jobs;    // nullptr: subs[0]'s sources roots[0 .. nroots) in order, from job job0 on,
+                            // job j's vector at j * n
+    uint32_t njobs, job0, nroots;
     uint32_t teams, team_ctas;
     const uint32_t *roots;  // engine ids, by WideJob::root0
-    const double *mult;
+    const double *mult;     // weights, likewise (nullptr: 1)
     double *jobbc;
-    RootStat *rstat;        // njobs * 16, zeroed
+    int *poison;            // several launches' stop word (nullptr: none): set by a launch that
+                            // stops, and a launch that finds it set does nothing
+    RootStat *rstat;        // njobs * 16, zeroed (nullptr: not wanted)
+    RootStat *total;        // or the sums over all sources, and the deepest level (zeroed)
     WideCtrl *ctrl;
     WideTeam *team;
     // per-team state, each array sized for the launch's largest graph
@@ -76,5 +86,61 @@ struct WideArgs {
     unsigned int trace_cap;
     unsigned int *trace_cnt;
 };
+
+// Adding the jobs of a graph: bc[map[v]] += sum over j < njobs of
+// jobbc[out0 + j * n + v].
+struct WideOut {
+    unsigned long long out0;
+    uint32_t njobs, n;
+    const uint32_t *map;
+    double *bc;
+};
+
+// The lists a wide form is made from (device arrays; vinfo and ext by engine
+// id, ext nullptr: bc is indexed by engine id).  A union of several graphs has
+// base[graphs + 1] (host), the first vertex of each.
+struct WideInput {
+    uint32_t n;
+    uint64_t nnz;
+    const uint32_t *offs, *adj;
+    const uint2 *vinfo;
+    const uint32_t *ext;
+    bool directed;
+    const uint32_t *base;
+    uint32_t graphs;
+    uint64_t big_nnz;  // entries of the largest graph
+};
+
+WideInput wide_input(const bcg_graph *g);  // of a graph's searched lists
+
+// A graph's (or union's) lists in the wide numbering.
+struct WideForm {
+    unsigned char *mem = nullptr;  // everything below on the device (nullptr: the caller's memory)
+    WideSub *d_subs = nullptr;     // one a graph
+    uint32_t *inv = nullptr, *map = nullptr;
+    std::vector<WideSub> subs;     // the host's copy (wide_form_make)
+};
+
+// Bytes of a form, and of the scratch that building it takes.
+size_t wide_form_bytes(const WideInput &in, size_t *scratch);
+// Enqueues the building in memory of that size on st; f.subs stays empty.
+int wide_form_enqueue(WideForm &f, const WideInput &in, unsigned char *mem, unsigned char *scratch, cudaStream_t st);
+// Allocates, builds on stream 0 and waits.
+int wide_form_make(WideForm &f, const WideInput &in);
+void wide_form_free(WideForm &f);
+
+// Fills a's state layout for graphs of up to n vertices; returns the stride.
+size_t wide_layout(WideArgs &a, size_t n, size_t nchunk, size_t nheavy);
+// Whether a graph with so many vertices that have an entry, and so many
+// entries, is shallow enough to be tried: mean degree 6 and up, or too few
+// vertices for more levels than a job holds.
+inline bool wide_shallow(uint64_t active, uint64_t nnz) { return nnz >= 6 * active || active + 2 < kWideLevels; }
+// Cuts the SMs into teams for njobs jobs on lists of so many entries (their
+// mean), a's layout being set.
+void wide_teams(WideArgs &a, uint64_t njobs, uint64_t entries);
+// One launch of a's jobs and the adding of their vectors: nouts entries of
+// outs (device; nmax vertices at most), or `one` when outs is nullptr.
+int wide_enqueue(const WideArgs &a, const WideOut *outs, uint32_t nouts, const WideOut &one, uint32_t nmax,
+                 cudaStream_t st);
 
 }  // namespace bcg

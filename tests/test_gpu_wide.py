@@ -121,3 +121,45 @@ def test_deep_search_leaves():
         assert_bc_close(G.bc(), ref, "deep")
         G.run(src)
         assert_bc_close(G.bc(), 2 * ref, "deep twice")
+
+
+def test_batch_of_shallow_graphs():
+    """A set that runs as wide searches: one to several jobs a graph, graphs of
+    one sorting block and of several, with an edgeless one, twice in a row."""
+    specs = ["rmat:scale=12,ef=16,a=0.57,b=0.19,c=0.19,seed=5", "er:scale=8,ef=8,seed=6", "er:scale=6,ef=6,seed=9",
+             "rmat:scale=9,ef=16,seed=11"]
+    graphs = [bcg.generate(s) for s in specs]
+    graphs += [bcg.from_pairs([[0, 1], [1, 2], [2, 3]], 5), (np.zeros(4, np.uint32), np.zeros(0, np.uint32))]
+    with bcg.Batch(graphs) as B:
+        for runs in (1, 2):
+            st = B.run()
+            assert st.batch_width == 16 and B.info()["captured"]
+            edges = 0
+            for i, (offs, adj) in enumerate(graphs):
+                ref, ost = oracle.bc(offs, adj, np.arange(len(offs) - 1), nthreads=oracle.max_threads())
+                assert_bc_close(B.bc(i), runs * ref, f"graph {i}")
+                edges += ost["teps_edges"]
+            assert st.teps_edges == edges
+
+
+def _cliques(size, count):
+    """Cliques in a row, neighbours joined by one edge: deep, one path a pair."""
+    pairs = []
+    for c in range(count):
+        b = c * size
+        pairs += [[b + i, b + j] for i in range(size) for j in range(i)]
+        if c:
+            pairs.append([b - 1, b])
+    return bcg.from_pairs(pairs, size * count)
+
+
+def test_batch_with_a_deep_graph():
+    """One graph of mean degree 7 and more than 62 levels: the packed schedule runs the set."""
+    graphs = [bcg.generate("er:scale=8,ef=8,seed=6"), _cliques(8, 60)]
+    with bcg.Batch(graphs) as B:
+        for runs in (1, 2):
+            st = B.run()
+            assert st.batch_width != 16 and st.max_depth > 62
+            for i, (offs, adj) in enumerate(graphs):
+                ref, _ = oracle.bc(offs, adj, np.arange(len(offs) - 1), nthreads=oracle.max_threads())
+                assert_bc_close(B.bc(i), runs * ref, f"graph {i}")

@@ -22,6 +22,19 @@
 // result is bitwise the same alone or in any mix.  S is 6 while the active graphs' 64-byte state rows
 // fit 64 MB (they then stay in L2), else 3.
 //
+// Wide waves.  A pool of shallow graphs (wide_shallow) runs its waves as
+// wide-batch searches (wide.cu) instead: a request's sources in its own order,
+// 16 a job, up to wave_batches jobs of a graph a wave; the jobs of graphs of
+// like size share a launch, in which a CTA or a few take a job.  Every job's
+// vector is added to its request's buffer in the request's job order, and a
+// job's sums do not depend on the launch, so here too the result is the same
+// alone or in any mix.  (24 requests, half exact, on ten graphs of 1,000 to
+// 30,000 vertices: 228 ms as packed waves, which pay barriers of the whole chip
+// for every sweep; 10 ms as wide ones.)  Nothing of a wave is added unless
+// all of its launches went through; a search of more than 62 levels stops it
+// and the waves behind it, their sources are taken back, and the pool is
+// served in packed waves from then on.
+//
 // Continuity.  bcg_server_step never waits for the GPU: it retires the waves
 // that have finished (their requests become done), admits what fits, and
 // keeps up to two waves queued on the server's stream, so the next wave is
@@ -30,6 +43,7 @@
 // threads may submit while a wave is on the GPU: such a request is admitted
 // at once if its buffer fits and joins the next wave that is planned.
 #include <algorithm>
+#include <cstring>
 #include <deque>
 #include <mutex>
 #include <unordered_map>
@@ -37,6 +51,7 @@
 
 #include "bcg_common.hpp"
 #include "engine_internal.hpp"
+#include "wide.cuh"
 
 using namespace bcg;
 
@@ -66,6 +81,11 @@ struct ServeWave {
     cudaEvent_t ev = nullptr;
     bool busy = false;
     std::vector<uint64_t> finishing;
+    // wide waves: jobs, sources and outputs; control words (and their copy)
+    unsigned char *h_jobs = nullptr, *d_jobs = nullptr, *d_stat = nullptr;
+    WideCtrl *h_ctrl = nullptr;
+    uint32_t spans = 0;                                   // launches of the wave (0: a packed wave)
+    std::vector<std::pair<uint64_t, size_t>> taken;       // requests and their sched before the wave
 };
 
 struct bcg_server {
@@ -91,6 +111,15 @@ struct bcg_server {
     double *d_slot_delta = nullptr;  // width * n per-slot dependencies of a batch
     uint64_t waves = 0;
     int sticky_error = BCG_OK;  // a failed wave leaves the server unusable
+    // wide waves
+    bool wide = false, packed = false;  // packed: the packed waves' buffers are there
+    WideForm form;
+    unsigned char *d_wstate = nullptr;
+    size_t wstate_bytes = 0;
+    double *d_jobbc = nullptr;
+    uint64_t cells = 0;          // doubles of d_jobbc: a wave's job vectors
+    int *d_poison = nullptr;
+    size_t off_wroots = 0, off_wouts = 0, wblob_bytes = 0;
 };
 
 namespace {
@@ -126,6 +155,219 @@ int admit(bcg_server *s) {
     return BCG_OK;
 }
 
+// Buffers of the packed waves.
+int packed_setup(bcg_server *s) {
+    const int rc = ensure_state(s->g, s->width);
+    if (rc) return rc;
+    if (cudaMalloc(&s->d_slot_delta, (size_t)s->width * s->g->n * sizeof(double)) != cudaSuccess)
+        return set_error(BCG_ERR_OOM, "per-slot dependency buffer");
+    for (ServeWave &w : s->slot) {
+        cudaError_t e;
+        if ((e = cudaMalloc(&w.d_blob, s->blob_bytes)) != cudaSuccess ||
+            (e = cudaMallocHost(&w.h_blob, s->blob_bytes)) != cudaSuccess ||
+            (e = cudaMalloc(&w.d_rstat, (size_t)s->wave_batches * s->width * sizeof(RootStat))) != cudaSuccess)
+            return set_error(BCG_ERR_CUDA, "server buffers: %s", cudaGetErrorString(e));
+    }
+    s->packed = true;
+    return BCG_OK;
+}
+
+constexpr uint32_t kMaxSpans = 8;  // launches of a wide wave
+
+void wide_clear(bcg_server *s) {
+    wide_form_free(s->form);
+    dev_free(s->d_wstate);
+    dev_free(s->d_jobbc);
+    s->d_wstate = nullptr;
+    s->d_jobbc = nullptr;
+    for (ServeWave &w : s->slot) {
+        dev_free(w.d_jobs);
+        dev_free(w.d_stat);
+        if (w.h_jobs) cudaFreeHost(w.h_jobs);
+        if (w.h_ctrl) cudaFreeHost(w.h_ctrl);
+        w.d_jobs = w.d_stat = w.h_jobs = nullptr;
+        w.h_ctrl = nullptr;
+    }
+    s->wide = false;
+}
+
+// Sets up the wide waves (s->wide = true) if every graph of the pool is
+// shallow and their buffers fit the budget beside the packed waves' (which a
+// deep search may still need).
+int wide_setup(bcg_server *s) {
+    bcg_graph *g = s->g;
+    const uint32_t G = s->ngraphs;
+    WideInput in = wide_input(g);
+    std::vector<uint32_t> ubase(s->base);  // the union keeps the caller's order
+    ubase.push_back(g->n);
+    in.graphs = G;
+    in.base = ubase.data();
+    in.big_nnz = 0;
+    uint32_t nmax = 1;
+    for (uint32_t i = 0; i < G; ++i) {
+        uint64_t act = 0;
+        for (uint32_t v = ubase[i]; v < ubase[i + 1]; ++v) act += s->hdeg[v] != 0;
+        if (!wide_shallow(act, s->gnnz[i])) return BCG_OK;
+        in.big_nnz = std::max<uint64_t>(in.big_nnz, s->gnnz[i]);
+        nmax = std::max(nmax, (uint32_t)act);
+    }
+    if (g->n >= (1u << 28)) return BCG_OK;
+    // a team's state for the largest graph, and up to 256 MB for more teams;
+    // job vectors for a wave of 148 of the largest graph's jobs, up to 256 MB
+    // (one at least)
+    WideArgs a{};
+    const size_t stride = wide_layout(a, nmax, in.big_nnz / kWideChunk * 2 + 1, in.big_nnz / kWideChunk + 1);
+    s->wstate_bytes = std::max(stride, std::min<size_t>(148 * stride, 256ull << 20));
+    s->cells = std::max<uint64_t>(nmax, std::min<uint64_t>(148ull * 8 * nmax, (256ull << 20) / 8));
+    const size_t jobs = (size_t)s->wave_batches * G;
+    s->off_wroots = up16(jobs * sizeof(WideJob));
+    s->off_wouts = s->off_wroots + up16(jobs * kWideSlots * 4);
+    s->wblob_bytes = s->off_wouts + jobs * sizeof(WideOut);
+    const size_t stat = kMaxSpans * (sizeof(WideCtrl) + kWideTeams * sizeof(WideTeam));
+    size_t scratch = 0;
+    const uint64_t extra =
+        wide_form_bytes(in, &scratch) + s->wstate_bytes + s->cells * 8 + kInFlight * (s->wblob_bytes + stat);
+    if (s->resident + extra + scratch > s->budget) return BCG_OK;
+    int rc = wide_form_make(s->form, in);
+    cudaError_t e = cudaSuccess;
+    if (!rc && ((e = dev_alloc(&s->d_wstate, s->wstate_bytes)) != cudaSuccess ||
+                (e = dev_alloc(&s->d_jobbc, s->cells * 8)) != cudaSuccess ||
+                (!s->d_poison && (e = cudaMalloc(&s->d_poison, sizeof(int))) != cudaSuccess) ||
+                (e = cudaMemset(s->d_poison, 0, sizeof(int))) != cudaSuccess))
+        rc = set_error(e == cudaErrorMemoryAllocation ? BCG_ERR_OOM : BCG_ERR_CUDA, "wide waves: %s", cudaGetErrorString(e));
+    for (ServeWave &w : s->slot)
+        if (!rc && ((e = dev_alloc(&w.d_jobs, s->wblob_bytes)) != cudaSuccess ||
+                    (e = cudaMallocHost(&w.h_jobs, s->wblob_bytes)) != cudaSuccess ||
+                    (e = dev_alloc(&w.d_stat, stat)) != cudaSuccess ||
+                    (e = cudaMallocHost(&w.h_ctrl, kMaxSpans * sizeof(WideCtrl))) != cudaSuccess))
+            rc = set_error(e == cudaErrorMemoryAllocation ? BCG_ERR_OOM : BCG_ERR_CUDA, "wide waves: %s", cudaGetErrorString(e));
+    CKS(cudaDeviceSynchronize());  // the buffers are ready for the server's stream
+    if (rc) {
+        wide_clear(s);
+        return rc == BCG_ERR_OOM ? (cudaGetLastError(), BCG_OK) : rc;
+    }
+    s->resident += extra;
+    s->wide = true;
+    return BCG_OK;
+}
+
+// A deep search stopped the oldest wave: nothing of it or of the waves behind
+// it was added.  Takes their sources back and goes on in packed waves.
+int take_back(bcg_server *s) {
+    CKS(cudaStreamSynchronize(s->stream));
+    for (auto it = s->inflight.rbegin(); it != s->inflight.rend(); ++it) {
+        ServeWave &w = s->slot[*it];
+        for (auto t = w.taken.rbegin(); t != w.taken.rend(); ++t) s->reqs[t->first].sched = t->second;
+        w.taken.clear();
+        w.finishing.clear();
+        w.busy = false;
+    }
+    s->inflight.clear();
+    // every admitted request that is not done, in admission order (ids ascend)
+    std::vector<uint64_t> ids;
+    for (auto &kv : s->reqs)
+        if (kv.second.d_out && !kv.second.done) ids.push_back(kv.first);
+    std::sort(ids.begin(), ids.end());
+    for (auto &q : s->queue) q.clear();
+    for (uint64_t id : ids) s->queue[s->reqs[id].graph].push_back(id);
+    wide_clear(s);
+    return packed_setup(s);
+}
+
+// Plans the next wide wave and enqueues it (enqueue_wave's wide form).
+int enqueue_wide_wave(bcg_server *s, ServeWave &w, int wi, bool *launched) {
+    std::vector<uint32_t> act;
+    for (uint32_t gi = 0; gi < s->ngraphs; ++gi)
+        if (!s->queue[gi].empty()) act.push_back(gi);
+    if (act.empty()) return BCG_OK;
+    // largest graphs first: graphs of like size share a launch
+    std::stable_sort(act.begin(), act.end(), [&](uint32_t x, uint32_t y) { return s->form.subs[x].n > s->form.subs[y].n; });
+    WideJob *jobs = reinterpret_cast<WideJob *>(w.h_jobs);
+    uint32_t *roots = reinterpret_cast<uint32_t *>(w.h_jobs + s->off_wroots);
+    WideOut *outs = reinterpret_cast<WideOut *>(w.h_jobs + s->off_wouts);
+    struct Span { uint32_t job0, njobs, nmax, nch, nheavy; uint64_t entries; };
+    std::vector<Span> spans;
+    uint32_t nj = 0, nr = 0, no = 0, nmax = 1;
+    uint64_t cells = 0;
+    w.finishing.clear();
+    w.taken.clear();
+    for (uint32_t gi : act) {
+        const WideSub &sub = s->form.subs[gi];
+        auto &q = s->queue[gi];
+        uint32_t used = 0;  // jobs of this graph
+        while (!q.empty()) {
+            Req &r = s->reqs[q.front()];
+            const size_t left = r.src.size() - r.sched;
+            const uint32_t take = (uint32_t)std::min<uint64_t>({(left + kWideSlots - 1) / kWideSlots,
+                                                                (uint64_t)s->wave_batches - used,
+                                                                sub.n ? (s->cells - cells) / sub.n : 0});
+            if (left && !take) break;  // the wave is full (for this graph)
+            w.taken.emplace_back(q.front(), r.sched);
+            if (take) {
+                if (spans.empty() || (sub.n < spans.back().nmax / 4 && spans.back().njobs >= 2 * 148 && spans.size() < kMaxSpans))
+                    spans.push_back(Span{nj, 0, sub.n, 1, 1, 0});
+                Span &l = spans.back();
+                l.nch = std::max({l.nch, sub.nchunk[0], sub.nchunk[1]});
+                l.nheavy = std::max(l.nheavy, sub.nheavy);
+                nmax = std::max(nmax, sub.n);
+                // (the map gives union ids: the buffer is addressed from the union's start)
+                double *out = reinterpret_cast<double *>(reinterpret_cast<uintptr_t>(r.d_out) -
+                                                         (uintptr_t)s->base[gi] * sizeof(double));
+                outs[no++] = WideOut{cells, take, sub.n, s->form.map + sub.base, out};
+                for (uint32_t j = 0; j < take; ++j) {
+                    const uint32_t k = (uint32_t)std::min<size_t>(kWideSlots, r.src.size() - r.sched);
+                    jobs[nj++] = WideJob{gi, nr, k, 0, cells};
+                    for (uint32_t i = 0; i < k; ++i) roots[nr++] = r.src[r.sched + i];
+                    r.sched += k;
+                    cells += sub.n;
+                    ++l.njobs;
+                    l.entries += s->gnnz[gi];
+                }
+                used += take;
+            }
+            if (r.sched < r.src.size()) break;
+            w.finishing.push_back(q.front());
+            q.pop_front();
+        }
+    }
+    w.spans = std::max<uint32_t>(1, (uint32_t)spans.size());
+    memset(w.h_ctrl, 0, kMaxSpans * sizeof(WideCtrl));
+    if (nj) {
+        // (one copy up to the last output that is used)
+        CKS(cudaMemcpyAsync(w.d_jobs, w.h_jobs, s->off_wroots + (size_t)nr * 4, cudaMemcpyHostToDevice, s->stream));
+        CKS(cudaMemcpyAsync(w.d_jobs + s->off_wouts, w.h_jobs + s->off_wouts, no * sizeof(WideOut), cudaMemcpyHostToDevice,
+                            s->stream));
+        CKS(cudaMemsetAsync(w.d_stat, 0, kMaxSpans * (sizeof(WideCtrl) + kWideTeams * sizeof(WideTeam)), s->stream));
+        WideArgs a{};
+        for (size_t k = 0; k < spans.size(); ++k) {
+            const Span &l = spans[k];
+            wide_layout(a, l.nmax, l.nch, l.nheavy);
+            wide_teams(a, l.njobs, l.entries / l.njobs, s->wstate_bytes);
+            a.subs = s->form.d_subs;
+            a.jobs = reinterpret_cast<const WideJob *>(w.d_jobs) + l.job0;
+            a.njobs = l.njobs;
+            a.split_ctas = 4;
+            a.roots = reinterpret_cast<const uint32_t *>(w.d_jobs + s->off_wroots);
+            a.jobbc = s->d_jobbc;
+            a.poison = s->d_poison;
+            a.ctrl = reinterpret_cast<WideCtrl *>(w.d_stat) + k;
+            a.team = reinterpret_cast<WideTeam *>(w.d_stat + kMaxSpans * sizeof(WideCtrl)) + k * kWideTeams;
+            a.state = s->d_wstate;
+            const int rc = wide_enqueue(a, nullptr, 0, WideOut{}, 1, s->stream);
+            if (rc) return rc;
+        }
+        const int rc = wide_chain(a, reinterpret_cast<const WideOut *>(w.d_jobs + s->off_wouts), no, nmax, s->stream);
+        if (rc) return rc;
+        CKS(cudaMemcpyAsync(w.h_ctrl, w.d_stat, kMaxSpans * sizeof(WideCtrl), cudaMemcpyDeviceToHost, s->stream));
+    }
+    CKS(cudaEventRecord(w.ev, s->stream));
+    w.busy = true;
+    s->inflight.push_back(wi);
+    ++s->waves;
+    *launched = true;
+    return BCG_OK;
+}
+
 // Retires the finished waves at the front of the queue (wait: block for the
 // oldest one first).
 int retire(bcg_server *s, bool wait) {
@@ -138,6 +380,17 @@ int retire(bcg_server *s, bool wait) {
             const cudaError_t q = cudaEventQuery(w.ev);
             if (q == cudaErrorNotReady) break;
             if (q != cudaSuccess) return set_error(BCG_ERR_CUDA, "wave event: %s", cudaGetErrorString(q));
+        }
+        if (w.spans) {
+            int error = 0, overflow = 0, deep = 0;
+            for (uint32_t k = 0; k < w.spans; ++k) {
+                error = w.h_ctrl[k].error ? w.h_ctrl[k].error : error;
+                overflow |= w.h_ctrl[k].overflow;
+                deep |= w.h_ctrl[k].deep;
+            }
+            if (deep && !error && !overflow) return take_back(s);
+            w.h_flags[0] = error;
+            w.h_flags[1] = overflow;
         }
         if (w.h_flags[1] || w.h_flags[0] == BCG_ERR_OVERFLOW) {
             s->sticky_error = BCG_ERR_OVERFLOW;
@@ -168,6 +421,8 @@ int enqueue_wave(bcg_server *s, bool *launched) {
         if (!s->slot[i].busy) { wi = i; break; }
     if (wi < 0) return BCG_OK;
     const uint32_t G = s->ngraphs, W = s->wave_batches;
+    if (s->wide) return enqueue_wide_wave(s, s->slot[wi], wi, launched);
+    s->slot[wi].spans = 0;
     // the graphs with work, and their active vertices (for the width rule)
     std::vector<uint32_t> act;
     uint64_t act_n = 0;
@@ -344,15 +599,7 @@ int bcg_server_create(uint32_t ngraphs, const uint32_t *const *offsets, const ui
     for (uint32_t gi = 1; gi < ngraphs; ++gi)
         if (s->grange[gi].x < s->grange[gi - 1].x)
             return fail(set_error(BCG_ERR_ARG, "the pool union does not keep the graphs in caller order"));
-    rc = ensure_state(s->g, s->width);
-    if (rc) return fail(rc);
-    if (cudaMalloc(&s->d_slot_delta, (size_t)s->width * s->g->n * sizeof(double)) != cudaSuccess)
-        return fail(set_error(BCG_ERR_OOM, "per-slot dependency buffer"));
     s->budget = hbm_budget_bytes;
-    s->resident = pool_bytes(s->g, s->width) + (uint64_t)s->width * s->g->n * sizeof(double);
-    if (s->resident > s->budget)
-        return fail(set_error(BCG_ERR_OOM, "the resident pool needs %llu bytes, over the %llu-byte budget",
-                              (unsigned long long)s->resident, (unsigned long long)s->budget));
     // wave schedule regions (a wave has at most wave_batches batches, each
     // with every graph active)
     const size_t W = wave_batches, G = ngraphs, S = s->width, R = W * G * S;
@@ -367,19 +614,22 @@ int bcg_server_create(uint32_t ngraphs, const uint32_t *const *offsets, const ui
     s->off_xrange = o; o += up16(W * G * 8);
     s->off_xout = o; o += up16(W * G * sizeof(SlotOut));
     s->blob_bytes = o;
+    s->resident = pool_bytes(s->g, s->width) + (uint64_t)s->width * s->g->n * sizeof(double);
+    if (s->resident > s->budget)
+        return fail(set_error(BCG_ERR_OOM, "the resident pool needs %llu bytes, over the %llu-byte budget",
+                              (unsigned long long)s->resident, (unsigned long long)s->budget));
+    s->resident += kInFlight * (o + W * S * sizeof(RootStat));
     cudaError_t e;
     if ((e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&s->result_stream, cudaStreamNonBlocking)) != cudaSuccess)
         return fail(set_error(BCG_ERR_CUDA, "server streams: %s", cudaGetErrorString(e)));
-    for (int i = 0; i < kInFlight; ++i) {
-        ServeWave &w = s->slot[i];
-        if ((e = cudaMalloc(&w.d_blob, o)) != cudaSuccess || (e = cudaMallocHost(&w.h_blob, o)) != cudaSuccess ||
-            (e = cudaMalloc(&w.d_rstat, W * S * sizeof(RootStat))) != cudaSuccess ||
-            (e = cudaMallocHost(&w.h_flags, 2 * sizeof(int))) != cudaSuccess ||
+    for (ServeWave &w : s->slot)
+        if ((e = cudaMallocHost(&w.h_flags, 2 * sizeof(int))) != cudaSuccess ||
             (e = cudaEventCreateWithFlags(&w.ev, cudaEventDisableTiming)) != cudaSuccess)
             return fail(set_error(BCG_ERR_CUDA, "server buffers: %s", cudaGetErrorString(e)));
-        s->resident += o + W * S * sizeof(RootStat);
-    }
+    rc = wide_setup(s);
+    if (!rc && !s->wide) rc = packed_setup(s);
+    if (rc) return fail(rc);
     *out = s;
     return BCG_OK;
 }
@@ -393,6 +643,8 @@ int bcg_server_destroy(bcg_server *s) {
         if (s->result_stream) cudaStreamSynchronize(s->result_stream);
         for (auto &kv : s->reqs)
             if (kv.second.d_out) cudaFree(kv.second.d_out);
+        wide_clear(s);
+        if (s->d_poison) cudaFree(s->d_poison);
         for (ServeWave &w : s->slot) {
             cudaFree(w.d_blob);
             cudaFree(w.d_rstat);

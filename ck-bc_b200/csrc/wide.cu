@@ -721,7 +721,8 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
         if (threadIdx.x == 0) {
             // four lanes take a vertex while its blocks are no more than
             // about half of a warp's share of a sweep
-            const uint32_t blocks = (sm.sub.offs[1][sm.sub.n] - sm.sub.offs[1][0]) / (128u * x.T * kWideWarps);
+            const uint32_t share = 128u * kWideWarps * (a.split_ctas ? a.split_ctas : x.T);
+            const uint32_t blocks = (sm.sub.offs[1][sm.sub.n] - sm.sub.offs[1][0]) / share;
             sm.nmed = sm.sub.nmed[blocks >= 32 ? 3 : (blocks >= 16 ? 2 : (blocks >= 8 ? 1 : 0))];
         }
         if (threadIdx.x < kWideSlots) {
@@ -948,6 +949,22 @@ __global__ void __launch_bounds__(256) k_wide_reduce(const WideCtrl *__restrict_
     }
 }
 
+// The same in strict job order, so that the bits do not depend on how the
+// jobs of a graph are spread over launches.
+__global__ void __launch_bounds__(256) k_wide_chain(const int *__restrict__ poison, const WideOut *__restrict__ outs,
+                                                    const double *__restrict__ jobbc) {
+    if (*poison) return;
+    const WideOut o = outs[blockIdx.y];
+    for (uint32_t v = blockIdx.x * 256 + threadIdx.x; v < o.n; v += gridDim.x * 256) {
+        const double *q = jobbc + o.out0 + v;
+        double *b = o.bc + o.map[v];
+        double s = *b;
+#pragma unroll 4
+        for (uint32_t j = 0; j < o.njobs; ++j) s += __ldcs(q + (size_t)j * o.n);
+        *b = s;
+    }
+}
+
 #define CKW(call)                                                                                  \
     do {                                                                                           \
         cudaError_t e_ = (call);                                                                   \
@@ -975,7 +992,7 @@ size_t wide_layout(WideArgs &a, size_t n, size_t nchunk, size_t nheavy) {
     return o;
 }
 
-void wide_teams(WideArgs &a, uint64_t njobs, uint64_t entries) {
+void wide_teams(WideArgs &a, uint64_t njobs, uint64_t entries, size_t state_bytes) {
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -984,11 +1001,11 @@ void wide_teams(WideArgs &a, uint64_t njobs, uint64_t entries) {
     // rows are well beyond L2 (fitted on 16-source jobs of R-MAT graphs: 0.1 M
     // entries 540 us on 1 CTA; 7.1 M entries 6,050 us on 13 and 590 us on 148;
     // 30 M entries 8,800 us on 29 and 1,590 us on 148).  The number of teams
-    // that ends first, its states within 1 GiB.
+    // that ends first, its states within state_bytes.
     constexpr double kFixed = 70.0, kEntry = 0.009, kBeyond = 1.1;
     double best = 0.0;
-    for (uint64_t t = 1; t <= std::min<uint64_t>(njobs, (uint64_t)nsm); ++t) {
-        if (t > 1 && (double)a.stride * (double)t > 1024.0 * 1024 * 1024) break;
+    for (uint64_t t = 1; t <= std::min<uint64_t>({njobs, (uint64_t)nsm, kWideTeams}); ++t) {
+        if (t > 1 && a.stride * t > state_bytes) break;
         const double rows = (double)t * (double)a.words * 32.0 * 128.0;
         const double job = kFixed + (double)entries * kEntry * (rows > 126e6 ? kBeyond : 1.0) / (double)(nsm / t);
         const double all = (double)((njobs + t - 1) / t) * job;
@@ -1011,6 +1028,14 @@ int wide_enqueue(const WideArgs &a, const WideOut *outs, uint32_t nouts, const W
     for (uint32_t o = 0; o < nouts; o += 65535u)
         k_wide_reduce<<<dim3(bx, std::min(65535u, nouts - o)), 256, 0, st>>>(a.ctrl, a.poison, outs ? outs + o : nullptr,
                                                                            one, a.jobbc);
+    CKW(cudaGetLastError());
+    return BCG_OK;
+}
+
+int wide_chain(const WideArgs &a, const WideOut *outs, uint32_t nouts, uint32_t nmax, cudaStream_t st) {
+    const unsigned bx = (unsigned)std::max<size_t>(1, std::min<size_t>(1024, ((size_t)nmax + 255) / 256));
+    for (uint32_t o = 0; o < nouts; o += 65535u)
+        k_wide_chain<<<dim3(bx, std::min(65535u, nouts - o)), 256, 0, st>>>(a.poison, outs + o, a.jobbc);
     CKW(cudaGetLastError());
     return BCG_OK;
 }

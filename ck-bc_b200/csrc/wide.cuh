@@ -15,6 +15,7 @@ namespace bcg {
 constexpr int kWideSlots = 16;       // sources of a job
 constexpr int kWideThreads = 640;    // one CTA per SM, 96 registers a thread
 constexpr int kWideWarps = kWideThreads / 32;
+constexpr uint32_t kWideTeams = 148;  // most teams of a launch
 constexpr uint32_t kWideLevels = 64;  // levels a job can hold (deeper searches run elsewhere)
 constexpr uint32_t kWideLight = 32;   // four lanes take a vertex of up to so many entries, or 2, 4, 8 times that
 constexpr uint32_t kWideChunk = 256;  // entries of a warp's share of a heavy vertex, at least
@@ -68,6 +69,8 @@ struct WideArgs {
                             // job j's vector at j * n
     uint32_t njobs, job0, nroots;
     uint32_t teams, team_ctas;
+    uint32_t split_ctas;    // team size the split of vertices by degree is made for (0: team_ctas);
+                            // fixed, a job's sums do not depend on the launch it runs in
     const uint32_t *roots;  // engine ids, by WideJob::root0
     const double *mult;     // weights, likewise (nullptr: 1)
     double *jobbc;
@@ -137,10 +140,14 @@ size_t wide_layout(WideArgs &a, size_t n, size_t nchunk, size_t nheavy);
 inline bool wide_shallow(uint64_t active, uint64_t nnz) { return nnz >= 6 * active || active + 2 < kWideLevels; }
 // Cuts the SMs into teams for njobs jobs on lists of so many entries (their
 // mean), a's layout being set.
-void wide_teams(WideArgs &a, uint64_t njobs, uint64_t entries);
+void wide_teams(WideArgs &a, uint64_t njobs, uint64_t entries, size_t state_bytes = 1ull << 30);
 // One launch of a's jobs and the adding of their vectors: nouts entries of
-// outs (device; nmax vertices at most), or `one` when outs is nullptr.
+// outs (device; nmax vertices at most; 0: nothing is added), or `one` when outs
+// is nullptr.
 int wide_enqueue(const WideArgs &a, const WideOut *outs, uint32_t nouts, const WideOut &one, uint32_t nmax,
                  cudaStream_t st);
+
+// Adds the vectors in strict job order (a.poison unset).
+int wide_chain(const WideArgs &a, const WideOut *outs, uint32_t nouts, uint32_t nmax, cudaStream_t st);
 
 }  // namespace bcg

@@ -163,3 +163,40 @@ def test_batch_with_a_deep_graph():
             for i, (offs, adj) in enumerate(graphs):
                 ref, _ = oracle.bc(offs, adj, np.arange(len(offs) - 1), nthreads=oracle.max_threads())
                 assert_bc_close(B.bc(i), runs * ref, f"graph {i}")
+
+
+def _served(pool, reqs, wave_batches=4):
+    out = {}
+    with bcg.Server(pool, 8 << 30, wave_batches) as S:
+        ids = [S.submit(g, src) for g, src in reqs]
+        while len(out) < len(ids):
+            for rid in S.wait():
+                out[rid] = S.result(rid)
+    return [out[i] for i in ids]
+
+
+@pytest.mark.parametrize("deep", [False, True])
+def test_served_waves(deep):
+    """Requests of one source to all, cut into several waves of 4 jobs a graph,
+    on graphs of unlike size (several launches a wave): against the oracle, and
+    bit for bit alone.  With a deep graph in the pool a wave stops, is taken
+    back and runs in packed waves, and nothing is added twice."""
+    pool = [bcg.generate("rmat:scale=12,ef=16,a=0.57,b=0.19,c=0.19,seed=5"), bcg.generate("er:scale=8,ef=8,seed=6"),
+            bcg.generate("er:scale=6,ef=6,seed=9")]
+    if deep:
+        pool.append(_cliques(8, 60))
+    rng = np.random.default_rng(2)
+    reqs = [(1, None), (0, np.array([5], dtype=np.uint32)), (2, None), (0, bcg.sample_sources(4096, 300, 3))]
+    reqs += [(int(g), np.sort(rng.choice(60, size=int(rng.integers(1, 60)), replace=False)).astype(np.uint32))
+             for g in rng.integers(0, len(pool), 8)]
+    if deep:
+        reqs.insert(3, (3, None))
+    served = _served(pool, reqs)
+    for i, (g, src) in enumerate(reqs):
+        offs, adj = pool[g]
+        s = np.arange(len(offs) - 1, dtype=np.uint32) if src is None else src
+        ref, _ = oracle.bc(offs, adj, s, nthreads=oracle.max_threads())
+        assert_bc_close(served[i], ref, f"request {i}")
+    if not deep:
+        for i in (0, 3, 6):
+            assert np.array_equal(served[i].view(np.uint64), _served(pool, [reqs[i]])[0].view(np.uint64)), i

@@ -164,7 +164,7 @@ int build_wide(bcg_batch *b) {
                 spans.push_back(Span{jobs.size(), 0, outs.size(), 0, 0, 0, s.n, 1, 1});
             Span &l = spans.back();
             if (l.nouts == 0 || r == 0) {
-                outs.push_back(WideOut{l.cells, 0, s.n, b->form.map + s.base, g->d_bc});
+                outs.push_back(WideOut{l.cells, 0, s.n, b->form.map + s.base, g->d_bc, nullptr});
                 ++l.nouts;
             }
             ++outs.back().njobs;

@@ -128,6 +128,16 @@ std::mutex g_pool_mu;
 std::vector<cudaMemPool_t> g_pools;  // per device, created on first use
 }  // namespace
 
+// What the pool keeps: 1 GiB more than is in use (its threshold counts used
+// memory too, so with larger graphs alive a fixed one would unmap every freed
+// buffer at the next synchronisation).
+static void pool_keep(cudaMemPool_t pool) {
+    uint64_t used = 0;
+    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) return;
+    uint64_t keep = used + (1ull << 30);
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+}
+
 cudaError_t tmp_alloc(void **p, size_t bytes, cudaStream_t st) {
     *p = nullptr;
     int dev = 0;
@@ -146,12 +156,13 @@ cudaError_t tmp_alloc(void **p, size_t bytes, cudaStream_t st) {
                 g_pools[dev] = nullptr;
                 return e;
             }
-            uint64_t keep = 1ull << 30;
-            cudaMemPoolSetAttribute(g_pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+            pool_keep(g_pools[dev]);
         }
         pool = g_pools[dev];
     }
-    return cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 16), pool, st);
+    const cudaError_t e2 = cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 16), pool, st);
+    if (e2 == cudaSuccess && bytes >= (16u << 20)) pool_keep(pool);
+    return e2;
 }
 
 cudaError_t tmp_free(void *p, cudaStream_t st) { return p ? cudaFreeAsync(p, st) : cudaSuccess; }
@@ -178,6 +189,10 @@ static void graph_free(bcg_graph *g) {
     dev_free(g->d_roots); dev_free(g->d_pend); dev_free(g->d_mult); dev_free(g->d_rstat);
     if (g->ev0) cudaEventDestroy(g->ev0);
     if (g->ev1) cudaEventDestroy(g->ev1);
+    {
+        std::lock_guard<std::mutex> lk(g_pool_mu);
+        if (g_pools.size() > (size_t)g->device && g_pools[g->device]) pool_keep(g_pools[g->device]);
+    }
     if (cur >= 0 && cur != g->device) cudaSetDevice(cur);
     delete g;
 }

@@ -9,8 +9,8 @@
 // same scratch.  No pruning; undirected graphs only.
 //
 // Setup: the first call on a device (with that device current) takes the
-// array's address with cudaGetSymbolAddress, which loads this module; the
-// address is kept per device for the life of the process.
+// array's address with cudaGetSymbolAddress, which loads this module, and loads
+// the kernels of both ways a call can take; the address is kept per device for the life of the process.
 //
 // Scratch that must start at zero and is cleared by every call: the status
 // block, the sweep control block, the tile marks, the hub arrival counters,
@@ -19,6 +19,12 @@
 // unvisited-tile ring, roots, the hub chunk slots, the saved accumulators) is
 // written before it is read.  One scratch per device: calls that overlap on the same device race
 // on it.
+//
+// Shallow graphs (wide_shallow) whose wide form and state fit the scratch go to
+// the wide-batch searches (wide.cu) on the same memory, and need no tiles; one
+// with a search of more than 62 levels or an overflowing count goes on as
+// below.  (100 sources at 4,000 vertices: 2.26 ms, half of it the tiles' one
+// thread and the rest sweeps of the whole chip; NOALLOC_MS ms.)
 //
 // Path counts: exact uint64 first; when one overflows (large grids, long
 // chains of diamonds), the accumulators saved before the sweep are put back
@@ -30,10 +36,12 @@
 
 #include "bcg_common.hpp"
 #include "engine.cuh"
+#include "wide.cuh"
 
 namespace bcg {
 
 int launch_sweep(int S, const BatchArgs &a, cudaStream_t st, int *grid_out, bool ext = false);
+void preload_sweep();
 
 namespace {
 
@@ -276,6 +284,13 @@ int na_scratch(unsigned char **out) {
             return set_error(e == cudaErrorNoKernelImageForDevice ? BCG_ERR_NOGPU : BCG_ERR_CUDA,
                              "cudaGetSymbolAddress of the no-allocation scratch on device %d: %s", dev,
                              cudaGetErrorString(e));
+        // every kernel a later call may need, so that none of them takes memory
+        cudaFuncAttributes at;
+        for (const void *k : {(const void *)k_na_check_offsets, (const void *)k_na_check_adj, (const void *)k_na_vinfo,
+                              (const void *)k_na_tiles, (const void *)k_na_roots})
+            cudaFuncGetAttributes(&at, k);
+        preload_sweep();
+        preload_wide();
         g_na_ptr[dev] = static_cast<unsigned char *>(p);
     }
     *out = g_na_ptr[dev];
@@ -292,6 +307,12 @@ const char *bad_name(uint32_t what) {
     }
 }
 
+// What the wide searches of a call use of the scratch: region A (the tiles to
+// the hub counters) for the teams' states, region B (the weights and the
+// per-root totals) for the form, its building, the control words and the job
+// vectors, or A where they are too large for B.
+constexpr size_t kRegionA = kOffTiles, kRegionAEnd = kOffRoots, kRegionB = kOffPend, kRegionBEnd = kOffBcSave;
+
 }  // namespace
 }  // namespace bcg
 
@@ -302,6 +323,71 @@ using namespace bcg;
         cudaError_t e_ = (call);                                                                     \
         if (e_ != cudaSuccess) return set_error(BCG_ERR_CUDA, "%s failed: %s", #call, cudaGetErrorString(e_)); \
     } while (0)
+
+// The wide searches on the call's copies in the scratch; *done = false: they
+// do not fit it, or stopped (d_bc is then as before).
+static int na_wide(unsigned char *scr, uint32_t n, uint64_t nnz, uint32_t nroots, double *d_bc, cudaStream_t st,
+                   bool *done) {
+    *done = false;
+    WideInput in{};
+    in.n = n;
+    in.nnz = in.big_nnz = nnz;
+    in.offs = reinterpret_cast<const uint32_t *>(scr + kOffOffs);
+    in.adj = reinterpret_cast<const uint32_t *>(scr + kOffAdj);
+    in.vinfo = reinterpret_cast<const uint2 *>(scr + kOffVinfo);
+    in.graphs = 1;
+    size_t scratch = 0;
+    const size_t form = wide_form_bytes(in, &scratch);
+    const uint64_t njobs = (nroots + kWideSlots - 1) / kWideSlots;
+    const size_t stat = up256(sizeof(WideCtrl) + kWideTeams * sizeof(WideTeam)), row = up256((size_t)n * sizeof(double));
+    size_t a0 = kRegionA, b0 = kRegionB;
+    // first come first served: B, then A
+    auto take = [&](size_t bytes) -> unsigned char * {
+        bytes = up256(bytes);
+        if (b0 + bytes <= kRegionBEnd) return b0 += bytes, scr + b0 - bytes;
+        if (a0 + bytes <= kRegionAEnd) return a0 += bytes, scr + a0 - bytes;
+        return nullptr;
+    };
+    unsigned char *mstat = take(stat), *mform = take(form), *mscr = take(scratch);
+    if (!mstat || !mform || !mscr) return BCG_OK;
+    // job vectors: as many as fit B's rest (one at least), for all jobs if need be several launches
+    uint64_t jl = std::min<uint64_t>(njobs, (kRegionBEnd - b0) / row);
+    if (!jl) jl = 1;
+    unsigned char *mjobs = take(jl * row);
+    WideArgs a{};
+    // (a heavy vertex has kWideChunk entries or more: the form's bounds)
+    wide_layout(a, n, 2 * (nnz / kWideChunk) + 1, nnz / kWideChunk + 1);
+    if (!mjobs || a0 + a.stride > kRegionAEnd) return BCG_OK;
+    wide_teams(a, jl, nnz, kRegionAEnd - a0);
+    WideForm f;
+    int rc = wide_form_enqueue(f, in, mform, mscr, st);
+    if (rc) return rc;
+    a.subs = f.d_subs;
+    a.nroots = nroots;
+    a.roots = reinterpret_cast<const uint32_t *>(scr + kOffRoots);
+    a.jobbc = reinterpret_cast<double *>(mjobs);
+    a.ctrl = reinterpret_cast<WideCtrl *>(mstat);
+    a.team = reinterpret_cast<WideTeam *>(mstat + sizeof(WideCtrl));
+    a.state = scr + a0;
+    double *save = reinterpret_cast<double *>(scr + kOffBcSave);
+    if (jl < njobs) NA_CK(cudaMemcpyAsync(save, d_bc, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    for (uint64_t j0 = 0; j0 < njobs; j0 += jl) {
+        a.job0 = (uint32_t)j0;
+        a.njobs = (uint32_t)std::min<uint64_t>(jl, njobs - j0);
+        NA_CK(cudaMemsetAsync(mstat, 0, stat, st));
+        if ((rc = wide_enqueue(a, nullptr, 1, WideOut{0, a.njobs, n, f.map, d_bc, f.d_subs}, n, st))) return rc;
+        WideCtrl c{};
+        NA_CK(cudaMemcpyAsync(&c, mstat, sizeof(c), cudaMemcpyDeviceToHost, st));
+        NA_CK(cudaStreamSynchronize(st));
+        if (c.error) return set_error(c.error, "device reported error %d (a bounded wait gave up)", c.error);
+        if (c.overflow || c.deep) {
+            if (jl < njobs) NA_CK(cudaMemcpyAsync(d_bc, save, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+            return BCG_OK;
+        }
+    }
+    *done = true;
+    return BCG_OK;
+}
 
 extern "C" int bcg_bc_noalloc(const uint32_t *d_offsets, const uint32_t *d_adj, uint32_t n, uint64_t nnz,
                               const uint32_t *d_sources, uint64_t nsrc, double *d_bc, int accumulate,
@@ -350,25 +436,38 @@ extern "C" int bcg_bc_noalloc(const uint32_t *d_offsets, const uint32_t *d_adj, 
         k_na_check_adj<<<blocks, 256, 0, st>>>(n, nnz, d_adjc, d_status);
     }
     k_na_vinfo<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, d_offsets, d_vinfo);
-    k_na_tiles<<<1, 1, 0, st>>>(n, d_offsets, d_tiles, d_tile_of, d_status);
-    k_na_roots<<<1, 1024, 0, st>>>(n, d_offsets, d_sources, (uint32_t)nsrc, d_roots, d_mult, d_pend, d_status);
-    NA_CK(cudaGetLastError());
+    // tiles are for the sweep kernel
+    bool wide = nsrc >= 4 && nnz && wide_shallow(n, nnz);
     NaStatus hs{};
-    NA_CK(cudaMemcpyAsync(&hs, d_status, sizeof(hs), cudaMemcpyDeviceToHost, st));
-    NA_CK(cudaStreamSynchronize(st));
-    if (hs.error)
-        return set_error(BCG_ERR_ARG, "invalid input: %s %llu", bad_name(hs.what), hs.index);
+    auto plan = [&](bool tiles) -> int {
+        if (tiles) k_na_tiles<<<1, 1, 0, st>>>(n, d_offsets, d_tiles, d_tile_of, d_status);
+        k_na_roots<<<1, 1024, 0, st>>>(n, d_offsets, d_sources, (uint32_t)nsrc, d_roots, d_mult, d_pend, d_status);
+        NA_CK(cudaGetLastError());
+        NA_CK(cudaMemcpyAsync(&hs, d_status, sizeof(hs), cudaMemcpyDeviceToHost, st));
+        NA_CK(cudaStreamSynchronize(st));
+        if (hs.error) return set_error(BCG_ERR_ARG, "invalid input: %s %llu", bad_name(hs.what), hs.index);
+        return BCG_OK;
+    };
+    rc = plan(!wide);
+    if (rc) return rc;
 
     if (!accumulate) NA_CK(cudaMemsetAsync(d_bc, 0, (size_t)n * sizeof(double), st));
+    if (hs.nroots == 0) {
+        NA_CK(cudaStreamSynchronize(st));
+        return BCG_OK;
+    }
+    if (wide) {
+        bool done = false;
+        rc = na_wide(scr, n, nnz, hs.nroots, d_bc, st, &done);
+        if (rc || done) return rc;
+        rc = plan(true);
+        if (rc) return rc;
+    }
     // the caller's accumulators before the sweep: a run whose uint64 path
     // counts overflow is redone with extended-range counts from this copy,
     // as bcg_run does in its automatic mode
     double *d_bc_save = reinterpret_cast<double *>(scr + kOffBcSave);
     NA_CK(cudaMemcpyAsync(d_bc_save, d_bc, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    if (hs.nroots == 0) {
-        NA_CK(cudaStreamSynchronize(st));
-        return BCG_OK;
-    }
     // the batch width bcg_run picks for a graph whose rows fit its state budget
     const uint32_t S = hs.nroots > 3 ? 6u : (hs.nroots > 1 ? 3u : 1u);
     const uint64_t nbatch = (hs.nroots + S - 1) / S;

@@ -313,7 +313,7 @@ int enqueue_wide_wave(bcg_server *s, ServeWave &w, int wi, bool *launched) {
                 // (the map gives union ids: the buffer is addressed from the union's start)
                 double *out = reinterpret_cast<double *>(reinterpret_cast<uintptr_t>(r.d_out) -
                                                          (uintptr_t)s->base[gi] * sizeof(double));
-                outs[no++] = WideOut{cells, take, sub.n, s->form.map + sub.base, out};
+                outs[no++] = WideOut{cells, take, sub.n, s->form.map + sub.base, out, nullptr};
                 for (uint32_t j = 0; j < take; ++j) {
                     const uint32_t k = (uint32_t)std::min<size_t>(kWideSlots, r.src.size() - r.sched);
                     jobs[nj++] = WideJob{gi, nr, k, 0, cells};

@@ -1412,6 +1412,14 @@ static int launch_impl(const BatchArgs &a, cudaStream_t st, int *grid_out) {
     return BCG_OK;
 }
 
+void preload_sweep() {
+    cudaFuncAttributes at;
+    for (const void *f : {(const void *)bc_sweep_kernel<1, false>, (const void *)bc_sweep_kernel<3, false>,
+                          (const void *)bc_sweep_kernel<6, false>, (const void *)bc_sweep_kernel<1, true>,
+                          (const void *)bc_sweep_kernel<3, true>, (const void *)bc_sweep_kernel<6, true>})
+        cudaFuncGetAttributes(&at, f);
+}
+
 int launch_sweep(int S, const BatchArgs &a, cudaStream_t st, int *grid_out, bool ext) {
     switch (S) {
         case 1: return ext ? launch_impl<1, true>(a, st, grid_out) : launch_impl<1, false>(a, st, grid_out);

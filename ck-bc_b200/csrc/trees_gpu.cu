@@ -103,6 +103,12 @@ __global__ void k_scan_add(uint32_t *__restrict__ out, const uint32_t *__restric
 
 }  // namespace
 
+void preload_scan() {
+    cudaFuncAttributes at;
+    cudaFuncGetAttributes(&at, (const void *)k_scan_block);
+    cudaFuncGetAttributes(&at, (const void *)k_scan_add);
+}
+
 uint64_t scan_scratch(uint64_t len) {
     uint64_t s = 0;
     for (uint64_t nb = (len + kScanBlock - 1) / kScanBlock; nb > 1; nb = (nb + kScanBlock - 1) / kScanBlock) s += nb;

@@ -856,9 +856,10 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
         const uint32_t D = d;
 
         // ---- what each source reached: a thread's vertices, four slots each
+        const bool counted = a.rstat || a.total;
         if (threadIdx.x < 3 * kWideSlots) sm.reach[threadIdx.x] = 0ull;
         __syncthreads();
-        {
+        if (counted) {
             uint32_t vis[4] = {0, 0, 0, 0};
             unsigned long long ws[4] = {0, 0, 0, 0}, mc[4] = {0, 0, 0, 0};
             for (uint32_t i = tid; i < n * 4u; i += nt) {  // n * 4 < 2^32 (checked on the host)
@@ -928,7 +929,8 @@ __global__ void __launch_bounds__(256) k_wide_reduce(const WideCtrl *__restrict_
     __shared__ double part[8][32];
     if (ctrl->error | ctrl->overflow | ctrl->deep) return;  // nothing of a stopped launch is kept
     if (poison && *poison) return;
-    const WideOut o = outs ? outs[blockIdx.y] : one;
+    WideOut o = outs ? outs[blockIdx.y] : one;
+    if (o.sub) o.n = o.sub->n;
     const unsigned lane = threadIdx.x & 31, p = threadIdx.x >> 5;
     for (uint32_t v0 = blockIdx.x * 32; v0 < o.n; v0 += gridDim.x * 32) {
         const uint32_t v = v0 + lane;
@@ -976,6 +978,13 @@ __global__ void __launch_bounds__(256) k_wide_chain(const int *__restrict__ pois
 size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
 
 }  // namespace
+
+void preload_wide() {
+    cudaFuncAttributes at;
+    cudaFuncGetAttributes(&at, (const void *)bc_wide_kernel);
+    cudaFuncGetAttributes(&at, (const void *)k_wide_reduce);
+    preload_wide_form();
+}
 
 size_t wide_layout(WideArgs &a, size_t n, size_t nchunk, size_t nheavy) {
     const size_t words = (n + 31) / 32;
@@ -1153,7 +1162,7 @@ int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t n
         a.job0 = (uint32_t)j0;
         a.rstat = reinterpret_cast<RootStat *>(w->stat + o_rstat) + j0 * kWideSlots;
         if (j0) CKW(cudaMemsetAsync(w->stat, 0, o_rstat, st));
-        if ((rc = wide_enqueue(a, nullptr, 1, WideOut{0, a.njobs, (uint32_t)n, w->form.map, g->d_bc}, (uint32_t)n, st)))
+        if ((rc = wide_enqueue(a, nullptr, 1, WideOut{0, a.njobs, (uint32_t)n, w->form.map, g->d_bc, nullptr}, (uint32_t)n, st)))
             return rc;
         res->launches += 2;
         const bool last = j0 + a.njobs >= njobs;

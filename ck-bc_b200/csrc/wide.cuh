@@ -97,6 +97,7 @@ struct WideOut {
     uint32_t njobs, n;
     const uint32_t *map;
     double *bc;
+    const WideSub *sub;  // set: n is its n (not known to the host)
 };
 
 // The lists a wide form is made from (device arrays; vinfo and ext by engine
@@ -132,6 +133,12 @@ int wide_form_enqueue(WideForm &f, const WideInput &in, unsigned char *mem, unsi
 int wide_form_make(WideForm &f, const WideInput &in);
 void wide_form_free(WideForm &f);
 
+// Loads the wide searches' kernels on the current device (CUDA would load each
+// at its first launch, which takes device memory).
+void preload_wide();
+void preload_wide_form();
+void preload_scan();
+
 // Fills a's state layout for graphs of up to n vertices; returns the stride.
 size_t wide_layout(WideArgs &a, size_t n, size_t nchunk, size_t nheavy);
 // Whether a graph with so many vertices that have an entry, and so many
@@ -140,7 +147,7 @@ size_t wide_layout(WideArgs &a, size_t n, size_t nchunk, size_t nheavy);
 inline bool wide_shallow(uint64_t active, uint64_t nnz) { return nnz >= 6 * active || active + 2 < kWideLevels; }
 // Cuts the SMs into teams for njobs jobs on lists of so many entries (their
 // mean), a's layout being set.
-void wide_teams(WideArgs &a, uint64_t njobs, uint64_t entries, size_t state_bytes = 1ull << 30);
+void wide_teams(WideArgs &a, uint64_t njobs, uint64_t entries, size_t state_bytes = 512ull << 20);
 // One launch of a's jobs and the adding of their vectors: nouts entries of
 // outs (device; nmax vertices at most; 0: nothing is added), or `one` when outs
 // is nullptr.

@@ -257,6 +257,14 @@ FormPlan plan_form(const WideInput &in) {
 
 }  // namespace
 
+void preload_wide_form() {
+    cudaFuncAttributes at;
+    for (const void *k : {(const void *)k_form_hist, (const void *)k_form_number, (const void *)k_form_rows,
+                          (const void *)k_form_fill, (const void *)k_form_subs})
+        cudaFuncGetAttributes(&at, k);
+    preload_scan();
+}
+
 size_t wide_form_bytes(const WideInput &in, size_t *scratch) {
     const FormPlan p = plan_form(in);
     *scratch = p.scratch;

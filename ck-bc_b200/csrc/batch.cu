@@ -100,6 +100,8 @@ void free_schedule(bcg_batch *b) {
     b->packed = false;
 }
 
+constexpr uint32_t kBatchSlots = 32;  // sources of a job: every graph has all its vertices searched
+
 void free_wide(bcg_batch *b) {
     wide_form_free(b->form);
     dev_free(b->d_wide); dev_free(b->d_stat); dev_free(b->d_state); dev_free(b->d_jobbc); dev_free(b->d_save);
@@ -158,7 +160,7 @@ int build_wide(bcg_batch *b) {
         const size_t r0 = roots.size();
         for (uint32_t v = ubase[p]; v < ubase[p + 1]; ++v)
             if (b->hdeg[v]) roots.push_back(v);
-        for (uint32_t r = 0; r < act[p]; r += kWideSlots) {
+        for (uint32_t r = 0; r < act[p]; r += kBatchSlots) {
             if (spans.empty() || spans.back().cells + s.n > kCells ||
                 (r == 0 && s.n < spans.back().nmax / 4 && spans.back().njobs >= 4 * 148))
                 spans.push_back(Span{jobs.size(), 0, outs.size(), 0, 0, 0, s.n, 1, 1});
@@ -168,7 +170,7 @@ int build_wide(bcg_batch *b) {
                 ++l.nouts;
             }
             ++outs.back().njobs;
-            jobs.push_back(WideJob{p, (uint32_t)(r0 + r), std::min<uint32_t>(kWideSlots, act[p] - r), 0, l.cells});
+            jobs.push_back(WideJob{p, (uint32_t)(r0 + r), std::min<uint32_t>(kBatchSlots, act[p] - r), 0, l.cells});
             ++l.njobs;
             l.cells += s.n;
             l.entries += gnnz[p];
@@ -184,7 +186,7 @@ int build_wide(bcg_batch *b) {
     size_t stat = 0, state = 0;
     for (const Span &l : spans) {
         bcg_batch::Launch L{};
-        state = std::max(state, (wide_layout(L.a, l.nmax, l.nch, l.nheavy), wide_teams(L.a, l.njobs, l.entries / l.njobs),
+        state = std::max(state, (wide_layout(L.a, kBatchSlots, l.nmax, l.nch, l.nheavy), wide_teams(L.a, l.njobs, l.entries / l.njobs),
                                  L.a.stride * L.a.teams));
         L.a.njobs = (uint32_t)l.njobs;
         L.outs = o_outs + l.out0 * sizeof(WideOut);
@@ -524,7 +526,7 @@ int bcg_batch_run(bcg_batch *b, bcg_stats *stats) {
             cv = t->wsum;
             md = t->depth;
             batches = b->njobs;
-            width = kWideSlots;
+            width = kBatchSlots;
         }
     }
     if (!b->wide) {

@@ -131,6 +131,7 @@ int scan_exclusive(const uint32_t *d_in, uint32_t *d_out, uint64_t len, uint32_t
 struct WideResult {
     bool done = false;
     uint64_t batches = 0, launches = 0;
+    uint32_t slots = 0;           // sources of a job
     std::vector<RootStat> rstat;  // per root, in order (padded to whole jobs)
 };
 int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, cudaStream_t st, WideResult *res);

@@ -172,6 +172,7 @@ int packed_setup(bcg_server *s) {
     return BCG_OK;
 }
 
+constexpr uint32_t kServeSlots = 32;  // sources of a job
 constexpr uint32_t kMaxSpans = 8;  // launches of a wide wave
 
 void wide_clear(bcg_server *s) {
@@ -216,12 +217,12 @@ int wide_setup(bcg_server *s) {
     // job vectors for a wave of 148 of the largest graph's jobs, up to 256 MB
     // (one at least)
     WideArgs a{};
-    const size_t stride = wide_layout(a, nmax, in.big_nnz / kWideChunk * 2 + 1, in.big_nnz / kWideChunk + 1);
+    const size_t stride = wide_layout(a, kServeSlots, nmax, in.big_nnz / kWideChunk * 2 + 1, in.big_nnz / kWideChunk + 1);
     s->wstate_bytes = std::max(stride, std::min<size_t>(148 * stride, 256ull << 20));
     s->cells = std::max<uint64_t>(nmax, std::min<uint64_t>(148ull * 8 * nmax, (256ull << 20) / 8));
     const size_t jobs = (size_t)s->wave_batches * G;
     s->off_wroots = up16(jobs * sizeof(WideJob));
-    s->off_wouts = s->off_wroots + up16(jobs * kWideSlots * 4);
+    s->off_wouts = s->off_wroots + up16(jobs * kServeSlots * 4);
     s->wblob_bytes = s->off_wouts + jobs * sizeof(WideOut);
     const size_t stat = kMaxSpans * (sizeof(WideCtrl) + kWideTeams * sizeof(WideTeam));
     size_t scratch = 0;
@@ -298,7 +299,7 @@ int enqueue_wide_wave(bcg_server *s, ServeWave &w, int wi, bool *launched) {
         while (!q.empty()) {
             Req &r = s->reqs[q.front()];
             const size_t left = r.src.size() - r.sched;
-            const uint32_t take = (uint32_t)std::min<uint64_t>({(left + kWideSlots - 1) / kWideSlots,
+            const uint32_t take = (uint32_t)std::min<uint64_t>({(left + kServeSlots - 1) / kServeSlots,
                                                                 (uint64_t)s->wave_batches - used,
                                                                 sub.n ? (s->cells - cells) / sub.n : 0});
             if (left && !take) break;  // the wave is full (for this graph)
@@ -315,7 +316,7 @@ int enqueue_wide_wave(bcg_server *s, ServeWave &w, int wi, bool *launched) {
                                                          (uintptr_t)s->base[gi] * sizeof(double));
                 outs[no++] = WideOut{cells, take, sub.n, s->form.map + sub.base, out, nullptr};
                 for (uint32_t j = 0; j < take; ++j) {
-                    const uint32_t k = (uint32_t)std::min<size_t>(kWideSlots, r.src.size() - r.sched);
+                    const uint32_t k = (uint32_t)std::min<size_t>(kServeSlots, r.src.size() - r.sched);
                     jobs[nj++] = WideJob{gi, nr, k, 0, cells};
                     for (uint32_t i = 0; i < k; ++i) roots[nr++] = r.src[r.sched + i];
                     r.sched += k;
@@ -341,7 +342,7 @@ int enqueue_wide_wave(bcg_server *s, ServeWave &w, int wi, bool *launched) {
         WideArgs a{};
         for (size_t k = 0; k < spans.size(); ++k) {
             const Span &l = spans[k];
-            wide_layout(a, l.nmax, l.nch, l.nheavy);
+            wide_layout(a, kServeSlots, l.nmax, l.nch, l.nheavy);
             wide_teams(a, l.njobs, l.entries / l.njobs, s->wstate_bytes);
             a.subs = s->form.d_subs;
             a.jobs = reinterpret_cast<const WideJob *>(w.d_jobs) + l.job0;

@@ -1,20 +1,24 @@
-// Wide-batch Brandes searches (sm_100a): 16 sources a job, for graphs whose
-// searches are a few levels deep.
+// Wide-batch Brandes searches (sm_100a): 16 or 32 sources a job, for graphs
+// whose searches are a few levels deep.
 //
 // What bounds it.  On a small-diameter graph nearly every vertex is in the
 // frontier of some source of a batch at the two or three middle levels, so a
 // level is a sparse-matrix times dense-matrix product: every vertex adds the
-// 16 values of each neighbour.  The rows are gathered from L2, and an SM
+// 16 (32) values of each neighbour.  The rows are gathered from L2, and an SM
 // takes in 64 bytes a clock from there.  So the design is about bytes per
 // (edge, source) and about whole rows per request:
-//   - 16 sources share a row: 64 bytes of 32-bit path counts forward, 128
-//     bytes of doubles backward, no level words in between.  A row holds the
+//   - 16 (32) sources share a row: 64 (128) bytes of 32-bit path counts
+//     forward, 128 (256) of doubles backward, no level words in between.  A row holds the
 //     value of the slots that sit exactly at the level being read and 0 in
 //     the others, so a gather needs no test per slot: 4 lanes take a row with
-//     one 16- or 32-byte load each and add.  (Measured on an R-MAT graph of
+//     one or two 16- or 32-byte loads each and add.  (Measured on an R-MAT graph of
 //     31 M entries: 141 us and 201 us a pass, 14 and 20 TB/s out of L2, the
 //     whole port; the 64-byte rows of levels and values of sweep.cu carry 6
-//     sources and take about 500 us.)
+//     sources and take about 500 us.)  The sweeps here reach 300 to 400 us:
+//     what is left is instructions (0.33 a cycle and scheduler, a third of
+//     them for ids, bits and vertices rather than rows) and the latency of
+//     rows.  32 sources a job share the first kind: 1,590 us a job of 16 and
+//     2,690 us one of 32 on the benchmark's graph.
 //   - a bit per vertex and level says whether any slot sits there, so a
 //     gather skips the rows of other vertices, rows are never cleared, and
 //     backward sweeps visit a level's vertices only.
@@ -23,10 +27,11 @@
 //     sweep reads levels and 64-bit counts (kFwdFull), with overflow checked.
 // All forward sweeps pull: no atomics on values, sums in a fixed order.
 //
-// Work split.  Vertices are numbered by descending degree class.  A vertex
-// of up to 32 entries is taken by four lanes (eight vertices of like degree a
-// warp), one of up to 256 by a warp (its edges dealt to the eight groups of
-// four lanes), a heavier one in chunks of 256 entries by one warp each, whose
+// Work split.  Vertices are numbered by descending degree class
+// (wide_form.cu).  A vertex of few entries (up to 32, or up to 256 where a warp
+// has much to do) is taken by four lanes, eight vertices of like degree a
+// warp; a heavier one by a warp, its edges dealt to the eight groups of four
+// lanes; the heaviest in chunks of 256 to 2,048 entries by one warp each, whose
 // sums meet in a buffer and are added in a fixed order by the chunk that
 // arrives last.  Warps draw items from a counter in shared memory, heaviest
 // first.
@@ -59,6 +64,7 @@ constexpr uint32_t kFull = 0xffffffffu;
 constexpr uint32_t kNone = 0xffffffffu;
 constexpr uint32_t kUnseen = 0xFFu;  // level byte of a vertex not reached yet
 constexpr uint32_t kEmpty = 0xFEu;   // level byte of a slot without a source
+constexpr double kWide32 = 1.5;      // time of a 32-source job's entries over a 16-source job's
 
 // What a sweep does: forward over 32-bit rows, forward over levels and
 // 64-bit counts, backward, backward at the deepest level (no child exists).
@@ -80,11 +86,22 @@ struct WideCtx {
 // The rows of level d.
 __device__ __forceinline__ unsigned char *rows_of(const WideCtx &x, uint32_t d) { return x.g0 + ((d & 1u) ? x.g01 : 0); }
 
+// What follows from a job's number of slots NS (16 or 32): a lane holds LS of
+// them, in a group of four lanes that takes a row together.
+template <int NS>
+struct Slots {
+    static constexpr int LS = NS / 4;
+    static constexpr int kLevels = LS / 4;    // words of a lane's levels
+    static constexpr int kRow32 = NS * 4;     // bytes of a row of counts,
+    static constexpr int kRow64 = NS * 8;     // of a row of doubles
+};
+
+template <int NS>
 struct WideSmem {
     WideSub sub;
     WideCtx x;
-    uint32_t roots[kWideSlots];
-    double mult[kWideSlots];
+    uint32_t roots[NS];
+    double mult[NS];
     uint32_t nmed;      // end of the vertices a warp takes alone (WideSub::nmed by degree bound)
     uint32_t next;      // items drawn in the current sweep
     uint32_t found;     // this CTA's part of WideTeam::any
@@ -93,8 +110,8 @@ struct WideSmem {
     uint32_t met[kWideLevels];  // vertices that some slot holds at a level, at most
     uint32_t left;              // vertices that some slot has not reached
     int ok;
-    uint32_t edges[kWideSlots + 1];             // entries of the sources before each
-    unsigned long long reach[3 * kWideSlots];   // this CTA's part of the sources' totals
+    uint32_t edges[NS + 1];             // entries of the sources before each
+    unsigned long long reach[3 * NS];   // this CTA's part of the sources' totals
     unsigned char list[kWideWarps][32];
 };
 
@@ -114,14 +131,35 @@ __device__ __forceinline__ void st32(void *p, const uint32_t (&w)[8]) {
                  "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "l"(p)
                  : "memory");
 }
-// A lane's part of row u of doubles (0 where u is kNone).  Not volatile: rows
-// do not change during the sweep that reads them, so the loads may move.
-__device__ __forceinline__ void ld_row(uint32_t u, const unsigned char *rows, double (&r)[4]) {
-    r[0] = r[1] = r[2] = r[3] = 0.0;
-    if (u != kNone)
-        asm("ld.global.cg.v4.f64 {%0,%1,%2,%3}, [%4];"
-            : "=d"(r[0]), "=d"(r[1]), "=d"(r[2]), "=d"(r[3])
-            : "l"(rows + (size_t)u * 128));
+// A lane's part of row u of doubles, or of 32-bit counts (0 where u is kNone).
+// Not volatile: rows do not change during the sweep that reads them, so the
+// loads may move.
+template <int N>
+__device__ __forceinline__ void ld_row(uint32_t u, const unsigned char *rows, double (&r)[N]) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) r[k] = 0.0;
+    if (u != kNone) {
+#pragma unroll
+        for (int k = 0; k < N; k += 4)
+            asm("ld.global.cg.v4.f64 {%0,%1,%2,%3}, [%4];"
+                : "=d"(r[k]), "=d"(r[k + 1]), "=d"(r[k + 2]), "=d"(r[k + 3])
+                : "l"(rows + (size_t)u * (32 * N) + 8 * k));
+    }
+}
+template <int N>
+__device__ __forceinline__ void ld_row(uint32_t u, const unsigned char *rows, uint32_t (&r)[N]) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) r[k] = 0u;
+    if (u != kNone) {
+        if constexpr (N == 4)
+            asm("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];"
+                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                : "l"(rows + (size_t)u * 64));
+        else
+            asm("ld.global.cg.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                : "l"(rows + (size_t)u * 128));
+    }
 }
 // An adjacency entry: streamed, so evicted before the rows.
 __device__ __forceinline__ uint32_t ld_adj(const uint32_t *p, unsigned long long pol) {
@@ -138,7 +176,8 @@ __device__ __forceinline__ bool wide_stopped(const WideCtrl *c) {
 // Barrier of a team: one arrival per CTA on the team's counter.  Returns
 // false when any CTA of the launch recorded an error; a waiting CTA sees that
 // too, so nobody waits for one that has left.
-__device__ bool team_sync(const WideArgs &a, const WideCtx &x, WideTeam *t, WideSmem &sm, unsigned long long wait_ns,
+template <int NS>
+__device__ bool team_sync(const WideArgs &a, const WideCtx &x, WideTeam *t, WideSmem<NS> &sm, unsigned long long wait_ns,
                           uint32_t slot, uint32_t level = 0) {
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -219,56 +258,66 @@ __device__ __forceinline__ void load_ids(uint32_t (&id)[4], const uint32_t *__re
 }
 
 // The first J of a lane's four edges: a group of four lanes takes its lanes'
-// edges one after the other, each lane 4 slots of a row, the next rows in
-// flight while the last are added.
-template <int KIND, int J, class T>
-__device__ __forceinline__ void add_rows(const unsigned char *rows, const uint32_t (&id)[4], T (&acc)[4]) {
+// edges one after the other, each lane LS slots of a row, the next rows in
+// flight (32 registers of them) while the last are added.
+template <int KIND, int J, int LS, class T>
+__device__ __forceinline__ void add_rows(const unsigned char *rows, const uint32_t (&id)[4], T (&acc)[LS]) {
     const unsigned sh = threadIdx.x & 28u;
     if constexpr (KIND == kFwd32) {
-        uint32_t part[4] = {0u, 0u, 0u, 0u};  // at most 16 counts below 2^28
-        uint4 r[2][4];
-        auto fetch = [&](int j, uint4 (&o)[4]) {
+        constexpr int U = 16 / LS;  // rows of a step
+        uint32_t part[LS];          // at most 16 counts below 2^28
+        uint32_t r[2][U][LS];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const uint32_t u = __shfl_sync(kFull, id[j], sh + q);
-                o[q] = make_uint4(0u, 0u, 0u, 0u);
-                if (u != kNone) o[q] = __ldcg(reinterpret_cast<const uint4 *>(rows + (size_t)u * 64));
+        for (int k = 0; k < LS; ++k) part[k] = 0u;
+        auto fetch = [&](int s, uint32_t (&o)[U][LS]) {
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                const int e = s * U + q;
+                ld_row(__shfl_sync(kFull, id[e >> 2], sh + (e & 3)), rows, o[q]);
             }
         };
+        constexpr int steps = 4 * J / U;
         fetch(0, r[0]);
 #pragma unroll
-        for (int j = 0; j < J; ++j) {
-            if (j + 1 < J) fetch(j + 1, r[(j + 1) & 1]);
-            const uint4 *o = r[j & 1];
-            part[0] += (o[0].x + o[1].x) + (o[2].x + o[3].x);
-            part[1] += (o[0].y + o[1].y) + (o[2].y + o[3].y);
-            part[2] += (o[0].z + o[1].z) + (o[2].z + o[3].z);
-            part[3] += (o[0].w + o[1].w) + (o[2].w + o[3].w);
+        for (int s = 0; s < steps; ++s) {
+            if (s + 1 < steps) fetch(s + 1, r[(s + 1) & 1]);
+#pragma unroll
+            for (int k = 0; k < LS; ++k) {
+                uint32_t t = r[s & 1][0][k] + r[s & 1][1][k];
+                if constexpr (U == 4) t += r[s & 1][2][k] + r[s & 1][3][k];
+                part[k] += t;
+            }
         }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) acc[k] += (T)part[k];
+        for (int k = 0; k < LS; ++k) acc[k] += (T)part[k];
     } else if constexpr (KIND == kBack) {
-        double r[2][2][4];
-        auto fetch = [&](int s, double (&o)[2][4]) {
+        constexpr int U = 8 / LS;
+        double r[2][U][LS];
+        auto fetch = [&](int s, double (&o)[U][LS]) {
 #pragma unroll
-            for (int q = 0; q < 2; ++q) ld_row(__shfl_sync(kFull, id[s >> 1], sh + 2 * (s & 1) + q), rows, o[q]);
+            for (int q = 0; q < U; ++q) {
+                const int e = s * U + q;
+                ld_row(__shfl_sync(kFull, id[e >> 2], sh + (e & 3)), rows, o[q]);
+            }
         };
+        constexpr int steps = 4 * J / U;
         fetch(0, r[0]);
 #pragma unroll
-        for (int s = 0; s < 2 * J; ++s) {
-            if (s + 1 < 2 * J) fetch(s + 1, r[(s + 1) & 1]);
+        for (int s = 0; s < steps; ++s) {
+            if (s + 1 < steps) fetch(s + 1, r[(s + 1) & 1]);
 #pragma unroll
-            for (int q = 0; q < 2; ++q)
+            for (int q = 0; q < U; ++q)
 #pragma unroll
-                for (int k = 0; k < 4; ++k) acc[k] += r[s & 1][q][k];
+                for (int k = 0; k < LS; ++k) acc[k] += r[s & 1][q][k];
         }
     }
 }
 
 // Adds the rows of a block's neighbours: every lane holds the ids of its own
 // four edges.  Ids that no slot holds at the level are dropped first.
-template <int KIND, class T>
-__device__ __forceinline__ void add_block(const WideCtx &x, uint32_t d, uint32_t (&id)[4], T (&acc)[4], bool &ovf) {
+template <int KIND, int NS, class T>
+__device__ __forceinline__ void add_block(const WideCtx &x, uint32_t d, uint32_t (&id)[4], T (&acc)[NS / 4], bool &ovf) {
+    constexpr int LS = NS / 4;
     const unsigned l = threadIdx.x & 3u, sh = threadIdx.x & 28u;
     const uint32_t *act = x.act + (size_t)(KIND == kBack ? d + 1 : d) * x.words;
     uint32_t wd[4];
@@ -284,16 +333,20 @@ __device__ __forceinline__ void add_block(const WideCtx &x, uint32_t d, uint32_t
             for (int q = 0; q < 4; ++q) {
                 const uint32_t u = __shfl_sync(kFull, id[j], sh + q);
                 if (u == kNone) continue;
-                uint32_t r[8];
-                ld32(x.sig + (size_t)u * kWideSlots + l * 4, r);
-                const uint32_t lv = __ldcg(reinterpret_cast<const uint32_t *>(x.lvl) + (size_t)u * 4 + l);
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (((lv >> (8 * k)) & 0xFFu) == d)
-                        acc[k] = wide_add<KIND>(acc[k], (T)((unsigned long long)r[2 * k + 1] << 32 | r[2 * k]), ovf);
+                for (int h = 0; h < LS; h += 4) {
+                    uint32_t r[8];
+                    ld32(x.sig + (size_t)u * NS + l * LS + h, r);
+                    const uint32_t lv =
+                        __ldcg(reinterpret_cast<const uint32_t *>(x.lvl) + (size_t)u * (NS / 4) + l * (LS / 4) + h / 4);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (((lv >> (8 * k)) & 0xFFu) == d)
+                            acc[h + k] = wide_add<KIND>(acc[h + k], (T)((unsigned long long)r[2 * k + 1] << 32 | r[2 * k]), ovf);
+                }
             }
     } else {
-        const unsigned char *rows = rows_of(x, KIND == kBack ? d + 1 : d) + l * (KIND == kFwd32 ? 16 : 32);
+        const unsigned char *rows = rows_of(x, KIND == kBack ? d + 1 : d) + l * (KIND == kFwd32 ? 4 * LS : 8 * LS);
         const bool low = id[0] != kNone || id[1] != kNone, high = id[2] != kNone || id[3] != kNone;
         if (__any_sync(kFull, high)) add_rows<KIND, 4>(rows, id, acc);
         else if (__any_sync(kFull, low)) add_rows<KIND, 2>(rows, id, acc);
@@ -301,126 +354,158 @@ __device__ __forceinline__ void add_block(const WideCtx &x, uint32_t d, uint32_t
 }
 
 // The eight groups' sums of a warp's vertex, added in a fixed order and dealt
-// out one slot a lane: lane 4g + l gets slot 4l + k, k = own_slot's low bits
-// (the lanes of groups g and g ^ 1 the same).
+// out one slot a lane (own_slot): lane 4g + l gets one of the slots LS * l ..,
+// which one by g's bits (16 slots: groups g and g ^ 1 get the same).
+template <int NS>
 __device__ __forceinline__ uint32_t own_slot() {
-    const unsigned lane = threadIdx.x & 31;
-    return 4u * (lane & 3u) + ((lane >> 3) & 3u);
+    const unsigned lane = threadIdx.x & 31, l = lane & 3u, g = lane >> 2;
+    if (NS == 16) return 4u * l + (g >> 1);
+    return 8u * l + g;
 }
-template <int KIND, class T>
-__device__ __forceinline__ T wide_fold(const T (&acc)[4], bool &ovf) {
+// Whether the lane is the one that stores its slot.
+template <int NS>
+__device__ __forceinline__ bool own_store() { return NS == 32 || !(threadIdx.x & 4u); }
+
+template <int KIND, int NS, class T>
+__device__ __forceinline__ T wide_fold(const T (&acc)[NS / 4], bool &ovf) {
+    constexpr int LS = NS / 4;
     const unsigned lane = threadIdx.x & 31;
-    T a0 = (lane & 16u) ? acc[2] : acc[0], a1 = (lane & 16u) ? acc[3] : acc[1];
-    const T b0 = (lane & 16u) ? acc[0] : acc[2], b1 = (lane & 16u) ? acc[1] : acc[3];
-    a0 = wide_add<KIND>(a0, (T)__shfl_xor_sync(kFull, b0, 16), ovf);
-    a1 = wide_add<KIND>(a1, (T)__shfl_xor_sync(kFull, b1, 16), ovf);
-    T c = (lane & 8u) ? a1 : a0;
-    const T e = (lane & 8u) ? a0 : a1;
-    c = wide_add<KIND>(c, (T)__shfl_xor_sync(kFull, e, 8), ovf);
-    return wide_add<KIND>(c, (T)__shfl_xor_sync(kFull, c, 4), ovf);
+    T a[LS];
+#pragma unroll
+    for (int k = 0; k < LS; ++k) a[k] = acc[k];
+#pragma unroll
+    for (int n = LS / 2, o = 16; n >= 1; n /= 2, o /= 2) {
+        const bool up = lane & (unsigned)o;
+#pragma unroll
+        for (int k = 0; k < n; ++k) {
+            const T keep = up ? a[n + k] : a[k], give = up ? a[k] : a[n + k];
+            a[k] = wide_add<KIND>(keep, (T)__shfl_xor_sync(kFull, give, o), ovf);
+        }
+    }
+    if (NS == 16) a[0] = wide_add<KIND>(a[0], (T)__shfl_xor_sync(kFull, a[0], 4), ovf);
+    return a[0];
 }
 
 // Finishing a vertex whose sums lie one slot a lane (wide_fold's order): the
-// whole warp calls, the lanes of even groups store.
+// whole warp calls.
+template <int NS>
 __device__ __forceinline__ uint32_t finish_fwd_warp(const WideCtx &x, uint32_t v, unsigned long long sum, uint32_t d,
                                                     uint32_t &found) {
-    const unsigned lane = threadIdx.x & 31;
-    const uint32_t k = own_slot();
-    const bool mine = !(lane & 4u);
-    unsigned char *lp = x.lvl + (size_t)v * kWideSlots + k;
+    const uint32_t k = own_slot<NS>();
+    unsigned char *lp = x.lvl + (size_t)v * NS + k;
     const uint32_t lv = __ldcg(lp);
     const bool fresh = lv == kUnseen && sum != 0ull;
     const bool got = __any_sync(kFull, fresh), left = __any_sync(kFull, lv == kUnseen && !fresh);
     if (got) {
         found |= 1u;
-        if (mine) reinterpret_cast<uint32_t *>(rows_of(x, d + 1) + (size_t)v * 64)[k] = fresh ? (uint32_t)sum : 0u;
-        if (mine && fresh) {
-            *lp = (unsigned char)(d + 1);
-            x.sig[(size_t)v * kWideSlots + k] = sum;
-            if (sum >> 28) found |= 2u;
+        if (own_store<NS>()) {
+            reinterpret_cast<uint32_t *>(rows_of(x, d + 1))[(size_t)v * NS + k] = fresh ? (uint32_t)sum : 0u;
+            if (fresh) {
+                *lp = (unsigned char)(d + 1);
+                x.sig[(size_t)v * NS + k] = sum;
+                if (sum >> 28) found |= 2u;
+            }
         }
     }
     return (got ? 1u : 0u) | (left ? 0u : 2u);
 }
 
+template <int NS>
 __device__ __forceinline__ void finish_back_warp(const WideCtx &x, const double *mult, uint32_t v, uint32_t reach,
                                                  double sum, uint32_t d) {
-    const unsigned lane = threadIdx.x & 31;
-    const uint32_t k = own_slot();
-    const uint32_t lv = __ldcg(x.lvl + (size_t)v * kWideSlots + k);
+    const uint32_t k = own_slot<NS>();
+    const uint32_t lv = __ldcg(x.lvl + (size_t)v * NS + k);
     double s = 0.0, xo = 0.0;
     if (lv == d) {
-        const double sg = (double)__ldcg(x.sig + (size_t)v * kWideSlots + k);
+        const double sg = (double)__ldcg(x.sig + (size_t)v * NS + k);
         const double delta = (double)reach + sg * sum;
         xo = (1.0 + delta) / sg;
         s = mult[k] * delta;
     }
-    if (!(lane & 4u)) reinterpret_cast<double *>(rows_of(x, d) + (size_t)v * 128)[k] = xo;
+    if (own_store<NS>()) reinterpret_cast<double *>(rows_of(x, d))[(size_t)v * NS + k] = xo;
 #pragma unroll
-    for (int o = 1; o <= 16; o = o == 2 ? 8 : 2 * o) s += __shfl_xor_sync(kFull, s, o);
+    for (int o = 1; o <= 16; o *= 2)
+        if (NS == 32 || o != 4) s += __shfl_xor_sync(kFull, s, o);
     // one add per vertex and sweep, sweeps ordered by the barrier
-    if (lane == 0) atomicAdd(x.bc + v, s);
+    if ((threadIdx.x & 31) == 0) atomicAdd(x.bc + v, s);
 }
 
-// Finishes vertex v from its sums (lane l of its group holds slots 4l ..
-// 4l + 3); every lane of the warp calls it, the ones without a vertex with
-// valid = false.  Forward: the slots not reached yet whose sum is not 0 are
-// at level d + 1.  Returns the bits of v's group: 1 some slot was reached, 2 none is left.
-__device__ __forceinline__ uint32_t finish_fwd(const WideCtx &x, uint32_t v, const unsigned long long (&acc)[4],
+// Finishes vertex v from its sums (lane l of its group holds slots LS * l ..);
+// every lane of the warp calls it, the ones without a vertex with valid =
+// false.  Forward: the slots not reached yet whose sum is not 0 are at level d
+// + 1.  Returns the bits of v's group: 1 some slot was reached, 2 none is left.
+template <int NS>
+__device__ __forceinline__ uint32_t finish_fwd(const WideCtx &x, uint32_t v, const unsigned long long (&acc)[NS / 4],
                                                bool valid, uint32_t d, uint32_t &found) {
-    const unsigned lane = threadIdx.x & 31, l = lane & 3u;
-    uint32_t *lp = reinterpret_cast<uint32_t *>(x.lvl) + (size_t)v * 4 + l;
-    const uint32_t lv = valid ? __ldcg(lp) : 0u;
-    uint32_t nl = lv, f[4];
+    constexpr int LS = NS / 4, LW = LS / 4;
+    const unsigned lane = threadIdx.x & 31, l = lane & 3u, sh = lane & 28u;
+    uint32_t *lp = reinterpret_cast<uint32_t *>(x.lvl) + (size_t)v * (NS / 4) + l * LW;
+    uint32_t nl[LW], f[LS];
+    bool got = false, left = false;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const bool fresh = ((lv >> (8 * k)) & 0xFFu) == kUnseen && acc[k] != 0ull;
-        f[k] = fresh ? (uint32_t)acc[k] : 0u;
-        if (fresh) {
-            nl = (nl & ~(0xFFu << (8 * k))) | ((d + 1) << (8 * k));
-            x.sig[(size_t)v * kWideSlots + 4 * l + k] = acc[k];
-            if (acc[k] >> 28) found |= 2u;
+    for (int h = 0; h < LW; ++h) {
+        const uint32_t lv = valid ? __ldcg(lp + h) : 0u;
+        nl[h] = lv;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int i = 4 * h + k;
+            const bool fresh = ((lv >> (8 * k)) & 0xFFu) == kUnseen && acc[i] != 0ull;
+            f[i] = fresh ? (uint32_t)acc[i] : 0u;
+            if (fresh) {
+                nl[h] = (nl[h] & ~(0xFFu << (8 * k))) | ((d + 1) << (8 * k));
+                x.sig[(size_t)v * NS + LS * l + i] = acc[i];
+                if (acc[i] >> 28) found |= 2u;
+            }
         }
+        if (nl[h] != lv) {
+            lp[h] = nl[h];
+            got = true;
+        }
+        left |= valid && __vcmpeq4(nl[h], kFull) != 0u;
     }
-    const unsigned got = __ballot_sync(kFull, nl != lv);
-    const unsigned left = __ballot_sync(kFull, valid && __vcmpeq4(nl, kFull) != 0u);
-    const unsigned sh = lane & ~3u;
-    if ((got >> sh) & 15u) {
+    const bool any = (__ballot_sync(kFull, got) >> sh) & 15u, rest = (__ballot_sync(kFull, left) >> sh) & 15u;
+    if (any) {
         found |= 1u;
-        *reinterpret_cast<uint4 *>(rows_of(x, d + 1) + (size_t)v * 64 + l * 16) = make_uint4(f[0], f[1], f[2], f[3]);
-        if (nl != lv) *lp = nl;
+        uint4 *row = reinterpret_cast<uint4 *>(rows_of(x, d + 1) + (size_t)v * (NS * 4) + l * (4 * LS));
+#pragma unroll
+        for (int h = 0; h < LW; ++h) row[h] = make_uint4(f[4 * h], f[4 * h + 1], f[4 * h + 2], f[4 * h + 3]);
     }
-    return (((got >> sh) & 15u) ? 1u : 0u) | (((left >> sh) & 15u) ? 0u : 2u);
+    return (any ? 1u : 0u) | (rest ? 0u : 2u);
 }
 
 // Backward: delta = reach + sigma * sum of X over the children, X = (1 +
 // delta) / sigma for the slots at level d, and the weighted delta into the
 // job's vector.
-__device__ __forceinline__ void finish_back(const WideCtx &x, const WideSmem &sm, uint32_t v, const double (&acc)[4],
-                                            bool valid, uint32_t d) {
+template <int NS>
+__device__ __forceinline__ void finish_back(const WideCtx &x, const WideSmem<NS> &sm, uint32_t v,
+                                            const double (&acc)[NS / 4], bool valid, uint32_t d) {
+    constexpr int LS = NS / 4, LW = LS / 4;
     const unsigned l = threadIdx.x & 3u;
     double s = 0.0;
     if (valid) {
-        const uint32_t lv = __ldcg(reinterpret_cast<const uint32_t *>(x.lvl) + (size_t)v * 4 + l);
-        uint32_t w[8];
-        uint32_t r[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) w[k] = 0u;
-        if (__vcmpeq4(lv, d * 0x01010101u)) {
-            const double reach = (double)sm.sub.vinfo[v].y;
-            ld32(x.sig + (size_t)v * kWideSlots + 4 * l, r);
+        for (int h = 0; h < LW; ++h) {
+            const uint32_t lv = __ldcg(reinterpret_cast<const uint32_t *>(x.lvl) + (size_t)v * (NS / 4) + l * LW + h);
+            uint32_t w[8];
+            uint32_t r[8];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                if (((lv >> (8 * k)) & 0xFFu) != d) continue;
-                const double sg = (double)((unsigned long long)r[2 * k + 1] << 32 | r[2 * k]);
-                const double delta = reach + sg * acc[k];
-                const double xo = (1.0 + delta) / sg;
-                w[2 * k] = (uint32_t)__double2loint(xo);
-                w[2 * k + 1] = (uint32_t)__double2hiint(xo);
-                s += sm.mult[4 * l + k] * delta;
+            for (int k = 0; k < 8; ++k) w[k] = 0u;
+            if (__vcmpeq4(lv, d * 0x01010101u)) {
+                const double reach = (double)sm.sub.vinfo[v].y;
+                ld32(x.sig + (size_t)v * NS + LS * l + 4 * h, r);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (((lv >> (8 * k)) & 0xFFu) != d) continue;
+                    const double sg = (double)((unsigned long long)r[2 * k + 1] << 32 | r[2 * k]);
+                    const double delta = reach + sg * acc[4 * h + k];
+                    const double xo = (1.0 + delta) / sg;
+                    w[2 * k] = (uint32_t)__double2loint(xo);
+                    w[2 * k + 1] = (uint32_t)__double2hiint(xo);
+                    s += sm.mult[LS * l + 4 * h + k] * delta;
+                }
             }
+            st32(rows_of(x, d) + (size_t)v * (NS * 8) + l * (8 * LS) + 32 * h, w);
         }
-        st32(rows_of(x, d) + (size_t)v * 128 + l * 32, w);
     }
     s += __shfl_xor_sync(kFull, s, 1);
     s += __shfl_xor_sync(kFull, s, 2);
@@ -430,8 +515,8 @@ __device__ __forceinline__ void finish_back(const WideCtx &x, const WideSmem &sm
 
 // One sweep over the team's share of the job's vertices.
 // (Not inlined: each kind then has the registers to itself.)
-template <int KIND>
-__device__ __noinline__ void wide_sweep(WideSmem &sm, uint32_t d) {
+template <int KIND, int NS>
+__device__ __noinline__ void wide_sweep(WideSmem<NS> &sm, uint32_t d) {
     const WideCtx &x = sm.x;
     using T = typename AccOf<KIND>::T;
     constexpr bool kForward = KIND == kFwd32 || KIND == kFwdFull;
@@ -509,7 +594,7 @@ __device__ __noinline__ void wide_sweep(WideSmem &sm, uint32_t d) {
                 const int i = __ffs(todo) - 1;
                 todo &= todo - 1;
                 const uint32_t vi = __shfl_sync(kFull, v, i), end = se;
-                T acc[4] = {0, 0, 0, 0};
+                T acc[NS / 4] = {};
                 uint32_t at = sb;
                 bool more;
 #pragma unroll 1
@@ -528,18 +613,18 @@ __device__ __noinline__ void wide_sweep(WideSmem &sm, uint32_t d) {
                         se = __shfl_sync(kFull, e1, __ffs(todo) - 1);
                         load_ids(nxt, adj, sb + lane, se, 32u, pol);
                     }
-                    if constexpr (kGather) add_block<KIND>(x, d, id, acc, ovf);
+                    if constexpr (kGather) add_block<KIND, NS>(x, d, id, acc, ovf);
                 } while (more);
-                T sum = wide_fold<KIND>(acc, ovf);
+                T sum = wide_fold<KIND, NS>(acc, ovf);
                 if (heavy) {
                     const uint32_t ci = it * cb + i;
                     const uint32_t c0 = g.cbeg[side][vi] - g.chunk0[side], nc = g.cbeg[side][vi + 1] - g.chunk0[side] - c0;
                     if (nc > 1) {
-                        // the chunks meet: the one that arrives last adds them,
-                        // half warps the even and the odd ones, in order
-                        const uint32_t k = own_slot();
+                        // the chunks meet: the one that arrives last adds them in
+                        // order (16 slots: half warps the even and the odd ones)
+                        const uint32_t k = own_slot<NS>();
                         T *part = reinterpret_cast<T *>(x.part);
-                        if (!(lane & 4u)) __stcg(part + (size_t)ci * kWideSlots + k, sum);
+                        if (own_store<NS>()) __stcg(part + (size_t)ci * NS + k, sum);
                         __syncwarp();
                         uint32_t last = 0;
                         if (lane == 0) {
@@ -551,14 +636,15 @@ __device__ __noinline__ void wide_sweep(WideSmem &sm, uint32_t d) {
                         if (!last) continue;
                         if (lane == 0) x.hcnt[vi] = 0u;
                         sum = 0;
+                        constexpr uint32_t step = NS == 16 ? 2u : 1u;
 #pragma unroll 4
-                        for (uint32_t q = (lane >> 2) & 1u; q < nc; q += 2)
-                            sum = wide_add<KIND>(sum, __ldcg(part + (size_t)(c0 + q) * kWideSlots + k), ovf);
-                        sum = wide_add<KIND>(sum, (T)__shfl_xor_sync(kFull, sum, 4), ovf);
+                        for (uint32_t q = NS == 16 ? (lane >> 2) & 1u : 0u; q < nc; q += step)
+                            sum = wide_add<KIND>(sum, __ldcg(part + (size_t)(c0 + q) * NS + k), ovf);
+                        if (NS == 16) sum = wide_add<KIND>(sum, (T)__shfl_xor_sync(kFull, sum, 4), ovf);
                     }
                 }
                 if constexpr (kForward) {
-                    const uint32_t b = finish_fwd_warp(x, vi, sum, d, found);
+                    const uint32_t b = finish_fwd_warp<NS>(x, vi, sum, d, found);
                     if (lane == 0) {
                         if (b & 1u) {
                             atomicOr(x.act + (size_t)(d + 1) * x.words + (vi >> 5), 1u << (vi & 31u));
@@ -570,7 +656,7 @@ __device__ __noinline__ void wide_sweep(WideSmem &sm, uint32_t d) {
                         }
                     }
                 } else {
-                    finish_back_warp(x, sm.mult, vi, g.vinfo[vi].y, sum, d);
+                    finish_back_warp<NS>(x, sm.mult, vi, g.vinfo[vi].y, sum, d);
                 }
             }
         } else {
@@ -614,7 +700,7 @@ __device__ __noinline__ void wide_sweep(WideSmem &sm, uint32_t d) {
             for (uint32_t i0 = 0; i0 < cnt; i0 += 8) {
                 const bool valid = ok;
                 const uint32_t v = vb + p;
-                T acc[4] = {0, 0, 0, 0};
+                T acc[NS / 4] = {};
                 if constexpr (kGather) {
                     const uint32_t b = sb, e = se;
                     const uint32_t nblk = max(1u, __reduce_max_sync(kFull, (e - b + 15u) / 16u));
@@ -629,13 +715,13 @@ __device__ __noinline__ void wide_sweep(WideSmem &sm, uint32_t d) {
                             pick(i0 + 8, ok, p, sb, se);
                             load_ids(nxt, adj, sb + (lane & 3u), se, 4u, pol);
                         }
-                        add_block<KIND>(x, d, id, acc, ovf);
+                        add_block<KIND, NS>(x, d, id, acc, ovf);
                     }
                 } else {
                     pick(i0 + 8, ok, p, sb, se);
                 }
                 if constexpr (kForward) {
-                    const uint32_t b = finish_fwd(x, v, acc, valid, d, found);
+                    const uint32_t b = finish_fwd<NS>(x, v, acc, valid, d, found);
                     const uint32_t bit = valid ? 1u << (v & 31u) : 0u;
                     const uint32_t am = __reduce_or_sync(kFull, (b & 1u) ? bit : 0u);
                     const uint32_t dm = __reduce_or_sync(kFull, (b & 2u) ? bit : 0u);
@@ -650,7 +736,7 @@ __device__ __noinline__ void wide_sweep(WideSmem &sm, uint32_t d) {
                         }
                     }
                 } else {
-                    finish_back(x, sm, v, acc, valid, d);
+                    finish_back<NS>(x, sm, v, acc, valid, d);
                 }
             }
             __syncwarp();
@@ -674,8 +760,9 @@ __device__ __forceinline__ void wide_trace(const WideArgs &a, uint32_t job, uint
     *a.trace_cnt = i + 1;
 }
 
+template <int NS>
 __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
-    __shared__ WideSmem sm;
+    __shared__ WideSmem<NS> sm;
     WideCtx &x = sm.x;
     const uint32_t team = blockIdx.x / a.team_ctas;
     if (team >= a.teams) return;
@@ -710,8 +797,8 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
         if (a.jobs) {
             J = a.jobs[job];
         } else {  // one graph's sources in order
-            J.root0 = (a.job0 + job) * kWideSlots;
-            J.nroots = min((uint32_t)kWideSlots, a.nroots - J.root0);
+            J.root0 = (a.job0 + job) * NS;
+            J.nroots = min((uint32_t)NS, a.nroots - J.root0);
             J.out = (unsigned long long)job * a.subs[0].n;
         }
         if (threadIdx.x < sizeof(WideSub) / 4)
@@ -725,7 +812,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
             const uint32_t blocks = (sm.sub.offs[1][sm.sub.n] - sm.sub.offs[1][0]) / share;
             sm.nmed = sm.sub.nmed[blocks >= 32 ? 3 : (blocks >= 16 ? 2 : (blocks >= 8 ? 1 : 0))];
         }
-        if (threadIdx.x < kWideSlots) {
+        if (threadIdx.x < NS) {
             const bool has = threadIdx.x < J.nroots;
             uint32_t r = kNone;
             if (has) r = sm.sub.inv[a.roots[J.root0 + threadIdx.x]];
@@ -739,20 +826,20 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
         if (threadIdx.x == 0) sm.left = n;
         if (threadIdx.x < 32) {
             // (16 lists of one graph: the sum may pass 2^32 only on graphs refused on the host)
-            const uint32_t r = lane < kWideSlots ? sm.roots[lane] : kNone;
+            const uint32_t r = lane < NS ? sm.roots[lane] : kNone;
             uint32_t s = r != kNone ? offs1[r + 1] - offs1[r] : 0u;
 #pragma unroll
-            for (int o = 1; o < kWideSlots; o <<= 1) {
+            for (int o = 1; o < NS; o <<= 1) {
                 const uint32_t y = __shfl_up_sync(kFull, s, o);
                 if (lane >= (unsigned)o) s += y;
             }
-            if (lane < kWideSlots) sm.edges[lane + 1] = s;
+            if (lane < NS) sm.edges[lane + 1] = s;
             if (lane == 0) sm.edges[0] = 0;
         }
         __syncthreads();
         // f(k, w) for every neighbour w of the source in slot k
         auto each_first = [&](auto f) {
-            for (uint32_t i = tid; i < sm.edges[kWideSlots]; i += nt) {
+            for (uint32_t i = tid; i < sm.edges[NS]; i += nt) {
                 int k = 0;
                 while (sm.edges[k + 1] <= i) ++k;
                 f(k, adj1[offs1[sm.roots[k]] + (i - sm.edges[k])]);
@@ -768,10 +855,12 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
             }
         }
         for (uint32_t v = tid; v < n; v += nt) {
-            uint32_t w[4] = {kFull, kFull, kFull, kFull};
+            uint32_t w[NS / 4];
+#pragma unroll
+            for (int k = 0; k < NS / 4; ++k) w[k] = kFull;
             bool root = false;
 #pragma unroll
-            for (int k = 0; k < kWideSlots; ++k) {
+            for (int k = 0; k < NS; ++k) {
                 const uint32_t r = sm.roots[k];
                 if (r == kNone) w[k >> 2] = (w[k >> 2] & ~(0xFFu << (8 * (k & 3)))) | (kEmpty << (8 * (k & 3)));
                 if (r == v) {
@@ -779,19 +868,22 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
                     root = true;
                 }
             }
-            reinterpret_cast<uint4 *>(x.lvl)[v] = make_uint4(w[0], w[1], w[2], w[3]);
+#pragma unroll
+            for (int h = 0; h < NS / 16; ++h)
+                reinterpret_cast<uint4 *>(x.lvl)[(size_t)v * (NS / 16) + h] =
+                    make_uint4(w[4 * h], w[4 * h + 1], w[4 * h + 2], w[4 * h + 3]);
             x.bc[v] = 0.0;
             if (root) {
-                uint32_t *row = reinterpret_cast<uint32_t *>(x.g0) + (size_t)v * kWideSlots;
-                for (int k = 0; k < kWideSlots; ++k) {
+                uint32_t *row = reinterpret_cast<uint32_t *>(x.g0) + (size_t)v * NS;
+                for (int k = 0; k < NS; ++k) {
                     row[k] = sm.roots[k] == v;
-                    if (sm.roots[k] == v) x.sig[(size_t)v * kWideSlots + k] = 1ull;
+                    if (sm.roots[k] == v) x.sig[(size_t)v * NS + k] = 1ull;
                 }
             }
         }
         for (uint32_t w = tid; w < (n + 31u) >> 5; w += nt) {
             uint32_t m = 0;
-            for (int k = 0; k < kWideSlots; ++k)
+            for (int k = 0; k < NS; ++k)
                 if (sm.roots[k] >> 5 == w && sm.roots[k] != kNone) m |= 1u << (sm.roots[k] & 31u);
             x.done[w] = 0;
             x.act[w] = m;
@@ -800,10 +892,10 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
         for (uint32_t i = tid; i < sm.sub.nheavy; i += nt) x.hcnt[i] = 0;
         // the rows of level 1 start from 0
         each_first([&](int k, uint32_t w) {
-            if (w != sm.roots[k]) x.sig[(size_t)w * kWideSlots + k] = 0ull;
-            uint4 *row = reinterpret_cast<uint4 *>(rows_of(x, 1) + (size_t)w * 64);
+            if (w != sm.roots[k]) x.sig[(size_t)w * NS + k] = 0ull;
+            uint4 *row = reinterpret_cast<uint4 *>(rows_of(x, 1) + (size_t)w * (NS * 4));
 #pragma unroll
-            for (int h = 0; h < 4; ++h) row[h] = make_uint4(0u, 0u, 0u, 0u);
+            for (int h = 0; h < NS / 4; ++h) row[h] = make_uint4(0u, 0u, 0u, 0u);
         });
         if (!team_sync(a, x, t, sm, wait_ns, 5)) return;
         wide_trace(a, job, 0, 0, n);
@@ -829,17 +921,17 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
                 // they are listed
                 each_first([&](int k, uint32_t w) {
                     if (w == sm.roots[k]) return;
-                    x.lvl[(size_t)w * kWideSlots + k] = 1;
-                    atomicAdd(x.sig + (size_t)w * kWideSlots + k, 1ull);
-                    atomicAdd(reinterpret_cast<uint32_t *>(rows_of(x, 1)) + (size_t)w * kWideSlots + k, 1u);
+                    x.lvl[(size_t)w * NS + k] = 1;
+                    atomicAdd(x.sig + (size_t)w * NS + k, 1ull);
+                    atomicAdd(reinterpret_cast<uint32_t *>(rows_of(x, 1)) + (size_t)w * NS + k, 1u);
                     atomicOr(x.act + x.words + (w >> 5), 1u << (w & 31u));
                 });
-                if (threadIdx.x == 0 && sm.edges[kWideSlots]) {
+                if (threadIdx.x == 0 && sm.edges[NS]) {
                     sm.found = 1;
-                    if (x.rank == 0) sm.count = sm.edges[kWideSlots];  // at most
+                    if (x.rank == 0) sm.count = sm.edges[NS];  // at most
                 }
-            } else if (big) wide_sweep<kFwdFull>(sm, d);
-            else wide_sweep<kFwd32>(sm, d);
+            } else if (big) wide_sweep<kFwdFull, NS>(sm, d);
+            else wide_sweep<kFwd32, NS>(sm, d);
             if (!team_sync(a, x, t, sm, wait_ns, d & 3, d + 1)) return;
             const uint32_t any = sm.any;
             wide_trace(a, job, 2, d, any);
@@ -857,14 +949,14 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
 
         // ---- what each source reached: a thread's vertices, four slots each
         const bool counted = a.rstat || a.total;
-        if (threadIdx.x < 3 * kWideSlots) sm.reach[threadIdx.x] = 0ull;
+        if (threadIdx.x < 3 * NS) sm.reach[threadIdx.x] = 0ull;
         __syncthreads();
         if (counted) {
             uint32_t vis[4] = {0, 0, 0, 0};
             unsigned long long ws[4] = {0, 0, 0, 0}, mc[4] = {0, 0, 0, 0};
-            for (uint32_t i = tid; i < n * 4u; i += nt) {  // n * 4 < 2^32 (checked on the host)
+            for (uint32_t i = tid; i < n * (NS / 4u); i += nt) {  // below 2^32 (checked on the host)
                 const uint32_t lv = __ldcg(reinterpret_cast<const uint32_t *>(x.lvl) + i);
-                const uint2 vi = sm.sub.vinfo[i >> 2];
+                const uint2 vi = sm.sub.vinfo[i / (NS / 4u)];
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     if (((lv >> (8 * k)) & 0xFFu) >= kWideLevels) continue;
@@ -873,41 +965,41 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
                     mc[k] += (unsigned long long)vi.x + 2ull * vi.y;
                 }
             }
-            // nt is a multiple of 4, so a thread's words all belong to slots 4 (lane & 3) ..
+            // nt is a multiple of 8, so a thread's words all belong to the same four slots
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 unsigned long long s0 = vis[k], s1 = ws[k], s2 = mc[k];
 #pragma unroll
-                for (int o = 4; o <= 16; o <<= 1) {
+                for (int o = NS / 4; o <= 16; o <<= 1) {
                     s0 += __shfl_xor_sync(kFull, s0, o);
                     s1 += __shfl_xor_sync(kFull, s1, o);
                     s2 += __shfl_xor_sync(kFull, s2, o);
                 }
-                if (lane < 4 && s0) {
+                if (lane < NS / 4 && s0) {
                     atomicAdd(&sm.reach[4 * lane + k], s0);
-                    atomicAdd(&sm.reach[kWideSlots + 4 * lane + k], s1);
-                    atomicAdd(&sm.reach[2 * kWideSlots + 4 * lane + k], s2);
+                    atomicAdd(&sm.reach[NS + 4 * lane + k], s1);
+                    atomicAdd(&sm.reach[2 * NS + 4 * lane + k], s2);
                 }
             }
         }
         __syncthreads();
-        if (threadIdx.x < kWideSlots && sm.reach[threadIdx.x] && a.total) {
+        if (threadIdx.x < NS && sm.reach[threadIdx.x] && a.total) {
             atomicAdd(&a.total->visited, sm.reach[threadIdx.x]);
-            atomicAdd(&a.total->wsum, sm.reach[kWideSlots + threadIdx.x]);
-            atomicAdd(&a.total->mc2, sm.reach[2 * kWideSlots + threadIdx.x]);
+            atomicAdd(&a.total->wsum, sm.reach[NS + threadIdx.x]);
+            atomicAdd(&a.total->mc2, sm.reach[2 * NS + threadIdx.x]);
             atomicMax(&a.total->depth, D);
-        } else if (threadIdx.x < kWideSlots && sm.reach[threadIdx.x] && a.rstat) {
-            RootStat *rs = a.rstat + (size_t)job * kWideSlots + threadIdx.x;
+        } else if (threadIdx.x < NS && sm.reach[threadIdx.x] && a.rstat) {
+            RootStat *rs = a.rstat + (size_t)job * NS + threadIdx.x;
             atomicAdd(&rs->visited, sm.reach[threadIdx.x]);
-            atomicAdd(&rs->wsum, sm.reach[kWideSlots + threadIdx.x]);
-            atomicAdd(&rs->mc2, sm.reach[2 * kWideSlots + threadIdx.x]);
+            atomicAdd(&rs->wsum, sm.reach[NS + threadIdx.x]);
+            atomicAdd(&rs->mc2, sm.reach[2 * NS + threadIdx.x]);
             rs->depth = D;
         }
 
         // ---- backward
         for (uint32_t e = D; e >= 1; --e) {
-            if (e == D) wide_sweep<kBackLast>(sm, e);
-            else wide_sweep<kBack>(sm, e);
+            if (e == D) wide_sweep<kBackLast, NS>(sm, e);
+            else wide_sweep<kBack, NS>(sm, e);
             if (!team_sync(a, x, t, sm, wait_ns, 4)) return;
             wide_trace(a, job, 3, e, 0);
         }
@@ -981,27 +1073,29 @@ size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
 
 void preload_wide() {
     cudaFuncAttributes at;
-    cudaFuncGetAttributes(&at, (const void *)bc_wide_kernel);
+    cudaFuncGetAttributes(&at, (const void *)bc_wide_kernel<16>);
+    cudaFuncGetAttributes(&at, (const void *)bc_wide_kernel<32>);
     cudaFuncGetAttributes(&at, (const void *)k_wide_reduce);
     preload_wide_form();
 }
 
-size_t wide_layout(WideArgs &a, size_t n, size_t nchunk, size_t nheavy) {
+size_t wide_layout(WideArgs &a, uint32_t slots, size_t n, size_t nchunk, size_t nheavy) {
     const size_t words = (n + 31) / 32;
-    size_t o = up256(n * 16);
+    size_t o = up256(n * slots);
+    a.slots = slots;
     a.o_done = o; o += up256(words * 4);
     a.o_act = o; o += up256(words * 4 * kWideLevels);
-    a.o_sig = o; o += up256(n * 128);
-    a.o_g0 = o; o += up256(n * 128);
-    a.o_g1 = o; o += up256(n * 128);
-    a.o_part = o; o += up256(std::max<size_t>(1, nchunk) * 128);
+    a.o_sig = o; o += up256(n * slots * 8);
+    a.o_g0 = o; o += up256(n * slots * 8);
+    a.o_g1 = o; o += up256(n * slots * 8);
+    a.o_part = o; o += up256(std::max<size_t>(1, nchunk) * slots * 8);
     a.o_hcnt = o; o += up256(std::max<size_t>(1, nheavy) * 4);
     a.stride = o;
     a.words = words;
     return o;
 }
 
-void wide_teams(WideArgs &a, uint64_t njobs, uint64_t entries, size_t state_bytes) {
+double wide_teams(WideArgs &a, uint64_t njobs, uint64_t entries, size_t state_bytes) {
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -1009,14 +1103,15 @@ void wide_teams(WideArgs &a, uint64_t njobs, uint64_t entries, size_t state_byte
     // its entries at 9 ns an entry and CTA, 1.1 times that once the teams'
     // rows are well beyond L2 (fitted on 16-source jobs of R-MAT graphs: 0.1 M
     // entries 540 us on 1 CTA; 7.1 M entries 6,050 us on 13 and 590 us on 148;
-    // 30 M entries 8,800 us on 29 and 1,590 us on 148).  The number of teams
-    // that ends first, its states within state_bytes.
-    constexpr double kFixed = 70.0, kEntry = 0.009, kBeyond = 1.1;
+    // 30 M entries 8,800 us on 29 and 1,590 us on 148), and a job of 32
+    // sources 1.3 to 1.7 times one of 16 (414 us on 3 CTAs, 2,690 us on 148).  The number of teams that ends first, its
+    // states within state_bytes.
+    const double entry = a.slots == 32 ? 0.009 * kWide32 : 0.009, fixed = 70.0, beyond = 1.1;
     double best = 0.0;
     for (uint64_t t = 1; t <= std::min<uint64_t>({njobs, (uint64_t)nsm, kWideTeams}); ++t) {
         if (t > 1 && a.stride * t > state_bytes) break;
-        const double rows = (double)t * (double)a.words * 32.0 * 128.0;
-        const double job = kFixed + (double)entries * kEntry * (rows > 126e6 ? kBeyond : 1.0) / (double)(nsm / t);
+        const double rows = (double)t * (double)a.words * 32.0 * 8.0 * a.slots;
+        const double job = fixed + (double)entries * entry * (rows > 126e6 ? beyond : 1.0) / (double)(nsm / t);
         const double all = (double)((njobs + t - 1) / t) * job;
         if (t == 1 || all < best) {
             best = all;
@@ -1024,13 +1119,27 @@ void wide_teams(WideArgs &a, uint64_t njobs, uint64_t entries, size_t state_byte
         }
     }
     a.team_ctas = (uint32_t)nsm / a.teams;
+    return best;
+}
+
+uint32_t wide_plan(WideArgs &a, uint64_t nroots, uint64_t entries, size_t n, size_t nchunk, size_t nheavy,
+                   size_t state_bytes) {
+    WideArgs b = a;
+    wide_layout(a, 16, n, nchunk, nheavy);
+    const double t16 = wide_teams(a, (nroots + 15) / 16, entries, state_bytes);
+    wide_layout(b, 32, n, nchunk, nheavy);
+    if (b.stride > state_bytes && a.stride <= state_bytes) return 16;
+    if (wide_teams(b, (nroots + 31) / 32, entries, state_bytes) >= t16) return 16;
+    a = b;
+    return 32;
 }
 
 int wide_enqueue(const WideArgs &a, const WideOut *outs, uint32_t nouts, const WideOut &one, uint32_t nmax,
                  cudaStream_t st) {
     WideArgs args = a;
     void *params[] = {&args};
-    CKW(cudaLaunchCooperativeKernel((const void *)bc_wide_kernel, dim3(a.teams * a.team_ctas), dim3(kWideThreads),
+    CKW(cudaLaunchCooperativeKernel(a.slots == 32 ? (const void *)bc_wide_kernel<32> : (const void *)bc_wide_kernel<16>,
+                                    dim3(a.teams * a.team_ctas), dim3(kWideThreads),
                                     params, 0, st));
     const unsigned bx = (unsigned)std::max<size_t>(1, ((size_t)nmax + 31) / 32);
     // (65535 graphs at most in the second dimension)
@@ -1049,35 +1158,21 @@ int wide_chain(const WideArgs &a, const WideOut *outs, uint32_t nouts, uint32_t 
     return BCG_OK;
 }
 
-// What a graph keeps for its wide runs (bcg_graph::wide): its wide form and
-// the buffers of its runs.
+// What a graph keeps for its wide runs (bcg_graph::wide): its wide form, and
+// one buffer for its runs.
 struct WideGraph {
     WideForm form;
-    unsigned char *state = nullptr, *blob = nullptr, *stat = nullptr;
-    double *jobbc = nullptr;
-    size_t state_cap = 0, blob_cap = 0, stat_cap = 0, jobbc_cap = 0;
+    unsigned char *mem = nullptr;
+    size_t cap = 0;
 };
 
 void wide_free(bcg_graph *g) {
     WideGraph *w = g->wide;
     if (!w) return;
     wide_form_free(w->form);
-    dev_free(w->state); dev_free(w->blob); dev_free(w->stat); dev_free(w->jobbc);
+    dev_free(w->mem);
     delete w;
     g->wide = nullptr;
-}
-
-// Grows *p to bytes (the old buffer may be in use on any stream).
-static int grow(unsigned char **p, size_t *cap, size_t bytes) {
-    if (*cap >= bytes) return BCG_OK;
-    if (*p) CKW(cudaDeviceSynchronize());
-    dev_free(*p);
-    *p = nullptr;
-    *cap = 0;
-    CKW(dev_alloc(p, bytes));
-    CKW(cudaStreamSynchronize(0));  // ready for any stream
-    *cap = bytes;
-    return BCG_OK;
 }
 
 WideInput wide_input(const bcg_graph *g) {
@@ -1097,44 +1192,57 @@ WideInput wide_input(const bcg_graph *g) {
 int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, cudaStream_t st, WideResult *res) {
     *res = WideResult{};
     int rc;
-    // out of memory anywhere: the caller's other kernels need less
-    auto give_up = [](int code) { return code == BCG_ERR_OOM ? (cudaGetLastError(), BCG_OK) : code; };
+    bool fresh = false;
+    // (out of memory: the caller's other kernels need less)
     if (!g->wide) {
         g->wide = new WideGraph();
         if ((rc = wide_form_make(g->wide->form, wide_input(g)))) {
             wide_free(g);
-            return give_up(rc);
+            return rc == BCG_ERR_OOM ? (cudaGetLastError(), BCG_OK) : rc;
         }
+        fresh = true;
     }
     WideGraph *w = g->wide;
-    const WideSub &b = w->form.subs[0];
-    const uint64_t njobs = (nroots + kWideSlots - 1) / kWideSlots;
+    const WideSub &b = w->form.subs[0];  // (bounds, on a small graph)
     const size_t n = b.n;
     WideArgs a{};
-    wide_layout(a, n, std::max(b.nchunk[0], b.nchunk[1]), b.nheavy);
-    wide_teams(a, njobs, g->nnz_pruned);
+    const uint32_t slots = wide_plan(a, nroots, g->nnz_pruned, n, std::max(b.nchunk[0], b.nchunk[1]), b.nheavy);
+    const uint64_t njobs = (nroots + slots - 1) / slots;
     // jobs of one launch: their vectors stay under 512 MB
     const uint64_t jl = std::min(njobs, std::max<uint64_t>(a.teams, (512ull << 20) / (n * 8 + 1)));
-    // control words, teams, per-source totals: one block, cleared together
+    // control words, teams, per-source totals (cleared together); weights and
+    // sources (one upload); job vectors; states
     const size_t o_team = sizeof(WideCtrl), o_rstat = o_team + a.teams * sizeof(WideTeam),
-                 stat = o_rstat + njobs * kWideSlots * sizeof(RootStat);
-    const size_t o_roots = up256(nroots * 8), blob = o_roots + up256(nroots * 4);
-    if ((rc = grow(&w->state, &w->state_cap, a.stride * a.teams)) ||
-        (rc = grow(reinterpret_cast<unsigned char **>(&w->jobbc), &w->jobbc_cap, jl * n * 8)) ||
-        (rc = grow(&w->blob, &w->blob_cap, blob)) || (rc = grow(&w->stat, &w->stat_cap, stat)))
-        return give_up(rc);
+                 stat = o_rstat + njobs * slots * sizeof(RootStat), o_blob = up256(stat), o_roots = up256(nroots * 8),
+                 blob = o_roots + up256(nroots * 4), o_jobbc = o_blob + up256(blob), o_state = o_jobbc + up256(jl * n * 8),
+                 need = o_state + a.stride * a.teams;
+    if (w->cap < need) {
+        if (w->mem) CKW(cudaDeviceSynchronize());  // earlier runs (any stream) are done with it
+        dev_free(w->mem);
+        w->mem = nullptr;
+        w->cap = 0;
+        const cudaError_t e = dev_alloc(&w->mem, need);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            return BCG_OK;
+        }
+        CKW(e);
+        w->cap = need;
+        fresh = true;
+    }
+    if (fresh && st != 0) CKW(cudaStreamSynchronize(0));  // what stream 0 made is ready for st
     std::vector<unsigned char> h(blob), hs(stat);
     memcpy(h.data(), mult, nroots * 8);
     memcpy(h.data() + o_roots, roots, nroots * 4);
-    CKW(cudaMemcpyAsync(w->blob, h.data(), blob, cudaMemcpyHostToDevice, st));
+    CKW(cudaMemcpyAsync(w->mem + o_blob, h.data(), blob, cudaMemcpyHostToDevice, st));
     a.subs = w->form.d_subs;
     a.nroots = (uint32_t)nroots;
-    a.mult = reinterpret_cast<const double *>(w->blob);
-    a.roots = reinterpret_cast<const uint32_t *>(w->blob + o_roots);
-    a.jobbc = w->jobbc;
-    a.state = w->state;
-    a.ctrl = reinterpret_cast<WideCtrl *>(w->stat);
-    a.team = reinterpret_cast<WideTeam *>(w->stat + o_team);
+    a.mult = reinterpret_cast<const double *>(w->mem + o_blob);
+    a.roots = reinterpret_cast<const uint32_t *>(w->mem + o_blob + o_roots);
+    a.jobbc = reinterpret_cast<double *>(w->mem + o_jobbc);
+    a.state = w->mem + o_state;
+    a.ctrl = reinterpret_cast<WideCtrl *>(w->mem);
+    a.team = reinterpret_cast<WideTeam *>(w->mem + o_team);
     TraceRec *d_trace = nullptr;
     unsigned int *d_tcnt = nullptr;
     const char *trace_path = getenv("BCG_TRACE_FILE");
@@ -1147,7 +1255,7 @@ int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t n
         a.trace = d_trace;
         a.trace_cnt = d_tcnt;
     }
-    CKW(cudaMemsetAsync(w->stat, 0, stat, st));
+    CKW(cudaMemsetAsync(w->mem, 0, stat, st));
     CKW(cudaEventRecord(g->ev0, st));
     // The jobs are added into bc on the device only if none of them stopped.
     // Several launches add one after the other, so bc is saved before them.
@@ -1160,14 +1268,14 @@ int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t n
     for (uint64_t j0 = 0; j0 < njobs; j0 += jl) {
         a.njobs = (uint32_t)std::min(jl, njobs - j0);
         a.job0 = (uint32_t)j0;
-        a.rstat = reinterpret_cast<RootStat *>(w->stat + o_rstat) + j0 * kWideSlots;
-        if (j0) CKW(cudaMemsetAsync(w->stat, 0, o_rstat, st));
-        if ((rc = wide_enqueue(a, nullptr, 1, WideOut{0, a.njobs, (uint32_t)n, w->form.map, g->d_bc, nullptr}, (uint32_t)n, st)))
+        a.rstat = reinterpret_cast<RootStat *>(w->mem + o_rstat) + j0 * slots;
+        if (j0) CKW(cudaMemsetAsync(w->mem, 0, o_rstat, st));
+        if ((rc = wide_enqueue(a, nullptr, 1, WideOut{0, a.njobs, (uint32_t)n, w->form.map, g->d_bc, w->form.d_subs}, (uint32_t)n, st)))
             return rc;
         res->launches += 2;
         const bool last = j0 + a.njobs >= njobs;
         if (last) CKW(cudaEventRecord(g->ev1, st));
-        CKW(cudaMemcpyAsync(hs.data(), w->stat, last ? stat : sizeof(WideCtrl), cudaMemcpyDeviceToHost, st));
+        CKW(cudaMemcpyAsync(hs.data(), w->mem, last ? stat : sizeof(WideCtrl), cudaMemcpyDeviceToHost, st));
         CKW(cudaStreamSynchronize(st));
         if (c->error || c->overflow || c->deep) break;
     }
@@ -1193,9 +1301,10 @@ int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t n
         res->launches = 0;
         return BCG_OK;
     }
-    res->rstat.resize(njobs * kWideSlots);
+    res->rstat.resize(njobs * slots);
     memcpy(res->rstat.data(), hs.data() + o_rstat, res->rstat.size() * sizeof(RootStat));
     res->batches = njobs;
+    res->slots = slots;
     res->done = true;
     return BCG_OK;
 }

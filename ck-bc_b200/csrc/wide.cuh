@@ -1,5 +1,5 @@
-// Types of the wide-batch searches (wide.cu): 16 sources a job, jobs spread
-// over teams of CTAs.
+// Types of the wide-batch searches (wide.cu): 16 or 32 sources a job, jobs
+// spread over teams of CTAs.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -12,7 +12,6 @@ struct bcg_graph;
 
 namespace bcg {
 
-constexpr int kWideSlots = 16;       // sources of a job
 constexpr int kWideThreads = 640;    // one CTA per SM, 96 registers a thread
 constexpr int kWideWarps = kWideThreads / 32;
 constexpr uint32_t kWideTeams = 148;  // most teams of a launch
@@ -39,7 +38,7 @@ struct WideSub {
     const uint32_t *inv;       // the engine's vertex id -> this numbering
 };
 
-// One job: up to 16 sources of one searched graph.
+// One job: up to `slots` sources of one searched graph.
 struct WideJob {
     uint32_t sub, root0, nroots, pad;
     unsigned long long out;  // its dependencies: bc[out .. out + n) of WideArgs::jobbc
@@ -68,6 +67,7 @@ struct WideArgs {
     const WideJob *jobs;    // nullptr: subs[0]'s sources roots[0 .. nroots) in order, from job job0 on,
                             // job j's vector at j * n
     uint32_t njobs, job0, nroots;
+    uint32_t slots;         // sources of a job: 16 or 32
     uint32_t teams, team_ctas;
     uint32_t split_ctas;    // team size the split of vertices by degree is made for (0: team_ctas);
                             // fixed, a job's sums do not depend on the launch it runs in
@@ -76,7 +76,7 @@ struct WideArgs {
     double *jobbc;
     int *poison;            // several launches' stop word (nullptr: none): set by a launch that
                             // stops, and a launch that finds it set does nothing
-    RootStat *rstat;        // njobs * 16, zeroed (nullptr: not wanted)
+    RootStat *rstat;        // njobs * slots, zeroed (nullptr: not wanted)
     RootStat *total;        // or the sums over all sources, and the deepest level (zeroed)
     WideCtrl *ctrl;
     WideTeam *team;
@@ -122,14 +122,14 @@ struct WideForm {
     unsigned char *mem = nullptr;  // everything below on the device (nullptr: the caller's memory)
     WideSub *d_subs = nullptr;     // one a graph
     uint32_t *inv = nullptr, *map = nullptr;
-    std::vector<WideSub> subs;     // the host's copy (wide_form_make)
+    std::vector<WideSub> subs;     // the host's copy (wide_form_make; of one small graph: bounds)
 };
 
 // Bytes of a form, and of the scratch that building it takes.
 size_t wide_form_bytes(const WideInput &in, size_t *scratch);
 // Enqueues the building in memory of that size on st; f.subs stays empty.
 int wide_form_enqueue(WideForm &f, const WideInput &in, unsigned char *mem, unsigned char *scratch, cudaStream_t st);
-// Allocates, builds on stream 0 and waits.
+// Allocates and builds on stream 0 (waits, but for one small graph).
 int wide_form_make(WideForm &f, const WideInput &in);
 void wide_form_free(WideForm &f);
 
@@ -139,15 +139,20 @@ void preload_wide();
 void preload_wide_form();
 void preload_scan();
 
-// Fills a's state layout for graphs of up to n vertices; returns the stride.
-size_t wide_layout(WideArgs &a, size_t n, size_t nchunk, size_t nheavy);
+// Fills a's state layout for jobs of 16 or 32 slots on graphs of up to n
+// vertices; returns the stride.
+size_t wide_layout(WideArgs &a, uint32_t slots, size_t n, size_t nchunk, size_t nheavy);
 // Whether a graph with so many vertices that have an entry, and so many
 // entries, is shallow enough to be tried: mean degree 6 and up, or too few
 // vertices for more levels than a job holds.
 inline bool wide_shallow(uint64_t active, uint64_t nnz) { return nnz >= 6 * active || active + 2 < kWideLevels; }
 // Cuts the SMs into teams for njobs jobs on lists of so many entries (their
-// mean), a's layout being set.
-void wide_teams(WideArgs &a, uint64_t njobs, uint64_t entries, size_t state_bytes = 512ull << 20);
+// mean), a's layout being set; returns the time in us this is expected to take.
+double wide_teams(WideArgs &a, uint64_t njobs, uint64_t entries, size_t state_bytes = 512ull << 20);
+// Layout and teams for nroots sources of one graph, in jobs of 16 or 32,
+// whichever is expected to end first; returns which.
+uint32_t wide_plan(WideArgs &a, uint64_t nroots, uint64_t entries, size_t n, size_t nchunk, size_t nheavy,
+                   size_t state_bytes = 512ull << 20);
 // One launch of a's jobs and the adding of their vectors: nouts entries of
 // outs (device; nmax vertices at most; 0: nothing is added), or `one` when outs
 // is nullptr.

@@ -348,14 +348,25 @@ int wide_form_enqueue(WideForm &f, const WideInput &in, unsigned char *mem, unsi
 int wide_form_make(WideForm &f, const WideInput &in) {
     size_t scratch_bytes = 0;
     const size_t bytes = wide_form_bytes(in, &scratch_bytes);
+    f.subs.resize(in.graphs);
+    // One small graph: everything in one block, and its description's bounds
+    // stand for it, so that the first run does not wait for the building.
+    const bool small = in.graphs == 1 && !in.directed && in.n <= (1u << 16);
+    CKF(dev_alloc(&f.mem, small ? bytes + scratch_bytes : bytes));
+    if (small) {
+        WideSub &s = f.subs[0];
+        s = WideSub{};
+        s.n = in.n;
+        s.nheavy = (uint32_t)(in.nnz / kWideChunk + 1);
+        s.nchunk[0] = s.nchunk[1] = (uint32_t)(2 * (in.nnz / kWideChunk) + 1);
+        return wide_form_enqueue(f, in, f.mem, f.mem + bytes, 0);
+    }
     unsigned char *scratch = nullptr;
-    CKF(dev_alloc(&f.mem, bytes));
     const cudaError_t e = dev_alloc(&scratch, scratch_bytes);
     int rc = BCG_OK;
     if (e != cudaSuccess)
         rc = set_error(e == cudaErrorMemoryAllocation ? BCG_ERR_OOM : BCG_ERR_CUDA, "wide form: %s", cudaGetErrorString(e));
     if (!rc) rc = wide_form_enqueue(f, in, f.mem, scratch, 0);
-    f.subs.resize(in.graphs);
     if (!rc && cudaMemcpy(f.subs.data(), f.d_subs, in.graphs * sizeof(WideSub), cudaMemcpyDeviceToHost) != cudaSuccess)
         rc = set_error(BCG_ERR_CUDA, "reading the wide form: %s", cudaGetErrorString(cudaGetLastError()));
     dev_free(scratch);  // ordered on stream 0, behind the building

@@ -1,9 +1,9 @@
-"""The wide-batch searches (16 sources a job, teams of CTAs) against the oracle.
+"""The wide-batch searches (16 or 32 sources a job, teams of CTAs) against the oracle.
 
 Plain runs of four roots or more go there on graphs of mean degree 6 and up.
 The cases sit at the edges of its work split: vertices of 31 to 33, 64, 256
 and several thousand entries (four lanes, a warp, chunks), vertex counts
-around 32-vertex words, one to 17 and 33 roots, several components, every
+around 32-vertex words, 1 to 65 roots (one job of 16 to several of 32), several components, every
 pruning mode, directed lists, counts of 2^28 and more (the 32-bit rows do not
 hold them), counts past 2^64 and searches of more than 62 levels (both leave
 the kernel: the run is redone).  The bar is the suite's 1e-9; path counts are
@@ -16,6 +16,7 @@ import oracle
 from test_gpu_parity import assert_bc_close
 
 pytestmark = pytest.mark.gpu
+WIDE = (16, 32)  # sources of a job
 
 
 def _rows(n, degrees, seed):
@@ -47,7 +48,7 @@ def test_matches_oracle(graphs, gname, flags):
     offs, adj = graphs[gname]
     n = len(offs) - 1
     live = np.nonzero(np.diff(offs))[0].astype(np.uint32)
-    for k in (4, 16, 17, 33):
+    for k in (1, 4, 16, 17, 33, 65):
         src = live[np.linspace(0, len(live) - 1, min(k, len(live))).astype(int)]
         ref, ost = oracle.bc(offs, adj, src, nthreads=oracle.max_threads())
         with bcg.Graph(offs, adj, flags) as G:
@@ -55,7 +56,7 @@ def test_matches_oracle(graphs, gname, flags):
             got = G.bc()
             G.run(src)
             twice = G.bc()
-        assert flags or st.batch_width == 16
+        assert flags or st.batch_width in WIDE
         assert_bc_close(got, ref, f"{gname} k={k} flags={flags}")
         assert_bc_close(twice, 2 * ref, f"{gname} k={k} flags={flags} accumulated")
         assert st.teps_edges == ost["teps_edges"] and st.skipped == ost["skipped"]
@@ -86,7 +87,7 @@ def test_directed():
     ref, ost = oracle.bc(offs, adj, src)
     with bcg.Graph(offs, adj, bcg.DIRECTED) as G:
         st = G.run(src)
-        assert st.batch_width == 16
+        assert st.batch_width in WIDE
         assert_bc_close(G.bc(), ref, "directed")
 
 
@@ -105,7 +106,7 @@ def test_large_counts(depth, ext):
     ref, _ = oracle.bc_q(offs, adj, src)
     with bcg.Graph(offs, adj) as G:
         st = G.run(src)
-        assert st.extended_sigma == ext and (ext or st.batch_width == 16)
+        assert st.extended_sigma == ext and (ext or st.batch_width in WIDE)
         assert_bc_close(G.bc(), ref, f"layers {depth}")
 
 
@@ -117,7 +118,7 @@ def test_deep_search_leaves():
     ref, _ = oracle.bc_q(offs, adj, src)
     with bcg.Graph(offs, adj) as G:
         st = G.run(src)
-        assert st.max_depth > 62 and st.batch_width != 16
+        assert st.max_depth > 62 and st.batch_width not in WIDE
         assert_bc_close(G.bc(), ref, "deep")
         G.run(src)
         assert_bc_close(G.bc(), 2 * ref, "deep twice")
@@ -133,7 +134,7 @@ def test_batch_of_shallow_graphs():
     with bcg.Batch(graphs) as B:
         for runs in (1, 2):
             st = B.run()
-            assert st.batch_width == 16 and B.info()["captured"]
+            assert st.batch_width in WIDE and B.info()["captured"]
             edges = 0
             for i, (offs, adj) in enumerate(graphs):
                 ref, ost = oracle.bc(offs, adj, np.arange(len(offs) - 1), nthreads=oracle.max_threads())
@@ -159,7 +160,7 @@ def test_batch_with_a_deep_graph():
     with bcg.Batch(graphs) as B:
         for runs in (1, 2):
             st = B.run()
-            assert st.batch_width != 16 and st.max_depth > 62
+            assert st.batch_width not in WIDE and st.max_depth > 62
             for i, (offs, adj) in enumerate(graphs):
                 ref, _ = oracle.bc(offs, adj, np.arange(len(offs) - 1), nthreads=oracle.max_threads())
                 assert_bc_close(B.bc(i), runs * ref, f"graph {i}")

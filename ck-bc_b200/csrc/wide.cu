@@ -44,7 +44,7 @@
 // adds the vectors in job order, so the result does not depend on which team
 // ran a job, nor on what else ran.
 //
-// Coherence.  Rows, levels and counts are read with .cg loads.  The bitmaps
+// Coherence.  Levels and counts are read with .cg loads.  The bitmaps and rows
 // are read through L1: they are written in one sweep and read in later ones,
 // and the barrier's acquire and fences order the two.
 #include <algorithm>
@@ -131,35 +131,44 @@ __device__ __forceinline__ void st32(void *p, const uint32_t (&w)[8]) {
                  "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "l"(p)
                  : "memory");
 }
-// A lane's part of row u of doubles, or of 32-bit counts (0 where u is kNone).
-// Not volatile: rows do not change during the sweep that reads them, so the
-// loads may move.
+// A lane's part of row u of doubles, or of 32-bit counts.  Not volatile: rows
+// do not change during the sweep that reads them, so the loads may move.
+// Through L1, which keeps the row of zeros that stands for ids to be left out:
+// no load or add needs a test.  Except for the doubles of 32 slots, where a row
+// of zeros costs as much as another (its 256 bytes go through the register
+// port all the same) and the rows drive the bitmaps out of L1: they are tested
+// and read past it.  (Benchmark's graph, the two large forward sweeps of a job
+// of 32: 377 and 493 us tested, 347 and 415 us with zeros; the two large
+// backward ones 437 and 664 us tested, 608 and 745 us with zeros.  4M-vertex
+// graph, job of 16, forward 1,442 -> 1,040 us, backward 1,702 -> 1,425 us.)
 template <int N>
-__device__ __forceinline__ void ld_row(uint32_t u, const unsigned char *rows, double (&r)[N]) {
+__device__ __forceinline__ void ld_row(uint32_t u, uint32_t zero, const unsigned char *rows, double (&r)[N]) {
+    if constexpr (N == 4) {
+        asm("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
+            : "=d"(r[0]), "=d"(r[1]), "=d"(r[2]), "=d"(r[3])
+            : "l"(rows + (size_t)u * 128));
+    } else {
 #pragma unroll
-    for (int k = 0; k < N; ++k) r[k] = 0.0;
-    if (u != kNone) {
+        for (int k = 0; k < N; ++k) r[k] = 0.0;
+        if (u != zero) {
 #pragma unroll
-        for (int k = 0; k < N; k += 4)
-            asm("ld.global.cg.v4.f64 {%0,%1,%2,%3}, [%4];"
-                : "=d"(r[k]), "=d"(r[k + 1]), "=d"(r[k + 2]), "=d"(r[k + 3])
-                : "l"(rows + (size_t)u * (32 * N) + 8 * k));
+            for (int k = 0; k < N; k += 4)
+                asm("ld.global.cg.v4.f64 {%0,%1,%2,%3}, [%4];"
+                    : "=d"(r[k]), "=d"(r[k + 1]), "=d"(r[k + 2]), "=d"(r[k + 3])
+                    : "l"(rows + (size_t)u * 256 + 8 * k));
+        }
     }
 }
 template <int N>
-__device__ __forceinline__ void ld_row(uint32_t u, const unsigned char *rows, uint32_t (&r)[N]) {
-#pragma unroll
-    for (int k = 0; k < N; ++k) r[k] = 0u;
-    if (u != kNone) {
-        if constexpr (N == 4)
-            asm("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];"
-                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                : "l"(rows + (size_t)u * 64));
-        else
-            asm("ld.global.cg.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                : "l"(rows + (size_t)u * 128));
-    }
+__device__ __forceinline__ void ld_row(uint32_t u, uint32_t, const unsigned char *rows, uint32_t (&r)[N]) {
+    if constexpr (N == 4)
+        asm("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+            : "l"(rows + (size_t)u * 64));
+    else
+        asm("ld.global.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+            : "l"(rows + (size_t)u * 128));
 }
 // An adjacency entry: streamed, so evicted before the rows.
 __device__ __forceinline__ uint32_t ld_adj(const uint32_t *p, unsigned long long pol) {
@@ -247,13 +256,14 @@ __device__ __forceinline__ T wide_add(T x, T y, bool &ovf) {
     return s;
 }
 
-// The ids of a lane's edges base + step * j, j < 4, below end.
+// The ids of a lane's edges base + step * j, j < 4, below end; past it zero,
+// the id of the row of zeros (the graph's number of vertices).
 __device__ __forceinline__ void load_ids(uint32_t (&id)[4], const uint32_t *__restrict__ adj, uint32_t base,
-                                         uint32_t end, uint32_t step, unsigned long long pol) {
+                                         uint32_t end, uint32_t step, uint32_t zero, unsigned long long pol) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const uint32_t e = base + step * j;
-        id[j] = e < end ? ld_adj(adj + e, pol) : kNone;
+        id[j] = e < end ? ld_adj(adj + e, pol) : zero;
     }
 }
 
@@ -261,7 +271,8 @@ __device__ __forceinline__ void load_ids(uint32_t (&id)[4], const uint32_t *__re
 // edges one after the other, each lane LS slots of a row, the next rows in
 // flight (32 registers of them) while the last are added.
 template <int KIND, int J, int LS, class T>
-__device__ __forceinline__ void add_rows(const unsigned char *rows, const uint32_t (&id)[4], T (&acc)[LS]) {
+__device__ __forceinline__ void add_rows(const unsigned char *rows, uint32_t zero, const uint32_t (&id)[4],
+                                         T (&acc)[LS]) {
     const unsigned sh = threadIdx.x & 28u;
     if constexpr (KIND == kFwd32) {
         constexpr int U = 16 / LS;  // rows of a step
@@ -273,7 +284,7 @@ __device__ __forceinline__ void add_rows(const unsigned char *rows, const uint32
 #pragma unroll
             for (int q = 0; q < U; ++q) {
                 const int e = s * U + q;
-                ld_row(__shfl_sync(kFull, id[e >> 2], sh + (e & 3)), rows, o[q]);
+                ld_row(__shfl_sync(kFull, id[e >> 2], sh + (e & 3)), zero, rows, o[q]);
             }
         };
         constexpr int steps = 4 * J / U;
@@ -297,7 +308,7 @@ __device__ __forceinline__ void add_rows(const unsigned char *rows, const uint32
 #pragma unroll
             for (int q = 0; q < U; ++q) {
                 const int e = s * U + q;
-                ld_row(__shfl_sync(kFull, id[e >> 2], sh + (e & 3)), rows, o[q]);
+                ld_row(__shfl_sync(kFull, id[e >> 2], sh + (e & 3)), zero, rows, o[q]);
             }
         };
         constexpr int steps = 4 * J / U;
@@ -314,25 +325,27 @@ __device__ __forceinline__ void add_rows(const unsigned char *rows, const uint32
 }
 
 // Adds the rows of a block's neighbours: every lane holds the ids of its own
-// four edges.  Ids that no slot holds at the level are dropped first.
+// four edges.  Ids that no slot holds at the level become the row of zeros.
 template <int KIND, int NS, class T>
-__device__ __forceinline__ void add_block(const WideCtx &x, uint32_t d, uint32_t (&id)[4], T (&acc)[NS / 4], bool &ovf) {
+__device__ __forceinline__ void add_block(const WideCtx &x, uint32_t d, uint32_t zero, uint32_t (&id)[4],
+                                          T (&acc)[NS / 4], bool &ovf) {
     constexpr int LS = NS / 4;
     const unsigned l = threadIdx.x & 3u, sh = threadIdx.x & 28u;
     const uint32_t *act = x.act + (size_t)(KIND == kBack ? d + 1 : d) * x.words;
     uint32_t wd[4];
+    // (zero's word may be the next level's first: in the array, and without effect)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) wd[j] = id[j] != kNone ? act[id[j] >> 5] : 0u;
+    for (int j = 0; j < 4; ++j) wd[j] = act[id[j] >> 5];
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-        if (!((wd[j] >> (id[j] & 31u)) & 1u)) id[j] = kNone;
+        if (!((wd[j] >> (id[j] & 31u)) & 1u)) id[j] = zero;
     if constexpr (KIND == kFwdFull) {
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll 1
             for (int q = 0; q < 4; ++q) {
                 const uint32_t u = __shfl_sync(kFull, id[j], sh + q);
-                if (u == kNone) continue;
+                if (u == zero) continue;
 #pragma unroll
                 for (int h = 0; h < LS; h += 4) {
                     uint32_t r[8];
@@ -347,9 +360,9 @@ __device__ __forceinline__ void add_block(const WideCtx &x, uint32_t d, uint32_t
             }
     } else {
         const unsigned char *rows = rows_of(x, KIND == kBack ? d + 1 : d) + l * (KIND == kFwd32 ? 4 * LS : 8 * LS);
-        const bool low = id[0] != kNone || id[1] != kNone, high = id[2] != kNone || id[3] != kNone;
-        if (__any_sync(kFull, high)) add_rows<KIND, 4>(rows, id, acc);
-        else if (__any_sync(kFull, low)) add_rows<KIND, 2>(rows, id, acc);
+        const bool low = id[0] != zero || id[1] != zero, high = id[2] != zero || id[3] != zero;
+        if (__any_sync(kFull, high)) add_rows<KIND, 4>(rows, zero, id, acc);
+        else if (__any_sync(kFull, low)) add_rows<KIND, 2>(rows, zero, id, acc);
     }
 }
 
@@ -587,7 +600,7 @@ __device__ __noinline__ void wide_sweep(WideSmem<NS> &sm, uint32_t d) {
             if (todo) {
                 sb = __shfl_sync(kFull, e0, __ffs(todo) - 1);
                 se = __shfl_sync(kFull, e1, __ffs(todo) - 1);
-                load_ids(nxt, adj, sb + lane, se, 32u, pol);
+                load_ids(nxt, adj, sb + lane, se, 32u, g.n, pol);
             }
 #pragma unroll 1
             while (todo) {
@@ -607,13 +620,13 @@ __device__ __noinline__ void wide_sweep(WideSmem<NS> &sm, uint32_t d) {
                     at += 128u;
                     more = at < end;
                     if (more) {
-                        load_ids(nxt, adj, at + lane, end, 32u, pol);
+                        load_ids(nxt, adj, at + lane, end, 32u, g.n, pol);
                     } else if (todo) {
                         sb = __shfl_sync(kFull, e0, __ffs(todo) - 1);
                         se = __shfl_sync(kFull, e1, __ffs(todo) - 1);
-                        load_ids(nxt, adj, sb + lane, se, 32u, pol);
+                        load_ids(nxt, adj, sb + lane, se, 32u, g.n, pol);
                     }
-                    if constexpr (kGather) add_block<KIND, NS>(x, d, id, acc, ovf);
+                    if constexpr (kGather) add_block<KIND, NS>(x, d, g.n, id, acc, ovf);
                 } while (more);
                 T sum = wide_fold<KIND, NS>(acc, ovf);
                 if (heavy) {
@@ -695,7 +708,7 @@ __device__ __noinline__ void wide_sweep(WideSmem<NS> &sm, uint32_t d) {
             bool ok;
             uint32_t p, sb, se, nxt[4];
             pick(0, ok, p, sb, se);
-            if constexpr (kGather) load_ids(nxt, adj, sb + (lane & 3u), se, 4u, pol);
+            if constexpr (kGather) load_ids(nxt, adj, sb + (lane & 3u), se, 4u, g.n, pol);
 #pragma unroll 1
             for (uint32_t i0 = 0; i0 < cnt; i0 += 8) {
                 const bool valid = ok;
@@ -710,12 +723,12 @@ __device__ __noinline__ void wide_sweep(WideSmem<NS> &sm, uint32_t d) {
 #pragma unroll
                         for (int j = 0; j < 4; ++j) id[j] = nxt[j];
                         if (k < nblk) {
-                            load_ids(nxt, adj, b + 16u * k + (lane & 3u), e, 4u, pol);
+                            load_ids(nxt, adj, b + 16u * k + (lane & 3u), e, 4u, g.n, pol);
                         } else if (i0 + 8 < cnt) {
                             pick(i0 + 8, ok, p, sb, se);
-                            load_ids(nxt, adj, sb + (lane & 3u), se, 4u, pol);
+                            load_ids(nxt, adj, sb + (lane & 3u), se, 4u, g.n, pol);
                         }
-                        add_block<KIND, NS>(x, d, id, acc, ovf);
+                        add_block<KIND, NS>(x, d, g.n, id, acc, ovf);
                     }
                 } else {
                     pick(i0 + 8, ok, p, sb, se);
@@ -890,6 +903,14 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
             x.act[x.words + w] = 0;
         }
         for (uint32_t i = tid; i < sm.sub.nheavy; i += nt) x.hcnt[i] = 0;
+        // the rows of zeros: row n of the counts' rows and of the doubles'
+        if (x.rank == 0 && threadIdx.x < NS) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                reinterpret_cast<uint32_t *>(rows_of(x, h))[(size_t)n * NS + threadIdx.x] = 0u;
+                reinterpret_cast<double *>(rows_of(x, h))[(size_t)n * NS + threadIdx.x] = 0.0;
+            }
+        }
         // the rows of level 1 start from 0
         each_first([&](int k, uint32_t w) {
             if (w != sm.roots[k]) x.sig[(size_t)w * NS + k] = 0ull;
@@ -1086,8 +1107,8 @@ size_t wide_layout(WideArgs &a, uint32_t slots, size_t n, size_t nchunk, size_t 
     a.o_done = o; o += up256(words * 4);
     a.o_act = o; o += up256(words * 4 * kWideLevels);
     a.o_sig = o; o += up256(n * slots * 8);
-    a.o_g0 = o; o += up256(n * slots * 8);
-    a.o_g1 = o; o += up256(n * slots * 8);
+    a.o_g0 = o; o += up256((n + 1) * slots * 8);
+    a.o_g1 = o; o += up256((n + 1) * slots * 8);
     a.o_part = o; o += up256(std::max<size_t>(1, nchunk) * slots * 8);
     a.o_hcnt = o; o += up256(std::max<size_t>(1, nheavy) * 4);
     a.stride = o;

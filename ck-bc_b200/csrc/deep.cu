@@ -5,19 +5,23 @@
 // 3,960 levels of about 1,060 vertices a source), so a level costs what its
 // chain of dependent loads and its barrier cost.  A sweep over the whole
 // chip pays a grid barrier and its work lists for every level and batch of
-// six sources: about 28 us.  Here a CTA, or a cluster of up to 8 where there
+// six sources: about 28 us.  Here a CTA, or a cluster of up to 16 where there
 // are fewer sources than would fill the chip, runs one source by itself: the
 // barrier is __syncthreads or the cluster's, and sources are independent.
-// (A level's states lie far apart, each load its own sector, and one SM has
-// only so many misses in flight: on the 2048 x 2048 grid a forward level takes
-// it 24 us and a backward one 13; clusters of 2, 4 and 8 take 16, 10 and 7,
-// and 8, 5 and 4.  On a 300 x 290 grid, 150 vertices a level, all take about 6
-// and 2.6: there it is the chain of latencies alone.)
+// A level's states lie far apart, each load its own sector: an SM issues one
+// of those in about 3 cycles and an atomic in about 10, so large frontiers
+// want several SMs.  (2048 x 2048 grid, a forward and a backward level
+// together, clusters of 4, 5, 8, 12 and 16: 14.0, 12.5, 9.2, 7.9 and 7.5 us.
+// 300 x 290 grid, 150 vertices a level: 9.1 us with one CTA, 6.3 with 4; there
+// it is a chain of latencies: on the way forward two round trips to L2 (1,300
+// cycles each), the sum and the queue (1,500), the barrier (1,600); on the way
+// back one round trip, the sum (1,000) and the barrier.)
 //   - vertices have at most 4 (or 8) neighbours, kept as one 16-byte (two)
 //     row, so there is no row start to look up first;
 //   - the frontier is a queue in shared memory that carries each vertex's
-//     neighbour row, read when the vertex was found; in a cluster every warp
-//     sends what it found to the queue of one CTA, in turn;
+//     neighbour row, read when the vertex was found; in a cluster it stays in
+//     the finder's CTA while the CTAs' shares are about even, and is dealt to
+//     all by the warp otherwise;
 //   - one pass a level: the vertices of level d read the states of their
 //     neighbours once, which gives both the sum over the parents (level d - 1,
 //     finished) and the neighbours not reached yet, which are claimed for
@@ -47,7 +51,8 @@ namespace bcg {
 
 namespace {
 
-constexpr int kDeepThreads = 1024;
+constexpr int kDeepThreads = 512;      // most of a CTA
+constexpr uint32_t kDeepCluster = 16;  // most CTAs of a source
 constexpr uint32_t kFull = 0xffffffffu;
 constexpr uint32_t kNone = 0xffffffffu;    // no neighbour
 constexpr uint32_t kUnseen = 0xffffffffu;  // level of a vertex not reached
@@ -94,17 +99,46 @@ __device__ __forceinline__ Row<D> ell_row(const uint32_t *ell, uint32_t v) {
     return r;
 }
 
-// States are written by other threads of the CTA: always read from L2.
+// States are written by other threads of the cluster: always read from L2.
 __device__ __forceinline__ void ld_state(const DeepState *p, unsigned long long &val, uint32_t &lvl, uint32_t &kids) {
     uint32_t a, b;
     asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(a), "=r"(b), "=r"(lvl), "=r"(kids) : "l"(p) : "memory");
     val = (unsigned long long)b << 32 | a;
 }
 
+// Adds the terms that bit q of `which` names, x[q], in order of q, one of
+// them a step: a warp takes as many steps as one of its lanes has terms (two
+// on most of a grid's levels, and the first costs no addition).
+template <int D, class T, class Add>
+__device__ __forceinline__ T add_terms(const unsigned long long (&x)[D], uint32_t which, Add add) {
+    T sum = T();
+#pragma unroll 1
+    for (bool first = true; which; first = false) {
+        const uint32_t q = (uint32_t)__ffs(which) - 1u;
+        which &= which - 1u;
+        unsigned long long t = x[0];
+#pragma unroll
+        for (int k = 1; k < D; ++k) t = q == (uint32_t)k ? x[k] : t;
+        sum = add(sum, t, first);
+    }
+    return sum;
+}
+
+__device__ __forceinline__ unsigned long long ld_val(const DeepState *p) {
+    unsigned long long v;
+    asm volatile("ld.global.cg.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
 // Entries a queue holds in shared memory (two queues); a larger frontier's
 // tail is read back from the order list.
 template <int D>
 constexpr uint32_t queue_cap() { return D == 4 ? 5000u : 2700u; }
+
+template <bool EXT>
+struct SumOf { using T = double; };
+template <>
+struct SumOf<true> { using T = unsigned long long; };
 
 template <int D>
 struct DeepSmem {
@@ -128,6 +162,7 @@ __device__ __forceinline__ T *peer(T *p, uint32_t C, uint32_t rank) {
 template <int D, bool EXT>
 __global__ void __launch_bounds__(kDeepThreads, 1) bc_deep_kernel(DeepArgs a) {
     extern __shared__ __align__(16) unsigned char deep_raw[];
+    static_assert(D <= 8, "neighbours of a row");
     DeepSmem<D> &sm = *reinterpret_cast<DeepSmem<D> *>(deep_raw);
     constexpr uint32_t Q = queue_cap<D>();
     const uint32_t C = a.cluster, s = blockIdx.x / C, rank = blockIdx.x % C;
@@ -149,34 +184,38 @@ __global__ void __launch_bounds__(kDeepThreads, 1) bc_deep_kernel(DeepArgs a) {
     if (tid < 3) sm.tot[tid] = 0ull;
     source_sync(C);
     // ---- forward: one pass a level
-    uint32_t d = 0, base = 0, size = 0;  // the level, its place in order, its size
+    const uint32_t logC = 31u - __clz(C);
+    uint32_t d = 0, base = 0;  // the level, its place in order
     unsigned long long vis = 0, wsum = 0, mc2 = 0;
     bool too_deep = false;
     for (;; ++d) {
-        // the level's vertices: cnt in this CTA's queue, at order[first ..]
-        const uint32_t ring = d % 3u;
-        uint32_t cnt, first = base;
-        if (C == 1) {
-            cnt = size = sm.cnt[ring];
-        } else {
-            const uint32_t mine = lane < C ? *peer(&sm.cnt[ring], C, lane) : 0u;
-            cnt = __shfl_sync(kFull, mine, rank);
+        const uint32_t ring = d % 3u, cnt = sm.cnt[ring];  // the level's vertices in this CTA's queue,
+        uint32_t size = cnt, first = base;                 // in all, and where this CTA's start in order
+        // (the other CTAs' counts are asked for here and used once the level's
+        // own loads are on their way)
+        const uint32_t mine = C == 1 ? 0u : (lane < C ? *peer(&sm.cnt[ring], C, lane) : 0u);
+        bool known = C == 1, deal = false;
+        auto counts = [&]() {
+            if (known) return;
+            known = true;
             size = __reduce_add_sync(kFull, mine);
-            first += __reduce_add_sync(kFull, lane < rank ? mine : 0u);
-        }
+            first = base + __reduce_add_sync(kFull, lane < rank ? mine : 0u);
+            // What a CTA finds stays with it while the CTAs' shares differ by
+            // little and cannot outgrow a queue; else the warps' finds are
+            // dealt to all.
+            const uint32_t most = __reduce_max_sync(kFull, mine);
+            deal = most > (size >> logC) + (size >> (logC + 2u)) + 32u || most > Q / (D - 1);
+        };
         // (one barrier a level: what a faster thread has written since is the
         // next level's, in another entry of the ring, with a higher stop level)
         if (d && sm.stop < d) {
             if (tid == 0 && rank == 0) a.ctrl->overflow = 1;
             break;
         }
-        too_deep = size && d > kMaxLevel;
-        if (!size || too_deep) break;
-        if (tid == 0 && rank == 0) lbeg[d] = base;
-        const uint32_t c = d & 1u, to = (d + 1u) % 3u, next = base + size;
+        const uint32_t c = d & 1u, to = (d + 1u) % 3u;
         int seen_stop = 0;
         if (tid == 0 && (d & 31u) == 0) seen_stop = *reinterpret_cast<volatile int *>(&a.ctrl->overflow);
-        for (uint32_t i0 = tid & ~31u; i0 < cnt; i0 += kDeepThreads) {
+        for (uint32_t i0 = tid & ~31u; i0 < cnt; i0 += blockDim.x) {
             const uint32_t i = i0 + lane;
             const bool has = i < cnt;
             uint32_t v = 0;
@@ -187,7 +226,6 @@ __global__ void __launch_bounds__(kDeepThreads, 1) bc_deep_kernel(DeepArgs a) {
                 if (i < Q) {
                     v = sm.v[c][i];
                     nb = sm.nb[c][i];
-                    order[first + i] = v;
                 } else {
                     v = __ldcg(order + first + i);
                     nb = ell_row<D>(a.ell, v);
@@ -195,42 +233,53 @@ __global__ void __launch_bounds__(kDeepThreads, 1) bc_deep_kernel(DeepArgs a) {
             }
             uint32_t lv[D];
             unsigned long long val[D];
-#pragma unroll
-            for (int q = 0; q < D; ++q) {
-                lv[q] = 0u;
-                uint32_t unused;
-                if (nb.u[q] != kNone) ld_state(state + nb.u[q], val[q], lv[q], unused);
-            }
-            uint32_t reach = 0;
-            if (has && a.vinfo) reach = a.vinfo[v].y;
-            // claim the neighbours not reached yet, their rows on the way
-            uint32_t old[D];
             Row<D> far[D];
 #pragma unroll
             for (int q = 0; q < D; ++q) {
-                old[q] = 0u;
-                if (nb.u[q] != kNone && lv[q] == kUnseen) {
-                    old[q] = atomicExch(&state[nb.u[q]].lvl, d + 1u);
+                lv[q] = d;
+                val[q] = 0ull;
+                uint32_t unused;
+                if (nb.u[q] != kNone) ld_state(state + nb.u[q], val[q], lv[q], unused);
+            }
+            // claim the neighbours not reached yet, their rows on the way (an
+            // SM issues an atomic in about 10 cycles: none is spent on others)
+#pragma unroll
+            for (int q = 0; q < D; ++q) {
+                if (lv[q] == kUnseen) {
+                    lv[q] = atomicExch(&state[nb.u[q]].lvl, d + 1u);
                     if (D == 4) far[q] = ell_row<D>(a.ell, nb.u[q]);
                 }
             }
+            uint32_t reach = 0;
+            if (has && a.vinfo) reach = a.vinfo[v].y;
+            counts();
+            if (has && i < Q) order[first + i] = v;
+            uint32_t won[D], total = 0;
+#pragma unroll
+            for (int q = 0; q < D; ++q) {
+                won[q] = __ballot_sync(kFull, lv[q] == kUnseen);
+                total += __popc(won[q]);
+            }
+            const uint32_t dest = deal ? ((i0 >> 5) + rank + d) & (C - 1u) : rank;
+            uint32_t at = 0;
+            if (total && lane == 0) at = dest == rank ? atomicAdd(&sm.cnt[to], total) : atomicAdd(peer(&sm.cnt[to], C, dest), total);
             if (has) {
-                unsigned long long sum = 0ull;
-                uint32_t kids = 0, deg = 0;
+                uint32_t kids = 0, parents = 0, deg = 0;
                 bool ovf = false;
 #pragma unroll
                 for (int q = 0; q < D; ++q) {
                     if (nb.u[q] == kNone) continue;
                     ++deg;
                     if (lv[q] == kUnseen || lv[q] == d + 1u) kids |= 1u << q;
-                    if (lv[q] + 1u != d) continue;
-                    if (EXT) {
-                        sum = ext_add(sum, val[q]);
-                    } else {
-                        sum += val[q];
-                        ovf |= sum < val[q];
-                    }
+                    if (lv[q] + 1u == d) parents |= 1u << q;
                 }
+                unsigned long long sum = add_terms<D, unsigned long long>(
+                    val, parents, [&](unsigned long long x, unsigned long long y, bool one) {
+                        if (one) return y;
+                        if (EXT) return ext_add(x, y);
+                        ovf |= x + y < y;
+                        return x + y;
+                    });
                 if (d == 0) sum = EXT ? kExtOne : 1ull;
                 *reinterpret_cast<uint4 *>(state + v) = make_uint4((uint32_t)sum, (uint32_t)(sum >> 32), d, kids);
                 if (ovf) seen_stop = 1;
@@ -238,21 +287,11 @@ __global__ void __launch_bounds__(kDeepThreads, 1) bc_deep_kernel(DeepArgs a) {
                 wsum += 1ull + reach;
                 mc2 += (unsigned long long)deg + 2ull * reach;
             }
-            unsigned won[D];
-            uint32_t total = 0;
-#pragma unroll
-            for (int q = 0; q < D; ++q) {
-                won[q] = __ballot_sync(kFull, old[q] == kUnseen);
-                total += __popc(won[q]);
-            }
+            __syncwarp();
             if (total) {
-                // a warp's finds go to one queue, the warps' in turn
-                const uint32_t dest = C == 1 ? 0u : ((i0 >> 5) + rank + d) % C;
-                uint32_t at = 0;
-                if (lane == 0) at = atomicAdd(peer(&sm.cnt[to], C, dest), total);
                 at = __shfl_sync(kFull, at, 0);
-                uint32_t *qv = peer(&sm.v[c ^ 1u][0], C, dest);
-                Row<D> *qn = peer(&sm.nb[c ^ 1u][0], C, dest);
+                uint32_t *qv = dest == rank ? &sm.v[c ^ 1u][0] : peer(&sm.v[c ^ 1u][0], C, dest);
+                Row<D> *qn = dest == rank ? &sm.nb[c ^ 1u][0] : peer(&sm.nb[c ^ 1u][0], C, dest);
 #pragma unroll
                 for (int q = 0; q < D; ++q) {
                     if ((won[q] >> lane) & 1u) {
@@ -261,7 +300,7 @@ __global__ void __launch_bounds__(kDeepThreads, 1) bc_deep_kernel(DeepArgs a) {
                             qv[p] = nb.u[q];
                             qn[p] = D == 4 ? far[q] : ell_row<D>(a.ell, nb.u[q]);
                         } else if (C == 1) {
-                            order[next + p] = nb.u[q];
+                            order[base + size + p] = nb.u[q];
                         } else {
                             a.ctrl->full = 1;  // the host runs it again with one CTA a source
                             seen_stop = 1;
@@ -271,12 +310,16 @@ __global__ void __launch_bounds__(kDeepThreads, 1) bc_deep_kernel(DeepArgs a) {
                 }
             }
         }
+        counts();
+        too_deep = size && d > kMaxLevel;
+        if (!size || too_deep) break;
+        if (tid == 0 && rank == 0) lbeg[d] = base;
         if (seen_stop)
             for (uint32_t k = 0; k < C; ++k) *peer(&sm.stop, C, k) = d;
         // (last read two barriers ago)
         if (tid == 0) sm.cnt[(d + 2u) % 3u] = 0;
         source_sync(C);
-        base = next;
+        base += size;
     }
     if (too_deep || (d && sm.stop < d)) {
         if (too_deep && tid == 0 && rank == 0) a.ctrl->deep = 1;
@@ -309,7 +352,8 @@ __global__ void __launch_bounds__(kDeepThreads, 1) bc_deep_kernel(DeepArgs a) {
     // thread is known (v1) and its row and state are loaded while level e is
     // worked on; of level e - 2 the vertex is loaded.
     // (a level's warps are dealt to the CTAs in turn)
-    const uint32_t t0 = ((tid >> 5) * C + rank) * 32u + lane, per = C * kDeepThreads;
+    const uint32_t t0 = ((tid >> 5) * C + rank) * 32u + lane, per = C * blockDim.x;
+    using Sum = typename SumOf<EXT>::T;
     struct Item {
         uint32_t v;
         Row<D> nb;
@@ -322,47 +366,42 @@ __global__ void __launch_bounds__(kDeepThreads, 1) bc_deep_kernel(DeepArgs a) {
         ld_state(state + it.v, it.sig, lvl, it.kids);
         it.reach = a.vinfo ? a.vinfo[it.v].y : 0u;
     };
+    auto kids_of = [&](const Item &it, unsigned long long (&x)[D]) {
+#pragma unroll
+        for (int q = 0; q < D; ++q)
+            if ((it.kids >> q) & 1u) x[q] = ld_val(state + it.nb.u[q]);
+    };
     auto finish = [&](const Item &it, const unsigned long long (&x)[D]) {
+        const Sum sum = add_terms<D, Sum>(x, it.kids, [&](Sum s, unsigned long long y, bool one) -> Sum {
+            if constexpr (EXT) return one ? y : ext_add(s, y);
+            else return s + __longlong_as_double((long long)y);
+        });
         double dl;
         unsigned long long xo;
-        if (EXT) {
-            unsigned long long sum = 0ull;
-#pragma unroll
-            for (int q = 0; q < D; ++q)
-                if ((it.kids >> q) & 1u) sum = ext_add(sum, x[q]);
+        if constexpr (EXT) {
             dl = (double)it.reach + ext_to_double(ext_mul(it.sig, sum));
             xo = ext_div(1.0 + dl, it.sig);
         } else {
-            double sum = 0.0;
-#pragma unroll
-            for (int q = 0; q < D; ++q)
-                if ((it.kids >> q) & 1u) sum += __longlong_as_double((long long)x[q]);
             dl = (double)it.reach + (double)it.sig * sum;
             xo = (unsigned long long)__double_as_longlong((1.0 + dl) / (double)it.sig);
         }
         *reinterpret_cast<uint4 *>(state + it.v) =
             make_uint4((uint32_t)xo, (uint32_t)(xo >> 32), (uint32_t)__double2loint(dl), (uint32_t)__double2hiint(dl));
     };
-    auto kids_of = [&](const Item &it, unsigned long long (&x)[D]) {
-#pragma unroll
-        for (int q = 0; q < D; ++q)
-            if ((it.kids >> q) & 1u) x[q] = __ldcg(&state[it.nb.u[q]].val);
-    };
     // starts of levels e, e - 1, e - 2
     uint32_t end = base, b0 = __ldcg(lbeg + depth), b1 = depth >= 2u ? __ldcg(lbeg + depth - 1) : 0u;
-    Item it{};
+    Item even{}, odd{};
     uint32_t v1 = 0;
     if (t0 < end - b0) {
-        it.v = __ldcg(order + b0 + t0);
-        load(it);
+        even.v = __ldcg(order + b0 + t0);
+        load(even);
     }
     if (depth >= 2u && t0 < b0 - b1) v1 = __ldcg(order + b1 + t0);
-    for (uint32_t e = depth; e >= 1u; --e) {
+    auto level = [&](uint32_t e, Item &it, Item &nx) {
         const uint32_t n0 = end - b0, n1 = e >= 2u ? b0 - b1 : 0u;
         const uint32_t b2 = e >= 3u ? __ldcg(lbeg + e - 2) : 0u;
         unsigned long long x[D];
         if (t0 < n0) kids_of(it, x);
-        Item nx{};
         nx.v = v1;
         if (t0 < n1) load(nx);
         if (t0 < n0) finish(it, x);
@@ -373,11 +412,15 @@ __global__ void __launch_bounds__(kDeepThreads, 1) bc_deep_kernel(DeepArgs a) {
             finish(it, x);
         }
         if (e >= 3u && t0 < b1 - b2) v1 = __ldcg(order + b2 + t0);
-        it = nx;
         end = b0;
         b0 = b1;
         b1 = b2;
         source_sync(C);
+    };
+    for (uint32_t e = depth; e >= 1u; --e) {
+        level(e, even, odd);
+        if (--e == 0u) break;
+        level(e, odd, even);
     }
     // the source's own dependencies do not count
     if (rank == 0 && tid == 0) state[a.roots[s]] = DeepState{1ull, 0u, 0u};
@@ -421,14 +464,24 @@ __global__ void k_deep_rows(uint32_t n, const uint32_t *__restrict__ offs, const
                              #call, cudaGetErrorString(e_));                                       \
     } while (0)
 
+// Launches a.nroots sources in clusters of up to `most` CTAs: as many a source
+// as leave every source room on the chip.  Clusters of more than 8 are not
+// promised by the architecture, and fewer of them fit than the SMs would
+// allow: the device is asked.
 template <int D, bool EXT>
-cudaError_t launch_deep(const DeepArgs &a, cudaStream_t st) {
+cudaError_t launch_deep(DeepArgs &a, uint32_t most, uint32_t nsm, cudaStream_t st) {
     const void *f = (const void *)bc_deep_kernel<D, EXT>;
     cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeepSmem<D>));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
+    a.cluster = 1;
+    while (a.cluster < most && a.nroots * 2 * a.cluster <= nsm) a.cluster *= 2;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(a.nroots * a.cluster);
-    cfg.blockDim = dim3(kDeepThreads);
+    // (threads, measured on 2048 x 2048 vertices: clusters of 16 25.1 ms with
+    // 256 and 26.5 with 512, of 8 30.1 and 29.8, of 4 45.8 and 42.0; 148
+    // sources of 1000 x 1000, a CTA each: 34.7 and 32.7)
+    cfg.blockDim = dim3(a.cluster >= 8 ? kDeepThreads / 2 : kDeepThreads);
     cfg.dynamicSmemBytes = sizeof(DeepSmem<D>);
     cfg.stream = st;
     cudaLaunchAttribute at{};
@@ -437,6 +490,15 @@ cudaError_t launch_deep(const DeepArgs &a, cudaStream_t st) {
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
+    if (a.cluster > 8) {
+        int fit = 0;
+        e = cudaOccupancyMaxActiveClusters(&fit, f, &cfg);
+        if (e != cudaSuccess || (uint32_t)fit < a.nroots) {
+            cudaGetLastError();
+            at.val.clusterDim.x = a.cluster = 8;
+            cfg.gridDim = dim3(a.nroots * 8u);
+        }
+    }
     DeepArgs args = a;
     void *params[] = {&args};
     return cudaLaunchKernelExC(&cfg, f, params);
@@ -523,9 +585,6 @@ static int deep_launch(bcg_graph *g, const uint32_t *roots, const double *mult, 
     memcpy(up_.data(), mult, nroots * sizeof(double));
     memcpy(up_.data() + (o_roots - o_mult), roots, nroots * sizeof(uint32_t));
     const bool several = slots < nroots;
-    // as many CTAs a source as leave every source room on the chip
-    a.cluster = 1;
-    while (a.cluster < most_ctas && slots * 2 * a.cluster <= (uint64_t)nsm) a.cluster *= 2;
     CKD(cudaEventRecord(g->ev0, st));
     CKD(cudaMemsetAsync(w->mem, 0, o_mult, st));  // control words and the sources' totals
     CKD(cudaMemcpyAsync(w->mem + o_mult, up_.data(), up_.size(), cudaMemcpyHostToDevice, st));
@@ -539,8 +598,8 @@ static int deep_launch(bcg_graph *g, const uint32_t *roots, const double *mult, 
         a.roots = reinterpret_cast<const uint32_t *>(w->mem + o_roots) + s0;
         a.rstat = reinterpret_cast<RootStat *>(w->mem + o_rstat) + s0;
         k_deep_init<<<nsm * 8, 256, 0, st>>>((uint64_t)a.nroots * n, a.state);
-        CKD(D == 4 ? (ext ? launch_deep<4, true>(a, st) : launch_deep<4, false>(a, st))
-                   : (ext ? launch_deep<8, true>(a, st) : launch_deep<8, false>(a, st)));
+        CKD(D == 4 ? (ext ? launch_deep<4, true>(a, most_ctas, nsm, st) : launch_deep<4, false>(a, most_ctas, nsm, st))
+                   : (ext ? launch_deep<8, true>(a, most_ctas, nsm, st) : launch_deep<8, false>(a, most_ctas, nsm, st)));
         k_deep_reduce<<<(n + 255) / 256, 256, 0, st>>>(a.ctrl, n, a.nroots,
                                                        reinterpret_cast<const double *>(w->mem + o_mult) + s0, a.state,
                                                        g->d_ext, g->d_bc);
@@ -568,7 +627,7 @@ static int deep_launch(bcg_graph *g, const uint32_t *roots, const double *mult, 
 
 int deep_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, bool ext, cudaStream_t st,
              DeepResult *res) {
-    return deep_launch(g, roots, mult, nroots, ext, 8, st, res);
+    return deep_launch(g, roots, mult, nroots, ext, kDeepCluster, st, res);
 }
 
 }  // namespace bcg

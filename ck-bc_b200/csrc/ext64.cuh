@@ -16,62 +16,30 @@ constexpr int kExtBias = 32768 + 48;
 constexpr unsigned long long kExtOne = 0x8000000000000000ull;  // 1.0: E = 32768, f = 0
 constexpr unsigned long long kExtFrac = (1ull << 48) - 1;
 
-__host__ __device__ __forceinline__ unsigned long long ext_pack(int e, unsigned long long m) {
-    // m in [2^48, 2^49); an exponent outside the encodable range saturates
-    if (e < 1) return 0ull;
-    if (e > 65535) return ~0ull;
-    return ((unsigned long long)e << 48) | (m & kExtFrac);
-}
-
-// s in [2^59, 2^61) stands for the value s * 2^(e - kExtBias - 11) (with more
-// nonzero bits below s when `sticky`); rounds it to a 49-bit significand.
-__host__ __device__ __forceinline__ unsigned long long ext_round(unsigned long long s, bool sticky, int e) {
-    if (s >= (1ull << 60)) {
-        sticky |= (s & 1ull) != 0;
-        s >>= 1;
-        ++e;
-    }
-    unsigned long long m = s >> 11;
-    const unsigned long long rb = s & 0x7FFull;
-    if (rb > 0x400ull || (rb == 0x400ull && (sticky || (m & 1ull)))) {
-        ++m;
-        if (m == (1ull << 49)) {
-            m >>= 1;
-            ++e;
-        }
-    }
-    return ext_pack(e, m);
+// s in [2^61, 2^63) stands for the value s * 2^(e - kExtBias - 13), its bit 0
+// set where more bits follow below; rounds it to a 49-bit significand.  (No
+// branch: the lanes of a warp round alike, and a chain of these operations is
+// what a level of a deep search waits for.)
+__host__ __device__ __forceinline__ unsigned long long ext_round(unsigned long long s, int e) {
+    const int up = (int)(s >> 62), sh = 13 + up;
+    const unsigned long long m = (s + ((1ull << (sh - 1)) - 1ull) + ((s >> sh) & 1ull)) >> sh;  // up to 2^49
+    const int f = e + up + (int)(m >> 49);
+    unsigned long long r = ((unsigned long long)(e + up) << 48) + (m - (1ull << 48));
+    r = f > 65535 ? ~0ull : r;  // an exponent outside the encodable range saturates
+    return f < 1 ? 0ull : r;
 }
 
 __host__ __device__ __forceinline__ unsigned long long ext_add(unsigned long long a, unsigned long long b) {
-    if (!a) return b;
-    if (!b) return a;
-    if (a < b) {
-        const unsigned long long t = a;
-        a = b;
-        b = t;
-    }
-    const int ea = (int)(a >> 48), eb = (int)(b >> 48);
-    const int d = ea - eb;
-    const unsigned long long A = ((a & kExtFrac) | (1ull << 48)) << 11;
-    const unsigned long long B = ((b & kExtFrac) | (1ull << 48)) << 11;
-    unsigned long long bs;
-    bool sticky;
-    if (d == 0) {
-        bs = B;
-        sticky = false;
-    } else if (d < 64) {
-        bs = B >> d;
-        sticky = (B << (64 - d)) != 0;
-    } else {
-        bs = 0;
-        sticky = true;
-    }
-    return ext_round(A + bs, sticky, ea);
+    const unsigned long long x = a < b ? b : a, y = a < b ? a : b;
+    const int e = (int)(x >> 48), gap = e - (int)(y >> 48), d = gap < 63 ? gap : 63;
+    const unsigned long long A = ((x & kExtFrac) | (1ull << 48)) << 13;
+    const unsigned long long B = y ? ((y & kExtFrac) | (1ull << 48)) << 13 : 0ull;
+    const unsigned long long t = B >> d;
+    const unsigned long long r = ext_round((A + t) | ((t << d) != B ? 1ull : 0ull), e);
+    return x ? r : 0ull;
 }
 
 __host__ __device__ __forceinline__ unsigned long long ext_mul(unsigned long long a, unsigned long long b) {
-    if (!a || !b) return 0ull;
     const unsigned long long ma = (a & kExtFrac) | (1ull << 48), mb = (b & kExtFrac) | (1ull << 48);
 #ifdef __CUDA_ARCH__
     const unsigned long long hi = __umul64hi(ma, mb), lo = ma * mb;
@@ -79,12 +47,12 @@ __host__ __device__ __forceinline__ unsigned long long ext_mul(unsigned long lon
     const unsigned __int128 p = (unsigned __int128)ma * mb;
     const unsigned long long hi = (unsigned long long)(p >> 64), lo = (unsigned long long)p;
 #endif
-    // p = ma * mb in [2^96, 2^98), value p * 2^(ea + eb - 2 bias); s = p >> 37 in
-    // [2^59, 2^61) stands for s * 2^(e - bias - 11) (ext_round's scaling), so
-    // e - bias - 11 = 37 + ea + eb - 2 bias, i.e. e = ea + eb - bias + 48
-    const unsigned long long s = (hi << 27) | (lo >> 37);
-    const bool sticky = (lo & ((1ull << 37) - 1)) != 0;
-    return ext_round(s, sticky, (int)(a >> 48) + (int)(b >> 48) - kExtBias + 48);
+    // p = ma * mb in [2^96, 2^98), value p * 2^(ea + eb - 2 bias); s = p >> 35 in
+    // [2^61, 2^63) stands for s * 2^(e - bias - 13) (ext_round's scaling), so
+    // e - bias - 13 = 35 + ea + eb - 2 bias, i.e. e = ea + eb - bias + 48
+    const unsigned long long s = (hi << 29) | (lo >> 35) | ((lo & ((1ull << 35) - 1)) ? 1ull : 0ull);
+    const unsigned long long r = ext_round(s, (int)(a >> 48) + (int)(b >> 48) - kExtBias + 48);
+    return a && b ? r : 0ull;
 }
 
 // x > 0 finite double -> extended value x * 2^k.
@@ -96,15 +64,15 @@ __host__ __device__ __forceinline__ unsigned long long ext_from_double(double x,
     const int be = (int)(bits >> 52);
     if (be != 0) {  // a normal number: its fields are the significand and exponent
         q = be - 1022;
-        return ext_round(((bits & ((1ull << 52) - 1)) | (1ull << 52)) << 8, false, q + k - 50 + kExtBias);
+        return ext_round(((bits & ((1ull << 52) - 1)) | (1ull << 52)) << 9, q + k - 49 + kExtBias);
     }
 #endif
     const double m = frexp(x, &q);  // x = m * 2^q, m in [0.5, 1)
     // 53-bit integer significand D = m * 2^53, x * 2^k = D * 2^(q - 53 + k);
-    // s = D * 2^8 in [2^60, 2^61) stands for s * 2^(e - bias - 11), so
-    // e = q + k - 50 + bias
+    // s = D * 2^9 in [2^61, 2^62) stands for s * 2^(e - bias - 13), so
+    // e = q + k - 49 + bias
     const unsigned long long D = (unsigned long long)ldexp(m, 53);
-    return ext_round(D << 8, false, q + k - 50 + kExtBias);
+    return ext_round(D << 9, q + k - 49 + kExtBias);
 }
 
 // Extended value -> double (inf / 0 outside the double range).

@@ -1,6 +1,6 @@
 """One CTA or cluster a source (graphs of at most 8 neighbours a vertex)
 against the oracle: both row widths (4 and 8 neighbours), frontiers from one
-vertex to more than a cluster's queues hold, few sources (clusters of 8) and
+vertex to more than a cluster's queues hold, few sources (clusters of 16) and
 more than the chip has SMs, path counts that fit uint64, that overflow it
 midway, and that are extended from the start, in every pruning mode.  The bar
 is the suite's 1e-9; the sums run in list order, so two runs give the same bits."""

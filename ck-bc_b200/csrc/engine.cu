@@ -18,12 +18,16 @@
 // (isolated in the pruned graph) still gets its exact bc, and vertices
 // outside a root's component get nothing from it (the reference adds
 // reach * (reach_v0 + 1) to them, cuda_kernels.cu:274, 1095).
+#include <sys/mman.h>
+
 #include <algorithm>
+#include <atomic>
 #include <cinttypes>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <thread>
 #include <unordered_map>
 #include <vector>
 
@@ -166,6 +170,50 @@ cudaError_t tmp_alloc(void **p, size_t bytes, cudaStream_t st) {
 }
 
 cudaError_t tmp_free(void *p, cudaStream_t st) { return p ? cudaFreeAsync(p, st) : cudaSuccess; }
+
+// Copies a result to the caller's (pageable) memory.  A result buffer is
+// usually fresh, and the copy then waits for one page fault after another: 32
+// MB take 1.6 ms into pages that are there and 7.0 ms into fresh huge ones.  So
+// two threads populate the pages ahead of the copy (no byte is changed; a range
+// that cannot be populated is left to the copy to report): 3.5 ms.  One thread
+// 4.3, three 3.8, four 4.0 to 4.8: their page clearing takes the copy's memory
+// bandwidth.  Below 4 MB a copy takes less than the threads' start is worth.
+static cudaError_t copy_out(void *dst, const void *src, size_t bytes) {
+#ifdef MADV_POPULATE_WRITE
+    constexpr uintptr_t kPart = 2u << 20;  // at multiples of a huge page, so that no two threads meet in one
+    constexpr size_t kCopy = 8u << 20, kLeast = 4u << 20;
+    if (bytes >= kLeast && std::thread::hardware_concurrency() >= 4) {
+        const uintptr_t a = ((uintptr_t)dst + 4095) & ~uintptr_t(4095), z = ((uintptr_t)dst + bytes) & ~uintptr_t(4095);
+        const uintptr_t a0 = a / kPart * kPart;
+        const size_t parts = (z - a0 + kPart - 1) / kPart;
+        std::atomic<size_t> next{0}, done{0};
+        auto populate = [&]() {
+            for (size_t p; (p = next.fetch_add(1)) < parts; done.fetch_add(1)) {
+                const uintptr_t b = std::max(a, a0 + p * kPart), e = std::min(z, a0 + (p + 1) * kPart);
+                (void)madvise((void *)b, e - b, MADV_POPULATE_WRITE);
+            }
+        };
+        std::thread help[2];
+        unsigned nt = 0;
+        try {
+            for (; nt < 2; ++nt) help[nt] = std::thread(populate);
+        } catch (...) {  // no thread to be had: one helper or none
+        }
+        cudaError_t e = cudaSuccess;
+        for (size_t at = 0; at < bytes && e == cudaSuccess; at += kCopy) {
+            const size_t m = std::min(kCopy, bytes - at);
+            // (parts are taken in order: with two more done than the copy
+            // needs, at most one of its own is still in work)
+            const size_t want = std::min(parts, (at + m + kPart - 1) / kPart + 2);
+            while (nt && done.load() < want) std::this_thread::yield();
+            e = cudaMemcpy((char *)dst + at, (const char *)src + at, m, cudaMemcpyDeviceToHost);
+        }
+        for (unsigned k = 0; k < nt; ++k) help[k].join();
+        return e;
+    }
+#endif
+    return cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost);
+}
 
 static void graph_free(bcg_graph *g) {
     if (!g) return;
@@ -880,7 +928,7 @@ int bcg_run_device(bcg_graph *g, const uint32_t *d_sources, uint64_t nsrc, void 
 int bcg_get_bc(bcg_graph *g, double *bc_host) {
     clear_error();
     if (!g || !bc_host) return set_error(BCG_ERR_ARG, "null argument");
-    CK(cudaMemcpy(bc_host, g->d_bc, (size_t)g->n * sizeof(double), cudaMemcpyDeviceToHost));
+    CK(copy_out(bc_host, g->d_bc, (size_t)g->n * sizeof(double)));
     return BCG_OK;
 }
 

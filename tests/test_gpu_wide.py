@@ -201,3 +201,24 @@ def test_served_waves(deep):
     if not deep:
         for i in (0, 3, 6):
             assert np.array_equal(served[i].view(np.uint64), _served(pool, [reqs[i]])[0].view(np.uint64)), i
+
+
+@pytest.mark.parametrize("n", [524287, 524288, 2000003])
+@pytest.mark.parametrize("shift", [0, 1, 511])
+def test_large_result_into_fresh_and_odd_buffers(n, shift):
+    """Results from about 4 MB on, at any 8-byte place of a fresh buffer or of
+    one in use: the same values, and nothing beside them."""
+    offs, adj = bcg.from_pairs([[i, i + 1] for i in range(50)] + [[n - 2, n - 1], [n - 3, n - 2]], n)
+    with bcg.Graph(offs, adj) as G:
+        G.run([0, 20, n - 1])
+        want = np.zeros(n)
+        want[1:50] = 49.0 - np.arange(49)  # from vertex 0
+        want[1:20] += np.arange(1, 20)     # from vertex 20
+        want[21:50] += 49.0 - np.arange(20, 49)
+        want[n - 2] = 1.0
+        for fill in (0.0, 3.5):
+            buf = np.zeros(n + 1024) if fill == 0.0 else np.full(n + 1024, fill)
+            out = buf[shift:shift + n]
+            assert bcg.lib().bcg_get_bc(G.h, out.ctypes.data_as(bcg._f64p)) == 0
+            assert np.array_equal(out, want)
+            assert np.all(buf[:shift] == fill) and np.all(buf[shift + n:] == fill)

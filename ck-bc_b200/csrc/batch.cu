@@ -207,6 +207,22 @@ int build_wide(bcg_batch *b) {
     CKB(cudaMemcpy(b->d_wide, jobs.data(), jobs.size() * sizeof(WideJob), cudaMemcpyHostToDevice));
     CKB(cudaMemcpy(b->d_wide + o_roots, roots.data(), roots.size() * 4, cudaMemcpyHostToDevice));
     CKB(cudaMemcpy(b->d_wide + o_outs, outs.data(), outs.size() * sizeof(WideOut), cudaMemcpyHostToDevice));
+    // a graph's sources in the order its jobs should take them, if there is
+    // memory for a second list (a set's jobs are of many graphs: 6.2 -> 5.6 ms
+    // on 48 R-MAT graphs)
+    uint32_t *tmp = nullptr;
+    if ((e = dev_alloc(&tmp, roots.size() * 8)) == cudaSuccess) {
+        CKB(cudaMemcpy(tmp, roots.data(), roots.size() * 4, cudaMemcpyHostToDevice));
+        uint32_t *to = reinterpret_cast<uint32_t *>(b->d_wide + o_roots);
+        size_t r = 0;
+        for (uint32_t p = 0; p < G && !rc; r += act[p], ++p)
+            if (act[p] > kBatchSlots)
+                rc = wide_order(b->form.d_subs + p, tmp + r, nullptr, act[p], tmp + roots.size() + r, to + r, nullptr, nullptr, 0);
+        dev_free(tmp);
+        if (rc) return give_up(rc);
+    } else {
+        cudaGetLastError();
+    }
     CKB(cudaDeviceSynchronize());  // everything is ready for the batch's stream
     size_t at = 0;
     for (size_t i = 0; i < spans.size(); ++i) {

@@ -153,6 +153,11 @@ double wide_teams(WideArgs &a, uint64_t njobs, uint64_t entries, size_t state_by
 // whichever is expected to end first; returns which.
 uint32_t wide_plan(WideArgs &a, uint64_t nroots, uint64_t entries, size_t n, size_t nchunk, size_t nheavy,
                    size_t state_bytes = 512ull << 20);
+// Puts a graph's nroots sources (and weights, unless nullptr) in the order in
+// which its jobs should take them; order (nullptr: not wanted) says which came
+// to each place.  key: nroots words of scratch.  Windows of 8192 sources.
+int wide_order(const WideSub *sub, const uint32_t *roots, const double *mult, uint32_t nroots, uint32_t *key,
+               uint32_t *roots_to, double *mult_to, uint32_t *order, cudaStream_t st);
 // One launch of a's jobs and the adding of their vectors: nouts entries of
 // outs (device; nmax vertices at most; 0: nothing is added), or `one` when outs
 // is nullptr.

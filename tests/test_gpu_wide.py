@@ -222,3 +222,29 @@ def test_large_result_into_fresh_and_odd_buffers(n, shift):
             assert bcg.lib().bcg_get_bc(G.h, out.ctypes.data_as(bcg._f64p)) == 0
             assert np.array_equal(out, want)
             assert np.all(buf[:shift] == fill) and np.all(buf[shift + n:] == fill)
+
+
+@pytest.mark.parametrize("k", [1, 31, 33, 300, 8191, 8192, 8193, 20000])
+def test_sources_out_of_order(k):
+    """Jobs take their sources in an order of their own: weights and totals
+    must follow.  Repeated sources (weights above 1), sources without an edge,
+    one and several windows of 8,192, against the same sources one by one in
+    the totals and the oracle in the values."""
+    offs, adj = bcg.generate("rmat:scale=15,ef=8,seed=9")
+    n = len(offs) - 1
+    rng = np.random.default_rng(k)
+    src = rng.permutation(n)[:k].astype(np.uint32)
+    if k > 32:
+        src[::7] = src[1]
+    few = min(k, 40)
+    ref, ost = oracle.bc_q(offs, adj, src[:few])
+    with bcg.Graph(offs, adj) as G:
+        G.run(src[:few])
+        assert_bc_close(G.bc(), ref, f"first {few}")
+        G.reset()
+        st = G.run(src)
+        whole = G.bc()
+        G.reset()
+        parts = [G.run(p) for p in np.array_split(src, max(1, k // 1000))]  # other jobs, other companions
+        assert_bc_close(whole, G.bc(), f"k={k}")
+        assert st.teps_edges == sum(p.teps_edges for p in parts) and st.skipped == sum(p.skipped for p in parts)

@@ -233,6 +233,7 @@ static void graph_free(bcg_graph *g) {
     dev_free(g->d_ext);
     wide_free(g);
     deep_free(g);
+    small_free(g);
     dev_free(g->d_rows); dev_free(g->d_ctrl);
     dev_free(g->d_roots); dev_free(g->d_pend); dev_free(g->d_mult); dev_free(g->d_rstat);
     if (g->ev0) cudaEventDestroy(g->ev0);
@@ -554,6 +555,20 @@ static int run_plan(bcg_graph *g, const RunPlan &p, cudaStream_t st, bcg_stats *
     // plain runs of a width that is not forced: the wide-batch kernel, or one
     // CTA a source on graphs of few neighbours (both wait for their results)
     const bool free_run = !debug && p.plain && !g->forced_width && (stats || g->sigma_mode == BCG_SIGMA_AUTO);
+    if (free_run && takes_wide(g, nroots) && small_takes(g, nroots)) {
+        SmallResult res;
+        rc = small_run(g, p.roots.data(), p.mult.data(), nroots, st, &res);
+        if (rc) return rc;
+        if (res.done) {
+            if (stats) {
+                stats->launches += res.launches;
+                stats->batches = nroots;
+                stats->batch_width = 1;
+                finish_stats(g, p, res.rstat, stats);
+            }
+            return BCG_OK;
+        }
+    }
     if (free_run && takes_wide(g, nroots)) {
         WideResult res;
         rc = wide_run(g, p.roots.data(), p.mult.data(), nroots, st, &res);

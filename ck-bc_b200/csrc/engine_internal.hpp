@@ -18,6 +18,7 @@ using bcg::kTileVerts;
 namespace bcg {
 struct WideGraph;  // wide.cu
 struct DeepGraph;  // deep.cu
+struct SmallGraph;  // small.cu
 
 // Pendant trees of a graph on the device (BCG_PRUNE_TREES, and one peeling
 // round for BCG_PRUNE_DEGREE1; trees_gpu.cu), caller's numbering.
@@ -90,6 +91,7 @@ struct bcg_graph {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     bcg::WideGraph *wide = nullptr;  // the graph's form for wide-batch runs (wide.cu), built by the first one
     bcg::DeepGraph *deep = nullptr;  // the same for deep runs (deep.cu)
+    bcg::SmallGraph *small = nullptr;  // and for small ones (small.cu)
     uint32_t max_deg = 0;            // largest degree in the searched graph
 };
 
@@ -149,6 +151,19 @@ bool deep_takes(const bcg_graph *g);
 int deep_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, bool ext, cudaStream_t st,
              DeepResult *res);
 void deep_free(bcg_graph *g);
+
+// Runs a CTA a source in shared memory on a small graph (small.cu); waits for
+// the result.  done = false: a count overflowed or memory ran out, and nothing
+// was added to bc.
+struct SmallResult {
+    bool done = false;
+    std::vector<RootStat> rstat;
+    uint64_t launches = 0;
+};
+bool small_takes(const bcg_graph *g, uint64_t nroots);
+int small_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, cudaStream_t st,
+              SmallResult *res);
+void small_free(bcg_graph *g);
 
 // Component-packed batches already on the device (see BatchArgs::xbeg).
 struct PackedRun {

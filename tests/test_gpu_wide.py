@@ -1,6 +1,7 @@
 """The wide-batch searches (16 or 32 sources a job, teams of CTAs) against the oracle.
 
-Plain runs of four roots or more go there on graphs of mean degree 6 and up.
+Plain runs go there on graphs of mean degree 6 and up that are not small (a
+large component beside them makes the small ones here large enough).
 The cases sit at the edges of its work split: vertices of 31 to 33, 64, 256
 and several thousand entries (four lanes, a warp, chunks), vertex counts
 around 32-vertex words, 1 to 65 roots (one job of 16 to several of 32), several components, every
@@ -27,12 +28,20 @@ def _rows(n, degrees, seed):
     return bcg.from_pairs(np.concatenate(pairs + [fill]), n)
 
 
+def _beside(offs, adj, undirected=True):
+    """The graph (vertices 0 .. n - 1) and a random component of 20,000 vertices."""
+    n = len(offs) - 1
+    own = np.stack([np.repeat(np.arange(n), np.diff(offs.astype(np.int64))), adj], 1)
+    far = np.random.default_rng(31).integers(n, n + 20000, (130000, 2))
+    return bcg.from_pairs(np.concatenate([own, far]), n + 20000, undirected=undirected)
+
+
 GRAPHS = {
-    "degrees": lambda: _rows(5000, [4000, 3000, 1025, 1024, 513, 512, 300, 257, 256, 255, 129, 128, 65, 64, 63, 33, 32, 31, 1], 3),
-    "word31": lambda: bcg.generate("er:scale=5,ef=6,seed=8"),
-    "word33": lambda: _rows(33, [30, 20], 4),
+    "degrees": lambda: _beside(*_rows(5000, [4000, 3000, 1025, 1024, 513, 512, 300, 257, 256, 255, 129, 128, 65, 64, 63, 33, 32, 31, 1], 3)),
+    "word31": lambda: _beside(*bcg.generate("er:scale=5,ef=6,seed=8")),
+    "word33": lambda: _beside(*_rows(33, [30, 20], 4)),
     "rmat13": lambda: bcg.generate("rmat:scale=13,ef=16,a=0.57,b=0.19,c=0.19,seed=3"),
-    "pendants": lambda: bcg.generate("rmat:scale=11,ef=16,seed=9,pendant_frac=0.1,pendant_mean=4"),
+    "pendants": lambda: _beside(*bcg.generate("rmat:scale=11,ef=16,seed=9,pendant_frac=0.1,pendant_mean=4")),
     "er15": lambda: bcg.generate("er:scale=15,ef=12,seed=6"),
 }
 
@@ -83,6 +92,7 @@ def test_directed():
     hub = np.stack([np.zeros(2000, int), rng.choice(np.arange(1, n), 2000, replace=False)], 1)
     into = np.stack([rng.choice(np.arange(2, n), 700, replace=False), np.ones(700, int)], 1)
     offs, adj = bcg.from_pairs(np.concatenate([rng.integers(0, n, (40000, 2)), hub, into]), n, undirected=False)
+    offs, adj = _beside(offs, adj, undirected=False)
     src = bcg.sample_sources(n, 100, 1)
     ref, ost = oracle.bc(offs, adj, src)
     with bcg.Graph(offs, adj, bcg.DIRECTED) as G:
@@ -101,7 +111,7 @@ def _layers(width, depth):
 @pytest.mark.parametrize("depth,ext", [(9, 0), (12, 0), (15, 0), (30, 1)])
 def test_large_counts(depth, ext):
     """16 paths more a layer: 2^28 is passed from depth 9 on, 2^64 at 18."""
-    offs, adj = _layers(16, depth)
+    offs, adj = _beside(*_layers(16, depth))
     src = np.arange(0, 16 * depth, 3, dtype=np.uint32)
     ref, _ = oracle.bc_q(offs, adj, src)
     with bcg.Graph(offs, adj) as G:
@@ -113,7 +123,7 @@ def test_large_counts(depth, ext):
 def test_deep_search_leaves():
     """Mean degree above 6, 120 levels: the run is redone by the sweep kernel,
     and what was in bc before stays."""
-    offs, adj = _layers(4, 120)
+    offs, adj = _beside(*_layers(4, 120))
     src = np.arange(0, 480, 30, dtype=np.uint32)
     ref, _ = oracle.bc_q(offs, adj, src)
     with bcg.Graph(offs, adj) as G:

@@ -98,7 +98,7 @@ struct bcg_graph {
 namespace bcg {
 
 // Device memory of graphs and of their creation, from a library-owned
-// stream-ordered pool of the current device that keeps up to 1 GiB reserved
+// stream-ordered pool of the current device that keeps up to 4 GiB reserved
 // once it is freed: creating and destroying graphs one after another then
 // neither maps fresh memory nor waits in cudaFree.  tmp_alloc / tmp_free are
 // ordered on stream st like a kernel; dev_alloc / dev_free on the default

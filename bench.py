@@ -673,8 +673,10 @@ def main():
     alg_bytes = 16.0 * edges + 56.0 * cverts + 8.0 * ran
     kern_s = sum(kern_ms) / 1e3
     achieved = alg_bytes / kern_s / 1e9
-    tps, tnote = traffic_per_source(args.prune, f"bcg::bc_sweep_kernel<{int(st.batch_width)}, "
-                                                f"{'true' if st.extended_sigma else 'false'}>")
+    w = int(st.batch_width)
+    # (16 and 32 sources a batch are the wide searches')
+    tps, tnote = traffic_per_source(args.prune, f"bcg::bc_wide_kernel<{w}>" if w >= 16 else
+                                    f"bcg::bc_sweep_kernel<{w}, {'true' if st.extended_sigma else 'false'}>")
     traffic = tps * (ran / args.steps) if tps is not None else None
     # the same bytes per search over the graph the kernel actually walks (the
     # pruned graph, one search per root however many sources it stands for)

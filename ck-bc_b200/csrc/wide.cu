@@ -15,10 +15,11 @@
 //     31 M entries: 141 us and 201 us a pass, 14 and 20 TB/s out of L2, the
 //     whole port; the 64-byte rows of levels and values of sweep.cu carry 6
 //     sources and take about 500 us.)  The sweeps here reach 300 to 400 us:
-//     what is left is instructions (0.33 a cycle and scheduler, a third of
-//     them for ids, bits and vertices rather than rows) and the latency of
-//     rows.  32 sources a job share the first kind: 1,590 us a job of 16 and
-//     2,690 us one of 32 on the benchmark's graph.
+//     what is left is the latency of ids, bits and rows (a warp waits half of
+//     its time for a load and a fifth at the sweeps' ends; 0.27 instructions a
+//     cycle and scheduler, the L2 28 % busy, hit rate 77 %).  32 sources a job
+//     share what is not rows: 1,590 us a job of 16 and 2,690 us one of 32 on
+//     the benchmark's graph, in the order given.
 //   - a bit per vertex and level says whether any slot sits there, so a
 //     gather skips the rows of other vertices, rows are never cleared, and
 //     backward sweeps visit a level's vertices only.
@@ -267,9 +268,19 @@ __device__ __forceinline__ void load_ids(uint32_t (&id)[4], const uint32_t *__re
     }
 }
 
+// Sets of rows that a lane holds, one being added and the others on their way
+// (a set: 16 registers).  Each sweep is a matter of rows in flight: with 512
+// threads of 128 registers three sets against two take 13.4 against 14.5 ms on
+// an Erdos-Renyi graph of 500k vertices (200 sources, jobs of 32), 2.48 against
+// 2.61 on a 100k-vertex R-MAT one, the same on the benchmark's; a fourth spills
+// (14.0, 2.70).  Jobs of 16: 5.86, 6.00 and 5.58 ms with two, three and four
+// sets at 4M vertices.
+template <int LS>
+constexpr int row_sets() { return LS == 4 ? 4 : 3; }
+
 // The first J of a lane's four edges: a group of four lanes takes its lanes'
 // edges one after the other, each lane LS slots of a row, the next rows in
-// flight (32 registers of them) while the last are added.
+// flight while the last are added.
 template <int KIND, int J, int LS, class T>
 __device__ __forceinline__ void add_rows(const unsigned char *rows, uint32_t zero, const uint32_t (&id)[4],
                                          T (&acc)[LS]) {
@@ -277,7 +288,8 @@ __device__ __forceinline__ void add_rows(const unsigned char *rows, uint32_t zer
     if constexpr (KIND == kFwd32) {
         constexpr int U = 16 / LS;  // rows of a step
         uint32_t part[LS];          // at most 16 counts below 2^28
-        uint32_t r[2][U][LS];
+        constexpr int P = row_sets<LS>();
+        uint32_t r[P][U][LS];
 #pragma unroll
         for (int k = 0; k < LS; ++k) part[k] = 0u;
         auto fetch = [&](int s, uint32_t (&o)[U][LS]) {
@@ -288,14 +300,15 @@ __device__ __forceinline__ void add_rows(const unsigned char *rows, uint32_t zer
             }
         };
         constexpr int steps = 4 * J / U;
-        fetch(0, r[0]);
+#pragma unroll
+        for (int s = 0; s < P - 1 && s < steps; ++s) fetch(s, r[s]);
 #pragma unroll
         for (int s = 0; s < steps; ++s) {
-            if (s + 1 < steps) fetch(s + 1, r[(s + 1) & 1]);
+            if (s + P - 1 < steps) fetch(s + P - 1, r[(s + P - 1) % P]);
 #pragma unroll
             for (int k = 0; k < LS; ++k) {
-                uint32_t t = r[s & 1][0][k] + r[s & 1][1][k];
-                if constexpr (U == 4) t += r[s & 1][2][k] + r[s & 1][3][k];
+                uint32_t t = r[s % P][0][k] + r[s % P][1][k];
+                if constexpr (U == 4) t += r[s % P][2][k] + r[s % P][3][k];
                 part[k] += t;
             }
         }
@@ -303,7 +316,8 @@ __device__ __forceinline__ void add_rows(const unsigned char *rows, uint32_t zer
         for (int k = 0; k < LS; ++k) acc[k] += (T)part[k];
     } else if constexpr (KIND == kBack) {
         constexpr int U = 8 / LS;
-        double r[2][U][LS];
+        constexpr int P = row_sets<LS>();
+        double r[P][U][LS];
         auto fetch = [&](int s, double (&o)[U][LS]) {
 #pragma unroll
             for (int q = 0; q < U; ++q) {
@@ -312,14 +326,15 @@ __device__ __forceinline__ void add_rows(const unsigned char *rows, uint32_t zer
             }
         };
         constexpr int steps = 4 * J / U;
-        fetch(0, r[0]);
+#pragma unroll
+        for (int s = 0; s < P - 1 && s < steps; ++s) fetch(s, r[s]);
 #pragma unroll
         for (int s = 0; s < steps; ++s) {
-            if (s + 1 < steps) fetch(s + 1, r[(s + 1) & 1]);
+            if (s + P - 1 < steps) fetch(s + P - 1, r[(s + P - 1) % P]);
 #pragma unroll
             for (int q = 0; q < U; ++q)
 #pragma unroll
-                for (int k = 0; k < LS; ++k) acc[k] += r[s & 1][q][k];
+                for (int k = 0; k < LS; ++k) acc[k] += r[s % P][q][k];
         }
     }
 }

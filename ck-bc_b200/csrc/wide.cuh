@@ -12,7 +12,11 @@ struct bcg_graph;
 
 namespace bcg {
 
-constexpr int kWideThreads = 640;    // one CTA per SM, 96 registers a thread
+// One CTA per SM.  Registers hold rows in flight, and 640 threads leave 96 a
+// thread, with spills in every sweep: 512 with 128 take 35.7 against 37.4 ms on
+// the benchmark's graph (1024 sources), 5.3 against 5.6 for 48 small graphs; 576
+// and 768 are slower than either.
+constexpr int kWideThreads = 512;
 constexpr int kWideWarps = kWideThreads / 32;
 constexpr uint32_t kWideTeams = 148;  // most teams of a launch
 constexpr uint32_t kWideLevels = 64;  // levels a job can hold (deeper searches run elsewhere)

@@ -362,7 +362,10 @@ int small_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t 
     a.out = nroots > 1 ? reinterpret_cast<double *>(w->mem + o_out) : nullptr;
     a.bc = g->d_bc;
     const void *f = (const void *)bc_small_kernel;
-    CKM(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared));
+    // (the limit belongs to the kernel, not to the launch: the same for every
+    // graph, so that threads running graphs of different sizes do not lower it
+    // for one another)
+    CKM(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallShared));
     CKM(cudaEventRecord(g->ev0, st));
     void *params[] = {&a};
     CKM(cudaLaunchKernel(f, dim3((unsigned)nroots), dim3(kSmallThreads), params, shared, st));

@@ -1297,7 +1297,10 @@ int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t n
         g->wide = new WideGraph();
         if ((rc = wide_form_make(g->wide->form, wide_input(g)))) {
             wide_free(g);
-            return rc == BCG_ERR_OOM ? (cudaGetLastError(), BCG_OK) : rc;
+            if (rc != BCG_ERR_OOM) return rc;
+            cudaGetLastError();
+            clear_error();
+            return BCG_OK;
         }
         fresh = true;
     }

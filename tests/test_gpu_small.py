@@ -122,3 +122,31 @@ def test_large_counts(width, depth, ext):
         st = G.run(src)
         assert st.extended_sigma == ext and (ext or st.batch_width == 1)
         assert_bc_close(G.bc(), ref, f"layers {width} {depth}")
+
+
+def test_threads_with_graphs_of_different_sizes():
+    """The kernel's shared-memory limit is the process's: a thread with a small graph must not lower it for another."""
+    import threading
+
+    sets = [_dense(n, nnz) for n, nnz in ((64, 400), (1000, 30000), (300, 8000), (1500, 60000))]
+    want = [oracle.bc_q(o, a, np.arange(4, dtype=np.uint32))[0] for o, a in sets]
+    got, errors = [None] * len(sets), []
+
+    def work(k):
+        try:
+            with bcg.Graph(*sets[k]) as g:
+                for _ in range(200):
+                    g.reset()
+                    g.run(np.arange(4, dtype=np.uint32))
+                got[k] = g.bc()
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(sets))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for w, b in zip(want, got):
+        assert_bc_close(b, w)

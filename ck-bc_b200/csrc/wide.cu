@@ -68,13 +68,15 @@ constexpr uint32_t kEmpty = 0xFEu;   // level byte of a slot without a source
 constexpr double kWide32 = 1.5;      // time of a 32-source job's entries over a 16-source job's
 
 // What a sweep does: forward over 32-bit rows, forward over levels and
-// 64-bit counts, backward, backward at the deepest level (no child exists).
-enum : int { kFwd32 = 0, kFwdFull = 1, kBack = 2, kBackLast = 3 };
+// 64-bit counts, backward, backward at the deepest level (no child exists),
+// forward from level 1 where every count is 1.
+enum : int { kFwd32 = 0, kFwdFull = 1, kBack = 2, kBackLast = 3, kFwdOnes = 4 };
 
 struct WideCtx {
     uint32_t T, rank;  // CTAs of the team, this one's place
     unsigned char *lvl;
     uint32_t *done, *act;  // bitmaps: all slots reached; by level: some slot at it
+    uint32_t *bits;        // by vertex: the slots that are at level 1 (of vertices where some slot is)
     size_t words;
     unsigned long long *sig;
     unsigned char *g0;  // rows of even levels,
@@ -381,6 +383,83 @@ __device__ __forceinline__ void add_block(const WideCtx &x, uint32_t d, uint32_t
     }
 }
 
+// Level 1.  Its counts are 1 (unless a list names a neighbour twice), so a row
+// is a word of 32 slots' bits, and a lane adds the words of its edges bit by bit
+// in kPlanes words: bit k of word p is bit p of slot k's sum.  Four edges take
+// about 20 instructions where their rows take 80 and 512 bytes.
+constexpr int kPlanes = 7;  // a lane has at most 64 edges: a chunk's by 32 lanes, or a light vertex's by 4
+static_assert(8 * kWideChunk / 32 < 1 << kPlanes && (kWideLight << 3) / 4 < 1 << kPlanes, "planes of a lane's sums");
+
+__device__ __forceinline__ void add_ones(const WideCtx &x, uint32_t d, const uint32_t (&id)[4], uint32_t (&pl)[kPlanes]) {
+    const uint32_t *act = x.act + (size_t)d * x.words;
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = act[id[j] >> 5];
+    uint32_t hit = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        w[j] = (w[j] >> (id[j] & 31u)) & 1u;
+        hit |= w[j];
+    }
+    if (!__any_sync(kFull, hit)) return;  // most blocks, where the sources have few neighbours
+    // (an id past the end is n: its bit may be another level's, its word is 0)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = w[j] ? x.bits[id[j]] : 0u;
+    const uint32_t s = w[0] ^ w[1] ^ w[2], c = (w[0] & w[1]) | (w[2] & (w[0] ^ w[1]));
+    const uint32_t ones = s ^ w[3], c2 = s & w[3], twos = c ^ c2, fours = c & c2;
+    uint32_t k = pl[0] & ones;
+    pl[0] ^= ones;
+    const uint32_t k1 = (pl[1] & twos) | (k & (pl[1] ^ twos));
+    pl[1] ^= twos ^ k;
+    k = (pl[2] & fours) | (k1 & (pl[2] ^ fours));
+    pl[2] ^= fours ^ k1;
+#pragma unroll
+    for (int p = 3; p < kPlanes; ++p) {
+        const uint32_t up = pl[p] & k;
+        pl[p] ^= k;
+        k = up;
+    }
+}
+
+// Bit l of lane k's result is bit k of lane l's word.
+__device__ __forceinline__ uint32_t transpose_bits(uint32_t x) {
+    const unsigned lane = threadIdx.x & 31;
+    constexpr uint32_t low[5] = {0x0000FFFFu, 0x00FF00FFu, 0x0F0F0F0Fu, 0x33333333u, 0x55555555u};
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+        const int s = 16 >> i;
+        const uint32_t y = __shfl_xor_sync(kFull, x, s);
+        x = (lane & (unsigned)s) ? (x & ~low[i]) | ((y >> s) & low[i]) : (x & low[i]) | ((y & low[i]) << s);
+    }
+    return x;
+}
+
+// A group's sums: slot LS * l + i of the four lanes' words into lane l's acc[i].
+template <int LS>
+__device__ __forceinline__ void ones_to_group(const uint32_t (&pl)[kPlanes], unsigned long long (&acc)[LS]) {
+    const unsigned l = threadIdx.x & 3u, sh = threadIdx.x & 28u;
+    uint32_t sum[LS];
+#pragma unroll
+    for (int i = 0; i < LS; ++i) sum[i] = 0u;
+#pragma unroll
+    for (int p = 0; p < kPlanes; ++p) {
+        if (!__any_sync(kFull, pl[p] != 0u)) continue;
+        uint32_t b[LS / 4];  // four slots' bytes each
+#pragma unroll
+        for (int h = 0; h < LS / 4; ++h) b[h] = 0u;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t y = __shfl_sync(kFull, pl[p], sh + q) >> (LS * l);
+#pragma unroll
+            for (int h = 0; h < LS / 4; ++h) b[h] += (((y >> (4 * h)) & 15u) * 0x00204081u) & 0x01010101u;
+        }
+#pragma unroll
+        for (int i = 0; i < LS; ++i) sum[i] += ((b[i / 4] >> (8 * (i & 3))) & 0xFFu) << p;
+    }
+#pragma unroll
+    for (int i = 0; i < LS; ++i) acc[i] = sum[i];
+}
+
 // The eight groups' sums of a warp's vertex, added in a fixed order and dealt
 // out one slot a lane (own_slot): lane 4g + l gets one of the slots LS * l ..,
 // which one by g's bits (16 slots: groups g and g ^ 1 get the same).
@@ -412,6 +491,16 @@ __device__ __forceinline__ T wide_fold(const T (&acc)[NS / 4], bool &ovf) {
     }
     if (NS == 16) a[0] = wide_add<KIND>(a[0], (T)__shfl_xor_sync(kFull, a[0], 4), ovf);
     return a[0];
+}
+
+// The warp's sums in the same places.
+template <int NS>
+__device__ __forceinline__ unsigned long long ones_to_warp(const uint32_t (&pl)[kPlanes]) {
+    uint32_t sum = 0;
+#pragma unroll
+    for (int p = 0; p < kPlanes; ++p)
+        if (__any_sync(kFull, pl[p] != 0u)) sum += (uint32_t)__popc(transpose_bits(pl[p])) << p;
+    return __shfl_sync(kFull, sum, own_slot<NS>());
 }
 
 // Finishing a vertex whose sums lie one slot a lane (wide_fold's order): the
@@ -547,7 +636,8 @@ template <int KIND, int NS>
 __device__ __noinline__ void wide_sweep(WideSmem<NS> &sm, uint32_t d) {
     const WideCtx &x = sm.x;
     using T = typename AccOf<KIND>::T;
-    constexpr bool kForward = KIND == kFwd32 || KIND == kFwdFull;
+    constexpr bool kForward = KIND == kFwd32 || KIND == kFwdFull || KIND == kFwdOnes;
+    constexpr bool kOnes = KIND == kFwdOnes;
     constexpr int side = kForward ? 0 : 1;
     const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const WideSub &g = sm.sub;
@@ -623,6 +713,7 @@ __device__ __noinline__ void wide_sweep(WideSmem<NS> &sm, uint32_t d) {
                 todo &= todo - 1;
                 const uint32_t vi = __shfl_sync(kFull, v, i), end = se;
                 T acc[NS / 4] = {};
+                uint32_t pl[kPlanes] = {};
                 uint32_t at = sb;
                 bool more;
 #pragma unroll 1
@@ -641,9 +732,12 @@ __device__ __noinline__ void wide_sweep(WideSmem<NS> &sm, uint32_t d) {
                         se = __shfl_sync(kFull, e1, __ffs(todo) - 1);
                         load_ids(nxt, adj, sb + lane, se, 32u, g.n, pol);
                     }
-                    if constexpr (kGather) add_block<KIND, NS>(x, d, g.n, id, acc, ovf);
+                    if constexpr (kOnes) add_ones(x, d, id, pl);
+                    else if constexpr (kGather) add_block<KIND, NS>(x, d, g.n, id, acc, ovf);
                 } while (more);
-                T sum = wide_fold<KIND, NS>(acc, ovf);
+                T sum;
+                if constexpr (kOnes) sum = ones_to_warp<NS>(pl);
+                else sum = wide_fold<KIND, NS>(acc, ovf);
                 if (heavy) {
                     const uint32_t ci = it * cb + i;
                     const uint32_t c0 = g.cbeg[side][vi] - g.chunk0[side], nc = g.cbeg[side][vi + 1] - g.chunk0[side] - c0;
@@ -729,6 +823,7 @@ __device__ __noinline__ void wide_sweep(WideSmem<NS> &sm, uint32_t d) {
                 const bool valid = ok;
                 const uint32_t v = vb + p;
                 T acc[NS / 4] = {};
+                uint32_t pl[kPlanes] = {};
                 if constexpr (kGather) {
                     const uint32_t b = sb, e = se;
                     const uint32_t nblk = max(1u, __reduce_max_sync(kFull, (e - b + 15u) / 16u));
@@ -743,8 +838,10 @@ __device__ __noinline__ void wide_sweep(WideSmem<NS> &sm, uint32_t d) {
                             pick(i0 + 8, ok, p, sb, se);
                             load_ids(nxt, adj, sb + (lane & 3u), se, 4u, g.n, pol);
                         }
-                        add_block<KIND, NS>(x, d, g.n, id, acc, ovf);
+                        if constexpr (kOnes) add_ones(x, d, id, pl);
+                        else add_block<KIND, NS>(x, d, g.n, id, acc, ovf);
                     }
+                    if constexpr (kOnes) ones_to_group<NS / 4>(pl, acc);
                 } else {
                     pick(i0 + 8, ok, p, sb, se);
                 }
@@ -805,6 +902,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
         x.done = reinterpret_cast<uint32_t *>(st + a.o_done);
         x.act = reinterpret_cast<uint32_t *>(st + a.o_act);
         x.words = a.words;
+        x.bits = reinterpret_cast<uint32_t *>(st + a.o_bits);
         x.sig = reinterpret_cast<unsigned long long *>(st + a.o_sig);
         x.g0 = st + a.o_g0;
         x.g01 = (ptrdiff_t)(a.o_g1 - a.o_g0);
@@ -917,6 +1015,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
             x.act[w] = m;
             x.act[x.words + w] = 0;
         }
+        if (x.rank == 0 && threadIdx.x == 0) x.bits[n] = 0u;
         for (uint32_t i = tid; i < sm.sub.nheavy; i += nt) x.hcnt[i] = 0;
         // the rows of zeros: row n of the counts' rows and of the doubles'
         if (x.rank == 0 && threadIdx.x < NS) {
@@ -929,6 +1028,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
         // the rows of level 1 start from 0
         each_first([&](int k, uint32_t w) {
             if (w != sm.roots[k]) x.sig[(size_t)w * NS + k] = 0ull;
+            x.bits[w] = 0u;
             uint4 *row = reinterpret_cast<uint4 *>(rows_of(x, 1) + (size_t)w * (NS * 4));
 #pragma unroll
             for (int h = 0; h < NS / 4; ++h) row[h] = make_uint4(0u, 0u, 0u, 0u);
@@ -939,6 +1039,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
         // ---- forward
         uint32_t d = 0;
         bool big = false;  // some count of level d is 2^28 or more
+        bool ones = false;  // every count of level 1 is 1
         for (;; ++d) {
             if (d + 2 >= kWideLevels) {
                 if (threadIdx.x == 0) {
@@ -958,15 +1059,17 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
                 each_first([&](int k, uint32_t w) {
                     if (w == sm.roots[k]) return;
                     x.lvl[(size_t)w * NS + k] = 1;
-                    atomicAdd(x.sig + (size_t)w * NS + k, 1ull);
+                    if (atomicAdd(x.sig + (size_t)w * NS + k, 1ull)) atomicOr(&sm.found, 8u);  // listed before
+                    atomicOr(x.bits + w, 1u << k);
                     atomicAdd(reinterpret_cast<uint32_t *>(rows_of(x, 1)) + (size_t)w * NS + k, 1u);
                     atomicOr(x.act + x.words + (w >> 5), 1u << (w & 31u));
                 });
                 if (threadIdx.x == 0 && sm.edges[NS]) {
-                    sm.found = 1;
+                    atomicOr(&sm.found, 1u);
                     if (x.rank == 0) sm.count = sm.edges[NS];  // at most
                 }
             } else if (big) wide_sweep<kFwdFull, NS>(sm, d);
+            else if (d == 1 && ones) wide_sweep<kFwdOnes, NS>(sm, d);
             else wide_sweep<kFwd32, NS>(sm, d);
             if (!team_sync(a, x, t, sm, wait_ns, d & 3, d + 1)) return;
             const uint32_t any = sm.any;
@@ -980,6 +1083,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
             }
             if (!(any & 1u)) break;
             big = (any & 2u) != 0;
+            ones = d == 0 && !(any & 8u);
         }
         const uint32_t D = d;
 
@@ -1189,6 +1293,7 @@ size_t wide_layout(WideArgs &a, uint32_t slots, size_t n, size_t nchunk, size_t 
     a.o_g1 = o; o += up256((n + 1) * slots * 8);
     a.o_part = o; o += up256(std::max<size_t>(1, nchunk) * slots * 8);
     a.o_hcnt = o; o += up256(std::max<size_t>(1, nheavy) * 4);
+    a.o_bits = o; o += up256((n + 1) * 4);
     a.stride = o;
     a.words = words;
     return o;

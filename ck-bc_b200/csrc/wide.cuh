@@ -52,7 +52,8 @@ struct WideJob {
 struct WideTeam {
     unsigned long long arrived;  // barrier arrivals since the launch (monotone)
     uint32_t job[2];             // next job, by parity of the current one
-    uint32_t any[4];             // ring: the forward sweep found a vertex (1), a count of 2^32 or more (2)
+    uint32_t any[4];             // ring: the forward sweep found a vertex (1), a count of 2^28 or more (2), an overflow (4),
+                                 // a neighbour listed twice at level 1 (8)
     unsigned long long count[4];  // ring: vertices the forward sweep found, and finished (upper half)
     uint32_t pad[16];
 };
@@ -87,7 +88,7 @@ struct WideArgs {
     // per-team state, each array sized for the launch's largest graph
     unsigned char *state;
     size_t stride;          // bytes of a team's state
-    size_t o_done, o_act, o_sig, o_g0, o_g1, o_part, o_hcnt;
+    size_t o_done, o_act, o_bits, o_sig, o_g0, o_g1, o_part, o_hcnt;
     size_t words;           // 32-vertex words of the largest graph (row length of act)
     TraceRec *trace;
     unsigned int trace_cap;

@@ -258,3 +258,47 @@ def test_sources_out_of_order(k):
         parts = [G.run(p) for p in np.array_split(src, max(1, k // 1000))]  # other jobs, other companions
         assert_bc_close(whole, G.bc(), f"k={k}")
         assert st.teps_edges == sum(p.teps_edges for p in parts) and st.skipped == sum(p.skipped for p in parts)
+
+
+@pytest.mark.parametrize("nsrc", [1, 16, 33])
+def test_sums_over_level_one(nsrc):
+    """Vertices with 1 to 4,500 neighbours next to a source, whose counts are added bit by bit: a lane of four or of 32
+    takes up to 64 of them, at the edges of a block, of a light vertex, a warp's and a chunk."""
+    mids = 4600
+    sinks = [1, 2, 3, 4, 5, 15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 511, 512, 513, 2047, 2048, 2049, 4500]
+    pairs = [np.stack([np.zeros(mids, int), np.arange(1, mids + 1)], 1)]
+    for i, k in enumerate(sinks):
+        pairs.append(np.stack([np.full(k, mids + 1 + i), np.arange(1, k + 1)], 1))
+    offs, adj = _beside(*bcg.from_pairs(np.concatenate(pairs), mids + 1 + len(sinks)))
+    src = np.concatenate([[0], np.arange(mids + len(sinks), mids + len(sinks) + 1 - nsrc, -1)]).astype(np.uint32)
+    ref, ost = oracle.bc(offs, adj, src)
+    with bcg.Graph(offs, adj) as G:
+        st = G.run(src)
+        assert st.batch_width in WIDE and st.visited == ost["visited"]
+        assert_bc_close(G.bc(), ref, f"{nsrc} sources")
+
+
+@pytest.mark.parametrize("repeats", [0, 1])
+def test_lists_that_name_a_neighbour_twice(repeats):
+    """A source's list with a repeated neighbour: a count of 2 at level 1, which no bit holds."""
+    rng = np.random.default_rng(5)
+    n = 30000
+    pairs = np.concatenate([rng.integers(0, n, (300000, 2))] + [np.stack([np.zeros(900, int), rng.integers(1, 400, 900)], 1)] * repeats)
+    key = pairs[:, 0] * n + pairs[:, 1]
+    pairs = pairs[np.argsort(pairs[:, 0], kind="stable")] if repeats else pairs[np.unique(key, return_index=True)[1]]
+    pairs = pairs[np.argsort(pairs[:, 0], kind="stable")]
+    offs = np.zeros(n + 1, dtype=np.uint32)
+    np.cumsum(np.bincount(pairs[:, 0], minlength=n), out=offs[1:])
+    adj = pairs[:, 1].astype(np.uint32)
+    src = np.arange(0, 40, dtype=np.uint32)
+    with bcg.Graph(offs, adj, bcg.DIRECTED) as G:
+        G.set_batch_width(6)
+        a = G.run(src)
+        want = G.bc()
+        G.reset()
+        G.set_batch_width(0)
+        b = G.run(src)
+        got = G.bc()
+    assert a.batch_width == 6 and b.batch_width in WIDE
+    assert a.teps_edges == b.teps_edges and a.visited == b.visited and a.max_depth == b.max_depth
+    assert_bc_close(got, want, "repeated neighbours")

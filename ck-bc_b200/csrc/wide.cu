@@ -26,6 +26,7 @@
 //   - path counts are 64-bit; the 32-bit rows are used while every count of
 //     the level is below 2^28 (the sweep that finds them says so), and otherwise the
 //     sweep reads levels and 64-bit counts (kFwdFull), with overflow checked.
+//   - level 1, whose counts are 1, is a word of bits a vertex (kFwdOnes).
 // All forward sweeps pull: no atomics on values, sums in a fixed order.
 //
 // Work split.  Vertices are numbered by descending degree class
@@ -403,6 +404,9 @@ __device__ __forceinline__ void add_block(const WideCtx &x, uint32_t d, uint32_t
 // is a word of 32 slots' bits, and a lane adds the words of its edges bit by bit
 // in kPlanes words: bit k of word p is bit p of slot k's sum.  Four edges take
 // about 20 instructions where their rows take 80 and 512 bytes.
+// (The sweep, 1M-vertex graph, 658 sources: 250 -> 196 us a job; kernel 35.7 ->
+// 34.8 ms, 100k-vertex R-MAT 2.56 -> 2.49, 48 small graphs 5.28 -> 5.17, a
+// 500k-vertex Erdos-Renyi graph, whose level 1 is next to empty, 13.4 -> 13.6.)
 constexpr int kPlanes = 7;  // a lane has at most 64 edges: a chunk's by 32 lanes, or a light vertex's by 4
 static_assert(8 * kWideChunk / 32 < 1 << kPlanes && (kWideLight << 3) / 4 < 1 << kPlanes, "planes of a lane's sums");
 

@@ -141,7 +141,7 @@ int build_wide(bcg_batch *b) {
         free_wide(b);
         return rc == BCG_ERR_OOM ? (cudaGetLastError(), BCG_OK) : rc;
     };
-    int rc = wide_form_make(b->form, in);
+    int rc = wide_form_make(b->form, in, false);
     if (rc) return give_up(rc);
     // jobs in union order (largest graphs first); a launch ends when its jobs'
     // vectors take 512 MB, or when the graphs have become a quarter of its

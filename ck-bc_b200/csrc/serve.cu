@@ -229,7 +229,7 @@ int wide_setup(bcg_server *s) {
     const uint64_t extra =
         wide_form_bytes(in, &scratch) + s->wstate_bytes + s->cells * 8 + kInFlight * (s->wblob_bytes + stat);
     if (s->resident + extra + scratch > s->budget) return BCG_OK;
-    int rc = wide_form_make(s->form, in);
+    int rc = wide_form_make(s->form, in, false);
     cudaError_t e = cudaSuccess;
     if (!rc && ((e = dev_alloc(&s->d_wstate, s->wstate_bytes)) != cudaSuccess ||
                 (e = dev_alloc(&s->d_jobbc, s->cells * 8)) != cudaSuccess ||
@@ -343,6 +343,9 @@ int enqueue_wide_wave(bcg_server *s, ServeWave &w, int wi, bool *launched) {
         for (size_t k = 0; k < spans.size(); ++k) {
             const Span &l = spans[k];
             wide_layout(a, kServeSlots, l.nmax, l.nch, l.nheavy);
+            if (a.stride > s->wstate_bytes)
+                return set_error(BCG_ERR_RANGE, "a team's state of %zu bytes is more than the %zu of the server's buffer", a.stride,
+                                 s->wstate_bytes);
             wide_teams(a, l.njobs, l.entries / l.njobs, s->wstate_bytes);
             a.subs = s->form.d_subs;
             a.jobs = reinterpret_cast<const WideJob *>(w.d_jobs) + l.job0;

@@ -1426,7 +1426,7 @@ int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t n
     // (out of memory: the caller's other kernels need less)
     if (!g->wide) {
         g->wide = new WideGraph();
-        if ((rc = wide_form_make(g->wide->form, wide_input(g)))) {
+        if ((rc = wide_form_make(g->wide->form, wide_input(g), true))) {
             wide_free(g);
             if (rc != BCG_ERR_OOM) return rc;
             cudaGetLastError();

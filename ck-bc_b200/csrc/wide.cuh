@@ -127,15 +127,18 @@ struct WideForm {
     unsigned char *mem = nullptr;  // everything below on the device (nullptr: the caller's memory)
     WideSub *d_subs = nullptr;     // one a graph
     uint32_t *inv = nullptr, *map = nullptr;
-    std::vector<WideSub> subs;     // the host's copy (wide_form_make; of one small graph: bounds)
+    std::vector<WideSub> subs;     // the host's copy (wide_form_make)
 };
 
 // Bytes of a form, and of the scratch that building it takes.
 size_t wide_form_bytes(const WideInput &in, size_t *scratch);
 // Enqueues the building in memory of that size on st; f.subs stays empty.
 int wide_form_enqueue(WideForm &f, const WideInput &in, unsigned char *mem, unsigned char *scratch, cudaStream_t st);
-// Allocates and builds on stream 0 (waits, but for one small graph).
-int wide_form_make(WideForm &f, const WideInput &in);
+// Allocates and builds on stream 0, and reads subs back.  bounds: the caller
+// takes subs' n, nheavy and nchunk for upper bounds (n counts the vertices
+// without an entry too) and its WideOut names the device's sub; of one small
+// graph nothing is read back then, and the building is not waited for.
+int wide_form_make(WideForm &f, const WideInput &in, bool bounds);
 void wide_form_free(WideForm &f);
 
 // Loads the wide searches' kernels on the current device (CUDA would load each
@@ -153,6 +156,8 @@ size_t wide_layout(WideArgs &a, uint32_t slots, size_t n, size_t nchunk, size_t 
 inline bool wide_shallow(uint64_t active, uint64_t nnz) { return nnz >= 6 * active || active + 2 < kWideLevels; }
 // Cuts the SMs into teams for njobs jobs on lists of so many entries (their
 // mean), a's layout being set; returns the time in us this is expected to take.
+// One team at least, also where its state alone is more than state_bytes: a
+// caller whose buffer is fixed looks at a.stride itself.
 double wide_teams(WideArgs &a, uint64_t njobs, uint64_t entries, size_t state_bytes = 512ull << 20);
 // Layout and teams for nroots sources of one graph, in jobs of 16 or 32,
 // whichever is expected to end first; returns which.

@@ -345,13 +345,13 @@ int wide_form_enqueue(WideForm &f, const WideInput &in, unsigned char *mem, unsi
     return BCG_OK;
 }
 
-int wide_form_make(WideForm &f, const WideInput &in) {
+int wide_form_make(WideForm &f, const WideInput &in, bool bounds) {
     size_t scratch_bytes = 0;
     const size_t bytes = wide_form_bytes(in, &scratch_bytes);
     f.subs.resize(in.graphs);
-    // One small graph: everything in one block, and its description's bounds
-    // stand for it, so that the first run does not wait for the building.
-    const bool small = in.graphs == 1 && !in.directed && in.n <= (1u << 16);
+    // One small graph whose bounds do: everything in one block, and the first
+    // run does not wait for the building.
+    const bool small = bounds && in.graphs == 1 && !in.directed && in.n <= (1u << 16);
     CKF(dev_alloc(&f.mem, small ? bytes + scratch_bytes : bytes));
     if (small) {
         WideSub &s = f.subs[0];

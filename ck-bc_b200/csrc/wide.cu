@@ -901,6 +901,33 @@ __device__ __noinline__ void wide_sweep(WideSmem<NS> &sm, uint32_t d) {
     }
 }
 
+// Whether a path count at level d + 1 passed 2^64, asked after a forward
+// sweep in which some sum did: the sweep sums every slot of a vertex, and what
+// a slot that was reached before sums is no count.  Summed again for the slots
+// that were open then (not reached now, or at level d + 1): a warp a vertex, a
+// lane a slot.  (Telling them apart in the sweep itself takes registers from
+// all of its kinds: 1 % of every run.)
+template <int NS>
+__device__ __noinline__ bool count_overflows(const WideSmem<NS> &sm, uint32_t d) {
+    const WideCtx &x = sm.x;
+    const WideSub &g = sm.sub;
+    const unsigned lane = threadIdx.x & 31;
+    const uint32_t w = x.rank * kWideWarps + (threadIdx.x >> 5);
+    bool ovf = false;
+    for (uint32_t v = w; v < g.n; v += x.T * kWideWarps) {
+        const uint32_t lv = lane < NS ? __ldcg(x.lvl + (size_t)v * NS + lane) : kEmpty;
+        const bool open = lv == kUnseen || lv == d + 1u;
+        if (!__any_sync(kFull, open)) continue;
+        unsigned long long sum = 0;
+        const uint32_t e1 = g.offs[0][v + 1];
+        for (uint32_t e = g.offs[0][v]; e < e1; ++e) {
+            const size_t at = (size_t)g.adj[0][e] * NS + lane;
+            if (open && __ldcg(x.lvl + at) == d) sum = wide_add<kFwdFull>(sum, __ldcg(x.sig + at), ovf);
+        }
+    }
+    return ovf;
+}
+
 __device__ __forceinline__ void wide_trace(const WideArgs &a, uint32_t job, uint32_t kind, uint32_t level,
                                            uint32_t info) {
     if (!a.trace || blockIdx.x != 0 || threadIdx.x != 0) return;
@@ -1101,11 +1128,11 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
             const uint32_t any = sm.any;
             wide_trace(a, job, 2, d, any);
             if (any & 4u) {
-                if (threadIdx.x == 0) {
+                if (count_overflows<NS>(sm, d)) {
                     a.ctrl->overflow = 1;
                     if (a.poison) *a.poison = 1;
                 }
-                return;
+                if (!team_sync(a, x, t, sm, wait_ns, 5)) return;
             }
             if (!(any & 1u)) break;
             big = (any & 2u) != 0;

@@ -52,8 +52,8 @@ struct WideJob {
 struct WideTeam {
     unsigned long long arrived;  // barrier arrivals since the launch (monotone)
     uint32_t job[2];             // next job, by parity of the current one
-    uint32_t any[4];             // ring: the forward sweep found a vertex (1), a count of 2^28 or more (2), an overflow (4),
-                                 // a neighbour listed twice at level 1 (8)
+    uint32_t any[4];             // ring: the forward sweep found a vertex (1), a count of 2^28 or more (2), a sum past 2^64 (4:
+                                 // count_overflows tells whether it is a count), a neighbour listed twice at level 1 (8)
     unsigned long long count[4];  // ring: vertices the forward sweep found, and finished (upper half)
     uint32_t pad[16];
 };

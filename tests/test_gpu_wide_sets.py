@@ -1,5 +1,6 @@
 """Batched and serving forms on the wide searches, where a set or pool is unlike the usual one: a single graph, most of
-whose vertices have no edge.  Against the oracle, within the suite's 1e-9; what no path passes is exactly 0."""
+whose vertices have no edge; path counts just below and just past 2^64.  Against the oracle, within the suite's 1e-9;
+what no path passes is exactly 0."""
 import numpy as np
 import pytest
 
@@ -63,3 +64,57 @@ def test_one_graph(gname):
     for got, want in zip(_serve([(offs, adj)], [(0, None), (0, k)]), (ref, part)):
         assert_bc_close(got, want, f"served {gname}")
         assert not np.any(got[alone])
+
+
+def _layers(width, depth):
+    """Complete bipartite layers (width^i paths to layer i + 1) and a triangle beside them, which keeps every vertex
+    unfinished: no source reaches both."""
+    ids = np.arange(width * depth).reshape(depth, width)
+    pairs = [np.stack(np.meshgrid(ids[i], ids[i + 1]), -1).reshape(-1, 2) for i in range(depth - 1)]
+    b = width * depth
+    return bcg.from_pairs(np.concatenate(pairs + [[[b, b + 1], [b + 1, b + 2], [b + 2, b]]]), b + 3)
+
+
+def _noalloc(offs, adj, src):
+    torch = pytest.importorskip("torch")
+    n = len(offs) - 1
+    o, a, s = (torch.from_numpy(x.view(np.int32)).cuda() for x in (offs, adj, src))
+    bc = torch.zeros(n, dtype=torch.float64, device="cuda")
+    bcg.bc_noalloc(o.data_ptr(), a.data_ptr(), n, len(adj), s.data_ptr(), len(src), bc.data_ptr())
+    return bc.cpu().numpy()
+
+
+@pytest.mark.parametrize("depth", [16, 17, 18])
+def test_counts_around_two_to_the_64(depth):
+    """16 paths more a layer: 2^60 is the largest count at depth 17, and a layer's sums of the one behind it, which are no
+    counts, reach 2^64.  At depth 18 a count does."""
+    offs, adj = _layers(16, depth)
+    n = len(offs) - 1
+    src = np.arange(n, dtype=np.uint32)
+    ref, ost = oracle.bc_q(offs, adj, src)
+    with bcg.Graph(offs, adj) as G:
+        st = G.run(src)
+        assert st.extended_sigma == (depth == 18)
+        assert_bc_close(G.bc(), ref, f"run, {depth} layers")
+    beside = bcg.from_pairs(np.concatenate([np.stack([np.repeat(np.arange(n), np.diff(offs.astype(np.int64))), adj], 1),
+                                            np.random.default_rng(31).integers(n, n + 20000, (130000, 2))]), n + 20000)
+    with bcg.Graph(*beside) as G:  # (too large for the small kernel)
+        st = G.run(src)
+        assert st.extended_sigma == (depth == 18) and (depth == 18 or st.batch_width in WIDE)
+        assert_bc_close(G.bc()[:n], ref, f"run, {depth} layers beside a component")
+    assert_bc_close(_noalloc(offs, adj, src), ref, f"no allocation, {depth} layers")
+    pool = [bcg.generate("er:scale=8,ef=8,seed=6"), (offs, adj)]
+    with bcg.Batch(pool) as B:
+        if depth < 18:
+            assert B.run().batch_width in WIDE
+            assert_bc_close(B.bc(1), ref, f"batch, {depth} layers")
+        else:
+            with pytest.raises(bcg.BcgError) as e:
+                B.run()
+            assert e.value.code == bcg.ERR_OVERFLOW
+    if depth < 18:
+        assert_bc_close(_serve(pool, [(1, None)])[0], ref, f"served, {depth} layers")
+    else:
+        with pytest.raises(bcg.BcgError) as e:
+            _serve(pool, [(1, None)])
+        assert e.value.code == bcg.ERR_OVERFLOW

@@ -31,9 +31,11 @@
 // alone or in any mix.  (24 requests, half exact, on ten graphs of 1,000 to
 // 30,000 vertices: 228 ms as packed waves, which pay barriers of the whole chip
 // for every sweep; 10 ms as wide ones.)  Nothing of a wave is added unless
-// all of its launches went through; a search of more than 62 levels stops it
-// and the waves behind it, their sources are taken back, and the pool is
-// served in packed waves from then on.
+// all of its launches went through.  A search of more than 62 levels ends its
+// own job only: the request starts over in packed waves, which take turns with
+// the wide ones.  Which of the two a request is served in depends on its graph
+// and sources alone, so its result does not depend on the other requests
+// there either.
 //
 // Continuity.  bcg_server_step never waits for the GPU: it retires the waves
 // that have finished (their requests become done), admits what fits, and
@@ -61,6 +63,7 @@ struct Req {
     uint32_t graph = 0;
     std::vector<uint32_t> src;  // union ids of the request's non-isolated sources, in order
     size_t sched = 0;           // sources already placed in a wave
+    bool packed = false;        // a wide wave met a search too deep for it: the request runs in packed waves
     double *d_out = nullptr;    // one accumulator per vertex of the graph (from admission on)
     size_t bytes = 0;
     bool done = false;
@@ -81,11 +84,12 @@ struct ServeWave {
     cudaEvent_t ev = nullptr;
     bool busy = false;
     std::vector<uint64_t> finishing;
-    // wide waves: jobs, sources and outputs; control words (and their copy)
-    unsigned char *h_jobs = nullptr, *d_jobs = nullptr, *d_stat = nullptr;
-    WideCtrl *h_ctrl = nullptr;
-    uint32_t spans = 0;                                   // launches of the wave (0: a packed wave)
-    std::vector<std::pair<uint64_t, size_t>> taken;       // requests and their sched before the wave
+    // wide waves: jobs, sources and outputs; teams, control words and the
+    // jobs' deep words (and a copy of the latter two)
+    unsigned char *h_jobs = nullptr, *d_jobs = nullptr, *d_stat = nullptr, *h_stat = nullptr;
+    uint32_t spans = 0;  // launches of the wave (0: a packed wave)
+    struct Part { uint64_t rid; uint32_t job0, njobs; };
+    std::vector<Part> parts;
 };
 
 struct bcg_server {
@@ -101,6 +105,8 @@ struct bcg_server {
     uint64_t next_id = 1;
     std::deque<uint64_t> pending;
     std::vector<std::deque<uint64_t>> queue;  // per graph: admitted requests with unscheduled sources, in order
+    std::vector<std::deque<uint64_t>> deep_queue;  // the same for those that a pool of wide waves runs in packed ones
+    bool deep_turn = false;                        // the last wave was one of queue
     std::deque<uint64_t> done;                // finished, not yet reported
     // wave schedule layout (one region per wave slot)
     size_t off_xbeg = 0, off_xroots = 0, off_xslot = 0, off_xpf = 0, off_xpu = 0, off_xtiles = 0, off_xrbeg = 0,
@@ -155,18 +161,25 @@ int admit(bcg_server *s) {
     return BCG_OK;
 }
 
-// Buffers of the packed waves.
+// Buffers of the packed waves.  After a failure the next call takes up what is
+// missing.
 int packed_setup(bcg_server *s) {
+    if (s->packed) return BCG_OK;
     const int rc = ensure_state(s->g, s->width);
     if (rc) return rc;
-    if (cudaMalloc(&s->d_slot_delta, (size_t)s->width * s->g->n * sizeof(double)) != cudaSuccess)
-        return set_error(BCG_ERR_OOM, "per-slot dependency buffer");
+    cudaError_t e = cudaSuccess;
+    auto take = [&](auto **p, size_t bytes) {
+        if (e == cudaSuccess && !*p && (e = cudaMalloc(p, bytes)) != cudaSuccess) *p = nullptr;
+    };
+    take(&s->d_slot_delta, (size_t)s->width * s->g->n * sizeof(double));
     for (ServeWave &w : s->slot) {
-        cudaError_t e;
-        if ((e = cudaMalloc(&w.d_blob, s->blob_bytes)) != cudaSuccess ||
-            (e = cudaMallocHost(&w.h_blob, s->blob_bytes)) != cudaSuccess ||
-            (e = cudaMalloc(&w.d_rstat, (size_t)s->wave_batches * s->width * sizeof(RootStat))) != cudaSuccess)
-            return set_error(BCG_ERR_CUDA, "server buffers: %s", cudaGetErrorString(e));
+        take(&w.d_blob, s->blob_bytes);
+        take(&w.d_rstat, (size_t)s->wave_batches * s->width * sizeof(RootStat));
+        if (e == cudaSuccess && !w.h_blob && (e = cudaMallocHost(&w.h_blob, s->blob_bytes)) != cudaSuccess) w.h_blob = nullptr;
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return set_error(e == cudaErrorMemoryAllocation ? BCG_ERR_OOM : BCG_ERR_CUDA, "server buffers: %s", cudaGetErrorString(e));
     }
     s->packed = true;
     return BCG_OK;
@@ -174,6 +187,8 @@ int packed_setup(bcg_server *s) {
 
 constexpr uint32_t kServeSlots = 32;  // sources of a job
 constexpr uint32_t kMaxSpans = 8;  // launches of a wide wave
+// ServeWave::d_stat: the launches' teams, their control words, the jobs' deep words
+constexpr size_t kTeamBytes = kMaxSpans * kWideTeams * sizeof(WideTeam), kCtrlBytes = kMaxSpans * sizeof(WideCtrl);
 
 void wide_clear(bcg_server *s) {
     wide_form_free(s->form);
@@ -185,9 +200,8 @@ void wide_clear(bcg_server *s) {
         dev_free(w.d_jobs);
         dev_free(w.d_stat);
         if (w.h_jobs) cudaFreeHost(w.h_jobs);
-        if (w.h_ctrl) cudaFreeHost(w.h_ctrl);
-        w.d_jobs = w.d_stat = w.h_jobs = nullptr;
-        w.h_ctrl = nullptr;
+        if (w.h_stat) cudaFreeHost(w.h_stat);
+        w.d_jobs = w.d_stat = w.h_jobs = w.h_stat = nullptr;
     }
     s->wide = false;
 }
@@ -224,7 +238,7 @@ int wide_setup(bcg_server *s) {
     s->off_wroots = up16(jobs * sizeof(WideJob));
     s->off_wouts = s->off_wroots + up16(jobs * kServeSlots * 4);
     s->wblob_bytes = s->off_wouts + jobs * sizeof(WideOut);
-    const size_t stat = kMaxSpans * (sizeof(WideCtrl) + kWideTeams * sizeof(WideTeam));
+    const size_t stat = kTeamBytes + kCtrlBytes + up16(jobs * 4);
     size_t scratch = 0;
     const uint64_t extra =
         wide_form_bytes(in, &scratch) + s->wstate_bytes + s->cells * 8 + kInFlight * (s->wblob_bytes + stat);
@@ -240,7 +254,7 @@ int wide_setup(bcg_server *s) {
         if (!rc && ((e = dev_alloc(&w.d_jobs, s->wblob_bytes)) != cudaSuccess ||
                     (e = cudaMallocHost(&w.h_jobs, s->wblob_bytes)) != cudaSuccess ||
                     (e = dev_alloc(&w.d_stat, stat)) != cudaSuccess ||
-                    (e = cudaMallocHost(&w.h_ctrl, kMaxSpans * sizeof(WideCtrl))) != cudaSuccess))
+                    (e = cudaMallocHost(&w.h_stat, kCtrlBytes + up16(jobs * 4))) != cudaSuccess))
             rc = set_error(e == cudaErrorMemoryAllocation ? BCG_ERR_OOM : BCG_ERR_CUDA, "wide waves: %s", cudaGetErrorString(e));
     CKS(cudaDeviceSynchronize());  // the buffers are ready for the server's stream
     if (rc) {
@@ -252,27 +266,18 @@ int wide_setup(bcg_server *s) {
     return BCG_OK;
 }
 
-// A deep search stopped the oldest wave: nothing of it or of the waves behind
-// it was added.  Takes their sources back and goes on in packed waves.
-int take_back(bcg_server *s) {
-    CKS(cudaStreamSynchronize(s->stream));
-    for (auto it = s->inflight.rbegin(); it != s->inflight.rend(); ++it) {
-        ServeWave &w = s->slot[*it];
-        for (auto t = w.taken.rbegin(); t != w.taken.rend(); ++t) s->reqs[t->first].sched = t->second;
-        w.taken.clear();
-        w.finishing.clear();
-        w.busy = false;
-    }
-    s->inflight.clear();
-    // every admitted request that is not done, in admission order (ids ascend)
-    std::vector<uint64_t> ids;
-    for (auto &kv : s->reqs)
-        if (kv.second.d_out && !kv.second.done) ids.push_back(kv.first);
-    std::sort(ids.begin(), ids.end());
-    for (auto &q : s->queue) q.clear();
-    for (uint64_t id : ids) s->queue[s->reqs[id].graph].push_back(id);
-    wide_clear(s);
-    return packed_setup(s);
+// A search of the request was too deep for the wide waves: it starts over in
+// packed ones.  (Waves that are still queued may add to its buffer: it is
+// cleared behind them.)
+int demote(bcg_server *s, uint64_t rid) {
+    Req &r = s->reqs[rid];
+    auto &q = s->queue[r.graph];
+    q.erase(std::remove(q.begin(), q.end(), rid), q.end());
+    r.packed = true;
+    r.sched = 0;
+    s->deep_queue[r.graph].push_back(rid);
+    CKS(cudaMemsetAsync(r.d_out, 0, r.bytes, s->stream));
+    return BCG_OK;
 }
 
 // Plans the next wide wave and enqueues it (enqueue_wave's wide form).
@@ -291,7 +296,7 @@ int enqueue_wide_wave(bcg_server *s, ServeWave &w, int wi, bool *launched) {
     uint32_t nj = 0, nr = 0, no = 0, nmax = 1;
     uint64_t cells = 0;
     w.finishing.clear();
-    w.taken.clear();
+    w.parts.clear();
     for (uint32_t gi : act) {
         const WideSub &sub = s->form.subs[gi];
         auto &q = s->queue[gi];
@@ -303,8 +308,8 @@ int enqueue_wide_wave(bcg_server *s, ServeWave &w, int wi, bool *launched) {
                                                                 (uint64_t)s->wave_batches - used,
                                                                 sub.n ? (s->cells - cells) / sub.n : 0});
             if (left && !take) break;  // the wave is full (for this graph)
-            w.taken.emplace_back(q.front(), r.sched);
             if (take) {
+                w.parts.push_back(ServeWave::Part{q.front(), nj, take});
                 if (spans.empty() || (sub.n < spans.back().nmax / 4 && spans.back().njobs >= 2 * 148 && spans.size() < kMaxSpans))
                     spans.push_back(Span{nj, 0, sub.n, 1, 1, 0});
                 Span &l = spans.back();
@@ -314,7 +319,7 @@ int enqueue_wide_wave(bcg_server *s, ServeWave &w, int wi, bool *launched) {
                 // (the map gives union ids: the buffer is addressed from the union's start)
                 double *out = reinterpret_cast<double *>(reinterpret_cast<uintptr_t>(r.d_out) -
                                                          (uintptr_t)s->base[gi] * sizeof(double));
-                outs[no++] = WideOut{cells, take, sub.n, s->form.map + sub.base, out, nullptr};
+                outs[no++] = WideOut{cells, take, sub.n, s->form.map + sub.base, out, nullptr, nj, 0};
                 for (uint32_t j = 0; j < take; ++j) {
                     const uint32_t k = (uint32_t)std::min<size_t>(kServeSlots, r.src.size() - r.sched);
                     jobs[nj++] = WideJob{gi, nr, k, 0, cells};
@@ -332,13 +337,14 @@ int enqueue_wide_wave(bcg_server *s, ServeWave &w, int wi, bool *launched) {
         }
     }
     w.spans = std::max<uint32_t>(1, (uint32_t)spans.size());
-    memset(w.h_ctrl, 0, kMaxSpans * sizeof(WideCtrl));
+    memset(w.h_stat, 0, kCtrlBytes);
     if (nj) {
+        uint32_t *deep_jobs = reinterpret_cast<uint32_t *>(w.d_stat + kTeamBytes + kCtrlBytes);
         // (one copy up to the last output that is used)
         CKS(cudaMemcpyAsync(w.d_jobs, w.h_jobs, s->off_wroots + (size_t)nr * 4, cudaMemcpyHostToDevice, s->stream));
         CKS(cudaMemcpyAsync(w.d_jobs + s->off_wouts, w.h_jobs + s->off_wouts, no * sizeof(WideOut), cudaMemcpyHostToDevice,
                             s->stream));
-        CKS(cudaMemsetAsync(w.d_stat, 0, kMaxSpans * (sizeof(WideCtrl) + kWideTeams * sizeof(WideTeam)), s->stream));
+        CKS(cudaMemsetAsync(w.d_stat, 0, kTeamBytes + kCtrlBytes + nj * sizeof(uint32_t), s->stream));
         WideArgs a{};
         for (size_t k = 0; k < spans.size(); ++k) {
             const Span &l = spans[k];
@@ -354,15 +360,16 @@ int enqueue_wide_wave(bcg_server *s, ServeWave &w, int wi, bool *launched) {
             a.roots = reinterpret_cast<const uint32_t *>(w.d_jobs + s->off_wroots);
             a.jobbc = s->d_jobbc;
             a.poison = s->d_poison;
-            a.ctrl = reinterpret_cast<WideCtrl *>(w.d_stat) + k;
-            a.team = reinterpret_cast<WideTeam *>(w.d_stat + kMaxSpans * sizeof(WideCtrl)) + k * kWideTeams;
+            a.deep_jobs = deep_jobs + l.job0;
+            a.ctrl = reinterpret_cast<WideCtrl *>(w.d_stat + kTeamBytes) + k;
+            a.team = reinterpret_cast<WideTeam *>(w.d_stat) + k * kWideTeams;
             a.state = s->d_wstate;
             const int rc = wide_enqueue(a, nullptr, 0, WideOut{}, 1, s->stream);
             if (rc) return rc;
         }
-        const int rc = wide_chain(a, reinterpret_cast<const WideOut *>(w.d_jobs + s->off_wouts), no, nmax, s->stream);
+        const int rc = wide_chain(a, reinterpret_cast<const WideOut *>(w.d_jobs + s->off_wouts), no, nmax, deep_jobs, s->stream);
         if (rc) return rc;
-        CKS(cudaMemcpyAsync(w.h_ctrl, w.d_stat, kMaxSpans * sizeof(WideCtrl), cudaMemcpyDeviceToHost, s->stream));
+        CKS(cudaMemcpyAsync(w.h_stat, w.d_stat + kTeamBytes, kCtrlBytes + nj * sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
     }
     CKS(cudaEventRecord(w.ev, s->stream));
     w.busy = true;
@@ -386,15 +393,12 @@ int retire(bcg_server *s, bool wait) {
             if (q != cudaSuccess) return set_error(BCG_ERR_CUDA, "wave event: %s", cudaGetErrorString(q));
         }
         if (w.spans) {
-            int error = 0, overflow = 0, deep = 0;
+            const WideCtrl *c = reinterpret_cast<const WideCtrl *>(w.h_stat);
+            w.h_flags[0] = w.h_flags[1] = 0;
             for (uint32_t k = 0; k < w.spans; ++k) {
-                error = w.h_ctrl[k].error ? w.h_ctrl[k].error : error;
-                overflow |= w.h_ctrl[k].overflow;
-                deep |= w.h_ctrl[k].deep;
+                if (c[k].error) w.h_flags[0] = c[k].error;
+                w.h_flags[1] |= c[k].overflow;
             }
-            if (deep && !error && !overflow) return take_back(s);
-            w.h_flags[0] = error;
-            w.h_flags[1] = overflow;
         }
         if (w.h_flags[1] || w.h_flags[0] == BCG_ERR_OVERFLOW) {
             s->sticky_error = BCG_ERR_OVERFLOW;
@@ -404,8 +408,19 @@ int retire(bcg_server *s, bool wait) {
             s->sticky_error = w.h_flags[0];
             return set_error(w.h_flags[0], "device reported error %d in a served wave", w.h_flags[0]);
         }
+        if (w.spans) {
+            const uint32_t *deep = reinterpret_cast<const uint32_t *>(w.h_stat + kCtrlBytes);
+            for (const ServeWave::Part &p : w.parts) {
+                if (s->reqs[p.rid].packed || std::find(deep + p.job0, deep + p.job0 + p.njobs, 1u) == deep + p.job0 + p.njobs) continue;
+                const int rc = demote(s, p.rid);
+                if (rc) return rc;
+            }
+            w.parts.clear();
+        }
         for (uint64_t rid : w.finishing) {
-            s->reqs[rid].done = true;
+            Req &r = s->reqs[rid];
+            if (w.spans && r.packed) continue;  // it finishes in a packed wave
+            r.done = true;
             s->done.push_back(rid);
         }
         w.finishing.clear();
@@ -425,13 +440,26 @@ int enqueue_wave(bcg_server *s, bool *launched) {
         if (!s->slot[i].busy) { wi = i; break; }
     if (wi < 0) return BCG_OK;
     const uint32_t G = s->ngraphs, W = s->wave_batches;
-    if (s->wide) return enqueue_wide_wave(s, s->slot[wi], wi, launched);
+    if (s->wide) {  // wide waves, in turns with packed ones where there is work for both
+        auto any = [](const std::vector<std::deque<uint64_t>> &qs) {
+            return std::any_of(qs.begin(), qs.end(), [](const std::deque<uint64_t> &q) { return !q.empty(); });
+        };
+        const bool deep = any(s->deep_queue) && (s->deep_turn || !any(s->queue));
+        if (!deep) {
+            s->deep_turn = true;
+            return enqueue_wide_wave(s, s->slot[wi], wi, launched);
+        }
+        s->deep_turn = false;
+        const int rc = packed_setup(s);
+        if (rc) return rc;
+    }
+    std::vector<std::deque<uint64_t>> &queue = s->wide ? s->deep_queue : s->queue;
     s->slot[wi].spans = 0;
     // the graphs with work, and their active vertices (for the width rule)
     std::vector<uint32_t> act;
     uint64_t act_n = 0;
     for (uint32_t gi = 0; gi < G; ++gi) {
-        if (s->queue[gi].empty()) continue;
+        if (queue[gi].empty()) continue;
         act.push_back(gi);
         act_n += s->gn[gi];
     }
@@ -445,7 +473,7 @@ int enqueue_wave(bcg_server *s, bool *launched) {
     w.finishing.clear();
     uint32_t nb = 0;
     for (size_t a = 0; a < act.size(); ++a) {
-        auto &q = s->queue[act[a]];
+        auto &q = queue[act[a]];
         const size_t cap = (size_t)W * S;
         while (!q.empty() && picks[a].size() < cap) {
             Req &r = s->reqs[q.front()];
@@ -580,6 +608,7 @@ int bcg_server_create(uint32_t ngraphs, const uint32_t *const *offsets, const ui
     s->gn.assign(n, n + ngraphs);
     s->wave_batches = wave_batches;
     s->queue.resize(ngraphs);
+    s->deep_queue.resize(ngraphs);
     // tiles that never cross a graph boundary: graph g owns tiles [x, y)
     std::vector<uint32_t> breaks(ngraphs);
     for (uint32_t i = 0; i < ngraphs; ++i) breaks[i] = s->base[i];

@@ -1095,11 +1095,16 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
         bool ones = false;  // every count of level 1 is 1
         for (;; ++d) {
             if (d + 2 >= kWideLevels) {
-                if (threadIdx.x == 0) {
-                    a.ctrl->deep = 1;
-                    if (a.poison) *a.poison = 1;
+                if (!a.deep_jobs) {
+                    if (threadIdx.x == 0) {
+                        a.ctrl->deep = 1;
+                        if (a.poison) *a.poison = 1;
+                    }
+                    return;
                 }
-                return;
+                if (x.rank == 0 && threadIdx.x == 0) a.deep_jobs[job] = 1u;
+                d = kWideLevels;  // the job is left
+                break;
             }
             for (uint32_t w = tid; w < (n + 31u) >> 5; w += nt) x.act[(size_t)(d + 2) * x.words + w] = 0;
             if (x.rank == 0 && threadIdx.x == 0) {
@@ -1138,9 +1143,10 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
             big = (any & 2u) != 0;
             ones = d == 0 && !(any & 8u);
         }
-        const uint32_t D = d;
+        const uint32_t D = d == kWideLevels ? 0u : d;
 
         // ---- what each source reached: a thread's vertices, four slots each
+        // (a job is left by callers that do not ask)
         const bool counted = a.rstat || a.total;
         if (threadIdx.x < 3 * NS) sm.reach[threadIdx.x] = 0ull;
         __syncthreads();
@@ -1239,9 +1245,13 @@ __global__ void __launch_bounds__(256) k_wide_reduce(const WideCtrl *__restrict_
 // The same in strict job order, so that the bits do not depend on how the
 // jobs of a graph are spread over launches.
 __global__ void __launch_bounds__(256) k_wide_chain(const int *__restrict__ poison, const WideOut *__restrict__ outs,
-                                                    const double *__restrict__ jobbc) {
+                                                    const double *__restrict__ jobbc,
+                                                    const uint32_t *__restrict__ deep_jobs) {
     if (*poison) return;
     const WideOut o = outs[blockIdx.y];
+    bool left = false;
+    for (uint32_t j = threadIdx.x; j < o.njobs; j += 256) left |= deep_jobs[o.job0 + j] != 0u;
+    if (__syncthreads_or(left)) return;
     for (uint32_t v = blockIdx.x * 256 + threadIdx.x; v < o.n; v += gridDim.x * 256) {
         const double *q = jobbc + o.out0 + v;
         double *b = o.bc + o.map[v];
@@ -1407,10 +1417,11 @@ int wide_enqueue(const WideArgs &a, const WideOut *outs, uint32_t nouts, const W
     return BCG_OK;
 }
 
-int wide_chain(const WideArgs &a, const WideOut *outs, uint32_t nouts, uint32_t nmax, cudaStream_t st) {
+int wide_chain(const WideArgs &a, const WideOut *outs, uint32_t nouts, uint32_t nmax, const uint32_t *deep_jobs,
+               cudaStream_t st) {
     const unsigned bx = (unsigned)std::max<size_t>(1, std::min<size_t>(1024, ((size_t)nmax + 255) / 256));
     for (uint32_t o = 0; o < nouts; o += 65535u)
-        k_wide_chain<<<dim3(bx, std::min(65535u, nouts - o)), 256, 0, st>>>(a.poison, outs + o, a.jobbc);
+        k_wide_chain<<<dim3(bx, std::min(65535u, nouts - o)), 256, 0, st>>>(a.poison, outs + o, a.jobbc, deep_jobs);
     CKW(cudaGetLastError());
     return BCG_OK;
 }

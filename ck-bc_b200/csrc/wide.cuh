@@ -81,6 +81,8 @@ struct WideArgs {
     double *jobbc;
     int *poison;            // several launches' stop word (nullptr: none): set by a launch that
                             // stops, and a launch that finds it set does nothing
+    uint32_t *deep_jobs;    // njobs words (zeroed): a job with a search of more levels than it holds
+                            // sets its word and is left; nullptr: such a job stops the launch
     RootStat *rstat;        // njobs * slots, zeroed (nullptr: not wanted)
     RootStat *total;        // or the sums over all sources, and the deepest level (zeroed)
     WideCtrl *ctrl;
@@ -103,6 +105,7 @@ struct WideOut {
     const uint32_t *map;
     double *bc;
     const WideSub *sub;  // set: n is its n (not known to the host)
+    uint32_t job0, pad;  // its first job's word of deep_jobs (wide_chain)
 };
 
 // The lists a wide form is made from (device arrays; vinfo and ext by engine
@@ -174,7 +177,9 @@ int wide_order(const WideSub *sub, const uint32_t *roots, const double *mult, ui
 int wide_enqueue(const WideArgs &a, const WideOut *outs, uint32_t nouts, const WideOut &one, uint32_t nmax,
                  cudaStream_t st);
 
-// Adds the vectors in strict job order (a.poison unset).
-int wide_chain(const WideArgs &a, const WideOut *outs, uint32_t nouts, uint32_t nmax, cudaStream_t st);
+// Adds the vectors in strict job order (a.poison unset); of an entry with a
+// job that was left, none.
+int wide_chain(const WideArgs &a, const WideOut *outs, uint32_t nouts, uint32_t nmax, const uint32_t *deep_jobs,
+               cudaStream_t st);
 
 }  // namespace bcg

@@ -1,5 +1,6 @@
 """Batched and serving forms on the wide searches, where a set or pool is unlike the usual one: a single graph, most of
-whose vertices have no edge; path counts just below and just past 2^64.  Against the oracle, within the suite's 1e-9;
+whose vertices have no edge; path counts just below and just past 2^64; graphs with searches too deep for wide waves.
+Against the oracle, within the suite's 1e-9;
 what no path passes is exactly 0."""
 import numpy as np
 import pytest
@@ -118,3 +119,34 @@ def test_counts_around_two_to_the_64(depth):
         with pytest.raises(bcg.BcgError) as e:
             _serve(pool, [(1, None)])
         assert e.value.code == bcg.ERR_OVERFLOW
+
+
+def _cliques(size, count):
+    """Cliques in a row, neighbours joined by one edge: two levels a clique, one path a pair."""
+    pairs = []
+    for c in range(count):
+        b = c * size
+        pairs += [[b + i, b + j] for i in range(size) for j in range(i)]
+        if c:
+            pairs.append([b - 1, b])
+    return bcg.from_pairs(pairs, size * count)
+
+
+@pytest.mark.parametrize("wave_batches", [1, 4, 64])
+def test_deep_searches_of_a_served_pool(wave_batches):
+    """A graph whose searches from the middle have 60 levels and from the ends 119, so some of its requests run in wide
+    waves and some in packed ones, found out in the first or only in a later wave; the other graph's requests beside
+    them.  Every request gives the bits that it gives alone."""
+    deep = _cliques(8, 60)
+    pool = [deep, bcg.generate("rmat:scale=10,ef=16,a=0.57,b=0.19,c=0.19,seed=5")]
+    middle, ends = np.arange(236, 244, dtype=np.uint32), np.array([0, 1, 478], dtype=np.uint32)
+    last = np.concatenate([np.tile(middle, 12), ends]).astype(np.uint32)  # 99 sources, the deep ones in the fourth job
+    reqs = [(1, None), (0, middle), (0, ends), (1, np.arange(0, 900, 7, dtype=np.uint32)), (0, None), (0, last),
+            (1, np.array([3], dtype=np.uint32)), (0, middle[:1]), (0, ends[:1])]
+    served = _serve(pool, reqs, wave_batches=wave_batches)
+    for i, (g, src) in enumerate(reqs):
+        offs, adj = pool[g]
+        ref, _ = oracle.bc(offs, adj, np.arange(len(offs) - 1) if src is None else src, nthreads=oracle.max_threads())
+        assert_bc_close(served[i], ref, f"request {i}")
+        alone = _serve(pool, [reqs[i]], wave_batches=wave_batches)[0]
+        assert np.array_equal(served[i].view(np.uint64), alone.view(np.uint64)), i

@@ -24,7 +24,8 @@
 //
 // Wide waves.  A pool of shallow graphs (wide_shallow) runs its waves as
 // wide-batch searches (wide.cu) instead: a request's sources in its own order,
-// 16 a job, up to wave_batches jobs of a graph a wave; the jobs of graphs of
+// 32 a job, up to wave_batches jobs of a graph a wave and at least one of every
+// graph with work (the vectors' memory is dealt in turn); the jobs of graphs of
 // like size share a launch, in which a CTA or a few take a job.  Every job's
 // vector is added to its request's buffer in the request's job order, and a
 // job's sums do not depend on the launch, so here too the result is the same
@@ -219,21 +220,23 @@ int wide_setup(bcg_server *s) {
     in.base = ubase.data();
     in.big_nnz = 0;
     uint32_t nmax = 1;
+    uint64_t nall = 0;
     for (uint32_t i = 0; i < G; ++i) {
         uint64_t act = 0;
         for (uint32_t v = ubase[i]; v < ubase[i + 1]; ++v) act += s->hdeg[v] != 0;
         if (!wide_shallow(act, s->gnnz[i])) return BCG_OK;
         in.big_nnz = std::max<uint64_t>(in.big_nnz, s->gnnz[i]);
         nmax = std::max(nmax, (uint32_t)act);
+        nall += act;
     }
     if (g->n >= (1u << 28)) return BCG_OK;
     // a team's state for the largest graph, and up to 256 MB for more teams;
     // job vectors for a wave of 148 of the largest graph's jobs, up to 256 MB
-    // (one at least)
+    // (one of every graph at least, so that a wave advances them all)
     WideArgs a{};
     const size_t stride = wide_layout(a, kServeSlots, nmax, in.big_nnz / kWideChunk * 2 + 1, in.big_nnz / kWideChunk + 1);
     s->wstate_bytes = std::max(stride, std::min<size_t>(148 * stride, 256ull << 20));
-    s->cells = std::max<uint64_t>(nmax, std::min<uint64_t>(148ull * 8 * nmax, (256ull << 20) / 8));
+    s->cells = std::max<uint64_t>({nmax, nall, std::min<uint64_t>(148ull * 8 * nmax, (256ull << 20) / 8)});
     const size_t jobs = (size_t)s->wave_batches * G;
     s->off_wroots = up16(jobs * sizeof(WideJob));
     s->off_wouts = s->off_wroots + up16(jobs * kServeSlots * 4);
@@ -297,16 +300,36 @@ int enqueue_wide_wave(bcg_server *s, ServeWave &w, int wi, bool *launched) {
     uint64_t cells = 0;
     w.finishing.clear();
     w.parts.clear();
-    for (uint32_t gi : act) {
+    // the wave's jobs of each graph, dealt in turn while their vectors fit
+    std::vector<uint32_t> quota(act.size(), 0), want(act.size(), 0);
+    for (size_t k = 0; k < act.size(); ++k) {
+        uint64_t jobs = 0;
+        for (auto it = s->queue[act[k]].begin(); it != s->queue[act[k]].end() && jobs < s->wave_batches; ++it) {
+            const Req &r = s->reqs[*it];
+            jobs += (r.src.size() - r.sched + kServeSlots - 1) / kServeSlots;
+        }
+        want[k] = (uint32_t)std::min<uint64_t>(jobs, s->wave_batches);
+    }
+    uint64_t dealt = 0;
+    for (bool more = true; more;) {
+        more = false;
+        for (size_t k = 0; k < act.size(); ++k) {
+            const uint32_t n = s->form.subs[act[k]].n;
+            if (quota[k] == want[k] || dealt + n > s->cells) continue;
+            ++quota[k];
+            dealt += n;
+            more = true;
+        }
+    }
+    for (size_t ai = 0; ai < act.size(); ++ai) {
+        const uint32_t gi = act[ai];
         const WideSub &sub = s->form.subs[gi];
         auto &q = s->queue[gi];
         uint32_t used = 0;  // jobs of this graph
         while (!q.empty()) {
             Req &r = s->reqs[q.front()];
             const size_t left = r.src.size() - r.sched;
-            const uint32_t take = (uint32_t)std::min<uint64_t>({(left + kServeSlots - 1) / kServeSlots,
-                                                                (uint64_t)s->wave_batches - used,
-                                                                sub.n ? (s->cells - cells) / sub.n : 0});
+            const uint32_t take = (uint32_t)std::min<uint64_t>((left + kServeSlots - 1) / kServeSlots, quota[ai] - used);
             if (left && !take) break;  // the wave is full (for this graph)
             if (take) {
                 w.parts.push_back(ServeWave::Part{q.front(), nj, take});

@@ -340,7 +340,8 @@ typedef struct bcg_server bcg_server;  /* opaque: a resident pool and its reques
 
 /* Uploads the pool (as bcg_batch_create) and sizes the wave schedule:
  * wave_batches = batches of S sources each graph may advance per wave
- * (1..65535).  Fails with BCG_ERR_OOM when the pool alone exceeds
+ * (1..65535; a pool of shallow graphs runs jobs of 32 sources instead, see
+ * bcg_server_step).  Fails with BCG_ERR_OOM when the pool alone exceeds
  * hbm_budget_bytes. */
 int bcg_server_create(uint32_t ngraphs, const uint32_t *const *offsets,
                       const uint32_t *const *adj, const uint32_t *n,
@@ -360,6 +361,11 @@ int bcg_server_submit(bcg_server *s, uint32_t graph, const uint32_t *sources, ui
  * waves queued (a wave: every graph with admitted requests runs up to
  * wave_batches * S of their unscheduled sources, oldest request first, all
  * graphs in one packed launch), then reports up to cap finished request ids.
+ * A pool whose graphs are all shallow (mean degree 6 and up, or a few
+ * vertices) runs its waves as wide-batch searches: every graph with admitted
+ * requests runs one to wave_batches jobs of 32 sources, as many as the wave's
+ * memory, dealt to the graphs in turn, allows; a request with a search of more
+ * than 62 levels is run again in packed waves, in turns with the wide ones.
  * A request's result is bitwise the same alone or in any mix. */
 int bcg_server_step(bcg_server *s, uint64_t *done_ids, uint32_t cap, uint32_t *ndone);
 /* bcg_server_step after waiting (without holding the lock) for the oldest

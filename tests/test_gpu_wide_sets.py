@@ -1,6 +1,6 @@
 """Batched and serving forms on the wide searches, where a set or pool is unlike the usual one: a single graph, most of
-whose vertices have no edge; path counts just below and just past 2^64; graphs with searches too deep for wide waves.
-Against the oracle, within the suite's 1e-9;
+whose vertices have no edge; path counts just below and just past 2^64; graphs with searches too deep for wide waves;
+waves whose memory is full.  Against the oracle, within the suite's 1e-9;
 what no path passes is exactly 0."""
 import numpy as np
 import pytest
@@ -150,3 +150,25 @@ def test_deep_searches_of_a_served_pool(wave_batches):
         assert_bc_close(served[i], ref, f"request {i}")
         alone = _serve(pool, [reqs[i]], wave_batches=wave_batches)[0]
         assert np.array_equal(served[i].view(np.uint64), alone.view(np.uint64)), i
+
+
+def test_a_full_wave_advances_every_graph():
+    """More jobs of the larger graph than a wave's memory holds (148 x 8 of its vectors): the smaller graph's request, the
+    last to be submitted, ends with the first wave all the same."""
+    pool = [bcg.generate("rmat:scale=11,ef=16,a=0.57,b=0.19,c=0.19,seed=5"), bcg.generate("er:scale=8,ef=8,seed=6")]
+    refs = [oracle.bc(o, a, np.arange(len(o) - 1), nthreads=oracle.max_threads())[0] for o, a in pool]
+    jobs = -(-np.count_nonzero(np.diff(pool[0][0])) // 32)
+    with bcg.Server(pool, 8 << 30, 60000) as S:
+        ids = [S.submit(0) for _ in range(5 * 148 * 8 // jobs)]  # five waves
+        small = S.submit(1)
+        first, out = None, {}
+        while len(out) <= len(ids):
+            done = S.wait()
+            first = first or done
+            for rid in done:
+                out[rid] = S.result(rid)
+    assert small in first and not set(ids) <= set(first)
+    assert_bc_close(out[small], refs[1], "small")
+    for rid in ids:
+        assert_bc_close(out[rid], refs[0], "large")
+        assert np.array_equal(out[rid].view(np.uint64), out[ids[0]].view(np.uint64))

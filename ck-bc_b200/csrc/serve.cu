@@ -46,6 +46,7 @@
 // threads may submit while a wave is on the GPU: such a request is admitted
 // at once if its buffer fits and joins the next wave that is planned.
 #include <algorithm>
+#include <cstdlib>
 #include <cstring>
 #include <deque>
 #include <mutex>
@@ -66,6 +67,7 @@ struct Req {
     size_t sched = 0;           // sources already placed in a wave
     bool packed = false;        // a wide wave met a search too deep for it: the request runs in packed waves
     double *d_out = nullptr;    // one accumulator per vertex of the graph (from admission on)
+    double *h_out = nullptr;    // or, once done, the result in host memory (make_room)
     size_t bytes = 0;
     bool done = false;
 };
@@ -148,11 +150,44 @@ uint64_t pool_bytes(const bcg_graph *g, uint32_t S) {
            8ull * (kMaxLevel + 3);
 }
 
-// Admits pending requests, FIFO, while their buffers fit the budget.
+// Moves the result of a finished request that nobody has fetched to host
+// memory; *moved = false when there is none (or no host memory).
+int make_room(bcg_server *s, bool *moved) {
+    *moved = false;
+    for (auto &kv : s->reqs) {
+        Req &r = kv.second;
+        if (!r.done || !r.d_out) continue;
+        double *h = static_cast<double *>(malloc(r.bytes));
+        if (!h) return BCG_OK;
+        cudaError_t e = cudaMemcpyAsync(h, r.d_out, r.bytes, cudaMemcpyDeviceToHost, s->result_stream);
+        if (e == cudaSuccess) e = cudaFreeAsync(r.d_out, s->result_stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s->result_stream);
+        if (e != cudaSuccess) {
+            free(h);
+            return set_error(BCG_ERR_CUDA, "moving a result to host memory: %s", cudaGetErrorString(e));
+        }
+        r.h_out = h;
+        r.d_out = nullptr;
+        s->admitted -= r.bytes;
+        *moved = true;
+        return BCG_OK;
+    }
+    return BCG_OK;
+}
+
+// Admits pending requests, FIFO, while their buffers fit the budget.  The wide
+// waves' buffers leave room for any one of them, but for fewer finished results
+// at a time than a pool without them: those give way to a request that waits.
 int admit(bcg_server *s) {
     while (!s->pending.empty()) {
         Req &r = s->reqs[s->pending.front()];
-        if (s->resident + s->admitted + r.bytes > s->budget) break;
+        if (s->resident + s->admitted + r.bytes > s->budget) {
+            bool moved = false;
+            const int rc = s->wide ? make_room(s, &moved) : BCG_OK;
+            if (rc) return rc;
+            if (!moved) break;
+            continue;
+        }
         CKS(cudaMallocAsync(reinterpret_cast<void **>(&r.d_out), r.bytes, s->stream));
         CKS(cudaMemsetAsync(r.d_out, 0, r.bytes, s->stream));
         s->admitted += r.bytes;
@@ -209,7 +244,7 @@ void wide_clear(bcg_server *s) {
 
 // Sets up the wide waves (s->wide = true) if every graph of the pool is
 // shallow and their buffers fit the budget beside the packed waves' (which a
-// deep search may still need).
+// deep search may still need) and the largest graph's result.
 int wide_setup(bcg_server *s) {
     bcg_graph *g = s->g;
     const uint32_t G = s->ngraphs;
@@ -245,7 +280,8 @@ int wide_setup(bcg_server *s) {
     size_t scratch = 0;
     const uint64_t extra =
         wide_form_bytes(in, &scratch) + s->wstate_bytes + s->cells * 8 + kInFlight * (s->wblob_bytes + stat);
-    if (s->resident + extra + scratch > s->budget) return BCG_OK;
+    const uint64_t result = *std::max_element(s->gn.begin(), s->gn.end()) * sizeof(double);
+    if (s->resident + extra + std::max<uint64_t>(scratch, result) > s->budget) return BCG_OK;
     int rc = wide_form_make(s->form, in, false);
     cudaError_t e = cudaSuccess;
     if (!rc && ((e = dev_alloc(&s->d_wstate, s->wstate_bytes)) != cudaSuccess ||
@@ -697,8 +733,10 @@ int bcg_server_destroy(bcg_server *s) {
         std::lock_guard<std::mutex> lock(s->mu);
         if (s->stream) cudaStreamSynchronize(s->stream);
         if (s->result_stream) cudaStreamSynchronize(s->result_stream);
-        for (auto &kv : s->reqs)
+        for (auto &kv : s->reqs) {
             if (kv.second.d_out) cudaFree(kv.second.d_out);
+            free(kv.second.h_out);
+        }
         wide_clear(s);
         if (s->d_poison) cudaFree(s->d_poison);
         for (ServeWave &w : s->slot) {
@@ -778,6 +816,12 @@ int bcg_server_result(bcg_server *s, uint64_t id, double *bc_host) {
     if (it == s->reqs.end()) return set_error(BCG_ERR_ARG, "unknown request %llu", (unsigned long long)id);
     Req &r = it->second;
     if (!r.done) return set_error(BCG_ERR_ARG, "request %llu is not finished", (unsigned long long)id);
+    if (r.h_out) {
+        memcpy(bc_host, r.h_out, r.bytes);
+        free(r.h_out);
+        s->reqs.erase(it);
+        return BCG_OK;
+    }
     // the last wave that wrote the buffer has completed: copy on the result
     // stream, so later waves queued on the server's stream keep running
     CKS(cudaMemcpyAsync(bc_host, r.d_out, r.bytes, cudaMemcpyDeviceToHost, s->result_stream));

@@ -351,7 +351,11 @@ int bcg_server_destroy(bcg_server *s);
  * vertex of the graph, i.e. exact BC).  Sources of degree 0 are skipped, as
  * in bcg_run.  Its result buffer (8 bytes per vertex of the graph) is
  * allocated when the request is admitted, first come first served, while the
- * pool plus admitted buffers fit the budget.  Every bcg_server_* call takes
+ * pool plus admitted buffers fit the budget.  The pool's bytes include buffers
+ * that only make it faster (those of the wide waves, see bcg_server_step): they
+ * are taken if the largest graph's result still fits beside them, and results
+ * that nobody has fetched then give way to a request that waits for room (the
+ * step that admits it waits for their copy to host memory).  Every bcg_server_* call takes
  * the server's lock: submit may be called from any thread, also while a wave
  * is on the GPU (the request joins the next wave planned). */
 int bcg_server_submit(bcg_server *s, uint32_t graph, const uint32_t *sources, uint64_t nsrc,

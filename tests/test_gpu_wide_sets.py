@@ -1,6 +1,6 @@
 """Batched and serving forms on the wide searches, where a set or pool is unlike the usual one: a single graph, most of
 whose vertices have no edge; path counts just below and just past 2^64; graphs with searches too deep for wide waves;
-waves whose memory is full.  Against the oracle, within the suite's 1e-9;
+waves whose memory is full; budgets that hold little beside the pool.  Against the oracle, within the suite's 1e-9;
 what no path passes is exactly 0."""
 import numpy as np
 import pytest
@@ -172,3 +172,28 @@ def test_a_full_wave_advances_every_graph():
     for rid in ids:
         assert_bc_close(out[rid], refs[0], "large")
         assert np.array_equal(out[rid].view(np.uint64), out[ids[0]].view(np.uint64))
+
+
+def test_budgets_close_to_the_pool():
+    """Whatever the budget leaves beside the pool's buffers, a request whose result fits beside the pool is taken and ends;
+    several end before the first is fetched."""
+    offs, adj = bcg.generate("er:scale=13,ef=8,seed=6")
+    n = len(offs) - 1
+    src = bcg.sample_sources(n, 70, 1)
+    ref, _ = oracle.bc(offs, adj, src, nthreads=oracle.max_threads())
+    with bcg.Server([(offs, adj)], 8 << 30) as S:
+        full = S.info()["resident_bytes"]
+    for budget in list(range(full - 8 * n, full + 3 * 8 * n, 2 * n)) + [full + 8 * n - 1, full + 8 * n, full + 8 * n + 1]:
+        with bcg.Server([(offs, adj)], budget) as S:
+            ids = [S.submit(0, src) for _ in range(4)]
+            done = set()
+            for _ in range(1000):
+                done |= set(S.wait())
+                if len(done) == 4:
+                    break
+                info = S.info()
+                assert info["resident_bytes"] + info["admitted_bytes"] <= budget
+            assert done == set(ids), budget - full
+            for rid in ids:
+                assert_bc_close(S.result(rid), ref, f"budget {budget - full} bytes from the wide buffers")
+            assert S.info()["admitted_bytes"] == 0

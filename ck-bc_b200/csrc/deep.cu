@@ -508,16 +508,12 @@ cudaError_t launch_deep(DeepArgs &a, uint32_t most, uint32_t nsm, cudaStream_t s
 
 // What a graph keeps for its deep runs (bcg_graph::deep).
 struct DeepGraph {
-    uint32_t *ell = nullptr;
+    Workspace ell;
     int width = 0;         // neighbours of a row
-    unsigned char *mem = nullptr;
-    size_t cap = 0;
 };
 
 void deep_free(bcg_graph *g) {
     if (!g->deep) return;
-    dev_free(g->deep->ell);
-    dev_free(g->deep->mem);
     delete g->deep;
     g->deep = nullptr;
 }
@@ -532,90 +528,98 @@ static int deep_launch(bcg_graph *g, const uint32_t *roots, const double *mult, 
     if (!g->deep) {
         DeepGraph *w = g->deep = new DeepGraph();
         w->width = D;
-        const cudaError_t e = dev_alloc(&w->ell, (size_t)n * D * sizeof(uint32_t));
-        if (e == cudaErrorMemoryAllocation) {
-            cudaGetLastError();
+        cudaError_t e = w->ell.take((size_t)n * D * sizeof(uint32_t), 0, true);
+        if (e == cudaSuccess) {
+            uint32_t *ell = reinterpret_cast<uint32_t *>(w->ell.mem);
+            if (D == 4) k_deep_rows<4><<<(n + 255) / 256, 256>>>(n, g->d_offs, g->d_adj, ell);
+            else k_deep_rows<8><<<(n + 255) / 256, 256>>>(n, g->d_offs, g->d_adj, ell);
+            if ((e = cudaGetLastError()) == cudaSuccess) e = cudaDeviceSynchronize();  // ready for any stream
+        }
+        if (e != cudaSuccess) {
             deep_free(g);
+            if (e != cudaErrorMemoryAllocation) CKD(e);
+            cudaGetLastError();
             return BCG_OK;
         }
-        CKD(e);
-        if (D == 4) k_deep_rows<4><<<(n + 255) / 256, 256>>>(n, g->d_offs, g->d_adj, w->ell);
-        else k_deep_rows<8><<<(n + 255) / 256, 256>>>(n, g->d_offs, g->d_adj, w->ell);
-        CKD(cudaGetLastError());
-        CKD(cudaDeviceSynchronize());  // ready for any stream
     }
     DeepGraph *w = g->deep;
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    // a source's share: states and order (20 bytes a vertex), level starts; up to one source a CTA, 16 GiB in all
+    // a source's share: states and order (20 bytes a vertex), level starts; up
+    // to one source a CTA, in what a workspace may keep, or half as many where
+    // there is no memory for them; launches of like size (148 sources of 2048 x
+    // 2048 vertices: 128 ms in one launch of 12.4 GB, 194 as 102 and 46, 151 as
+    // 74 and 74)
     auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
     const size_t per = 20 * (size_t)n + (kMaxLevel + 3) * sizeof(uint32_t);
-    const uint64_t slots = std::max<uint64_t>(1, std::min<uint64_t>({nroots, (uint64_t)nsm, (16ull << 30) / per}));
+    uint64_t slots = std::max<uint64_t>(1, std::min<uint64_t>({nroots, (uint64_t)nsm, kWorkKeep / per}));
     size_t o = up(sizeof(DeepCtrl));
     const size_t o_rstat = o; o += up(nroots * sizeof(RootStat));
     const size_t o_mult = o; o += up(nroots * sizeof(double));
     const size_t o_roots = o; o += up(nroots * sizeof(uint32_t));
-    const size_t o_state = o; o += up(slots * n * sizeof(DeepState));
-    const size_t o_order = o; o += up(slots * n * sizeof(uint32_t));
-    const size_t o_lbeg = o; o += up(slots * (kMaxLevel + 3) * sizeof(uint32_t));
-    if (w->cap < o) {
-        CKD(cudaDeviceSynchronize());  // earlier runs (any stream) are done with the old buffer
-        dev_free(w->mem);
-        w->mem = nullptr;
-        w->cap = 0;
-        const cudaError_t e = dev_alloc(&w->mem, o);
-        if (e == cudaErrorMemoryAllocation) {
-            cudaGetLastError();
-            return BCG_OK;
-        }
-        CKD(e);
-        CKD(cudaDeviceSynchronize());
-        w->cap = o;
+    const size_t o_state = o;
+    Workspace ws;
+    size_t o_order = 0, o_lbeg = 0;
+    for (;; slots /= 2) {
+        const uint64_t launches = (nroots + slots - 1) / slots;
+        slots = (nroots + launches - 1) / launches;
+        o_order = o_state + up(slots * n * sizeof(DeepState));
+        o_lbeg = o_order + up(slots * n * sizeof(uint32_t));
+        const cudaError_t e = ws.take(o_lbeg + up(slots * (kMaxLevel + 3) * sizeof(uint32_t)), st);
+        if (e == cudaSuccess) break;
+        if (e != cudaErrorMemoryAllocation) CKD(e);
+        cudaGetLastError();
+        if (slots == 1) return BCG_OK;
     }
+    unsigned char *const mem = ws.mem;
     DeepArgs a{};
     a.n = n;
-    a.ell = w->ell;
+    a.ell = reinterpret_cast<const uint32_t *>(w->ell.mem);
     a.vinfo = g->trees ? g->d_vinfo : nullptr;
-    a.state = reinterpret_cast<DeepState *>(w->mem + o_state);
-    a.order = reinterpret_cast<uint32_t *>(w->mem + o_order);
-    a.lbeg = reinterpret_cast<uint32_t *>(w->mem + o_lbeg);
-    a.ctrl = reinterpret_cast<DeepCtrl *>(w->mem);
+    a.state = reinterpret_cast<DeepState *>(mem + o_state);
+    a.order = reinterpret_cast<uint32_t *>(mem + o_order);
+    a.lbeg = reinterpret_cast<uint32_t *>(mem + o_lbeg);
+    a.ctrl = reinterpret_cast<DeepCtrl *>(mem);
     std::vector<unsigned char> up_(o_state - o_mult), down(o_mult);
     memcpy(up_.data(), mult, nroots * sizeof(double));
     memcpy(up_.data() + (o_roots - o_mult), roots, nroots * sizeof(uint32_t));
     const bool several = slots < nroots;
     CKD(cudaEventRecord(g->ev0, st));
-    CKD(cudaMemsetAsync(w->mem, 0, o_mult, st));  // control words and the sources' totals
-    CKD(cudaMemcpyAsync(w->mem + o_mult, up_.data(), up_.size(), cudaMemcpyHostToDevice, st));
+    CKD(cudaMemsetAsync(mem, 0, o_mult, st));  // control words and the sources' totals
+    CKD(cudaMemcpyAsync(mem + o_mult, up_.data(), up_.size(), cudaMemcpyHostToDevice, st));
     if (several) {  // launches add to bc one after the other: what it was before them
-        if (!g->d_bc_save) CKD(dev_alloc(&g->d_bc_save, (size_t)g->n * sizeof(double)));
+        if (!g->d_bc_save) CKD(tmp_alloc(&g->d_bc_save, (size_t)g->n * sizeof(double), st));
         CKD(cudaMemcpyAsync(g->d_bc_save, g->d_bc, (size_t)g->n * sizeof(double), cudaMemcpyDeviceToDevice, st));
     }
     const DeepCtrl *c = reinterpret_cast<const DeepCtrl *>(down.data());
     for (uint64_t s0 = 0; s0 < nroots; s0 += slots) {
         a.nroots = (uint32_t)std::min<uint64_t>(slots, nroots - s0);
-        a.roots = reinterpret_cast<const uint32_t *>(w->mem + o_roots) + s0;
-        a.rstat = reinterpret_cast<RootStat *>(w->mem + o_rstat) + s0;
+        a.roots = reinterpret_cast<const uint32_t *>(mem + o_roots) + s0;
+        a.rstat = reinterpret_cast<RootStat *>(mem + o_rstat) + s0;
         k_deep_init<<<nsm * 8, 256, 0, st>>>((uint64_t)a.nroots * n, a.state);
         CKD(D == 4 ? (ext ? launch_deep<4, true>(a, most_ctas, nsm, st) : launch_deep<4, false>(a, most_ctas, nsm, st))
                    : (ext ? launch_deep<8, true>(a, most_ctas, nsm, st) : launch_deep<8, false>(a, most_ctas, nsm, st)));
         k_deep_reduce<<<(n + 255) / 256, 256, 0, st>>>(a.ctrl, n, a.nroots,
-                                                       reinterpret_cast<const double *>(w->mem + o_mult) + s0, a.state,
+                                                       reinterpret_cast<const double *>(mem + o_mult) + s0, a.state,
                                                        g->d_ext, g->d_bc);
         CKD(cudaGetLastError());
         res->launches += 3;
         const bool last = s0 + a.nroots >= nroots;
         if (last) CKD(cudaEventRecord(g->ev1, st));
-        CKD(cudaMemcpyAsync(down.data(), w->mem, last ? o_mult : sizeof(DeepCtrl), cudaMemcpyDeviceToHost, st));
+        CKD(cudaMemcpyAsync(down.data(), mem, last ? o_mult : sizeof(DeepCtrl), cudaMemcpyDeviceToHost, st));
         CKD(cudaStreamSynchronize(st));
+        ws.waited = last || c->overflow || c->deep || c->full;
         if (c->overflow || c->deep || c->full) break;
     }
     if (c->overflow || c->deep || c->full) {
         if (several)
             CKD(cudaMemcpyAsync(g->d_bc, g->d_bc_save, (size_t)g->n * sizeof(double), cudaMemcpyDeviceToDevice, st));
         // frontiers that do not fit the clusters' queues: one CTA a source
-        if (c->full) return deep_launch(g, roots, mult, nroots, ext, 1, st, res);
+        if (c->full) {
+            ws.leave();
+            return deep_launch(g, roots, mult, nroots, ext, 1, st, res);
+        }
         res->overflow = c->overflow != 0;
         return BCG_OK;
     }

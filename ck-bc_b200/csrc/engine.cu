@@ -134,16 +134,55 @@ std::vector<cudaMemPool_t> g_pools;  // per device, created on first use
 
 // What the pool keeps: 4 GiB more than is in use (its threshold counts used
 // memory too, so with larger graphs alive a fixed one would unmap every freed
-// buffer at the next synchronisation).  Unmapping and mapping again costs tens
-// of milliseconds a GiB; the buffers of a run on a graph of 4M vertices and
-// 130M entries are 2.3 GiB beside the graph's 0.7, so that with 1 GiB kept the
-// first run on the next such graph took 71 ms, and with 4 GiB 12.
+// buffer at the next synchronisation), left workspaces counted among the 4.
+// Unmapping and mapping again takes about 7 ms a GiB each, and now and then 300
+// to 900 ms where the machine is shared; the buffers of a run on a graph of 4M
+// vertices and 130M entries are 2.3 GiB beside the graph's 0.7, so that with 1
+// GiB kept the first run on the next such graph took 71 ms, and with 4 GiB 12.
 constexpr uint64_t kPoolKeep = 4ull << 30;
-static void pool_keep(cudaMemPool_t pool) {
+
+// Workspaces that runs have left, oldest first, and the graphs alive, by device
+// (g_pool_mu).  A large pool buffer that is freed and allocated again is mapped
+// again from the pool's pieces, 1 to 2 ms each for the 0.7 GB of a run and the
+// 0.14 GB of a form of the benchmark's graph, and on a shared machine up to 1.6
+// s (15 of 60 creations with a run): a buffer that stays as it is takes none
+// of that.
+struct LeftWork {
+    unsigned char *mem;
+    size_t cap;
+};
+struct DeviceWork {
+    std::vector<LeftWork> left;
+    uint64_t bytes = 0;
+    uint32_t graphs = 0;
+};
+static std::vector<DeviceWork> g_work;
+
+static DeviceWork &device_work(int dev) {
+    if (g_work.size() <= (size_t)dev) g_work.resize((size_t)dev + 1);
+    return g_work[dev];
+}
+
+// (g_pool_mu held)
+static void pool_keep(int dev) {
+    const cudaMemPool_t pool = g_pools[dev];
     uint64_t used = 0;
     if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) return;
-    uint64_t keep = used + kPoolKeep;
+    uint64_t keep = used + kPoolKeep - std::min(kPoolKeep, device_work(dev).bytes);
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+}
+
+// Gives left workspaces back, oldest first, until `keep` bytes are left
+// (g_pool_mu held; the device is current).
+static void drop_work(int dev, uint64_t keep) {
+    DeviceWork &w = device_work(dev);
+    size_t k = 0;
+    for (; w.bytes > keep; ++k) {
+        cudaFreeAsync(w.left[k].mem, 0);
+        w.bytes -= w.left[k].cap;
+    }
+    w.left.erase(w.left.begin(), w.left.begin() + (ptrdiff_t)k);
+    if (k) pool_keep(dev);
 }
 
 cudaError_t tmp_alloc(void **p, size_t bytes, cudaStream_t st) {
@@ -164,16 +203,74 @@ cudaError_t tmp_alloc(void **p, size_t bytes, cudaStream_t st) {
                 g_pools[dev] = nullptr;
                 return e;
             }
-            pool_keep(g_pools[dev]);
+            pool_keep(dev);
         }
         pool = g_pools[dev];
     }
-    const cudaError_t e2 = cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 16), pool, st);
-    if (e2 == cudaSuccess && bytes >= (16u << 20)) pool_keep(pool);
+    cudaError_t e2 = cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 16), pool, st);
+    if (e2 == cudaErrorMemoryAllocation) {  // once more without what is only kept
+        cudaGetLastError();
+        {
+            std::lock_guard<std::mutex> lk(g_pool_mu);
+            drop_work(dev, 0);
+        }
+        cudaDeviceSynchronize();
+        cudaMemPoolTrimTo(pool, 0);
+        e2 = cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 16), pool, st);
+    }
+    if (e2 == cudaSuccess && bytes >= (16u << 20)) {
+        std::lock_guard<std::mutex> lk(g_pool_mu);
+        pool_keep(dev);
+    }
     return e2;
 }
 
 cudaError_t tmp_free(void *p, cudaStream_t st) { return p ? cudaFreeAsync(p, st) : cudaSuccess; }
+
+cudaError_t Workspace::take(size_t bytes, cudaStream_t st, bool keep) {
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    waited = false;
+    {
+        // the smallest that does, unless it is far larger (another run may want it)
+        const size_t most = keep ? bytes + bytes / 8 + (2u << 20) : 8 * bytes + (64u << 20);
+        std::lock_guard<std::mutex> lk(g_pool_mu);
+        DeviceWork &w = device_work(device);
+        size_t best = w.left.size();
+        for (size_t k = 0; k < w.left.size(); ++k)
+            if (w.left[k].cap >= bytes && w.left[k].cap <= most &&
+                (best == w.left.size() || w.left[k].cap < w.left[best].cap))
+                best = k;
+        if (best < w.left.size()) {
+            mem = w.left[best].mem;
+            cap = w.left[best].cap;
+            w.bytes -= cap;
+            w.left.erase(w.left.begin() + (ptrdiff_t)best);
+            return cudaSuccess;
+        }
+    }
+    const size_t all = (bytes + (2u << 20) - 1) / (2u << 20) * (2u << 20);
+    const cudaError_t e2 = tmp_alloc(&mem, all, st);
+    if (e2 == cudaSuccess) cap = all;
+    return e2;
+}
+
+void Workspace::leave() {
+    if (!mem) return;
+    int cur = -1;
+    cudaGetDevice(&cur);
+    if (cur != device) cudaSetDevice(device);
+    if (!waited) cudaDeviceSynchronize();
+    {
+        std::lock_guard<std::mutex> lk(g_pool_mu);
+        DeviceWork &w = device_work(device);
+        w.left.push_back(LeftWork{mem, cap});
+        w.bytes += cap;
+        if (w.left.size() > 8 || w.bytes > kWorkKeep) drop_work(device, std::min(kWorkKeep, w.bytes - w.left.front().cap));
+    }
+    mem = nullptr;
+    if (cur >= 0 && cur != device) cudaSetDevice(cur);
+}
 
 // Copies a result to the caller's (pageable) memory.  A result buffer is
 // usually fresh, and the copy then waits for one page fault after another: 32
@@ -237,14 +334,15 @@ static void graph_free(bcg_graph *g) {
     dev_free(g->d_ext);
     wide_free(g);
     deep_free(g);
-    small_free(g);
     dev_free(g->d_rows); dev_free(g->d_ctrl);
     dev_free(g->d_roots); dev_free(g->d_pend); dev_free(g->d_mult); dev_free(g->d_rstat);
     if (g->ev0) cudaEventDestroy(g->ev0);
     if (g->ev1) cudaEventDestroy(g->ev1);
     {
         std::lock_guard<std::mutex> lk(g_pool_mu);
-        if (g_pools.size() > (size_t)g->device && g_pools[g->device]) pool_keep(g_pools[g->device]);
+        DeviceWork &w = device_work(g->device);
+        if (g->counted && --w.graphs == 0) drop_work(g->device, kPoolKeep);
+        if (g_pools.size() > (size_t)g->device && g_pools[g->device]) pool_keep(g->device);
     }
     if (cur >= 0 && cur != g->device) cudaSetDevice(cur);
     delete g;
@@ -646,7 +744,7 @@ static int run_plan(bcg_graph *g, const RunPlan &p, cudaStream_t st, bcg_stats *
     const bool autoext = g->sigma_mode == 0;
     bool ext = g->sigma_mode == 2;
     if (autoext) {
-        if (!g->d_bc_save) CK(dev_alloc(&g->d_bc_save, (size_t)g->n * sizeof(double)));
+        if (!g->d_bc_save) CK(tmp_alloc(&g->d_bc_save, (size_t)g->n * sizeof(double), st));
         CK(cudaMemcpyAsync(g->d_bc_save, g->d_bc, (size_t)g->n * sizeof(double), cudaMemcpyDeviceToDevice, st));
     }
     for (;;) {
@@ -819,6 +917,11 @@ static int graph_create_impl(const uint32_t *offsets, const uint32_t *adj, uint3
     if (flags & BCG_PRUNE_TREES) flags &= ~BCG_PRUNE_DEGREE1;
     bcg_graph *g = new bcg_graph();
     cudaGetDevice(&g->device);
+    {
+        std::lock_guard<std::mutex> lk(g_pool_mu);
+        ++device_work(g->device).graphs;
+        g->counted = true;
+    }
     g->n = n;
     g->nnz = nnz;
     g->flags = flags;

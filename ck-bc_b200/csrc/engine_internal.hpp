@@ -6,6 +6,7 @@
 
 #include "bcg.h"
 #include "engine.cuh"
+#include "workspace.hpp"
 
 using bcg::Ctrl;
 using bcg::kNoRoot;
@@ -18,7 +19,6 @@ using bcg::kTileVerts;
 namespace bcg {
 struct WideGraph;  // wide.cu
 struct DeepGraph;  // deep.cu
-struct SmallGraph;  // small.cu
 
 // Pendant trees of a graph on the device (BCG_PRUNE_TREES, and one peeling
 // round for BCG_PRUNE_DEGREE1; trees_gpu.cu), caller's numbering.
@@ -91,8 +91,8 @@ struct bcg_graph {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     bcg::WideGraph *wide = nullptr;  // the graph's form for wide-batch runs (wide.cu), built by the first one
     bcg::DeepGraph *deep = nullptr;  // the same for deep runs (deep.cu)
-    bcg::SmallGraph *small = nullptr;  // and for small ones (small.cu)
     uint32_t max_deg = 0;            // largest degree in the searched graph
+    bool counted = false;            // among the graphs alive (engine.cu)
 };
 
 namespace bcg {
@@ -115,6 +115,7 @@ cudaError_t dev_alloc(T **p, size_t bytes) {
     return tmp_alloc(reinterpret_cast<void **>(p), bytes, 0);
 }
 inline cudaError_t dev_free(void *p) { return tmp_free(p, 0); }
+
 
 // ext: sigma and X as extended-range numbers (ext64.cuh) instead of uint64 / double
 int launch_sweep(int S, const BatchArgs &a, cudaStream_t st, int *grid_out, bool ext = false);
@@ -163,7 +164,6 @@ struct SmallResult {
 bool small_takes(const bcg_graph *g, uint64_t nroots);
 int small_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, cudaStream_t st,
               SmallResult *res);
-void small_free(bcg_graph *g);
 
 // Component-packed batches already on the device (see BatchArgs::xbeg).
 struct PackedRun {

@@ -160,7 +160,7 @@ int make_room(bcg_server *s, bool *moved) {
         double *h = static_cast<double *>(malloc(r.bytes));
         if (!h) return BCG_OK;
         cudaError_t e = cudaMemcpyAsync(h, r.d_out, r.bytes, cudaMemcpyDeviceToHost, s->result_stream);
-        if (e == cudaSuccess) e = cudaFreeAsync(r.d_out, s->result_stream);
+        if (e == cudaSuccess) e = tmp_free(r.d_out, s->result_stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->result_stream);
         if (e != cudaSuccess) {
             free(h);
@@ -188,7 +188,7 @@ int admit(bcg_server *s) {
             if (!moved) break;
             continue;
         }
-        CKS(cudaMallocAsync(reinterpret_cast<void **>(&r.d_out), r.bytes, s->stream));
+        CKS(tmp_alloc(&r.d_out, r.bytes, s->stream));
         CKS(cudaMemsetAsync(r.d_out, 0, r.bytes, s->stream));
         s->admitted += r.bytes;
         s->queue[r.graph].push_back(s->pending.front());
@@ -205,7 +205,7 @@ int packed_setup(bcg_server *s) {
     if (rc) return rc;
     cudaError_t e = cudaSuccess;
     auto take = [&](auto **p, size_t bytes) {
-        if (e == cudaSuccess && !*p && (e = cudaMalloc(p, bytes)) != cudaSuccess) *p = nullptr;
+        if (e == cudaSuccess && !*p && (e = tmp_alloc(p, bytes, s->stream)) != cudaSuccess) *p = nullptr;
     };
     take(&s->d_slot_delta, (size_t)s->width * s->g->n * sizeof(double));
     for (ServeWave &w : s->slot) {
@@ -286,7 +286,7 @@ int wide_setup(bcg_server *s) {
     cudaError_t e = cudaSuccess;
     if (!rc && ((e = dev_alloc(&s->d_wstate, s->wstate_bytes)) != cudaSuccess ||
                 (e = dev_alloc(&s->d_jobbc, s->cells * 8)) != cudaSuccess ||
-                (!s->d_poison && (e = cudaMalloc(&s->d_poison, sizeof(int))) != cudaSuccess) ||
+                (!s->d_poison && (e = dev_alloc(&s->d_poison, sizeof(int))) != cudaSuccess) ||
                 (e = cudaMemset(s->d_poison, 0, sizeof(int))) != cudaSuccess))
         rc = set_error(e == cudaErrorMemoryAllocation ? BCG_ERR_OOM : BCG_ERR_CUDA, "wide waves: %s", cudaGetErrorString(e));
     for (ServeWave &w : s->slot)
@@ -734,21 +734,21 @@ int bcg_server_destroy(bcg_server *s) {
         if (s->stream) cudaStreamSynchronize(s->stream);
         if (s->result_stream) cudaStreamSynchronize(s->result_stream);
         for (auto &kv : s->reqs) {
-            if (kv.second.d_out) cudaFree(kv.second.d_out);
+            dev_free(kv.second.d_out);
             free(kv.second.h_out);
         }
         wide_clear(s);
-        if (s->d_poison) cudaFree(s->d_poison);
+        dev_free(s->d_poison);
         for (ServeWave &w : s->slot) {
-            cudaFree(w.d_blob);
-            cudaFree(w.d_rstat);
+            dev_free(w.d_blob);
+            dev_free(w.d_rstat);
             if (w.h_blob) cudaFreeHost(w.h_blob);
             if (w.h_flags) cudaFreeHost(w.h_flags);
             if (w.ev) cudaEventDestroy(w.ev);
         }
         if (s->stream) cudaStreamDestroy(s->stream);
         if (s->result_stream) cudaStreamDestroy(s->result_stream);
-        cudaFree(s->d_slot_delta);
+        dev_free(s->d_slot_delta);
         if (s->g) bcg_graph_destroy(s->g);
     }
     delete s;
@@ -825,7 +825,7 @@ int bcg_server_result(bcg_server *s, uint64_t id, double *bc_host) {
     // the last wave that wrote the buffer has completed: copy on the result
     // stream, so later waves queued on the server's stream keep running
     CKS(cudaMemcpyAsync(bc_host, r.d_out, r.bytes, cudaMemcpyDeviceToHost, s->result_stream));
-    CKS(cudaFreeAsync(r.d_out, s->result_stream));
+    CKS(tmp_free(r.d_out, s->result_stream));
     CKS(cudaStreamSynchronize(s->result_stream));
     s->admitted -= r.bytes;
     s->reqs.erase(it);

@@ -288,19 +288,6 @@ __global__ void __launch_bounds__(256) k_small_reduce(const SmallCtrl *__restric
 
 }  // namespace
 
-// What a graph keeps for its small runs (bcg_graph::small).
-struct SmallGraph {
-    unsigned char *mem = nullptr;
-    size_t cap = 0;
-};
-
-void small_free(bcg_graph *g) {
-    if (!g->small) return;
-    dev_free(g->small->mem);
-    delete g->small;
-    g->small = nullptr;
-}
-
 // Everything of a source must fit a CTA's shared memory, and two rounds of the
 // SMs must do: one source or 148 take the same time, 296 twice that, while the
 // wide searches' time hardly grows.  (Whole call, these against the wide
@@ -331,35 +318,27 @@ int small_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t 
     const size_t o_rstat = sizeof(SmallCtrl), o_mult = o_rstat + nroots * sizeof(RootStat),
                  o_roots = o_mult + nroots * sizeof(double), blob = o_roots + nroots * sizeof(uint32_t), o_out = up(blob),
                  need = o_out + (nroots > 1 ? nroots * a.n * sizeof(double) : 0);
-    if (!g->small) g->small = new SmallGraph();
-    SmallGraph *w = g->small;
-    if (w->cap < need) {
-        if (w->mem) CKM(cudaDeviceSynchronize());  // earlier runs (any stream) are done with it
-        dev_free(w->mem);
-        w->mem = nullptr;
-        w->cap = 0;
-        const cudaError_t e = dev_alloc(&w->mem, need);
-        if (e == cudaErrorMemoryAllocation) {
-            cudaGetLastError();
-            return BCG_OK;
-        }
-        CKM(e);
-        w->cap = need;
-        if (st != 0) CKM(cudaStreamSynchronize(0));  // ready for st
+    Workspace ws;
+    const cudaError_t took = ws.take(need, st);
+    if (took == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return BCG_OK;
     }
+    CKM(took);
+    unsigned char *const mem = ws.mem;
     std::vector<unsigned char> h(blob);
     memcpy(h.data() + o_mult, mult, nroots * sizeof(double));
     memcpy(h.data() + o_roots, roots, nroots * sizeof(uint32_t));
-    CKM(cudaMemcpyAsync(w->mem, h.data(), blob, cudaMemcpyHostToDevice, st));
+    CKM(cudaMemcpyAsync(mem, h.data(), blob, cudaMemcpyHostToDevice, st));
     a.offs = g->d_offs;
     a.adj = g->d_adj;
     a.vinfo = g->trees ? g->d_vinfo : nullptr;
     a.ext = g->d_ext;
-    a.ctrl = reinterpret_cast<SmallCtrl *>(w->mem);
-    a.rstat = reinterpret_cast<RootStat *>(w->mem + o_rstat);
-    a.mult = reinterpret_cast<const double *>(w->mem + o_mult);
-    a.roots = reinterpret_cast<const uint32_t *>(w->mem + o_roots);
-    a.out = nroots > 1 ? reinterpret_cast<double *>(w->mem + o_out) : nullptr;
+    a.ctrl = reinterpret_cast<SmallCtrl *>(mem);
+    a.rstat = reinterpret_cast<RootStat *>(mem + o_rstat);
+    a.mult = reinterpret_cast<const double *>(mem + o_mult);
+    a.roots = reinterpret_cast<const uint32_t *>(mem + o_roots);
+    a.out = nroots > 1 ? reinterpret_cast<double *>(mem + o_out) : nullptr;
     a.bc = g->d_bc;
     const void *f = (const void *)bc_small_kernel;
     // (the limit belongs to the kernel, not to the launch: the same for every
@@ -374,8 +353,9 @@ int small_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t 
         CKM(cudaGetLastError());
     }
     CKM(cudaEventRecord(g->ev1, st));
-    CKM(cudaMemcpyAsync(h.data(), w->mem, o_mult, cudaMemcpyDeviceToHost, st));
+    CKM(cudaMemcpyAsync(h.data(), mem, o_mult, cudaMemcpyDeviceToHost, st));
     CKM(cudaStreamSynchronize(st));
+    ws.waited = true;
     if (reinterpret_cast<const SmallCtrl *>(h.data())->overflow) return BCG_OK;  // the caller's other kernels extend the counts
     res->rstat.resize(nroots);
     memcpy(res->rstat.data(), h.data() + o_rstat, nroots * sizeof(RootStat));

@@ -1426,19 +1426,15 @@ int wide_chain(const WideArgs &a, const WideOut *outs, uint32_t nouts, uint32_t 
     return BCG_OK;
 }
 
-// What a graph keeps for its wide runs (bcg_graph::wide): its wide form, and
-// one buffer for its runs.
+// What a graph keeps for its wide runs (bcg_graph::wide).
 struct WideGraph {
     WideForm form;
-    unsigned char *mem = nullptr;
-    size_t cap = 0;
 };
 
 void wide_free(bcg_graph *g) {
     WideGraph *w = g->wide;
     if (!w) return;
     wide_form_free(w->form);
-    dev_free(w->mem);
     delete w;
     g->wide = nullptr;
 }
@@ -1492,33 +1488,27 @@ int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t n
                  o_blob = up256(stat), o_roots = up256(nroots * 8), blob = o_roots + up256(nroots * 4),
                  o_sorted = o_blob + up256(blob), o_jobbc = o_sorted + (sorted ? blob + up256(nroots * 4) : 0),
                  o_state = o_jobbc + up256(jl * n * 8), need = o_state + a.stride * a.teams;
-    if (w->cap < need) {
-        if (w->mem) CKW(cudaDeviceSynchronize());  // earlier runs (any stream) are done with it
-        dev_free(w->mem);
-        w->mem = nullptr;
-        w->cap = 0;
-        const cudaError_t e = dev_alloc(&w->mem, need);
-        if (e == cudaErrorMemoryAllocation) {
-            cudaGetLastError();
-            return BCG_OK;
-        }
-        CKW(e);
-        w->cap = need;
-        fresh = true;
+    Workspace ws;
+    const cudaError_t took = ws.take(need, st);
+    if (took == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return BCG_OK;
     }
-    if (fresh && st != 0) CKW(cudaStreamSynchronize(0));  // what stream 0 made is ready for st
+    CKW(took);
+    unsigned char *const mem = ws.mem;
+    if (fresh && st != 0) CKW(cudaStreamSynchronize(0));  // the form that stream 0 made is ready for st
     std::vector<unsigned char> h(blob), hs(stat);
     memcpy(h.data(), mult, nroots * 8);
     memcpy(h.data() + o_roots, roots, nroots * 4);
-    CKW(cudaMemcpyAsync(w->mem + o_blob, h.data(), blob, cudaMemcpyHostToDevice, st));
+    CKW(cudaMemcpyAsync(mem + o_blob, h.data(), blob, cudaMemcpyHostToDevice, st));
     a.subs = w->form.d_subs;
     a.nroots = (uint32_t)nroots;
-    a.mult = reinterpret_cast<const double *>(w->mem + o_blob);
-    a.roots = reinterpret_cast<const uint32_t *>(w->mem + o_blob + o_roots);
-    a.jobbc = reinterpret_cast<double *>(w->mem + o_jobbc);
-    a.state = w->mem + o_state;
-    a.ctrl = reinterpret_cast<WideCtrl *>(w->mem);
-    a.team = reinterpret_cast<WideTeam *>(w->mem + o_team);
+    a.mult = reinterpret_cast<const double *>(mem + o_blob);
+    a.roots = reinterpret_cast<const uint32_t *>(mem + o_blob + o_roots);
+    a.jobbc = reinterpret_cast<double *>(mem + o_jobbc);
+    a.state = mem + o_state;
+    a.ctrl = reinterpret_cast<WideCtrl *>(mem);
+    a.team = reinterpret_cast<WideTeam *>(mem + o_team);
     TraceRec *d_trace = nullptr;
     unsigned int *d_tcnt = nullptr;
     const char *trace_path = getenv("BCG_TRACE_FILE");
@@ -1531,20 +1521,20 @@ int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t n
         a.trace = d_trace;
         a.trace_cnt = d_tcnt;
     }
-    CKW(cudaMemsetAsync(w->mem, 0, stat, st));
+    CKW(cudaMemsetAsync(mem, 0, stat, st));
     CKW(cudaEventRecord(g->ev0, st));
     // The jobs are added into bc on the device only if none of them stopped.
     // Several launches add one after the other, so bc is saved before them.
     const bool several = jl < njobs;
     if (several) {
-        if (!g->d_bc_save) CKW(dev_alloc(&g->d_bc_save, (size_t)g->n * sizeof(double)));
+        if (!g->d_bc_save) CKW(tmp_alloc(&g->d_bc_save, (size_t)g->n * sizeof(double), st));
         CKW(cudaMemcpyAsync(g->d_bc_save, g->d_bc, (size_t)g->n * sizeof(double), cudaMemcpyDeviceToDevice, st));
     }
     if (sorted) {
-        unsigned char *to = w->mem + o_sorted;
+        unsigned char *to = mem + o_sorted;
         if ((rc = wide_order(a.subs, a.roots, a.mult, (uint32_t)nroots, reinterpret_cast<uint32_t *>(to + blob),
                              reinterpret_cast<uint32_t *>(to + o_roots), reinterpret_cast<double *>(to),
-                             reinterpret_cast<uint32_t *>(w->mem + o_order), st)))
+                             reinterpret_cast<uint32_t *>(mem + o_order), st)))
             return rc;
         a.roots = reinterpret_cast<const uint32_t *>(to + o_roots);
         a.mult = reinterpret_cast<const double *>(to);
@@ -1554,15 +1544,16 @@ int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t n
     for (uint64_t j0 = 0; j0 < njobs; j0 += jl) {
         a.njobs = (uint32_t)std::min(jl, njobs - j0);
         a.job0 = (uint32_t)j0;
-        a.rstat = reinterpret_cast<RootStat *>(w->mem + o_rstat) + j0 * slots;
-        if (j0) CKW(cudaMemsetAsync(w->mem, 0, o_rstat, st));
+        a.rstat = reinterpret_cast<RootStat *>(mem + o_rstat) + j0 * slots;
+        if (j0) CKW(cudaMemsetAsync(mem, 0, o_rstat, st));
         if ((rc = wide_enqueue(a, nullptr, 1, WideOut{0, a.njobs, (uint32_t)n, w->form.map, g->d_bc, w->form.d_subs}, (uint32_t)n, st)))
             return rc;
         res->launches += 2;
         const bool last = j0 + a.njobs >= njobs;
         if (last) CKW(cudaEventRecord(g->ev1, st));
-        CKW(cudaMemcpyAsync(hs.data(), w->mem, last ? stat : sizeof(WideCtrl), cudaMemcpyDeviceToHost, st));
+        CKW(cudaMemcpyAsync(hs.data(), mem, last ? stat : sizeof(WideCtrl), cudaMemcpyDeviceToHost, st));
         CKW(cudaStreamSynchronize(st));
+        ws.waited = last || c->error || c->overflow || c->deep;
         if (c->error || c->overflow || c->deep) break;
     }
     if (d_trace) {

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "engine.cuh"
+#include "workspace.hpp"
 
 struct bcg_graph;
 
@@ -127,7 +128,7 @@ WideInput wide_input(const bcg_graph *g);  // of a graph's searched lists
 
 // A graph's (or union's) lists in the wide numbering.
 struct WideForm {
-    unsigned char *mem = nullptr;  // everything below on the device (nullptr: the caller's memory)
+    Workspace mem;                 // everything below on the device (empty: the caller's memory)
     WideSub *d_subs = nullptr;     // one a graph
     uint32_t *inv = nullptr, *map = nullptr;
     std::vector<WideSub> subs;     // the host's copy (wide_form_make)

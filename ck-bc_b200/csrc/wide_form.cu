@@ -352,30 +352,29 @@ int wide_form_make(WideForm &f, const WideInput &in, bool bounds) {
     // One small graph whose bounds do: everything in one block, and the first
     // run does not wait for the building.
     const bool small = bounds && in.graphs == 1 && !in.directed && in.n <= (1u << 16);
-    CKF(dev_alloc(&f.mem, small ? bytes + scratch_bytes : bytes));
+    CKF(f.mem.take(small ? bytes + scratch_bytes : bytes, 0, true));
     if (small) {
         WideSub &s = f.subs[0];
         s = WideSub{};
         s.n = in.n;
         s.nheavy = (uint32_t)(in.nnz / kWideChunk + 1);
         s.nchunk[0] = s.nchunk[1] = (uint32_t)(2 * (in.nnz / kWideChunk) + 1);
-        return wide_form_enqueue(f, in, f.mem, f.mem + bytes, 0);
+        return wide_form_enqueue(f, in, f.mem.mem, f.mem.mem + bytes, 0);
     }
-    unsigned char *scratch = nullptr;
-    const cudaError_t e = dev_alloc(&scratch, scratch_bytes);
-    int rc = BCG_OK;
-    if (e != cudaSuccess)
-        rc = set_error(e == cudaErrorMemoryAllocation ? BCG_ERR_OOM : BCG_ERR_CUDA, "wide form: %s", cudaGetErrorString(e));
-    if (!rc) rc = wide_form_enqueue(f, in, f.mem, scratch, 0);
+    Workspace scratch;
+    CKF(scratch.take(scratch_bytes, 0));
+    int rc = wide_form_enqueue(f, in, f.mem.mem, scratch.mem, 0);
     if (!rc && cudaMemcpy(f.subs.data(), f.d_subs, in.graphs * sizeof(WideSub), cudaMemcpyDeviceToHost) != cudaSuccess)
         rc = set_error(BCG_ERR_CUDA, "reading the wide form: %s", cudaGetErrorString(cudaGetLastError()));
-    dev_free(scratch);  // ordered on stream 0, behind the building
+    scratch.waited = rc == BCG_OK;
     return rc;
 }
 
 void wide_form_free(WideForm &f) {
-    dev_free(f.mem);
-    f = WideForm{};
+    f.mem.leave();
+    f.d_subs = nullptr;
+    f.inv = f.map = nullptr;
+    f.subs.clear();
 }
 
 }  // namespace bcg

@@ -154,7 +154,10 @@ int bcg_graph_create_device(const uint32_t *d_offsets, const uint32_t *d_adj,
 /* Frees every device buffer of the graph (fincuda cuda_kernels.cu:1201-1232)
  * after the device has finished all queued work.  Graph buffers come from a
  * stream-ordered memory pool of the library (one per device) that keeps up
- * to 4 GiB reserved once freed, so the next creation reuses the memory. */
+ * to 4 GiB reserved once freed, so the next creation reuses the memory.  The
+ * buffers that runs work in are left there for later runs on any graph, up to
+ * 8 GiB a device while graphs are alive; a library allocation that would fail
+ * gets what is only kept. */
 int bcg_graph_destroy(bcg_graph *g);
 
 /* Sets every bc value of the graph to 0. */

@@ -456,6 +456,76 @@ __global__ void k_deep_rows(uint32_t n, const uint32_t *__restrict__ offs, const
     for (int q = 0; q < D; ++q) ell[(size_t)v * D + q] = (uint32_t)q < deg ? adj[e0 + q] : kNone;
 }
 
+// ---------------------------------------------------------------------------
+// Whether a search's frontier grows faster than a mesh's.  kProbes CTAs search
+// from vertices spread over the graph until a level of more than 16 + 8 d^2
+// vertices is met (a lattice in three dimensions has up to 6 d^2 + 2), or the
+// growth is a plane's at level 16 (8 d at most), or kProbeDepth levels or
+// kProbeVerts vertices hold neither.  About 2 us a level, once a graph.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kProbes = 8, kProbeDepth = 40, kProbeVerts = 32768, kProbeScan = 65536;
+constexpr int kProbeThreads = 512;
+
+// seen: kProbes bitmaps of `words` words (zeroed); queue: kProbes x (kProbeVerts
+// + 8 x kProbeThreads); vote: {probes that started, probes that met a level so
+// wide} (zeroed).
+template <int D>
+__global__ void __launch_bounds__(kProbeThreads) k_deep_probe(uint32_t n, const uint32_t *__restrict__ ell, uint32_t words,
+                                                              uint32_t *__restrict__ seen, uint32_t *__restrict__ queue,
+                                                              uint32_t *__restrict__ vote) {
+    __shared__ uint32_t start, end;
+    const uint32_t b = blockIdx.x, tid = threadIdx.x;
+    uint32_t *bits = seen + (size_t)b * words, *q = queue + (size_t)b * (kProbeVerts + 8 * kProbeThreads);
+    if (tid == 0) {
+        start = kNone;
+        end = 1;
+    }
+    __syncthreads();
+    // the first vertex with a neighbour in the probe's part
+    const uint32_t v0 = (uint32_t)((unsigned long long)n * b / kProbes), v1 = (uint32_t)((unsigned long long)n * (b + 1) / kProbes);
+    for (uint32_t v = v0; v < v1 && v - v0 < kProbeScan; v += kProbeThreads) {
+        if (v + tid < v1 && ell[(size_t)(v + tid) * D] != kNone) atomicMin(&start, v + tid);
+        __syncthreads();
+        const bool found = start != kNone;
+        __syncthreads();
+        if (found) break;
+    }
+    if (start == kNone) return;
+    if (tid == 0) {
+        q[0] = start;
+        bits[start >> 5] = 1u << (start & 31u);
+        atomicAdd(vote, 1u);
+    }
+    __syncthreads();
+    uint32_t d = 0, from = 0, to = 1;  // level d is q[from .. to)
+    while (d < kProbeDepth && to < kProbeVerts) {
+        for (uint32_t i = from + tid; i < to; i += kProbeThreads) {
+            const Row<D> r = ell_row<D>(ell, q[i]);
+#pragma unroll
+            for (int k = 0; k < D; ++k) {
+                const uint32_t u = r.u[k];
+                if (u == kNone) continue;
+                const uint32_t bit = 1u << (u & 31u);
+                if (atomicOr(bits + (u >> 5), bit) & bit) continue;
+                const uint32_t at = atomicAdd(&end, 1u);
+                if (at < kProbeVerts + 8 * kProbeThreads) q[at] = u;
+            }
+        }
+        __syncthreads();
+        const uint32_t last = min(end, kProbeVerts + 8 * kProbeThreads);
+        __syncthreads();
+        from = to;
+        to = last;
+        ++d;
+        const uint32_t size = to - from;
+        if (size > 16u + 8u * d * d) {
+            if (tid == 0) atomicAdd(vote + 1, 1u);
+            return;
+        }
+        if (!size || (d == 16 && size <= 8u * d)) return;
+    }
+}
+
 #define CKD(call)                                                                                  \
     do {                                                                                           \
         cudaError_t e_ = (call);                                                                   \
@@ -464,27 +534,24 @@ __global__ void k_deep_rows(uint32_t n, const uint32_t *__restrict__ offs, const
                              #call, cudaGetErrorString(e_));                                       \
     } while (0)
 
-// Launches a.nroots sources in clusters of up to `most` CTAs: as many a source
-// as leave every source room on the chip.  Clusters of more than 8 are not
-// promised by the architecture, and fewer of them fit than the SMs would
-// allow: the device is asked.
+// The launch of a.nroots sources in clusters of up to `most` CTAs (a.cluster):
+// as many a source as leave every source room on the chip.  Clusters of more
+// than 8 are not promised by the architecture, and fewer of them fit than the
+// SMs would allow: the device is asked.
 template <int D, bool EXT>
-cudaError_t launch_deep(DeepArgs &a, uint32_t most, uint32_t nsm, cudaStream_t st) {
+cudaError_t deep_config(DeepArgs &a, uint32_t most, uint32_t nsm, cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at) {
     const void *f = (const void *)bc_deep_kernel<D, EXT>;
     cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeepSmem<D>));
     if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     a.cluster = 1;
     while (a.cluster < most && a.nroots * 2 * a.cluster <= nsm) a.cluster *= 2;
-    cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(a.nroots * a.cluster);
     // (threads, measured on 2048 x 2048 vertices: clusters of 16 25.1 ms with
     // 256 and 26.5 with 512, of 8 30.1 and 29.8, of 4 45.8 and 42.0; 148
     // sources of 1000 x 1000, a CTA each: 34.7 and 32.7)
     cfg.blockDim = dim3(a.cluster >= 8 ? kDeepThreads / 2 : kDeepThreads);
     cfg.dynamicSmemBytes = sizeof(DeepSmem<D>);
-    cfg.stream = st;
-    cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeClusterDimension;
     at.val.clusterDim.x = a.cluster;
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
@@ -499,9 +566,19 @@ cudaError_t launch_deep(DeepArgs &a, uint32_t most, uint32_t nsm, cudaStream_t s
             cfg.gridDim = dim3(a.nroots * 8u);
         }
     }
+    return cudaSuccess;
+}
+
+template <int D, bool EXT>
+cudaError_t launch_deep(DeepArgs &a, uint32_t most, uint32_t nsm, cudaStream_t st) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    const cudaError_t e = deep_config<D, EXT>(a, most, nsm, cfg, at);
+    if (e != cudaSuccess) return e;
+    cfg.stream = st;
     DeepArgs args = a;
     void *params[] = {&args};
-    return cudaLaunchKernelExC(&cfg, f, params);
+    return cudaLaunchKernelExC(&cfg, (const void *)bc_deep_kernel<D, EXT>, params);
 }
 
 }  // namespace
@@ -509,7 +586,8 @@ cudaError_t launch_deep(DeepArgs &a, uint32_t most, uint32_t nsm, cudaStream_t s
 // What a graph keeps for its deep runs (bcg_graph::deep).
 struct DeepGraph {
     Workspace ell;
-    int width = 0;         // neighbours of a row
+    int width = 0;       // neighbours of a row
+    bool broad = false;  // frontiers grow faster than a mesh's (k_deep_probe)
 };
 
 void deep_free(bcg_graph *g) {
@@ -520,40 +598,66 @@ void deep_free(bcg_graph *g) {
 
 bool deep_takes(const bcg_graph *g) { return !(g->flags & BCG_DIRECTED) && g->max_deg >= 1 && g->max_deg <= 8; }
 
+// Makes g->deep, unless it is there; stays nullptr where there is no memory.
+static int deep_make(bcg_graph *g) {
+    if (g->deep) return BCG_OK;
+    const uint32_t n = g->tile_n ? g->tile_n : g->n, words = (n + 31u) / 32u;
+    const int D = g->max_deg <= 4 ? 4 : 8;
+    DeepGraph *w = g->deep = new DeepGraph();
+    w->width = D;
+    Workspace probe;
+    const size_t o_seen = 256, o_queue = o_seen + (size_t)kProbes * words * 4,
+                 probe_bytes = o_queue + (size_t)kProbes * (kProbeVerts + 8 * kProbeThreads) * 4;
+    uint32_t vote[2] = {0, 0};
+    cudaError_t e = w->ell.take((size_t)n * D * sizeof(uint32_t), 0, true);
+    if (e == cudaSuccess) e = probe.take(probe_bytes, 0);
+    if (e == cudaSuccess) e = cudaMemsetAsync(probe.mem, 0, o_queue, 0);
+    if (e == cudaSuccess) {
+        uint32_t *ell = reinterpret_cast<uint32_t *>(w->ell.mem), *at = reinterpret_cast<uint32_t *>(probe.mem);
+        uint32_t *seen = reinterpret_cast<uint32_t *>(probe.mem + o_seen), *queue = reinterpret_cast<uint32_t *>(probe.mem + o_queue);
+        if (D == 4) {
+            k_deep_rows<4><<<(n + 255) / 256, 256>>>(n, g->d_offs, g->d_adj, ell);
+            k_deep_probe<4><<<kProbes, kProbeThreads>>>(n, ell, words, seen, queue, at);
+        } else {
+            k_deep_rows<8><<<(n + 255) / 256, 256>>>(n, g->d_offs, g->d_adj, ell);
+            k_deep_probe<8><<<kProbes, kProbeThreads>>>(n, ell, words, seen, queue, at);
+        }
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaMemcpy(vote, at, sizeof(vote), cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess) e = cudaDeviceSynchronize();  // ready for any stream
+        probe.waited = e == cudaSuccess;
+    }
+    if (e != cudaSuccess) {
+        deep_free(g);
+        if (e != cudaErrorMemoryAllocation) CKD(e);
+        cudaGetLastError();
+    } else {
+        w->broad = vote[1] && 2 * vote[1] >= vote[0];
+    }
+    return BCG_OK;
+}
+
+// Most sources of a launch: one a CTA, in what a workspace may keep.
+static uint64_t deep_slots(uint32_t n, uint64_t nroots, uint32_t nsm) {
+    const size_t per = 20 * (size_t)n + (kMaxLevel + 3) * sizeof(uint32_t);
+    return std::max<uint64_t>(1, std::min<uint64_t>({nroots, (uint64_t)nsm, kWorkKeep / per}));
+}
+
 static int deep_launch(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, bool ext,
                        uint32_t most_ctas, cudaStream_t st, DeepResult *res) {
     *res = DeepResult{};
     const uint32_t n = g->tile_n ? g->tile_n : g->n;
     const int D = g->max_deg <= 4 ? 4 : 8;
-    if (!g->deep) {
-        DeepGraph *w = g->deep = new DeepGraph();
-        w->width = D;
-        cudaError_t e = w->ell.take((size_t)n * D * sizeof(uint32_t), 0, true);
-        if (e == cudaSuccess) {
-            uint32_t *ell = reinterpret_cast<uint32_t *>(w->ell.mem);
-            if (D == 4) k_deep_rows<4><<<(n + 255) / 256, 256>>>(n, g->d_offs, g->d_adj, ell);
-            else k_deep_rows<8><<<(n + 255) / 256, 256>>>(n, g->d_offs, g->d_adj, ell);
-            if ((e = cudaGetLastError()) == cudaSuccess) e = cudaDeviceSynchronize();  // ready for any stream
-        }
-        if (e != cudaSuccess) {
-            deep_free(g);
-            if (e != cudaErrorMemoryAllocation) CKD(e);
-            cudaGetLastError();
-            return BCG_OK;
-        }
-    }
     DeepGraph *w = g->deep;
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    // a source's share: states and order (20 bytes a vertex), level starts; up
-    // to one source a CTA, in what a workspace may keep, or half as many where
-    // there is no memory for them; launches of like size (148 sources of 2048 x
+    // a source's share: states and order (20 bytes a vertex), level starts; half
+    // as many sources where there is no memory; launches of like size (148 sources of 2048 x
     // 2048 vertices: 128 ms in one launch of 12.4 GB, 194 as 102 and 46, 151 as
     // 74 and 74)
     auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
-    const size_t per = 20 * (size_t)n + (kMaxLevel + 3) * sizeof(uint32_t);
-    uint64_t slots = std::max<uint64_t>(1, std::min<uint64_t>({nroots, (uint64_t)nsm, kWorkKeep / per}));
+    uint64_t slots = deep_slots(n, nroots, (uint32_t)nsm);
     size_t o = up(sizeof(DeepCtrl));
     const size_t o_rstat = o; o += up(nroots * sizeof(RootStat));
     const size_t o_mult = o; o += up(nroots * sizeof(double));
@@ -629,9 +733,52 @@ static int deep_launch(bcg_graph *g, const uint32_t *roots, const double *mult, 
     return BCG_OK;
 }
 
+// Where frontiers are broad the queues of a cluster run over, and one CTA a
+// source takes 33 ns a vertex (of three neighbours) where the sweep kernel
+// takes 0.3 to 0.5 ms and 1.3 ns a vertex for six sources at once.  The widest
+// level of a random 3-regular graph or a binary tree has a quarter of the
+// vertices, of a 4-regular one or a tree of 3 children a third, of a tree of 7
+// children 0.72: queues that hold that with room for uneven shares do (at 0.80
+// of them a tree's ran over, at 0.81 none of the others').  Random 3-regular graph, 1, 6, 24, 48 and 148
+// sources, clusters or one CTA a source against the sweep kernel: 2^16 vertices
+// 0.22, 0.23, 0.44, 1.3 and 2.2 ms against 0.36, 0.55, 1.9, 3.8 and 12; 2^18
+// vertices 0.48, 0.50, 7.0, 8.1 and 10 against 0.49, 0.89, 3.4, 6.6 and 21; 2^20
+// vertices 18, 29, 34, 36 and 45 against 0.9, 2.4, 9.2, 18 and 57.  Complete
+// binary tree of 2^20 vertices 11, 14, 16, 16 and 17 against 0.7, 1.4, 4.8, 9.5
+// and 27.  The rule takes the faster in all of these, or one within 8 % of it, as
+// it does on 4-regular graphs and trees of 3 and 7 children (2^14 to 2^21
+// vertices, 1 to 400 sources).
 int deep_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, bool ext, cudaStream_t st,
              DeepResult *res) {
-    return deep_launch(g, roots, mult, nroots, ext, kDeepCluster, st, res);
+    *res = DeepResult{};
+    const int rc = deep_make(g);
+    if (rc || !g->deep) return rc;
+    uint32_t most = kDeepCluster;
+    if (g->deep->broad) {
+        const uint32_t n = g->tile_n ? g->tile_n : g->n;
+        int dev = 0, nsm = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+        const uint64_t slots = deep_slots(n, nroots, (uint32_t)nsm), rounds = (nroots + slots - 1) / slots;
+        DeepArgs a{};
+        a.nroots = (uint32_t)((nroots + rounds - 1) / rounds);
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute at{};
+        if (g->max_deg <= 4) CKD((deep_config<4, false>(a, kDeepCluster, (uint32_t)nsm, cfg, at)));
+        else CKD((deep_config<8, false>(a, kDeepCluster, (uint32_t)nsm, cfg, at)));
+        const double queues = (double)a.cluster * (g->max_deg <= 4 ? queue_cap<4>() : queue_cap<8>());
+        if (a.cluster == 1 || n > queues * (g->max_deg <= 3 ? 3.3 : (g->max_deg == 4 ? 1.7 : 1.2))) {
+            // a CTA's search of so many vertices takes as long as `ratio` of the
+            // sweep kernel's for six sources, and those have a fixed part of so
+            // many vertices more
+            const double mean = (double)g->nnz_pruned / n;
+            const double fixed = mean >= 3.5 ? 200e3 : (mean >= 2.5 ? 230e3 : (g->max_deg > 4 ? 400e3 : 600e3));
+            const double ratio = mean >= 3.5 ? (n <= (1u << 17) ? 24.0 : 33.0) : (mean >= 2.5 ? 19.0 : (g->max_deg > 4 ? 24.0 : (g->max_deg > 3 ? 27.0 : 22.0)));
+            if ((double)((nroots + 5) / 6) * (fixed + n) <= ratio * n * rounds) return BCG_OK;
+            most = 1;
+        }
+    }
+    return deep_launch(g, roots, mult, nroots, ext, most, st, res);
 }
 
 }  // namespace bcg

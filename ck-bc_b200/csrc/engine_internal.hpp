@@ -142,7 +142,8 @@ void wide_free(bcg_graph *g);
 
 // Runs one CTA a source on a graph of at most 8 neighbours a vertex (deep.cu);
 // as wide_run otherwise.  overflow: a uint64 count wrapped (done = false, bc as
-// before).  done and overflow false: no memory, or more levels than kMaxLevel.
+// before).  done and overflow false: no memory, more levels than kMaxLevel, or
+// frontiers so broad that the sweep kernel is faster.
 struct DeepResult {
     bool done = false, overflow = false;
     uint64_t launches = 0;

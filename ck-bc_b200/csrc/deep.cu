@@ -446,6 +446,21 @@ __global__ void k_deep_reduce(const DeepCtrl *__restrict__ ctrl, uint32_t n, uin
     if (sum != 0.0) bc[ext ? ext[v] : v] += sum;
 }
 
+// What a source's search says of searches from the vertices that it reached
+// (k_levels_low's bound): order's first `reached`, by level from lbeg.
+__global__ void k_deep_low(uint32_t reached, uint32_t depth, const uint32_t *__restrict__ order,
+                           const uint32_t *__restrict__ lbeg, uint8_t *__restrict__ low) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= reached) return;
+    uint32_t l = 0, end = depth;  // the last level that starts at i or before
+    while (l < end) {
+        const uint32_t mid = (l + end + 1) / 2;
+        if (lbeg[mid] <= i) l = mid;
+        else end = mid - 1;
+    }
+    low[order[i]] = (uint8_t)min(max(l, depth - l), 255u);
+}
+
 template <int D>
 __global__ void k_deep_rows(uint32_t n, const uint32_t *__restrict__ offs, const uint32_t *__restrict__ adj,
                             uint32_t *__restrict__ ell) {
@@ -643,7 +658,7 @@ static uint64_t deep_slots(uint32_t n, uint64_t nroots, uint32_t nsm) {
     return std::max<uint64_t>(1, std::min<uint64_t>({nroots, (uint64_t)nsm, kWorkKeep / per}));
 }
 
-static int deep_launch(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, bool ext,
+static int deep_launch(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, bool ext, bool note,
                        uint32_t most_ctas, cudaStream_t st, DeepResult *res) {
     *res = DeepResult{};
     const uint32_t n = g->tile_n ? g->tile_n : g->n;
@@ -722,7 +737,7 @@ static int deep_launch(bcg_graph *g, const uint32_t *roots, const double *mult, 
         // frontiers that do not fit the clusters' queues: one CTA a source
         if (c->full) {
             ws.leave();
-            return deep_launch(g, roots, mult, nroots, ext, 1, st, res);
+            return deep_launch(g, roots, mult, nroots, ext, note, 1, st, res);
         }
         res->overflow = c->overflow != 0;
         return BCG_OK;
@@ -730,6 +745,17 @@ static int deep_launch(bcg_graph *g, const uint32_t *roots, const double *mult, 
     res->rstat.resize(nroots);
     memcpy(res->rstat.data(), down.data() + o_rstat, nroots * sizeof(RootStat));
     res->done = true;
+    if (note) {  // (the last launch's first source; its states are not needed any more)
+        const RootStat &rs = res->rstat[(nroots - 1) / slots * slots];
+        uint8_t *d_low = mem + o_state;
+        std::vector<uint8_t> low(n);
+        CKD(cudaMemsetAsync(d_low, 0, n, st));
+        k_deep_low<<<(unsigned)((rs.visited + 255) / 256), 256, 0, st>>>((uint32_t)rs.visited, rs.depth, a.order, a.lbeg, d_low);
+        CKD(cudaGetLastError());
+        CKD(cudaMemcpyAsync(low.data(), d_low, n, cudaMemcpyDeviceToHost, st));
+        CKD(cudaStreamSynchronize(st));
+        merge_levels(g, low);
+    }
     return BCG_OK;
 }
 
@@ -748,8 +774,8 @@ static int deep_launch(bcg_graph *g, const uint32_t *roots, const double *mult, 
 // and 27.  The rule takes the faster in all of these, or one within 8 % of it, as
 // it does on 4-regular graphs and trees of 3 and 7 children (2^14 to 2^21
 // vertices, 1 to 400 sources).
-int deep_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, bool ext, cudaStream_t st,
-             DeepResult *res) {
+int deep_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, bool ext, bool note,
+             cudaStream_t st, DeepResult *res) {
     *res = DeepResult{};
     const int rc = deep_make(g);
     if (rc || !g->deep) return rc;
@@ -778,7 +804,7 @@ int deep_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t n
             most = 1;
         }
     }
-    return deep_launch(g, roots, mult, nroots, ext, most, st, res);
+    return deep_launch(g, roots, mult, nroots, ext, note, most, st, res);
 }
 
 }  // namespace bcg

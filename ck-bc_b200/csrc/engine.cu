@@ -619,6 +619,69 @@ static bool takes_wide(const bcg_graph *g, uint64_t nroots) {
     return wide_shallow(n, g->nnz_pruned) && (g->nnz_pruned >= 6ull * n || !deep_takes(g));
 }
 
+// Whether one of the roots is known to have more levels than a wide job holds.
+static bool known_deep(const bcg_graph *g, const std::vector<uint32_t> &roots) {
+    if (g->levels_low.empty()) return false;
+    return std::any_of(roots.begin(), roots.end(), [&](uint32_t r) { return g->levels_low[r] >= kWideLevels - 2; });
+}
+
+// low[v]: the most of what a search from source t says of one from v on an
+// undirected graph, where v is at t's level l and t's deepest level is D: l
+// levels lead back to t, and D - l at least to what is farthest from t.
+__global__ void k_deepest(uint32_t n, const unsigned char *__restrict__ rows, uint32_t row, uint32_t S,
+                          uint32_t *__restrict__ deepest) {
+    __shared__ uint32_t m[6];
+    if (threadIdx.x < 6) m[threadIdx.x] = 0;
+    __syncthreads();
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+        for (uint32_t k = 0; k < S; ++k) {
+            const uint32_t l = reinterpret_cast<const uint16_t *>(rows + (size_t)v * row)[k];
+            if (l != kUnvisited && l > m[k]) atomicMax(&m[k], l);
+        }
+    __syncthreads();
+    if (threadIdx.x < S) atomicMax(deepest + threadIdx.x, m[threadIdx.x]);
+}
+__global__ void k_levels_low(uint32_t n, const unsigned char *__restrict__ rows, uint32_t row, uint32_t S,
+                             const uint32_t *__restrict__ deepest, uint8_t *__restrict__ low) {
+    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= n) return;
+    uint32_t m = 0;
+    for (uint32_t k = 0; k < S; ++k) {
+        const uint32_t l = reinterpret_cast<const uint16_t *>(rows + (size_t)v * row)[k];
+        if (l != kUnvisited) m = max(m, max(l, deepest[k] - l));
+    }
+    low[v] = (uint8_t)min(m, 255u);
+}
+
+void merge_levels(bcg_graph *g, const std::vector<uint8_t> &low) {
+    if (g->levels_low.size() != low.size()) g->levels_low.assign(low.size(), 0);
+    for (size_t v = 0; v < low.size(); ++v) g->levels_low[v] = std::max(g->levels_low[v], low[v]);
+}
+
+// Keeps what the sweep kernel's last batch (done, its levels still in the state
+// rows) says of the levels of searches from every vertex.  A run that is known
+// to be too deep for the wide searches is not tried there: they would stop, so
+// the result is the same bits either way.  (Nothing is kept where there is no
+// memory.)
+static void note_levels(bcg_graph *g, uint32_t S, cudaStream_t st) {
+    const uint32_t n = g->tile_n ? g->tile_n : g->n;
+    Workspace ws;
+    std::vector<uint8_t> low(n);
+    if (ws.take(256 + (size_t)n, st) == cudaSuccess) {
+        uint32_t *deepest = reinterpret_cast<uint32_t *>(ws.mem);
+        uint8_t *d_low = ws.mem + 256;
+        cudaMemsetAsync(deepest, 0, 256, st);
+        k_deepest<<<std::min<uint32_t>(148 * 4, (n + 255) / 256), 256, 0, st>>>(n, g->d_rows, (uint32_t)row_bytes((int)S), S, deepest);
+        k_levels_low<<<(n + 255) / 256, 256, 0, st>>>(n, g->d_rows, (uint32_t)row_bytes((int)S), S, deepest, d_low);
+        if (cudaMemcpyAsync(low.data(), d_low, n, cudaMemcpyDeviceToHost, st) == cudaSuccess &&
+            cudaStreamSynchronize(st) == cudaSuccess) {
+            ws.waited = true;
+            merge_levels(g, low);
+        }
+    }
+    cudaGetLastError();
+}
+
 // Totals of the plan's roots (rs in plan order) and the kernels' time.
 static void finish_stats(bcg_graph *g, const RunPlan &p, const std::vector<RootStat> &rs, bcg_stats *stats) {
     uint64_t teps = 0, vis = 0, cv = 0, se = 0;
@@ -657,6 +720,9 @@ static int run_plan(bcg_graph *g, const RunPlan &p, cudaStream_t st, bcg_stats *
     // plain runs of a width that is not forced: the wide-batch kernel, or one
     // CTA a source on graphs of few neighbours (both wait for their results)
     const bool free_run = !debug && p.plain && !g->forced_width && (stats || g->sigma_mode == BCG_SIGMA_AUTO);
+    // (what one kernel finds holds for the next: a count that passes 2^64 does
+    // so in each of them, so no other tries uint64)
+    bool overflow = false, too_deep = false;
     if (free_run && takes_wide(g, nroots) && small_takes(g, nroots)) {
         SmallResult res;
         rc = small_run(g, p.roots.data(), p.mult.data(), nroots, st, &res);
@@ -670,8 +736,9 @@ static int run_plan(bcg_graph *g, const RunPlan &p, cudaStream_t st, bcg_stats *
             }
             return BCG_OK;
         }
+        overflow = res.overflow;
     }
-    if (free_run && takes_wide(g, nroots)) {
+    if (free_run && !overflow && takes_wide(g, nroots) && !known_deep(g, p.roots)) {
         WideResult res;
         rc = wide_run(g, p.roots.data(), p.mult.data(), nroots, st, &res);
         if (rc) return rc;
@@ -684,14 +751,17 @@ static int run_plan(bcg_graph *g, const RunPlan &p, cudaStream_t st, bcg_stats *
             }
             return BCG_OK;
         }
+        overflow = res.overflow;
+        too_deep = res.deep && !(g->flags & BCG_DIRECTED);
     }
+    if (overflow && g->sigma_mode == BCG_SIGMA_EXACT) return set_error(BCG_ERR_OVERFLOW, "a shortest-path count exceeded 2^64");
     if (free_run && deep_takes(g)) {
         DeepResult res;
-        bool extended = g->sigma_mode == BCG_SIGMA_EXTENDED;
-        rc = deep_run(g, p.roots.data(), p.mult.data(), nroots, extended, st, &res);
+        bool extended = overflow || g->sigma_mode == BCG_SIGMA_EXTENDED;
+        rc = deep_run(g, p.roots.data(), p.mult.data(), nroots, extended, too_deep, st, &res);
         if (!rc && res.overflow && g->sigma_mode == BCG_SIGMA_AUTO) {
-            extended = true;
-            rc = deep_run(g, p.roots.data(), p.mult.data(), nroots, true, st, &res);
+            overflow = extended = true;
+            rc = deep_run(g, p.roots.data(), p.mult.data(), nroots, true, too_deep, st, &res);
         }
         if (rc) return rc;
         if (res.overflow) return set_error(BCG_ERR_OVERFLOW, "a shortest-path count exceeded 2^64");
@@ -742,8 +812,8 @@ static int run_plan(bcg_graph *g, const RunPlan &p, cudaStream_t st, bcg_stats *
     // automatic mode a run whose counts overflow is redone in extended mode
     // from a saved copy of the accumulators.
     const bool autoext = g->sigma_mode == 0;
-    bool ext = g->sigma_mode == 2;
-    if (autoext) {
+    bool ext = overflow || g->sigma_mode == 2;
+    if (autoext && !ext) {
         if (!g->d_bc_save) CK(tmp_alloc(&g->d_bc_save, (size_t)g->n * sizeof(double), st));
         CK(cudaMemcpyAsync(g->d_bc_save, g->d_bc, (size_t)g->n * sizeof(double), cudaMemcpyDeviceToDevice, st));
     }
@@ -821,6 +891,7 @@ static int run_plan(bcg_graph *g, const RunPlan &p, cudaStream_t st, bcg_stats *
     }
     dev_free(d_trace);
     dev_free(d_tcnt);
+    if (too_deep) note_levels(g, S, st);
     if (!stats) return BCG_OK;
     if (stats) {
         std::vector<RootStat> rs(slots);

@@ -93,6 +93,9 @@ struct bcg_graph {
     bcg::DeepGraph *deep = nullptr;  // the same for deep runs (deep.cu)
     uint32_t max_deg = 0;            // largest degree in the searched graph
     bool counted = false;            // among the graphs alive (engine.cu)
+    // by searched vertex: levels that a search from it has at least, as far as
+    // deep runs have shown (empty: nothing known; 255: that many or more)
+    std::vector<uint8_t> levels_low;
 };
 
 namespace bcg {
@@ -132,7 +135,8 @@ int scan_exclusive(const uint32_t *d_in, uint32_t *d_out, uint64_t len, uint32_t
 // done = false: the graph is too deep for it, a count overflowed or memory ran
 // out; bc is as before and nothing else was changed.
 struct WideResult {
-    bool done = false;
+    bool done = false, overflow = false;  // overflow: a path count of the run passes 2^64
+    bool deep = false;                    // a search has more levels than a job holds
     uint64_t batches = 0, launches = 0;
     uint32_t slots = 0;           // sources of a job
     std::vector<RootStat> rstat;  // per root, in order (padded to whole jobs)
@@ -150,15 +154,18 @@ struct DeepResult {
     std::vector<RootStat> rstat;
 };
 bool deep_takes(const bcg_graph *g);
-int deep_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, bool ext, cudaStream_t st,
-             DeepResult *res);
+// note: what the first source's search says of the others' levels is kept (merge_levels).
+int deep_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, bool ext, bool note,
+             cudaStream_t st, DeepResult *res);
 void deep_free(bcg_graph *g);
+// Keeps the larger of what is known and low, by searched vertex.
+void merge_levels(bcg_graph *g, const std::vector<uint8_t> &low);
 
 // Runs a CTA a source in shared memory on a small graph (small.cu); waits for
 // the result.  done = false: a count overflowed or memory ran out, and nothing
 // was added to bc.
 struct SmallResult {
-    bool done = false;
+    bool done = false, overflow = false;  // as WideResult::overflow
     std::vector<RootStat> rstat;
     uint64_t launches = 0;
 };

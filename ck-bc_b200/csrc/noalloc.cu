@@ -325,10 +325,11 @@ using namespace bcg;
     } while (0)
 
 // The wide searches on the call's copies in the scratch; *done = false: they
-// do not fit it, or stopped (d_bc is then as before).
+// do not fit it, or stopped (d_bc is then as before; *overflow: because a path
+// count passes 2^64).
 static int na_wide(unsigned char *scr, uint32_t n, uint64_t nnz, uint32_t nroots, double *d_bc, cudaStream_t st,
-                   bool *done) {
-    *done = false;
+                   bool *done, bool *overflow) {
+    *done = *overflow = false;
     WideInput in{};
     in.n = n;
     in.nnz = in.big_nnz = nnz;
@@ -383,6 +384,7 @@ static int na_wide(unsigned char *scr, uint32_t n, uint64_t nnz, uint32_t nroots
         NA_CK(cudaStreamSynchronize(st));
         if (c.error) return set_error(c.error, "device reported error %d (a bounded wait gave up)", c.error);
         if (c.overflow || c.deep) {
+            *overflow = c.overflow != 0;
             if (jl < njobs) NA_CK(cudaMemcpyAsync(d_bc, save, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, st));
             return BCG_OK;
         }
@@ -458,9 +460,10 @@ extern "C" int bcg_bc_noalloc(const uint32_t *d_offsets, const uint32_t *d_adj, 
         NA_CK(cudaStreamSynchronize(st));
         return BCG_OK;
     }
+    bool overflow = false;
     if (wide) {
         bool done = false;
-        rc = na_wide(scr, n, nnz, hs.nroots, d_bc, st, &done);
+        rc = na_wide(scr, n, nnz, hs.nroots, d_bc, st, &done, &overflow);
         if (rc || done) return rc;
         rc = plan(true);
         if (rc) return rc;
@@ -507,7 +510,7 @@ extern "C" int bcg_bc_noalloc(const uint32_t *d_offsets, const uint32_t *d_adj, 
     a.mark_ratio = 8;
     if (const char *e = getenv("BCG_CHILD_MARK_RATIO")) a.mark_ratio = (uint32_t)std::min(strtoul(e, nullptr, 10), 1024ul);
     a.directed = 0;
-    for (int pass = 0; pass < 2; ++pass) {
+    for (int pass = overflow ? 1 : 0; pass < 2; ++pass) {
         const bool ext = pass == 1;
         if (ext) {
             // overflow: restore the accumulators and clear the scratch the

@@ -356,7 +356,8 @@ int small_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t 
     CKM(cudaMemcpyAsync(h.data(), mem, o_mult, cudaMemcpyDeviceToHost, st));
     CKM(cudaStreamSynchronize(st));
     ws.waited = true;
-    if (reinterpret_cast<const SmallCtrl *>(h.data())->overflow) return BCG_OK;  // the caller's other kernels extend the counts
+    res->overflow = reinterpret_cast<const SmallCtrl *>(h.data())->overflow != 0;
+    if (res->overflow) return BCG_OK;  // the caller's other kernels extend the counts
     res->rstat.resize(nroots);
     memcpy(res->rstat.data(), h.data() + o_rstat, nroots * sizeof(RootStat));
     res->launches = nroots > 1 ? 2 : 1;

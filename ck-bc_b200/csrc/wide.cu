@@ -1572,10 +1572,12 @@ int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t n
     }
     if (c->error) return set_error(c->error, "device reported error %d (a bounded wait gave up)", c->error);
     if (c->overflow || c->deep) {
-        // an overflowing count or a deep search: the caller runs the sweep kernel
+        // an overflowing count or a deep search: for the caller's other kernels
         if (several)
             CKW(cudaMemcpyAsync(g->d_bc, g->d_bc_save, (size_t)g->n * sizeof(double), cudaMemcpyDeviceToDevice, st));
         res->launches = 0;
+        res->overflow = c->overflow != 0;
+        res->deep = c->deep != 0;
         return BCG_OK;
     }
     res->rstat.resize(njobs * slots);

@@ -143,6 +143,9 @@ int build_wide(bcg_batch *b) {
     };
     int rc = wide_form_make(b->form, in, false);
     if (rc) return give_up(rc);
+    // (the total of edges below is a half of all sources' entries together,
+    // which takes an even number of each: the packed schedule halves its own)
+    if (b->form.subs[0].loops) return give_up(BCG_OK);
     // jobs in union order (largest graphs first); a launch ends when its jobs'
     // vectors take 512 MB, or when the graphs have become a quarter of its
     // first one's size and it has work for four rounds of the chip
@@ -537,7 +540,7 @@ int bcg_batch_run(bcg_batch *b, bcg_stats *stats) {
             if (rc) return rc;
         } else {
             const RootStat *t = reinterpret_cast<const RootStat *>(hs.data() + b->o_total);
-            teps = t->mc2 / 2;  // every source's share is even
+            teps = t->mc2 / 2;  // every source's share is even (no loops)
             vis = t->visited;
             cv = t->wsum;
             md = t->depth;

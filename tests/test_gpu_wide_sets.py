@@ -1,6 +1,7 @@
 """Batched and serving forms on the wide searches, where a set or pool is unlike the usual one: a single graph, most of
 whose vertices have no edge; path counts just below and just past 2^64; graphs with searches too deep for wide waves;
-waves whose memory is full; budgets that hold little beside the pool.  Against the oracle, within the suite's 1e-9;
+waves whose memory is full; budgets that hold little beside the pool;
+loops in the lists.  Against the oracle, within the suite's 1e-9;
 what no path passes is exactly 0."""
 import numpy as np
 import pytest
@@ -197,3 +198,23 @@ def test_budgets_close_to_the_pool():
             for rid in ids:
                 assert_bc_close(S.result(rid), ref, f"budget {budget - full} bytes from the wide buffers")
             assert S.info()["admitted_bytes"] == 0
+
+
+def test_totals_with_loops():
+    """A list that names its own vertex makes a component's entries odd: the edges of a set are halved source by source,
+    as in a run."""
+    offs, adj = bcg.generate("rmat:scale=10,ef=16,a=0.57,b=0.19,c=0.19,seed=5")
+    rows = [list(adj[offs[v]:offs[v + 1]]) for v in range(1024)]
+    rows[7].append(7)
+    o = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.uint32)
+    a = np.array([w for r in rows for w in r], dtype=np.uint32)
+    src = np.nonzero(np.diff(o))[0].astype(np.uint32)
+    with bcg.Graph(o, a) as G:
+        G.set_batch_width(6)
+        want = G.run(src)
+        bc = G.bc()
+    with bcg.Batch([(o, a)]) as B:
+        for runs in (1, 2):
+            st = B.run()
+            assert st.teps_edges == want.teps_edges and st.visited == want.visited
+            assert_bc_close(B.bc(0), runs * bc, "a loop")

@@ -191,8 +191,8 @@ __device__ __forceinline__ bool wide_stopped(const WideCtrl *c) {
 // false when any CTA of the launch recorded an error; a waiting CTA sees that
 // too, so nobody waits for one that has left.
 template <int NS>
-__device__ bool team_sync(const WideArgs &a, const WideCtx &x, WideTeam *t, WideSmem<NS> &sm, unsigned long long wait_ns,
-                          uint32_t slot, uint32_t level = 0) {
+__device__ bool team_sync(const WideArgs &a, const WideCtx &x, WideTeam *t, WideSmem<NS> &sm, uint32_t slot,
+                          uint32_t level = 0) {
     __syncthreads();
     if (threadIdx.x == 0) {
         bool ok = true;
@@ -215,7 +215,7 @@ __device__ bool team_sync(const WideArgs &a, const WideCtx &x, WideTeam *t, Wide
                     if (v >= target) break;
                     if ((++spins & 63u) == 0) {
                         if (wide_stopped(a.ctrl)) break;
-                        if (wide_ns() - t0 > wait_ns) {
+                        if (wide_ns() - t0 > kDefaultWaitNs) {
                             atomicCAS(&a.ctrl->error, 0, BCG_ERR_TIMEOUT);
                             if (a.poison) *a.poison = 1;
                             break;
@@ -945,7 +945,6 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
     if (team >= a.teams) return;
     if (a.poison && *reinterpret_cast<volatile int *>(a.poison)) return;
     WideTeam *t = a.team + team;
-    const unsigned long long wait_ns = a.ctrl->wait_ns ? a.ctrl->wait_ns : kDefaultWaitNs;
     if (threadIdx.x == 0) {
         unsigned char *st = a.state + (size_t)team * a.stride;
         x.T = a.team_ctas;
@@ -1086,7 +1085,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
 #pragma unroll
             for (int h = 0; h < NS / 4; ++h) row[h] = make_uint4(0u, 0u, 0u, 0u);
         });
-        if (!team_sync(a, x, t, sm, wait_ns, 5)) return;
+        if (!team_sync(a, x, t, sm, 5)) return;
         wide_trace(a, job, 0, 0, n);
 
         // ---- forward
@@ -1129,7 +1128,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
             } else if (big) wide_sweep<kFwdFull, NS>(sm, d);
             else if (d == 1 && ones) wide_sweep<kFwdOnes, NS>(sm, d);
             else wide_sweep<kFwd32, NS>(sm, d);
-            if (!team_sync(a, x, t, sm, wait_ns, d & 3, d + 1)) return;
+            if (!team_sync(a, x, t, sm, d & 3, d + 1)) return;
             const uint32_t any = sm.any;
             wide_trace(a, job, 2, d, any);
             if (any & 4u) {
@@ -1137,7 +1136,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
                     a.ctrl->overflow = 1;
                     if (a.poison) *a.poison = 1;
                 }
-                if (!team_sync(a, x, t, sm, wait_ns, 5)) return;
+                if (!team_sync(a, x, t, sm, 5)) return;
             }
             if (!(any & 1u)) break;
             big = (any & 2u) != 0;
@@ -1199,10 +1198,10 @@ __global__ void __launch_bounds__(kWideThreads, 1) bc_wide_kernel(WideArgs a) {
         for (uint32_t e = D; e >= 1; --e) {
             if (e == D) wide_sweep<kBackLast, NS>(sm, e);
             else wide_sweep<kBack, NS>(sm, e);
-            if (!team_sync(a, x, t, sm, wait_ns, 4)) return;
+            if (!team_sync(a, x, t, sm, 4)) return;
             wide_trace(a, job, 3, e, 0);
         }
-        if (D == 0 && !team_sync(a, x, t, sm, wait_ns, 4)) return;
+        if (D == 0 && !team_sync(a, x, t, sm, 4)) return;
         job = *reinterpret_cast<volatile uint32_t *>(&t->job[par]);
         __syncthreads();
     }

@@ -64,8 +64,7 @@ static_assert(sizeof(WideTeam) == 128, "one line per team");
 struct WideCtrl {
     int error, overflow, deep;   // any of them set ends the launch
     uint32_t next_job;           // first job not handed out
-    unsigned long long wait_ns;
-    uint32_t pad[26];
+    uint32_t pad[28];
 };
 static_assert(sizeof(WideCtrl) == 128, "one line");
 

@@ -24,6 +24,9 @@ all-gathered over NCCL and added in rank order (bit-reproducible).
   roofline  algorithmic bytes of the sweep kernel = sum over sources of
          16*m_comp + 56*n_comp + 8 (int32 ids, uint64 sigma, FP64 delta/bc),
          divided by its CUDA-event time; peak = MEASURED_PEAKS.json hbm_gbs.
+         A run on the wide searches, which read the lists once for 16 or 32
+         sources, is set against the gather of rows out of L2 instead: 4 bytes
+         forward and 8 backward per searched entry and source.
   cpu_baseline  the oracle (CPU Brandes restatement, all host threads) on a
          bounded sample of the same workload's sources, rank 0 at N=1.
 --impl reference: the reference program has no CPU Brandes; its path is timed
@@ -688,6 +691,15 @@ def main():
                              "bytes_per_launch": s_bytes / args.steps,
                              "note": "16 B per searched edge + 56 B per searched vertex + 8 B per root, over the "
                                      "pruned graph each root's search walks"}}
+    if w >= 16:
+        # two entries an edge; what a plain kernel gathers of 256-byte rows of
+        # the benchmark graph's neighbours, measured
+        l2_peak = 20000.0
+        gathered = 24.0 * s_edges
+        roofline.update({"bound": "l2 gather", "achieved": gathered / kern_s / 1e9, "peak": l2_peak,
+                         "frac": gathered / kern_s / 1e9 / l2_peak, "peak_kind": "measured (rows of 256 bytes out of L2)",
+                         "alg_bytes_per_launch": gathered / args.steps})
+        del roofline["searched"]
     if tnote:
         roofline["traffic_note"] = tnote
 

@@ -16,13 +16,13 @@
 //
 // Sets of shallow graphs (wide_shallow: every graph of mean degree 6 and up, or
 // of a few vertices) do not run that schedule: their sources go to the
-// wide-batch searches (wide.cu), 16 of one graph a job, a CTA or a few to a
+// wide-batch searches (wide.cu), 32 of one graph a job, a CTA or a few to a
 // job, largest graphs first, in as many launches as the job vectors' memory
 // asks for, captured the same way.  One with a search of more than 62 levels
-// goes back to the packed schedule.  (48 graphs of 250 to 2,500 vertices: the
-// packed schedule advances all by six sources a batch and pays about 13
-// barriers of the whole chip for it, 108 ms; a CTA that runs 16 sources of one
-// graph has no such barrier: 6.8 ms.)
+// goes back to the packed schedule, and one with loops stays there.  (48 graphs
+// of 250 to 2,500 vertices: the packed schedule advances all by six sources a
+// batch and pays about 13 barriers of the whole chip for it, 108 ms; a CTA that
+// runs 32 sources of one graph has no such barrier: 5.2 ms.)
 //
 // The autotuner times a prefix of the schedule for each candidate batch width
 // S in {1, 3, 6} and tile shape (vertices x adjacency entries per tile), keeps

@@ -323,10 +323,10 @@ int bcg_batch_get_bc(bcg_batch *b, uint32_t graph, double *bc_host);
  * 16x128, 16x64} (vertices x adjacency entries per tile), keeps the fastest per
  * root and resets the accumulators.  Any output pointer may be NULL.  A set
  * that runs as wide-batch searches (every graph of mean degree 6 or more, or of
- * a few vertices) has nothing to tune: the current shape is reported. */
+ * a few vertices, and no list with its own vertex) has nothing to tune: the current shape is reported. */
 int bcg_batch_autotune(bcg_batch *b, uint32_t sample_batches, uint32_t *width,
                        uint32_t *tile_vertices, uint32_t *tile_entries);
-/* Schedule length (packed batches, or jobs of 16 sources of a set that runs as
+/* Schedule length (packed batches, or jobs of 32 sources of a set that runs as
  * wide-batch searches), width and tile shape of the packed schedule, and whether runs
  * replay a captured CUDA graph (1) or launch directly (0). */
 int bcg_batch_info(bcg_batch *b, uint32_t *nbatch, uint32_t *width, uint32_t *tile_vertices,

@@ -175,3 +175,32 @@ def test_a_count_past_two_to_the_64_is_found_once(tmp_path, monkeypatch):
             G.run(src)
         assert e.value.code == bcg.ERR_OVERFLOW and not np.any(G.bc())
         assert _attempts(trace, "# wide") == 2 and _attempts(trace, "# width") == 1
+
+
+def test_a_run_of_several_launches():
+    """Job vectors of more than 512 MB: the launches add one after the other, and when the last one meets a deep search
+    (ordered last by what it reaches), what the others added is taken back and the sweep kernel runs it all."""
+    rmat = bcg.generate("rmat:scale=18,ef=8,a=0.57,b=0.19,c=0.19,seed=3")
+    n = len(rmat[0]) - 1
+    own = np.stack([np.repeat(np.arange(n), np.diff(rmat[0].astype(np.int64))), rmat[1]], 1)
+    o, a = _cliques(8, 60)
+    tail = np.stack([np.repeat(np.arange(480), np.diff(o.astype(np.int64))), a], 1) + n
+    offs, adj = bcg.from_pairs(np.concatenate([own, tail]), n + 480)
+    live = np.nonzero(np.diff(rmat[0]))[0].astype(np.uint32)
+    jobs = (512 << 20) // (8 * (len(live) + 480)) + 20
+    src = live[np.sort(np.random.default_rng(1).choice(len(live), 32 * jobs, replace=False))]
+    ends = np.array([n, n + 479], dtype=np.uint32)
+    with bcg.Graph(offs, adj) as G:
+        parts = [G.run(p) for p in np.array_split(src, 4)]
+        want = G.bc()
+        G.reset()
+        st = G.run(src)
+        assert st.batch_width == 32 and st.batches == jobs
+        assert st.teps_edges == sum(p.teps_edges for p in parts) and st.visited == sum(p.visited for p in parts)
+        assert_bc_close(G.bc(), want, "one call")
+        G.run(ends)
+        both = G.bc()
+        G.reset()
+        st = G.run(np.concatenate([src, ends]))
+        assert st.batch_width == 6 and st.max_depth > 100
+        assert_bc_close(G.bc(), both, "with a deep search")

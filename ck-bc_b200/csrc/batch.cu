@@ -141,11 +141,13 @@ int build_wide(bcg_batch *b) {
         free_wide(b);
         return rc == BCG_ERR_OOM ? (cudaGetLastError(), BCG_OK) : rc;
     };
-    int rc = wide_form_make(b->form, in, false);
-    if (rc) return give_up(rc);
     // (the total of edges below is a half of all sources' entries together,
     // which takes an even number of each: the packed schedule halves its own)
-    if (b->form.subs[0].loops) return give_up(BCG_OK);
+    bool loops = false;
+    int rc = wide_loops(in, &loops);
+    if (rc || loops) return give_up(rc);
+    rc = wide_form_make(b->form, in, false);
+    if (rc) return give_up(rc);
     // jobs in union order (largest graphs first); a launch ends when its jobs'
     // vectors take 512 MB, or when the graphs have become a quarter of its
     // first one's size and it has work for four rounds of the chip

@@ -34,8 +34,7 @@ struct WideSub {
     uint32_t n, nheavy, chunk_len, pad;
     uint32_t nmed[4];
     uint32_t nchunk[2];
-    uint32_t base;             // the graph's first position in its union
-    uint32_t loops;            // 1: some list of the union names its own vertex
+    uint32_t base, pad2;       // the graph's first position in its union
     uint32_t chunk0[2];        // its first chunk there
     const uint32_t *offs[2], *adj[2];  // entries from offs[..][v] on in adj
     const uint2 *chunk[2];     // {union position of the vertex, index of the chunk within it}
@@ -144,6 +143,8 @@ int wide_form_enqueue(WideForm &f, const WideInput &in, unsigned char *mem, unsi
 // graph nothing is read back then, and the building is not waited for.
 int wide_form_make(WideForm &f, const WideInput &in, bool bounds);
 void wide_form_free(WideForm &f);
+// Whether some list names its own vertex (waits).
+int wide_loops(const WideInput &in, bool *loops);
 
 // Loads the wide searches' kernels on the current device (CUDA would load each
 // at its first launch, which takes device memory).

@@ -116,13 +116,12 @@ __global__ void k_form_rows(uint32_t n, const uint32_t *__restrict__ perm, const
                             const uint32_t *__restrict__ toffs, const uint2 *__restrict__ vinfo,
                             const uint32_t *__restrict__ ext, uint32_t chunk, uint32_t *__restrict__ len0,
                             uint32_t *__restrict__ len1, uint32_t *__restrict__ ch0, uint32_t *__restrict__ ch1,
-                            uint2 *__restrict__ vi2, uint32_t *__restrict__ map, uint32_t *__restrict__ loops) {
+                            uint2 *__restrict__ vi2, uint32_t *__restrict__ map) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i > n) return;
     if (i == n) {
         len1[n] = ch1[n] = 0;
         if (toffs) len0[n] = ch0[n] = 0;
-        *loops = 0;
         return;
     }
     const uint32_t v = perm[i];
@@ -143,34 +142,35 @@ __global__ void k_form_rows(uint32_t n, const uint32_t *__restrict__ perm, const
 __global__ void k_form_fill(uint32_t n, const uint32_t *__restrict__ perm, const uint32_t *__restrict__ inv,
                             const uint32_t *__restrict__ offs, const uint32_t *__restrict__ adj,
                             const uint32_t *__restrict__ offs2, uint32_t *__restrict__ adj2,
-                            const uint32_t *__restrict__ cbeg, uint2 *__restrict__ chunk, uint32_t *__restrict__ loops) {
+                            const uint32_t *__restrict__ cbeg, uint2 *__restrict__ chunk) {
     const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const unsigned lane = threadIdx.x & 31;
     if (w >= n) return;
     const uint32_t v = perm[w], e0 = offs[v], len = offs[v + 1] - e0, o = offs2[w];
-    bool loop = false;
-    for (uint32_t i = lane; i < len; i += 32) {
-        const uint32_t u = adj[e0 + i];
-        loop |= u == v;
-        adj2[o + i] = inv[u];
-    }
-    if (loop) *loops = 1;
+    for (uint32_t i = lane; i < len; i += 32) adj2[o + i] = inv[adj[e0 + i]];
     const uint32_t c0 = cbeg[w], c1 = cbeg[w + 1];
     for (uint32_t c = c0 + lane; c < c1; c += 32) chunk[c] = make_uint2((uint32_t)w, c - c0);
+}
+
+// One warp a vertex.
+__global__ void k_form_loops(uint32_t n, const uint32_t *__restrict__ offs, const uint32_t *__restrict__ adj,
+                             uint32_t *__restrict__ loops) {
+    const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (w >= n) return;
+    for (uint32_t e = offs[w] + (threadIdx.x & 31u); e < offs[w + 1]; e += 32)
+        if (adj[e] == (uint32_t)w) *loops = 1;
 }
 
 // The graphs' descriptions.  proto: everything that is the same for all, with
 // pointers to the union's arrays.
 __global__ void k_form_subs(uint32_t graphs, const FormGraph *__restrict__ list, FormGraph one,
-                            const uint32_t *__restrict__ hist, const uint32_t *__restrict__ loops, WideSub proto,
-                            WideSub *__restrict__ subs) {
+                            const uint32_t *__restrict__ hist, WideSub proto, WideSub *__restrict__ subs) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= graphs) return;
     const FormGraph g = list ? list[i] : one;
     WideSub s = proto;
     auto before = [&](uint32_t key) { return hist[g.hist + key * g.nb] - g.base; };  // vertices of lower keys
     s.base = g.base;
-    s.loops = *loops;
     s.n = before(kKeyZero);
     s.nheavy = before(degree_key(proto.chunk_len + 1u) + 1u);
     for (uint32_t b = 0; b < 4; ++b) s.nmed[b] = max(s.nheavy, before(degree_key(kWideLight << b)));
@@ -216,7 +216,7 @@ struct FormPlan {
     // form
     size_t subs, inv, map, vinfo, offs[2], adj[2], cbeg[2], chunks[2], bytes;
     // scratch
-    size_t perm, hist, scan, toffs, tadj, cursor, fblocks, fgraphs, loops, scratch;
+    size_t perm, hist, scan, toffs, tadj, cursor, fblocks, fgraphs, scratch;
 };
 
 FormPlan plan_form(const WideInput &in) {
@@ -260,7 +260,6 @@ FormPlan plan_form(const WideInput &in) {
     p.cursor = take(in.directed ? n1 * 4 : 0);
     p.fblocks = take(in.base ? (size_t)p.blocks * sizeof(FormBlock) : 0);
     p.fgraphs = take(in.base ? (size_t)in.graphs * sizeof(FormGraph) : 0);
-    p.loops = take(4);
     p.scratch = o;
     return p;
 }
@@ -286,7 +285,7 @@ int wide_form_enqueue(WideForm &f, const WideInput &in, unsigned char *mem, unsi
     const uint32_t n = in.n;
     auto u32 = [](unsigned char *b, size_t o) { return reinterpret_cast<uint32_t *>(b + o); };
     uint32_t *perm = u32(scratch, p.perm), *hist = u32(scratch, p.hist), *scan = u32(scratch, p.scan);
-    uint32_t *toffs = nullptr, *tadj = nullptr, *loops = u32(scratch, p.loops);
+    uint32_t *toffs = nullptr, *tadj = nullptr;
     int rc;
     if (in.directed) {
         toffs = u32(scratch, p.toffs);
@@ -328,7 +327,7 @@ int wide_form_enqueue(WideForm &f, const WideInput &in, unsigned char *mem, unsi
     k_form_number<<<p.blocks, 256, 0, st>>>(n, blocks, graphs, one, in.offs, toffs, hist, perm, f.inv);
     k_form_rows<<<fblocks((uint64_t)n + 1, 256), 256, 0, st>>>(n, perm, in.offs, toffs, in.vinfo, in.ext, p.chunk,
                                                                u32(mem, p.offs[0]), u32(mem, p.offs[1]),
-                                                               u32(mem, p.cbeg[0]), u32(mem, p.cbeg[1]), vinfo, f.map, loops);
+                                                               u32(mem, p.cbeg[0]), u32(mem, p.cbeg[1]), vinfo, f.map);
     CKF(cudaGetLastError());
     WideSub proto{};
     proto.chunk_len = p.chunk;
@@ -348,9 +347,9 @@ int wide_form_enqueue(WideForm &f, const WideInput &in, unsigned char *mem, unsi
         const bool t = in.directed && d == 0;
         k_form_fill<<<fblocks((uint64_t)n * 32, 256), 256, 0, st>>>(n, perm, f.inv, t ? toffs : in.offs, t ? tadj : in.adj,
                                                                     o, u32(mem, p.adj[d]), c,
-                                                                    reinterpret_cast<uint2 *>(mem + p.chunks[d]), loops);
+                                                                    reinterpret_cast<uint2 *>(mem + p.chunks[d]));
     }
-    k_form_subs<<<fblocks(in.graphs, 128), 128, 0, st>>>(in.graphs, graphs, one, hist, loops, proto, f.d_subs);
+    k_form_subs<<<fblocks(in.graphs, 128), 128, 0, st>>>(in.graphs, graphs, one, hist, proto, f.d_subs);
     CKF(cudaGetLastError());
     return BCG_OK;
 }
@@ -378,6 +377,20 @@ int wide_form_make(WideForm &f, const WideInput &in, bool bounds) {
         rc = set_error(BCG_ERR_CUDA, "reading the wide form: %s", cudaGetErrorString(cudaGetLastError()));
     scratch.waited = rc == BCG_OK;
     return rc;
+}
+
+int wide_loops(const WideInput &in, bool *loops) {
+    Workspace ws;
+    uint32_t found = 0;
+    CKF(ws.take(4, 0));
+    uint32_t *d_found = reinterpret_cast<uint32_t *>(ws.mem);
+    CKF(cudaMemsetAsync(d_found, 0, 4, 0));
+    k_form_loops<<<fblocks((uint64_t)in.n * 32, 256), 256>>>(in.n, in.offs, in.adj, d_found);
+    CKF(cudaGetLastError());
+    CKF(cudaMemcpy(&found, d_found, 4, cudaMemcpyDeviceToHost));
+    ws.waited = true;
+    *loops = found != 0;
+    return BCG_OK;
 }
 
 void wide_form_free(WideForm &f) {

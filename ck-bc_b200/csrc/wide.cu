@@ -1455,7 +1455,6 @@ WideInput wide_input(const bcg_graph *g) {
 int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t nroots, cudaStream_t st, WideResult *res) {
     *res = WideResult{};
     int rc;
-    bool fresh = false;
     // (out of memory: the caller's other kernels need less)
     if (!g->wide) {
         g->wide = new WideGraph();
@@ -1466,7 +1465,7 @@ int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t n
             clear_error();
             return BCG_OK;
         }
-        fresh = true;
+        if (st != 0) CKW(cudaStreamSynchronize(0));  // the form that stream 0 made is ready for any stream
     }
     WideGraph *w = g->wide;
     const WideSub &b = w->form.subs[0];  // (bounds, on a small graph)
@@ -1495,7 +1494,6 @@ int wide_run(bcg_graph *g, const uint32_t *roots, const double *mult, uint64_t n
     }
     CKW(took);
     unsigned char *const mem = ws.mem;
-    if (fresh && st != 0) CKW(cudaStreamSynchronize(0));  // the form that stream 0 made is ready for st
     std::vector<unsigned char> h(blob), hs(stat);
     memcpy(h.data(), mult, nroots * 8);
     memcpy(h.data() + o_roots, roots, nroots * 4);

@@ -129,7 +129,9 @@ namespace bcg {
 
 namespace {
 std::mutex g_pool_mu;
-std::vector<cudaMemPool_t> g_pools;  // per device, created on first use
+// per device, created on first use (never destroyed: a graph may outlive the
+// library's own static objects)
+std::vector<cudaMemPool_t> &g_pools = *new std::vector<cudaMemPool_t>;
 }  // namespace
 
 // What the pool keeps: 4 GiB more than is in use (its threshold counts used
@@ -156,7 +158,7 @@ struct DeviceWork {
     uint64_t bytes = 0;
     uint32_t graphs = 0;
 };
-static std::vector<DeviceWork> g_work;
+static std::vector<DeviceWork> &g_work = *new std::vector<DeviceWork>;
 
 static DeviceWork &device_work(int dev) {
     if (g_work.size() <= (size_t)dev) g_work.resize((size_t)dev + 1);
